@@ -35,9 +35,8 @@
 // rolling_ic_gpu (src/rolling_ic.cu:306-540) / np_rolling_ic
 // (fc/_cpu_core.py:271-293) for the IC; the reference sorts with CUB's global
 // segmented radix sort instead.
-#include "block_sort.cuh"
-#include "fcb_kernels.h"
 #include "learned_sort.cuh"
+#include "row_io.cuh"
 
 namespace fcb {
 namespace {
@@ -50,120 +49,6 @@ constexpr uint32_t kFacMask = 1u << 29;     //                bit 29 factor mask
 constexpr uint32_t kCellValid = 1u << 28;   // factor valid (finite and mask)
 constexpr uint32_t kCellJoint = 1u << 29;   // factor and returns valid
 constexpr uint32_t kCellDrop = 1u << 30;    // returns valid, factor not
-
-__host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~size_t(15); }
-
-// Row loads in the vector layout: thread tid owns columns 4*(j*NT + tid) + k.
-template <int NT, int V, bool STREAM>
-FCB_DEV void load_row_f32(const float* __restrict__ row, int N, float (&x)[4 * V]) {
-  const bool al = (reinterpret_cast<uintptr_t>(row) & 15u) == 0;
-  const float qnan = __uint_as_float(kQuietNanBits);
-#pragma unroll
-  for (int j = 0; j < V; ++j) {
-    const int i0 = 4 * (j * NT + static_cast<int>(threadIdx.x));
-    if (al && i0 + 3 < N) {
-      const float4* p = reinterpret_cast<const float4*>(row + i0);
-      const float4 q = STREAM ? __ldcs(p) : __ldg(p);
-      x[4 * j] = q.x;
-      x[4 * j + 1] = q.y;
-      x[4 * j + 2] = q.z;
-      x[4 * j + 3] = q.w;
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) x[4 * j + k] = (i0 + k < N) ? row[i0 + k] : qnan;
-    }
-  }
-}
-
-template <int NT, int V>
-FCB_DEV void load_words(const uint32_t* __restrict__ row, int N, uint32_t (&w)[4 * V]) {
-#pragma unroll
-  for (int j = 0; j < V; ++j) {
-    const int i0 = 4 * (j * NT + static_cast<int>(threadIdx.x));
-    if (i0 + 3 < N) {
-      const uint4 q = __ldg(reinterpret_cast<const uint4*>(row + i0));
-      w[4 * j] = q.x;
-      w[4 * j + 1] = q.y;
-      w[4 * j + 2] = q.z;
-      w[4 * j + 3] = q.w;
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) w[4 * j + k] = (i0 + k < N) ? row[i0 + k] : 0u;
-    }
-  }
-}
-
-// 0/1 bytes in the vector layout (all ones when there is no mask).
-template <int NT, int V>
-FCB_DEV void load_mask4(const uint8_t* __restrict__ row, int N, uint32_t (&m)[4 * V]) {
-  const bool al = (reinterpret_cast<uintptr_t>(row) & 3u) == 0;
-#pragma unroll
-  for (int j = 0; j < V; ++j) {
-    const int i0 = 4 * (j * NT + static_cast<int>(threadIdx.x));
-    if (row == nullptr) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) m[4 * j + k] = (i0 + k < N) ? 1u : 0u;
-    } else if (al && i0 + 3 < N) {
-      const uint32_t q = __ldcs(reinterpret_cast<const unsigned int*>(row + i0));
-#pragma unroll
-      for (int k = 0; k < 4; ++k) m[4 * j + k] = ((q >> (8 * k)) & 0xFFu) ? 1u : 0u;
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) m[4 * j + k] = (i0 + k < N && row[i0 + k] != 0) ? 1u : 0u;
-    }
-  }
-}
-
-template <int NT, int V>
-FCB_DEV void store_row_f32v(float* __restrict__ row, int N, const float (&v)[4 * V]) {
-  const bool al = (reinterpret_cast<uintptr_t>(row) & 15u) == 0;
-#pragma unroll
-  for (int j = 0; j < V; ++j) {
-    const int i0 = 4 * (j * NT + static_cast<int>(threadIdx.x));
-    if (al && i0 + 3 < N) {
-      __stcs(reinterpret_cast<float4*>(row + i0), make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (i0 + k < N) row[i0 + k] = v[4 * j + k];
-    }
-  }
-}
-
-// Order-preserving compaction offsets in the vector layout: the column order
-// is the (j, tid, k) order, so cell (j, k) of this thread goes to
-//   sum_{j' < j} total_j' + (flagged cells of vector j in threads < tid)
-//   + (flagged cells k' < k of this thread's vector j).
-// Per-vector counts (0..4 per thread, <= 4*NT per block) are packed into
-// 12-bit fields, five per 64-bit word, so one block scan serves five vectors.
-// Returns the block total; base[j] receives the first two terms.
-template <int NT, int V>
-FCB_DEV int compact_bases(uint32_t flags, int (&base)[V], unsigned long long* scratch) {
-  static_assert(4 * NT < 4096, "12-bit count fields");
-  static_assert(4 * V <= 32, "one flag bit per cell");
-  constexpr int PER = 5, K = (V + PER - 1) / PER;
-  int run = 0;
-#pragma unroll
-  for (int q = 0; q < K; ++q) {
-    unsigned long long packed = 0;
-#pragma unroll
-    for (int jj = 0; jj < PER; ++jj) {
-      const int j = q * PER + jj;
-      if (j < V) packed |= static_cast<unsigned long long>(__popc((flags >> (4 * j)) & 0xFu)) << (12 * jj);
-    }
-    unsigned long long tot;
-    const unsigned long long ex = block_exclusive_sum(packed, scratch, tot);
-#pragma unroll
-    for (int jj = 0; jj < PER; ++jj) {
-      const int j = q * PER + jj;
-      if (j < V) {
-        base[j] = run + static_cast<int>((ex >> (12 * jj)) & 0xFFFull);
-        run += static_cast<int>((tot >> (12 * jj)) & 0xFFFull);
-      }
-    }
-  }
-  return run;
-}
 
 // Shared-memory layout of the rank kernels (bytes; every region 16-aligned).
 struct BucketLayout {  // k_ric_learned
@@ -178,22 +63,6 @@ struct BucketLayout {  // k_ric_learned
     total = o;
   }
 };
-template <int NT>
-struct SortedLayout {  // k_ric_radix and k_ric_prep
-  size_t red, dw, scratch, k0, k1, i0, i1, total;
-  __host__ __device__ explicit SortedLayout(int n) {
-    size_t o = 0;
-    red = o; o += 1024;
-    dw = o; o = al16(o + size_t((n + 31) / 32 + 1) * 8);
-    scratch = o; o = al16(o + SortScratch<NT>::bytes);
-    k0 = o; o = al16(o + size_t(n) * 4 + 16);
-    k1 = o; o = al16(o + size_t(n) * 4 + 16);
-    i0 = o; o = al16(o + size_t(n) * 2 + 16);
-    i1 = o; o = al16(o + size_t(n) * 2 + 16);
-    total = o;
-  }
-};
-
 // Exclusive per-word prefix counts of the drop bitmap: dw[k] low half = the
 // bits of returns positions 32k..32k+31, high half = set bits before word k.
 // One warp; the bitmap must be complete (a barrier after the last atomicOr).
@@ -847,202 +716,6 @@ __global__ void __launch_bounds__(NT) k_ric_list_batch(const RicPanel* __restric
 }
 
 // ---------------------------------------------------------------------------
-// cs_rank and parameter_scan of one plane: one CTA per date
-// ---------------------------------------------------------------------------
-// cs_rank: valid = finite & mask; the valid cells are compacted in column
-// order, radix-sorted by key (of -x for descending), and each cell's rank is
-// its sorted position + 1 (replaces cs_rank_gpu, src/cross_sectional_rank.cu:
-// 228-372, which runs CUB's global segmented sort).
-template <int NT, int V>
-__global__ void __launch_bounds__(NT) k_csr(const float* __restrict__ X, const uint8_t* __restrict__ mask, int N,
-                                            int desc, float* __restrict__ out) {
-  constexpr int C = 4 * V;
-  extern __shared__ __align__(16) uint8_t sm[];
-  const SortedLayout<NT> L(N);
-  unsigned long long* scan64 = reinterpret_cast<unsigned long long*>(sm + L.red);
-  uint32_t* k0 = reinterpret_cast<uint32_t*>(sm + L.k0);
-  uint32_t* k1 = reinterpret_cast<uint32_t*>(sm + L.k1);
-  uint16_t* i0 = reinterpret_cast<uint16_t*>(sm + L.i0);
-  uint16_t* i1 = reinterpret_cast<uint16_t*>(sm + L.i1);
-  const int tid = static_cast<int>(threadIdx.x);
-  const size_t row = static_cast<size_t>(blockIdx.x) * N;
-  float x[C];
-  uint32_t mk[C];
-  load_row_f32<NT, V, true>(X + row, N, x);
-  load_mask4<NT, V>(mask != nullptr ? mask + row : nullptr, N, mk);
-  uint32_t valid = 0u;
-#pragma unroll
-  for (int c = 0; c < C; ++c) valid |= ((finite_f32(x[c]) && mk[c]) ? 1u : 0u) << c;
-  int base[V];
-  const int m = compact_bases<NT, V>(valid, base, scan64);
-#pragma unroll
-  for (int j = 0; j < V; ++j) {
-    int p = base[j];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int c = 4 * j + k;
-      if ((valid >> c) & 1u) {
-        k0[p] = key_f32(desc ? -x[c] : x[c]);
-        i0[p] = static_cast<uint16_t>(4 * (j * NT + tid) + k);
-        ++p;
-      }
-    }
-  }
-  __syncthreads();
-  uint32_t* ks;
-  uint16_t* is;
-  block_radix_sort<NT, C, uint32_t>(k0, i0, k1, i1, m, sm + L.scratch, &ks, &is);
-  uint32_t* RK = (ks == k0) ? k1 : k0;
-  for (int p = tid; p < m; p += NT) RK[is[p]] = static_cast<uint32_t>(p + 1);
-  __syncthreads();
-  const float qnan = __uint_as_float(kQuietNanBits);
-  float v[C];
-#pragma unroll
-  for (int c = 0; c < C; ++c)
-    v[c] = ((valid >> c) & 1u) ? static_cast<float>(RK[4 * ((c >> 2) * NT + tid) + (c & 3)]) : qnan;
-  store_row_f32v<NT, V>(out + row, N, v);
-}
-
-// parameter_scan: one ascending sort of the finite cells serves all four
-// groups (asc / desc x masked / unmasked).  With S the start and E the end of
-// a cell's tie group in sorted order, C the count of masked-valid cells before
-// a sorted position and m / mt the finite / masked-valid totals:
-//   asc unmasked  p + 1                  asc masked   C[p] + 1
-//   desc unmasked m - E + (p - S) + 1    desc masked  mt - C[E] + (C[p] - C[S]) + 1
-// (descending ranks keep ties by ascending column, the contract of
-// fc/_cpu_core.py:57-78 / :295-301; replaces the reference's four rank
-// pipelines, src/cross_sectional_rank.cu:401-664).  Shared memory stays at
-// the sort's 12 bytes per cell: tie-group starts go to a bitmap (the sorted
-// keys are then free for C and E), and the ascending and descending pairs of
-// ranks pass through one per-column buffer in turn.
-template <int NT, int V>
-__global__ void __launch_bounds__(NT) k_pscan(const float* __restrict__ X, const uint8_t* __restrict__ mask, int N,
-                                              ScanOut outs) {
-  constexpr int C = 4 * V;
-  extern __shared__ __align__(16) uint8_t sm[];
-  const SortedLayout<NT> L(N);
-  unsigned long long* scan64 = reinterpret_cast<unsigned long long*>(sm + L.red);
-  uint32_t* scan32 = reinterpret_cast<uint32_t*>(sm + L.red);
-  uint32_t* bits = reinterpret_cast<uint32_t*>(sm + L.dw);  // tie-group start per sorted position
-  uint32_t* k0 = reinterpret_cast<uint32_t*>(sm + L.k0);
-  uint32_t* k1 = reinterpret_cast<uint32_t*>(sm + L.k1);
-  uint16_t* i0 = reinterpret_cast<uint16_t*>(sm + L.i0);
-  uint16_t* i1 = reinterpret_cast<uint16_t*>(sm + L.i1);
-  const int tid = static_cast<int>(threadIdx.x);
-  const size_t row = static_cast<size_t>(blockIdx.x) * N;
-  for (int k = tid; k < (N + 31) / 32 + 1; k += NT) bits[k] = 0u;
-  float x[C];
-  uint32_t mk[C];
-  load_row_f32<NT, V, true>(X + row, N, x);
-  load_mask4<NT, V>(mask != nullptr ? mask + row : nullptr, N, mk);
-  uint32_t fin = 0u, msk = 0u;
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    fin |= (finite_f32(x[c]) ? 1u : 0u) << c;
-    msk |= (mk[c] ? 1u : 0u) << c;
-  }
-  int base[V];
-  const int m = compact_bases<NT, V>(fin, base, scan64);  // its barriers publish the bitmap clear
-#pragma unroll
-  for (int j = 0; j < V; ++j) {
-    int p = base[j];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int c = 4 * j + k;
-      if ((fin >> c) & 1u) {
-        k0[p] = key_f32(x[c]);
-        i0[p] = static_cast<uint16_t>((4 * (j * NT + tid) + k) | (((msk >> c) & 1u) << 15));
-        ++p;
-      }
-    }
-  }
-  __syncthreads();
-  uint32_t* ks;
-  uint16_t* is;
-  block_radix_sort<NT, C, uint32_t>(k0, i0, k1, i1, m, sm + L.scratch, &ks, &is);
-  uint16_t* S = (is == i0) ? i1 : i0;                                // group start per sorted position
-  uint32_t* O = (ks == k0) ? k1 : k0;                                // two ranks per column
-  uint16_t* Cn = reinterpret_cast<uint16_t*>(ks);                    // m + 1 entries, over the sorted keys
-  uint16_t* GE = reinterpret_cast<uint16_t*>(ks) + (N + 1);          // group end by group start
-  // pass 1: per chunk, masked-valid count, last group start, start bits
-  const int per = (m + NT - 1) / NT;
-  const int b0 = tid * per, b1 = min(m, b0 + per);
-  uint32_t cm = 0;
-  int last = -1;
-  for (int p = b0; p < b1; ++p) {
-    cm += is[p] >> 15;
-    if (p == 0 || ks[p] != ks[p - 1]) {
-      last = p;
-      atomicOr(&bits[p >> 5], 1u << (p & 31));
-    }
-  }
-  uint32_t mt;
-  uint32_t c = block_exclusive_sum(cm, scan32, mt);  // barriers: ks reads done, bits complete
-  // exclusive max-scan of the chunks' last group starts (identity -1)
-  int inc = last;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(kFull, inc, o);
-    if (lane_id() >= static_cast<unsigned>(o)) inc = max(inc, u);
-  }
-  const int wi = tid >> 5;
-  int* sc = reinterpret_cast<int*>(scan64);
-  if (lane_id() == 31) sc[wi] = inc;
-  __syncthreads();
-  int carry = -1;
-  for (int i = 0; i < wi; ++i) carry = max(carry, sc[i]);
-  const int up = __shfl_up_sync(kFull, inc, 1);
-  if (lane_id() > 0) carry = max(carry, up);
-  // pass 2: S, the masked-valid prefix C and the group ends E
-  auto is_start = [&](int p) { return ((bits[p >> 5] >> (p & 31)) & 1u) != 0u; };
-  for (int p = b0; p < b1; ++p) {
-    if (is_start(p)) carry = p;
-    S[p] = static_cast<uint16_t>(carry);
-    Cn[p] = static_cast<uint16_t>(c);
-    c += is[p] >> 15;
-    if (p == m - 1 || is_start(p + 1)) GE[carry] = static_cast<uint16_t>(p + 1);
-  }
-  if (tid == 0) Cn[m] = static_cast<uint16_t>(mt);
-  __syncthreads();
-  const float qnan = __uint_as_float(kQuietNanBits);
-  // pass 3, twice: the ascending pair (groups 0 | 1), then the descending pair
-  // (groups 2 | 3), each stored by column and written out
-  for (int half = 0; half < 2; ++half) {
-    if (outs.out[2 * half] == nullptr && outs.out[2 * half + 1] == nullptr) continue;  // uniform
-    for (int p = tid; p < m; p += NT) {
-      const uint32_t id = is[p];
-      const uint32_t cp = Cn[p];
-      uint32_t lo = 0u, hi;
-      if (half == 0) {
-        hi = static_cast<uint32_t>(p + 1);
-        if (id & 0x8000u) lo = cp + 1u;
-      } else {
-        const int s0 = S[p], e0 = GE[s0];
-        hi = static_cast<uint32_t>(m - e0 + (p - s0) + 1);
-        if (id & 0x8000u) lo = mt - Cn[e0] + (cp - Cn[s0]) + 1u;
-      }
-      O[id & 0x3FFFu] = lo | (hi << 16);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int g2 = 0; g2 < 2; ++g2) {
-      float* dst = outs.out[2 * half + g2];
-      if (dst == nullptr) continue;  // uniform
-      const int sh = g2 ? 16 : 0;
-      float v[C];
-#pragma unroll
-      for (int cc = 0; cc < C; ++cc) {
-        const uint32_t r =
-            ((fin >> cc) & 1u) ? ((O[4 * ((cc >> 2) * NT + tid) + (cc & 3)] >> sh) & 0xFFFFu) : 0u;
-        v[cc] = r ? static_cast<float>(r) : qnan;
-      }
-      store_row_f32v<NT, V>(dst + row, N, v);
-    }
-    __syncthreads();  // O is rewritten by the second half
-  }
-}
-
-// ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
 namespace {
@@ -1108,50 +781,6 @@ RicPrep ric_prep_carve(void* base, int T, int N, int F) {
   return rp;
 }
 
-
-namespace {
-template <int NT, int V>
-cudaError_t csr_launch(const float* X, const uint8_t* mask, int T, int N, int desc, float* out, cudaStream_t st) {
-  const size_t smem = SortedLayout<NT>(N).total;
-  cudaError_t e = cudaFuncSetAttribute(k_csr<NT, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e != cudaSuccess) return e;
-  k_csr<NT, V><<<T, NT, smem, st>>>(X, mask, N, desc, out);
-  return cudaGetLastError();
-}
-template <int NT, int V>
-cudaError_t pscan_launch(const float* X, const uint8_t* mask, int T, int N, ScanOut outs, cudaStream_t st) {
-  const size_t smem = SortedLayout<NT>(N).total;
-  if (smem > kMaxSmemPerBlock) return cudaErrorInvalidValue;
-  cudaError_t e =
-      cudaFuncSetAttribute(k_pscan<NT, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e != cudaSuccess) return e;
-  k_pscan<NT, V><<<T, NT, smem, st>>>(X, mask, N, outs);
-  return cudaGetLastError();
-}
-}  // namespace
-
-
-// The per-date rank kernels stage nothing through mbarriers, so `status` has
-// nothing to report; it is kept for the callers' uniform interface.
-cudaError_t launch_cs_rank(const float* X, const uint8_t* mask, int T, int N, int desc, float* out, int* status,
-                           cudaStream_t st) {
-  (void)status;
-  if (N < 1 || N > kSmemRankCap) return cudaErrorInvalidValue;
-  if (N <= 2048) return csr_launch<256, 2>(X, mask, T, N, desc, out, st);
-  if (N <= 5120) return csr_launch<256, 5>(X, mask, T, N, desc, out, st);
-  if (N <= 8192) return csr_launch<512, 4>(X, mask, T, N, desc, out, st);
-  return csr_launch<512, 8>(X, mask, T, N, desc, out, st);
-}
-
-cudaError_t launch_param_scan(const float* X, const uint8_t* mask, int T, int N, ScanOut outs, int* status,
-                              cudaStream_t st) {
-  (void)status;
-  if (N < 1 || N > kSmemRankCap) return cudaErrorInvalidValue;
-  if (N <= 2048) return pscan_launch<256, 2>(X, mask, T, N, outs, st);
-  if (N <= 5120) return pscan_launch<256, 5>(X, mask, T, N, outs, st);
-  if (N <= 8192) return pscan_launch<512, 4>(X, mask, T, N, outs, st);
-  return pscan_launch<512, 8>(X, mask, T, N, outs, st);
-}
 
 namespace {
 template <int NT, int V>
