@@ -2,12 +2,13 @@
 //
 // Rank + IC of f32 panels: the per-(date, factor) kernels of the single-panel
 // entry points in batched form.  Panels are grouped by the kernel variant
-// their width needs (N up to 2048 / 5120 / 8192 / 16384; the first two
-// boundaries are tunable), and each variant is one returns-preparation
-// launch over all its panels' dates, one rank launch over all their
-// (date, factor) sections and, with learned splitters, one launch that ranks
-// the sections handed back to the radix sort -- the same device bodies, so
-// results are those of the single-panel calls bit for bit.
+// their width needs (N up to 1024 / 2048 / 3072 / 5120 / 8192 / 16384; how far
+// the narrow and the middle ones reach is tunable), and each variant is one
+// returns-preparation launch over all its panels' dates and one rank launch
+// over all their (date, factor) sections -- the same device bodies, so results
+// are those of the single-panel calls bit for bit.  A panel's CDF model changes
+// nothing here: the value-spread buckets rank its sections faster than the
+// model's do, with the same results.
 //
 // Rank + IC of f64 panels: every (panel, date) pair is one work item.  Items are grouped by
 // the block size their cross-section needs (256 / 512 / 1024 threads; the
@@ -203,21 +204,20 @@ int occupancy(const fcb_batch& b, int k, int* occ) {
 // f32 panels: the kernel variant of a panel of width N under the current
 // configuration (a panel may be served by a wider variant than it needs).
 int variant_of(const fcb_batch& b, int N) {
-  if (N <= std::min(b.cfg.nt_small_max, ric_variant_cap(0))) return 0;
-  if (N <= std::min(b.cfg.nt_mid_max, ric_variant_cap(1))) return 1;
-  if (N <= ric_variant_cap(2)) return 2;
-  return 3;
+  if (N <= std::min(b.cfg.nt_small_max, ric_variant_cap(1))) return N <= ric_variant_cap(0) ? 0 : 1;
+  if (N <= std::min(b.cfg.nt_mid_max, ric_variant_cap(3))) return N <= ric_variant_cap(2) ? 2 : 3;
+  if (N <= ric_variant_cap(4)) return 4;
+  return 5;
 }
 
 // f32 panels: per variant, the panel descriptors (order 1: widest work
-// first), their date and section offsets and the fallback list, uploaded in
-// one buffer.
+// first) and their date and section offsets, uploaded in one buffer.
 int plan_items(fcb_batch& b) {
   std::vector<int> idx[kRicVariants];
   for (size_t i = 0; i < b.p.size(); ++i) idx[variant_of(b, b.p[i].N)].push_back(static_cast<int>(i));
   auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
   size_t total = 0;
-  size_t o_pan[kRicVariants], o_od[kRicVariants], o_oi[kRicVariants], o_cnt[kRicVariants], o_items[kRicVariants];
+  size_t o_pan[kRicVariants], o_od[kRicVariants], o_oi[kRicVariants];
   long long ndates[kRicVariants] = {}, nitems[kRicVariants] = {};
   for (int k = 0; k < kRicVariants; ++k) {
     if (b.cfg.order == 1)
@@ -237,10 +237,6 @@ int plan_items(fcb_batch& b) {
     total += al(np * sizeof(int));
     o_oi[k] = total;
     total += al(np * sizeof(int));
-    o_cnt[k] = total;
-    total += 256;
-    o_items[k] = total;
-    total += al(static_cast<size_t>(nitems[k]) * sizeof(int));
   }
   if (b.ric_cap < total) {
     cudaFree(b.d_ric);
@@ -274,12 +270,6 @@ int plan_items(fcb_batch& b) {
       a.min_valid = b.min_valid;
       a.ranks_out = q.ranks_out;
       a.ic_out = q.ic_out;
-      if (q.model != nullptr) {
-        a.cdf_table = q.model->table[q.model->cur];
-        a.cdf_zrange = q.model->zrange[q.model->cur];
-        v.learned = true;
-      }
-      a.learn_cap = b.cfg.learn_cap > 0 ? b.cfg.learn_cap : kLearnCapDefault;
       hp[j] = RicPanel{a, b.preps[i]};
       hd[j] = od;
       hi[j] = oi;
@@ -292,7 +282,6 @@ int plan_items(fcb_batch& b) {
     v.panels = reinterpret_cast<const RicPanel*>(base + o_pan[k]);
     v.off_dates = reinterpret_cast<const int*>(base + o_od[k]);
     v.off_items = reinterpret_cast<const int*>(base + o_oi[k]);
-    v.fb = RicList{reinterpret_cast<int*>(base + o_cnt[k]), reinterpret_cast<int*>(base + o_items[k])};
   }
   FCB_BTRY(cudaMemcpy(b.d_ric, host.data(), total, cudaMemcpyHostToDevice));
   return FCB_OK;
@@ -367,16 +356,10 @@ int enqueue(fcb_batch& b, cudaStream_t s0) {
     if (b.cls_cnt[k] == 0) continue;
     cudaStream_t st = (b.cfg.concurrent && k > 0) ? b.s[k] : s0;
     const int2* items = b.d_items + b.cls_off[k];
-    if (b.dtx == FCB_DTYPE_F32)
-      FCB_BTRY(launch_rank_ic_batch<float, float>(kClassNt[k], b.learned,
-                                                  static_cast<const RankIcArgs<float, float>*>(b.d_args), items,
+    FCB_BTRY(launch_rank_ic_batch<double, double>(kClassNt[k], false,
+                                                  static_cast<const RankIcArgs<double, double>*>(b.d_args), items,
                                                   b.cls_cnt[k], b.d_ctr + k, b.cls_grid[k], b.cls_smem[k],
                                                   b.d_status, st, nullptr));
-    else
-      FCB_BTRY(launch_rank_ic_batch<double, double>(kClassNt[k], false,
-                                                    static_cast<const RankIcArgs<double, double>*>(b.d_args), items,
-                                                    b.cls_cnt[k], b.d_ctr + k, b.cls_grid[k], b.cls_smem[k],
-                                                    b.d_status, st, nullptr));
   }
   // factor_corr of every panel: one batched launch per kernel kind, on the
   // last branch, alongside the rank + IC kernels (it reads only the factor
@@ -395,8 +378,6 @@ int build_graph(fcb_batch& b) {
   b.drop_graph();
   int r = plan(b);
   if (r != FCB_OK) return r;
-  // the scheduling knob learn_cap lives in the panel arguments (f32: in the
-  // descriptors plan() uploaded)
   if (b.dtx != FCB_DTYPE_F32 && (r = upload_args<double, double>(b)) != FCB_OK) return r;
   FCB_BTRY(cudaStreamBeginCapture(b.s[0], cudaStreamCaptureModeRelaxed));
   r = enqueue(b, b.s[0]);
@@ -663,18 +644,10 @@ extern "C" int fcb_batch_run_per_panel(fcb_batch* b, void* stream) {
       a.min_valid = b->min_valid;
       a.ranks_out = q.ranks_out;
       a.ic_out = q.ic_out;
-      const bool lrn = q.model != nullptr;
-      if (lrn) {
-        a.cdf_table = q.model->table[q.model->cur];
-        a.cdf_zrange = q.model->zrange[q.model->cur];
-        a.learn_cap = b->cfg.learn_cap > 0 ? b->cfg.learn_cap : kLearnCapDefault;
-      }
       // as the single-panel entry points: several factors go through the
       // prepared returns and per-(date, factor) items, one factor per date
       if (a.F >= 2 && ric_items_fit(a.N))
-        FCB_BTRY(launch_rank_ic_items(a, b->preps[i], lrn, s));
-      else if (lrn)
-        FCB_BTRY(launch_rank_ic_learned(a, b->d_status, s));
+        FCB_BTRY(launch_rank_ic_items(a, b->preps[i], false, s));
       else
         FCB_BTRY(launch_rank_ic<float, float>(a, b->d_status, s));
     } else {
@@ -804,7 +777,6 @@ extern "C" int fcb_batch_autotune(fcb_batch* b, int reps, const char* cache_path
   // coordinate descent over the knobs, each alternative tried once
   const int small_opts[] = {1024, 2048, 4096};
   const int cps_opts[] = {0, 1, 2};
-  const int cap_opts[] = {64, 128, 256, 512};
   auto consider = [&](const fcb_batch_config& c) -> int {
     if (!valid_cfg(c)) return FCB_OK;
     b->cfg = c;
@@ -844,14 +816,6 @@ extern "C" int fcb_batch_autotune(fcb_batch* b, int reps, const char* cache_path
       if (c.concurrent == v) continue;
       c.concurrent = v;
       if ((r = consider(c)) != FCB_OK) return r;
-    }
-    if (b->learned) {
-      for (int v : cap_opts) {
-        fcb_batch_config c = best;
-        if (c.learn_cap == v) continue;
-        c.learn_cap = v;
-        if ((r = consider(c)) != FCB_OK) return r;
-      }
     }
     b->cfg = best;
     b->drop_graph();
@@ -900,14 +864,6 @@ extern "C" int fcb_batch_autotune(fcb_batch* b, int reps, const char* cache_path
     if (c.concurrent == v) continue;
     c.concurrent = v;
     if ((r = consider(c)) != FCB_OK) return r;
-  }
-  if (b->learned) {
-    for (int v : cap_opts) {
-      fcb_batch_config c = best;
-      if (c.learn_cap == v) continue;
-      c.learn_cap = v;
-      if ((r = consider(c)) != FCB_OK) return r;
-    }
   }
   b->cfg = best;
   b->drop_graph();

@@ -785,7 +785,7 @@ extern "C" int fcb_rank_ic_panel(const float* x, const float* r, const uint8_t* 
     if (learned) ws.poll_fit();
     if (learned && ws.model_ready) {
       const int e = fcb::rank_ic_learned_ld(dx[j], dr[j], dfm[j], drm[j], F, tc, N, min_valid, drk[j], dic + t0, T,
-                                            ws.model, 0, nullptr, s_c);
+                                            ws.model, 0, nullptr, true, s_c);
       if (e != 0) return e;
       ++ws.learned_chunks;
     } else {

@@ -179,15 +179,14 @@ cudaError_t launch_factor_corr(const void* X, int dtype, const uint8_t* mask, lo
 // stock i in the stable ascending order of the date's valid returns, bits
 // 14-27 the position where its tie group starts, bit 28 returns valid, bit 29
 // factor mask (N <= 16384; rows 16-byte aligned).  fb_count / fb_items: the
-// sections (t*F + f) the learned kernel hands to the radix kernel.
+// sections (t*F + f) the learned kernel hands back.
 struct RicPrep {
   uint32_t* word;
   int* fb_count;
   int* fb_items;
   int ld;
 };
-// A device list of sections (item ids) handed from the learned kernel to the
-// radix kernel.
+// A device list of sections (item ids) that the learned kernel hands back.
 struct RicList {
   int* count;
   int* items;
@@ -197,10 +196,9 @@ RicPrep ric_prep_carve(void* base, int T, int N, int F);
 // True when the per-(date, factor) kernels take N (f32 factors and returns).
 bool ric_items_fit(int N);
 // Batched form: the panels of one size variant (variant v serves N up to
-// ric_variant_cap(v): 2048, 5120, 8192, 16384) in one returns launch, one rank
-// launch and (learned) one fallback launch; items are a panel's dates (returns
-// pass) or its (date, factor) sections, in panel order.
-constexpr int kRicVariants = 4;
+// ric_variant_cap(v)) in one returns launch and one rank launch; items are a
+// panel's dates (returns pass) or its (date, factor) sections, in panel order.
+constexpr int kRicVariants = 6;
 int ric_variant_cap(int variant);
 struct RicPanel {
   RankIcArgs<float, float> a;
@@ -211,14 +209,12 @@ struct RicBatchVariant {
   const int* off_dates;    // device, exclusive prefix of the panels' T (np entries)
   const int* off_items;    // device, exclusive prefix of the panels' T*F (np entries)
   int np, dates, items, maxN;
-  bool learned;            // some panel has a model (its sections take the learned body)
-  RicList fb;              // the variant's fallback list (items entries)
 };
 cudaError_t launch_rank_ic_items_batch(int variant, const RicBatchVariant& v, cudaStream_t st);
 // Rank + IC of F >= 1 f32 factor panels against one f32 returns panel: the
-// returns pass, then one CTA per (date, factor) -- learned splitters (with the
-// radix kernel taking the sections they hand back) or radix.  Requires
-// rank_f_out == rank_r_out == nullptr.
+// returns pass, then one CTA per (date, factor) -- value-spread buckets, or
+// learned splitters (with the former taking the sections they hand back).
+// Requires rank_f_out == rank_r_out == nullptr.
 cudaError_t launch_rank_ic_items(const RankIcArgs<float, float>& a, RicPrep rp, bool learned, cudaStream_t st);
 // Stream-ordered scratch for the entry points that take no workspace: a
 // library-private memory pool per device that keeps freed blocks cached.

@@ -23,10 +23,6 @@
 namespace fcb {
 namespace {
 
-// Threads of one SM the plane kernels are compiled for: 64 registers each.
-// Fewer registers (three 512-thread CTAs per SM) spill and take longer.
-constexpr int kSmThreads = 1024;
-
 // cs_rank by radix: valid = finite & mask; the valid cells are compacted in
 // column order, radix-sorted by key (of -x for descending), and each cell's
 // rank is its sorted position + 1.
@@ -241,10 +237,7 @@ __global__ void __launch_bounds__(NT, kSmThreads / NT) k_csr(const float* __rest
     csr_radix<NT, V>(X, mask, N, desc, out, sm);
     return;
   }
-  const uint32_t mem_s = smem_u32(sm + L.mem);
-  const uint32_t* tie = reinterpret_cast<const uint32_t*>(sm + L.cnt);
-  if (T.heavy) spread_heavy<NT, V>(L, sm);
-  spread_positions<NT, V>(mem_s, mem_s + 8u * T.m, tie, key, W);
+  spread_positions<NT, V, false>(L, sm, T.m, T.heavy, key, W);
   float v[C];
 #pragma unroll
   for (int c = 0; c < C; ++c)
@@ -253,7 +246,7 @@ __global__ void __launch_bounds__(NT, kSmThreads / NT) k_csr(const float* __rest
 }
 
 // parameter_scan: the finite cells' buckets serve all four groups.  With less,
-// q and t of spread_ties, U[p] the finite cells outside the mask among the
+// q and t of spread_positions, U[p] the finite cells outside the mask among the
 // first p sorted positions (a bitmap over positions) and m / mu the finite
 // cells / those outside the mask:
 //   asc unmasked  less + t + 1           asc masked   the same - U[less + t]
@@ -270,7 +263,7 @@ __global__ void __launch_bounds__(NT, kSmThreads / NT) k_pscan(const float* __re
   const int tid = static_cast<int>(threadIdx.x);
   const size_t row = static_cast<size_t>(blockIdx.x) * N;
   uint32_t* bits = reinterpret_cast<uint32_t*>(sm + L.bits);
-  const int nbw = N / 16 + 2;
+  const int nbw = mark_words(N);
   for (int k = tid; k < nbw; k += NT) bits[k] = 0u;  // spread_place's barriers publish the clear
   uint32_t key[C], W[C], out_of_mask = 0u;
   {
@@ -289,16 +282,12 @@ __global__ void __launch_bounds__(NT, kSmThreads / NT) k_pscan(const float* __re
     pscan_radix<NT, V>(X, mask, N, outs, sm);
     return;
   }
-  const uint32_t mem_s = smem_u32(sm + L.mem);
   static_assert(kSpreadMaxBucket < 512, "ties fit 9-bit fields");
   // W[c] becomes less | t << 14 | q << 23, q = 0 for the cells not ranked
-  const uint32_t* tie = reinterpret_cast<const uint32_t*>(sm + L.cnt);
-  if (T.heavy) spread_heavy<NT, V>(L, sm);
+  spread_positions<NT, V, true>(L, sm, T.m, T.heavy, key, W);
 #pragma unroll
-  for (int c = 0; c < C; ++c) {
-    W[c] = spread_ties(mem_s, tie, W[c], key[c], cell_col<NT>(c));
+  for (int c = 0; c < C; ++c)
     if ((out_of_mask >> c) & 1u) mark_set(bits, (W[c] & 0x3FFFu) + ((W[c] >> 14) & 0x1FFu));
-  }
   if (__syncthreads_or(out_of_mask != 0u)) {
     if (tid < 32) mark_prefix(bits, nbw);
     __syncthreads();

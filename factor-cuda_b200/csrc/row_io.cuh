@@ -134,14 +134,19 @@ FCB_DEV int compact_bases(uint32_t flags, int (&base)[V], unsigned long long* sc
   return run;
 }
 
+// Words of a bitmap over sorted positions 0 .. n (see mark_set), or of one bit
+// per position with room to spare.
+__host__ __device__ inline int mark_words(int n) { return n / 16 + 2; }
+
 // Shared-memory layout of the radix-sorted forms (bytes; every region 16-aligned).
 template <int NT>
 struct SortedLayout {
-  size_t red, dw, scratch, k0, k1, i0, i1, total;
+  size_t red, dw, dw2, scratch, k0, k1, i0, i1, total;
   __host__ __device__ explicit SortedLayout(int n) {
     size_t o = 0;
     red = o; o += 1024;
-    dw = o; o = al16(o + size_t((n + 31) / 32 + 1) * 8);
+    dw = o; o = al16(o + size_t(mark_words(n)) * 4);   // two bitmaps over positions
+    dw2 = o; o = al16(o + size_t(mark_words(n)) * 4);  // for the kernels' own use
     scratch = o; o = al16(o + SortScratch<NT>::bytes);
     k0 = o; o = al16(o + size_t(n) * 4 + 16);
     k1 = o; o = al16(o + size_t(n) * 4 + 16);

@@ -26,18 +26,22 @@
 
 namespace fcb {
 
+// Threads of one SM the section kernels are compiled for: 64 registers each.
+// Fewer registers (three 512-thread CTAs per SM) spill and take longer.
+constexpr int kSmThreads = 1024;
+
 // Largest bucket, and largest mean bucket seen by a cell (sum of squared
 // sizes over cells), that the in-bucket counts take.  The largest bucket also
-// bounds the 9-bit fields of W and of the tie words.
+// bounds the 9-bit fields of the tie words.
 constexpr uint32_t kSpreadMaxBucket = 500;
 constexpr uint32_t kSpreadMeanBucket = 24;
 // Equal neighbours (columns 2i, 2i + 1) above which a section goes to its
 // radix form before any bucket is counted: twice their number estimates the
 // mean number of cells that share a cell's value.
 constexpr uint32_t kSpreadMaxEqualPairs = 8;
-// A bucket above this size is ranked by warps, 32 of its words at a time
-// against all of them, and not by its cells' own threads, whose warps would
-// wait for the longest loop.
+// A bucket above this size (a few equal values, as a rule) is ranked by warps,
+// 32 of its words at a time against all of them, and not by its cells' own
+// threads, whose warps would wait for the longest loop.
 constexpr uint32_t kSpreadHeavy = 16;
 // A section whose bins hold, by the mean over its cells, more than this
 // fraction of it is a cluster far narrower than its range.
@@ -46,21 +50,25 @@ constexpr uint32_t kSpreadBinShare = 8;
 template <int NT, int V>
 struct SpreadLayout {
   static constexpr int K = 2 * NT;  // bins: two per thread
+  static_assert(V <= 4, "the list of heavy buckets fits the bins");
   // counters one thread scans: they cover every bucket (a power of two where
   // that wastes little; 32 for V = 4 would spill)
   static constexpr int P = V == 1 ? 8 : V <= 3 ? 16 : 4 * V + 4;
-  size_t red, tab, bits, cnt, mem, total;
+  size_t red, tab, knots, bits, bits2, cnt, mem, total;
   int S;  // counter stride: bucket b is counter (b % P) * S + b / P
   __host__ __device__ explicit SpreadLayout(int n) {
     size_t o = 0;
     red = o; o += 1024;
     tab = o; o += size_t(K) * 4;
-    bits = o; o = al16(o + size_t(n / 16 + 2) * 4);
+    knots = tab; o = tab + size_t(K > kCdfKnots ? K : kCdfKnots) * 4;  // k_ric_learned's table
+    bits = o; o = al16(o + size_t(mark_words(n)) * 4);   // two bitmaps over positions
+    bits2 = o; o = al16(o + size_t(mark_words(n)) * 4);  // for the kernels' own use
     S = ((n + K + P - 1) / P + 3) & ~3;  // at most n + K buckets
     cnt = o; o += size_t(P) * S * 4;
     mem = o; o = al16(o + size_t(n + 4) * 8);  // the four words after the last cell's are the pad
     total = o;
   }
+  static_assert(4 * V * NT + K <= P * NT, "one scan step covers every bucket");
 };
 
 // One word per warp in shared memory -> block result, in every thread.
@@ -113,7 +121,7 @@ FCB_DEV void smem_store2_if(bool p, uint32_t addr, uint32_t lo, uint32_t hi) {
 
 struct SpreadTotals {
   int m;           // valid cells
-  bool heavy;      // some bucket may be above kSpreadHeavy
+  bool heavy;      // some bucket is above kSpreadHeavy
   uint32_t range;  // largest valid key less the smallest
 };
 
@@ -144,40 +152,93 @@ FCB_DEV void bucket_scan(uint32_t* cnt, int S, uint32_t* red) {
   }
 }
 
-// The scanned buckets above kSpreadHeavy, one item (start | size << 14 | part
-// << 23) per 32 words; *items (0 before) counts them.
-FCB_DEV void list_heavy(const uint32_t* cnt, int counters, uint32_t* list, uint32_t* items) {
-  for (int i = static_cast<int>(threadIdx.x); i < counters; i += static_cast<int>(blockDim.x)) {
-    const uint32_t w = cnt[i], n = w >> 14;
-    if (n > kSpreadHeavy && n <= kSpreadMaxBucket) {  // n of an empty bucket at 2^14 reads 1
-      const uint32_t parts = (n + 31u) / 32u, at = atomicAdd(items, parts);
-      for (uint32_t k = 0; k < parts; ++k) list[at + k] = w | (k << 23);
-    }
-  }
-}
-
 // Column of cell c of this thread in the vector layout.
 template <int NT>
 FCB_DEV uint32_t cell_col(int c) { return 4u * ((c >> 2) * NT + threadIdx.x) + (c & 3); }
 
+// Counts the cells (key[c] <= range) into their buckets: buckets(j, b) gives
+// the buckets of the four cells of vector j (anything for the others).  The
+// counters are zero before.  W[c] becomes the counter index | slot << 16, with
+// slot the cell's arrival number in its bucket, so that the largest slot is
+// the largest bucket's size less one and twice the slots' sum is the sum of
+// squared sizes less m.  Ends with a barrier.  red: words [160, 224).
+struct CountTotals {
+  uint32_t largest, squares;  // largest bucket; sum of squared sizes less m
+};
+template <int NT, int V, typename Buckets>
+FCB_DEV CountTotals count_cells(const uint32_t (&key)[4 * V], uint32_t range, const SpreadLayout<NT, V>& L, uint8_t* sm,
+                                uint32_t (&W)[4 * V], Buckets buckets) {
+  constexpr int NW = NT / 32, P = SpreadLayout<NT, V>::P;
+  uint32_t* red = reinterpret_cast<uint32_t*>(sm + L.red);
+  const uint32_t cnt_s = smem_u32(sm + L.cnt);
+  uint32_t sum = 0u, mx = 0u;
+#pragma unroll
+  for (int j = 0; j < V; ++j) {
+    uint32_t b[4];
+    buckets(j, b);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = 4 * j + k;
+      const uint32_t q = (b[k] % P) * L.S + b[k] / P;
+      const uint32_t s = smem_fetch_inc_if(key[c] <= range, cnt_s + 4u * q);
+      sum += s;
+      mx = max(mx, s);
+      W[c] = q | (s << 16);
+    }
+  }
+  sum = __reduce_add_sync(kFull, sum);
+  mx = __reduce_max_sync(kFull, mx);
+  if (lane_id() == 0) {
+    red[160 + (threadIdx.x >> 5)] = sum;
+    red[192 + (threadIdx.x >> 5)] = mx;
+  }
+  __syncthreads();
+  return CountTotals{warps_max<NW>(red + 192) + 1u, 2u * warps_sum<NW>(red + 160)};
+}
+
+// Scans the counters and scatters the cells into their bucket slots: W[c] of
+// a counted cell becomes its bucket's start | size << 14, 0 for the others;
+// mem holds the (key << 32 | column) words grouped by bucket, then four
+// all-ones words.  Ends with a barrier.
+template <int NT, int V>
+FCB_DEV void scatter_cells(const uint32_t (&key)[4 * V], uint32_t range, int m, const SpreadLayout<NT, V>& L,
+                           uint8_t* sm, uint32_t (&W)[4 * V]) {
+  uint32_t* cnt = reinterpret_cast<uint32_t*>(sm + L.cnt);
+  const uint32_t cnt_s = smem_u32(cnt), mem_s = smem_u32(sm + L.mem);
+  bucket_scan<NT / 32, SpreadLayout<NT, V>::P>(cnt, L.S, reinterpret_cast<uint32_t*>(sm + L.red));
+  if (threadIdx.x < 4) reinterpret_cast<unsigned long long*>(sm + L.mem)[m + threadIdx.x] = ~0ull;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < V; ++j) {  // four cells' loads in flight at a time
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[k] = smem_load_if(key[4 * j + k] <= range, cnt_s + 4u * (W[4 * j + k] & 0xFFFFu));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = 4 * j + k;
+      const uint32_t p = (w[k] & 0x3FFFu) + (W[c] >> 16);
+      smem_store2_if(key[c] <= range, mem_s + 8u * p, cell_col<NT>(c), key[c]);
+      W[c] = w[k];
+    }
+  }
+  __syncthreads();
+}
+
 // Places the valid cells (key[c] != kInvalidKey32) in bucket slots.  key[c]
 // becomes the distance from the smallest valid key, above T.range for the
 // invalid cells.  On true, W[c] of a valid cell is its bucket's start | size
-// << 14 and its own slot in the bucket << 23, 0 for the others; mem holds the
-// (distance << 32 | column) words of the valid cells grouped by bucket, then
-// four all-ones words.  On false (crowded buckets) shared memory holds nothing
+// << 14 and mem its words (scatter_cells).  On false (crowded buckets) shared memory holds nothing
 // of use.  Uniform across
 // the block; every thread calls; ends with a barrier.  T.m == 0 returns true
-// with nothing placed.
+// with nothing placed but the pad.
 template <int NT, int V>
 FCB_DEV bool spread_place(uint32_t (&key)[4 * V], const SpreadLayout<NT, V>& L, uint8_t* sm, uint32_t (&W)[4 * V],
                           SpreadTotals& T) {
   constexpr int C = 4 * V, NW = NT / 32, K = SpreadLayout<NT, V>::K, P = SpreadLayout<NT, V>::P;
-  static_assert(4 * NT * V + K <= P * NT, "one scan step covers every bucket");
   uint32_t* red = reinterpret_cast<uint32_t*>(sm + L.red);
   uint32_t* tab = reinterpret_cast<uint32_t*>(sm + L.tab);
   uint32_t* cnt = reinterpret_cast<uint32_t*>(sm + L.cnt);
-  const uint32_t tab_s = smem_u32(tab), cnt_s = smem_u32(cnt), mem_s = smem_u32(sm + L.mem);
+  const uint32_t tab_s = smem_u32(tab);
   const int tid = static_cast<int>(threadIdx.x), wi = tid >> 5;
   // ---- key range; clear the bins and the bucket counters
   *reinterpret_cast<uint2*>(tab + 2 * tid) = make_uint2(0u, 0u);
@@ -210,6 +271,8 @@ FCB_DEV bool spread_place(uint32_t (&key)[4 * V], const SpreadLayout<NT, V>& L, 
     T.range = 0u;
 #pragma unroll
     for (int c = 0; c < C; ++c) W[c] = 0u;
+    if (tid < 4) reinterpret_cast<unsigned long long*>(sm + L.mem)[tid] = ~0ull;
+    __syncthreads();  // (the caller also reuses red)
     return true;
   }
   T.range = range;
@@ -245,51 +308,21 @@ FCB_DEV bool spread_place(uint32_t (&key)[4 * V], const SpreadLayout<NT, V>& L, 
     *reinterpret_cast<uint2*>(tab + 2 * tid) = make_uint2(ex | (w0 << 16), (ex + w0) | (w1 << 16));
   }
   __syncthreads();
-  // ---- bucket of every cell, counted; the returned count is the cell's slot
-  // in the bucket, so twice their sum is the sum of squared sizes less m
-  uint32_t sum = 0u, any = 0u;
-#pragma unroll
-  for (int j = 0; j < V; ++j) {  // four cells' loads in flight at a time
+  // ---- counts, scan, scatter
+  const CountTotals ct = count_cells<NT, V>(key, range, L, sm, W, [&](int j, uint32_t (&b)[4]) {
     uint32_t bw[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < 4; ++k)  // four cells' loads in flight at a time
       bw[k] = smem_load_if(key[4 * j + k] <= range, tab_s + 4u * __umulhi(key[4 * j + k], scale));
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int c = 4 * j + k;
-      const uint32_t b = (bw[k] & 0xFFFFu) + __umulhi(key[c] * scale, bw[k] >> 16);
-      const uint32_t q = (b % P) * L.S + b / P;
-      const uint32_t s = smem_fetch_inc_if(key[c] <= range, cnt_s + 4u * q);
-      sum += s;
-      any |= s;
-      W[c] = q | (s << 16);
-    }
-  }
-  sum = __reduce_add_sync(kFull, sum);
-  if (lane_id() == 0) red[160 + wi] = sum;
-  T.heavy = __syncthreads_or(any >= kSpreadHeavy);  // a slot above 15
-  sum = 2u * warps_sum<NW>(red + 160) + static_cast<uint32_t>(T.m);
-  if (sum > kSpreadMaxBucket * kSpreadMaxBucket || sum > kSpreadMeanBucket * static_cast<uint32_t>(T.m)) {
+    for (int k = 0; k < 4; ++k) b[k] = (bw[k] & 0xFFFFu) + __umulhi(key[4 * j + k] * scale, bw[k] >> 16);
+  });
+  if (ct.largest > kSpreadMaxBucket || ct.squares > (kSpreadMeanBucket - 1u) * static_cast<uint32_t>(T.m)) {
     __syncthreads();  // the caller reuses the shared memory
     return false;
   }
-  bucket_scan<NW, P>(cnt, L.S, red);
-  if (tid < 4) reinterpret_cast<unsigned long long*>(sm + L.mem)[T.m + tid] = ~0ull;
-  __syncthreads();
-  // ---- scatter
-#pragma unroll
-  for (int j = 0; j < V; ++j) {
-    uint32_t w[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) w[k] = smem_load_if(key[4 * j + k] <= range, cnt_s + 4u * (W[4 * j + k] & 0xFFFFu));
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int c = 4 * j + k;
-      smem_store2_if(key[c] <= range, mem_s + 8u * ((w[k] & 0x3FFFu) + (W[c] >> 16)), cell_col<NT>(c), key[c]);
-      W[c] = w[k] + ((W[c] >> 16) << 23);
-    }
-  }
-  __syncthreads();
+  T.heavy = ct.largest > kSpreadHeavy;
+  scatter_cells<NT, V>(key, range, T.m, L, sm, W);
   return true;
 }
 
@@ -299,96 +332,112 @@ FCB_DEV unsigned long long smem_load64(uint32_t addr) {
   return v;
 }
 
-// Tie words of the buckets above kSpreadHeavy, one per slot, over the bucket
-// counters: less | t << 14 | q << 23 (see spread_ties).  The buckets are listed
+// What a cell's words count in its bucket, from slot k on.
+struct InBucket {
+  uint32_t before = 0u, less = 0u, le = 0u;  // smaller words; smaller keys; keys no larger
+  template <bool TIES>
+  FCB_DEV void add(unsigned long long o, unsigned long long mine) {
+    before += o < mine ? 1u : 0u;
+    if (TIES) {
+      less += static_cast<uint32_t>(o >> 32) < static_cast<uint32_t>(mine >> 32) ? 1u : 0u;
+      le += static_cast<uint32_t>(o >> 32) <= static_cast<uint32_t>(mine >> 32) ? 1u : 0u;
+    }
+  }
+  // the bucket starts at s: the sorted position, or the tie word
+  template <bool TIES>
+  FCB_DEV uint32_t result(uint32_t s) const {
+    return TIES ? (s + less) | ((before - less) << 14) | ((le - less) << 23) : s + before;
+  }
+};
+
+// The scanned buckets above kSpreadHeavy, one item (start | part << 16, size)
+// per 32 words; *items (0 before) counts them.
+FCB_DEV void list_heavy(const uint32_t* cnt, int counters, uint2* list, uint32_t* items) {
+  for (int i = static_cast<int>(threadIdx.x); i < counters; i += static_cast<int>(blockDim.x)) {
+    const uint32_t w = cnt[i], n = w >> 14;
+    if (n > kSpreadHeavy) {  // (an empty bucket at 2^14 reads n = 1)
+      const uint32_t parts = (n + 31u) / 32u, at = atomicAdd(items, parts);
+      for (uint32_t k = 0; k < parts; ++k) list[at + k] = make_uint2((w & 0x3FFFu) | (k << 16), n);
+    }
+  }
+}
+
+// Buckets above kSpreadHeavy: a word per column, over the bucket counters, with
+// the cell's sorted position or (TIES) its tie word.  The buckets are listed
 // where the bins were; each warp takes 32 words of one against all of its
-// words (broadcast reads).  Call when T.heavy (uniform); ends with a barrier.
-template <int NT, int V>
-FCB_DEV void spread_heavy(const SpreadLayout<NT, V>& L, uint8_t* sm) {
-  constexpr int P = SpreadLayout<NT, V>::P;
+// words (broadcast reads).  Call when some bucket is that large (uniform);
+// ends with a barrier.
+template <int NT, int V, bool TIES>
+FCB_DEV void rank_heavy(const SpreadLayout<NT, V>& L, uint8_t* sm) {
   uint32_t* red = reinterpret_cast<uint32_t*>(sm + L.red);
-  uint32_t* list = reinterpret_cast<uint32_t*>(sm + L.tab);
-  uint32_t* tie = reinterpret_cast<uint32_t*>(sm + L.cnt);
+  uint2* list = reinterpret_cast<uint2*>(sm + L.tab);
+  uint32_t* by_col = reinterpret_cast<uint32_t*>(sm + L.cnt);
   const uint32_t mem_s = smem_u32(sm + L.mem);
-  list_heavy(tie, P * L.S, list, &red[224]);
+  list_heavy(by_col, SpreadLayout<NT, V>::P * L.S, list, &red[224]);
   __syncthreads();
   const int items = static_cast<int>(red[224]);
   for (int it = static_cast<int>(threadIdx.x >> 5); it < items; it += NT / 32) {
-    const uint32_t w = list[it], s = w & 0x3FFFu, n = (w >> 14) & 0x1FFu, i = (w >> 23) * 32u + lane_id();
+    const uint2 w = list[it];
+    const uint32_t s = w.x & 0xFFFFu, n = w.y, i = (w.x >> 16) * 32u + lane_id();
     const unsigned long long mine = i < n ? smem_load64(mem_s + 8u * (s + i)) : 0ull;
-    const uint32_t key = static_cast<uint32_t>(mine >> 32);
-    uint32_t less = 0u, le = 0u, before = 0u;
+    InBucket ib;
 #pragma unroll 4
-    for (uint32_t k = 0; k < n; ++k) {
-      const unsigned long long o = smem_load64(mem_s + 8u * (s + k));
-      const uint32_t ok = static_cast<uint32_t>(o >> 32);
-      less += ok < key ? 1u : 0u;
-      le += ok <= key ? 1u : 0u;
-      before += o < mine ? 1u : 0u;
-    }
-    if (i < n) tie[s + i] = (s + less) | ((before - less) << 14) | ((le - less) << 23);
+    for (uint32_t k = 0; k < n; ++k) ib.add<TIES>(smem_load64(mem_s + 8u * (s + k)), mine);
+    if (i < n) by_col[static_cast<uint32_t>(mine)] = ib.result<TIES>(s);
   }
   __syncthreads();
 }
 
-// Sorted position of every cell, in place of its W: its bucket's start plus
-// the smaller words in its bucket (0 for the cells with W = 0, which read
-// nothing of use).  The first four slots of four cells at a time are compared
-// in straight line, so that their loads overlap; slots past a bucket's end
-// hold larger words, and lanes with nothing (more) to compare share the pad's
-// all-ones words, which costs no bank conflict.  tie: spread_heavy's words.
-template <int NT, int V>
-FCB_DEV void spread_positions(uint32_t mem_s, uint32_t pad_s, const uint32_t* tie, const uint32_t (&key)[4 * V],
+// Sorted position of every cell, in place of its W (of no use for the cells
+// with W = 0).  TIES: its tie word instead, less | t << 14 | q << 23 (q = 0 for
+// the cells with W = 0): less = sorted position of its first equal key, t equal
+// keys at smaller columns (position less + t), q equal keys in all.
+// The first four slots of four cells at a time are compared in straight line,
+// so that their loads overlap: slots past a bucket's end hold larger words,
+// and lanes with nothing (more) to compare share the pad's all-ones words,
+// which costs no bank conflict.  by_col: rank_heavy's results.
+template <int NT, int V, bool TIES>
+FCB_DEV void spread_positions(const SpreadLayout<NT, V>& L, uint8_t* sm, int m, bool heavy, const uint32_t (&key)[4 * V],
                               uint32_t (&W)[4 * V]) {
+  const uint32_t* by_col = reinterpret_cast<const uint32_t*>(sm + L.cnt);
+  const uint32_t mem_s = smem_u32(sm + L.mem), pad_s = mem_s + 8u * static_cast<uint32_t>(m);
+  if (heavy) rank_heavy<NT, V, TIES>(L, sm);  // uniform
 #pragma unroll
   for (int j = 0; j < V; ++j) {
     uint32_t r[4], most = 0u;
+    InBucket ib[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int c = 4 * j + k;
-      const uint32_t n = (W[c] >> 14) & 0x1FFu, s = W[c] & 0x3FFFu, a = mem_s + 8u * s;
+      const uint32_t n = W[c] >> 14, s = W[c] & 0x3FFFu, a = mem_s + 8u * s;
       const uint32_t a01 = n > 1u ? a : pad_s;  // a bucket of one is the cell itself
       const uint32_t a23 = n > 2u ? a + 16u : pad_s;
       const unsigned long long mine = (static_cast<unsigned long long>(key[c]) << 32) | cell_col<NT>(c);
-      const unsigned long long o0 = smem_load64(a01), o1 = smem_load64(a01 + 8u);
-      const unsigned long long o2 = smem_load64(a23), o3 = smem_load64(a23 + 8u);
-      r[k] = s + (o0 < mine ? 1u : 0u) + (o1 < mine ? 1u : 0u) + (o2 < mine ? 1u : 0u) + (o3 < mine ? 1u : 0u);
-      most = max(most, n);
+      ib[k].add<TIES>(smem_load64(a01), mine);
+      ib[k].add<TIES>(smem_load64(a01 + 8u), mine);
+      ib[k].add<TIES>(smem_load64(a23), mine);
+      ib[k].add<TIES>(smem_load64(a23 + 8u), mine);
+      r[k] = ib[k].result<TIES>(s);
+      if (TIES && n <= 1u) r[k] = s | (n << 23);  // the pad does not hold the cell itself
+      most = max(most, W[c]);
     }
-    if (most > 4u) {
+    if (most >= (5u << 14)) {  // some bucket of more than four
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int c = 4 * j + k;
-        const uint32_t n = (W[c] >> 14) & 0x1FFu, s = W[c] & 0x3FFFu;
+        const uint32_t n = W[c] >> 14, s = W[c] & 0x3FFFu;
         if (n > kSpreadHeavy) {
-          const uint32_t v = tie[s + (W[c] >> 23)];
-          r[k] = (v & 0x3FFFu) + ((v >> 14) & 0x1FFu);
-        } else {
+          r[k] = by_col[cell_col<NT>(c)];
+        } else if (n > 4u) {
           const unsigned long long mine = (static_cast<unsigned long long>(key[c]) << 32) | cell_col<NT>(c);
-          for (uint32_t i = 4u; i < n; ++i) r[k] += smem_load64(mem_s + 8u * (s + i)) < mine ? 1u : 0u;
+          for (uint32_t i = 4u; i < n; ++i) ib[k].add<TIES>(smem_load64(mem_s + 8u * (s + i)), mine);
+          r[k] = ib[k].result<TIES>(s);
         }
       }
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) W[4 * j + k] = r[k];
   }
-}
-
-// One cell with its ties, less | t << 14 | q << 23 (0 for a cell with W = 0):
-// less = sorted position of its first equal key, t equal keys at smaller
-// columns (position less + t), q equal keys in all, itself included.
-FCB_DEV uint32_t spread_ties(uint32_t mem_s, const uint32_t* tie, uint32_t w, uint32_t key, uint32_t i) {
-  const uint32_t s = w & 0x3FFFu, n = (w >> 14) & 0x1FFu;
-  if (n > kSpreadHeavy) return tie[s + (w >> 23)];
-  uint32_t v = s | (n == 1u ? 1u << 23 : 0u);  // a bucket of one is the cell itself
-  if (n > 1u)
-    for (uint32_t k = 0; k < n; ++k) {
-      const unsigned long long o = smem_load64(mem_s + 8u * (s + k));
-      const uint32_t ok = static_cast<uint32_t>(o >> 32);
-      v += ok < key ? 1u : 0u;
-      if (ok == key) v += (1u << 23) + (static_cast<uint32_t>(o) < i ? 1u << 14 : 0u);
-    }
-  return v;
 }
 
 // Bitmap over sorted positions, 16 positions per word: bits 0-15 the marks,
@@ -407,7 +456,9 @@ FCB_DEV void mark_prefix(uint32_t* bits, int nwords) {  // one warp
 }
 FCB_DEV uint32_t marks_before(const uint32_t* bits, uint32_t p) {
   const uint32_t v = bits[p >> 4];
-  return (v >> 16) + __popc(v & ((1u << (p & 15u)) - 1u));
+  uint32_t below;
+  asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(below) : "r"(p & 15u));  // the bits below p's
+  return (v >> 16) + __popc(v & below);
 }
 
 }  // namespace fcb

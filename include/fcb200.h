@@ -297,8 +297,10 @@ int fcb_cdf_model_load(fcb_cdf_model* m, const float* params, const float* zrang
  * for one batch of n <= 256 samples, by the training kernel's own
  * forward/backward code.  Host pointers; for checking. */
 int fcb_cdf_grad(const float* params, const float* z, const float* u, int n, float* grad, float* loss);
-/* Learned rank + IC over device panels (as fcb_dev_rank_ic_panel); d_stats
- * (NULL = off) receives (F,T,4) ints: outcome (1 learned, 2 bucket overflow,
+/* Learned rank + IC over device panels (as fcb_dev_rank_ic_panel).  Ranks and
+ * IC do not depend on the model; without d_stats, panels of several factors
+ * take the value-spread buckets of fcb_dev_rank_ic_panel, which are faster.
+ * d_stats (NULL = off) receives (F,T,4) ints: outcome (1 learned, 2 bucket overflow,
  * 3 order check rejected -- with several factors, a staged CDF table that
  * is not non-decreasing within [0, 1]; with one factor, the ranked keys out
  * of order --, 4 unusable scale; 2-4 fell back to radix), the largest
@@ -385,10 +387,9 @@ int fcb_dev_factor_corr_noalloc(const void* d_x, int dtype, const uint8_t* d_mas
  * computes, for every panel, what fcb_dev_rank_ic_panel (cs_rank ranks +
  * rolling_ic) and fcb_factor_corr compute for it alone -- bit for bit.
  * Rank + IC of f32 panels runs the single-panel per-(date, factor) kernels in
- * batched form: per kernel variant (N up to 2048 / 5120 / 8192 / 16384), one
- * returns launch over every date of its panels, one rank launch over every
- * (date, factor) section and, with learned splitters, one launch ranking the
- * sections handed back to the radix sort.  f64 panels run persistent kernels
+ * batched form: per kernel variant (see fcb_batch_config), one returns launch
+ * over every date of its panels and one rank launch over every (date, factor)
+ * section.  f64 panels run persistent kernels
  * taking (panel, date) items from device queues.  factor_corr follows; the
  * sequence is captured once into a CUDA graph and replayed.  All pointers are
  * DEVICE pointers owned by the caller and must stay valid for the batch's
@@ -410,14 +411,15 @@ typedef struct fcb_panel {
   double* ic_out;              /* (F,T) rolling IC                               */
   double* corr_out;            /* (F,F) factor_corr over the panel's (t,i) rows
                                   (fmask broadcast per column; F <= 128) or NULL */
-  const fcb_cdf_model* model;  /* learned splitters for this panel's factors
-                                  (f32 only, fitted, model F == F) or NULL       */
+  const fcb_cdf_model* model;  /* a CDF model of this panel's factors (f32 only,
+                                  fitted, model F == F) or NULL; results do not
+                                  depend on it                                   */
 } fcb_panel;
 
 /* Scheduling knobs.  None of them changes a result.  f32 panels: a panel of
- * width N runs in the narrowest kernel variant whose range holds it, the
- * first two ranges being N <= min(nt_small_max, 2048) and
- * N <= min(nt_mid_max, 5120) (then 8192, 16384); ctas_per_sm is not used.
+ * width N runs in the narrowest kernel variant whose range holds it: up to
+ * 1024 and 2048 (N <= nt_small_max), 3072 and 5120 (N <= nt_mid_max), 8192,
+ * 16384; ctas_per_sm and learn_cap are not used.
  * f64 panels: size classes of 256 / 512 / 1024-thread persistent CTAs. */
 typedef struct fcb_batch_config {
   int nt_small_max;  /* f64: largest N ranked by 256-thread CTAs (1..4096)       */
@@ -427,7 +429,7 @@ typedef struct fcb_batch_config {
   int concurrent;    /* 1: size classes (variants) run side by side; 0: one
                         after another, each on the whole GPU                    */
   int order;         /* 1: longest panels / items first; 0: panel order         */
-  int learn_cap;     /* largest learned bucket before the radix fallback         */
+  int learn_cap;     /* not used (kept for the layout)                           */
 } fcb_batch_config;
 
 void fcb_batch_default_config(fcb_batch_config* cfg);
