@@ -25,7 +25,7 @@ using namespace fcb;
 // ---------------------------------------------------------------------------
 enum Slot : int {
   S_X = 0, S_X2, S_MASK, S_MASK2, S_OUT, S_OUT1, S_OUT2, S_OUT3, S_STATUS, S_IC, S_RF, S_RR,
-  S_SC_RAW, S_SC_C, S_SC_M, S_SC_ST, S_SC_SUM, S_FB_LIST, S_FB_CNT,
+  S_SC_RAW, S_SC_C, S_SC_M, S_SC_AB, S_SC_ST, S_SC_SUM, S_FB_LIST, S_FB_CNT,
   S_FC_COLPART, S_FC_COLSTAT, S_FC_GRAM, S_FC_FLAGS, S_FC_FBPART,
   S_PC_MU, S_PC_XH, S_PC_XM, S_PC_XL, S_PC_QH, S_PC_QM, S_PC_QL, S_PC_M16, S_PC_X32, S_PC_Q32, S_PC_M32, S_PC_TILES, S_PC_X, S_PC_MASK,
   S_PC_OUT, S_PC_CPART, S_GSCR, S_RICPREP, S_FCT_WORK,
@@ -847,31 +847,28 @@ extern "C" int fcb_dev_stock_corr(const void* d_x, int dtype, const uint8_t* d_m
   fcb_workspace& ws = *wsp;
   FCB_TRY(ws.bind());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int Tp = (T + 31) / 32 * 32;
-  double *xraw, *xc, *mc, *sum;
-  ColStat* st;
-  int *fbl, *fbc;
-  FCB_TRY(ws.get(S_SC_RAW, static_cast<size_t>(N) * Tp * 8, &xraw));
-  FCB_TRY(ws.get(S_SC_C, static_cast<size_t>(N) * Tp * 8, &xc));
-  FCB_TRY(ws.get(S_SC_M, static_cast<size_t>(N) * Tp * 8, &mc));
-  FCB_TRY(ws.get(S_SC_ST, static_cast<size_t>(N) * sizeof(ColStat), &st));
-  FCB_TRY(ws.get(S_SC_SUM, 64, &sum));
+  const size_t Tp = static_cast<size_t>((T + 31) / 32 * 32);
+  ScWork w{};
+  FCB_TRY(ws.get(S_SC_RAW, N * Tp * 8, &w.xraw));
+  FCB_TRY(ws.get(S_SC_C, N * Tp * 8, &w.xc));
+  FCB_TRY(ws.get(S_SC_M, sc_masks_bytes(T, N), &w.masks));
+  FCB_TRY(ws.get(S_SC_AB, sc_pairs_bytes(N), &w.ab));
+  FCB_TRY(ws.get(S_SC_ST, static_cast<size_t>(N) * sizeof(ColStat), &w.st));
+  FCB_TRY(ws.get(S_SC_SUM, 64, &w.summary));
   const size_t upper = static_cast<size_t>(N) * (N - 1) / 2;
-  FCB_TRY(ws.get(S_FB_LIST, (upper > 0 ? upper : 1) * 4, &fbl));
-  FCB_TRY(ws.get(S_FB_CNT, 64, &fbc));
-  FCB_TRY(launch_stock_corr_prep(d_x, dtype, d_mask, T, N, Tp, xraw, xc, mc, st, sum, s));
-  // the domain check and the path flag are read on the host before the Gram pass
-  double hs[3];
-  FCB_TRY(cudaMemcpyAsync(hs, sum, sizeof(hs), cudaMemcpyDeviceToHost, s));
+  FCB_TRY(ws.get(S_FB_LIST, (upper > 0 ? upper : 1) * 4, &w.fb_list));
+  FCB_TRY(launch_stock_corr(d_x, dtype, d_mask, T, N, w, d_out, s));
+  // the domain check, the path flag and the fallback count, read once at the end
+  ScSummary h;
+  FCB_TRY(cudaMemcpyAsync(&h, w.summary, sizeof(h), cudaMemcpyDeviceToHost, s));
   FCB_TRY(cudaStreamSynchronize(s));
-  if (hs[0] > 1e150 || hs[1] < 1e-150) return FCB_ERR_CAP4;
-  if (selected_path) *selected_path = hs[2] != 0.0 ? 0 : 1;
-  FCB_TRY(cudaMemsetAsync(fbc, 0, sizeof(int), s));
-  FCB_TRY(launch_stock_corr_gram(xraw, xc, mc, st, T, N, Tp, d_out, fbl, fbc, s));
-  int hfb = 0;
-  FCB_TRY(cudaMemcpyAsync(&hfb, fbc, sizeof(int), cudaMemcpyDeviceToHost, s));
-  FCB_TRY(cudaStreamSynchronize(s));
-  if (fallback_count) *fallback_count = hfb;
+  double mx, mn;
+  const unsigned long long mn_bits = ~h.min_abs_inv;
+  std::memcpy(&mx, &h.max_abs, 8);
+  std::memcpy(&mn, &mn_bits, 8);
+  if (mx > 1e150 || mn < 1e-150) return FCB_ERR_CAP4;  // (mn is a NaN when no valid cell is nonzero)
+  if (selected_path) *selected_path = h.masked ? 1 : 0;
+  if (fallback_count) *fallback_count = h.flagged;
   return FCB_OK;
 }
 
@@ -1158,8 +1155,9 @@ uint64_t budget_dev_factor_corr(int dtype, long long R, int F) {
 uint64_t budget_dev_stock_corr(int T, int N) {
   const size_t Tp = static_cast<size_t>((T + 31) / 32 * 32);
   const size_t upper = static_cast<size_t>(N) * (N - 1) / 2;
-  return 3 * slot_bytes(static_cast<size_t>(N) * Tp * 8) + slot_bytes(static_cast<size_t>(N) * sizeof(ColStat)) + 64 +
-         slot_bytes((upper > 0 ? upper : 1) * 4) + 64;
+  return 2 * slot_bytes(static_cast<size_t>(N) * Tp * 8) + slot_bytes(sc_masks_bytes(T, N)) +
+         slot_bytes(sc_pairs_bytes(N)) + slot_bytes(static_cast<size_t>(N) * sizeof(ColStat)) + 64 +
+         slot_bytes((upper > 0 ? upper : 1) * 4);
 }
 }  // namespace
 

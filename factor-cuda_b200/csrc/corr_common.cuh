@@ -1,0 +1,70 @@
+// corr_common.cuh -- what the FP64 correlations share: compensated sums, the
+// Pearson finalize with its gates, and the FP64 matrix instruction.
+#pragma once
+
+#include "fcb_common.cuh"
+
+namespace fcb {
+
+constexpr double kBigPos = 1e300;
+constexpr double kCancelRatio = 3.0;
+constexpr double kConstVarRel = 1e-10;
+constexpr double kTiny = 1e-300;
+constexpr int kTwoPassKahanT = 2048;
+
+struct Kahan {
+  double s = 0.0, c = 0.0;
+  FCB_DEV void add(double x) {
+    const double y = x - c;
+    const double t = s + y;
+    c = (t - s) - y;
+    s = t;
+  }
+  FCB_DEV void merge(const Kahan& o) {
+    add(o.s);
+    add(-o.c);
+  }
+};
+
+FCB_DEV double dnan() { return __longlong_as_double(0x7ff8000000000000ll); }
+
+FCB_DEV double safe_pearson(double sxy, double sxx, double syy) {
+  if (!(sxx > 0.0 && syy > 0.0) || !isfinite(sxx) || !isfinite(syy) || !isfinite(sxy)) return dnan();
+  const double r = (sxy / sqrt(sxx)) / sqrt(syy);
+  return isfinite(r) ? r : dnan();
+}
+
+// Decide from the centred moment sums of one pair whether the Gram value is
+// trustworthy; returns NaN + flag when the pair must go to the fallback.
+FCB_DEV double finalize_pair(double n, double sx, double sy, double sxy, double sx2, double sy2, double mux,
+                             double muy, bool& flag) {
+  flag = false;
+  if (n < 2.0) return dnan();
+  const double rn = 1.0 / n, mx = sx * rn, my = sy * rn;  // one division for all
+  const double cov = fma(-mx, sy, sxy);
+  const double vx = fma(-mx, sx, sx2);
+  const double vy = fma(-my, sy, sy2);
+  // uncentred sums of the reference's one-pass Gram, reconstructed
+  const double sxr = sx + n * mux;
+  const double syr = sy + n * muy;
+  const double sx2r = sx2 + 2.0 * mux * sx + n * mux * mux;
+  const double sy2r = sy2 + 2.0 * muy * sy + n * muy * muy;
+  const double qxx = sxr * sxr * rn, qyy = syr * syr * rn;
+  bool fix = (fabs(sxr * syr * rn) > kCancelRatio * fabs(cov)) || (fabs(qxx) > kCancelRatio * fabs(vx)) ||
+             (fabs(qyy) > kCancelRatio * fabs(vy));
+  const double xmag = fmax(fabs(sx2r), fabs(qxx));
+  const double ymag = fmax(fabs(sy2r), fabs(qyy));
+  if (fabs(vx) <= kConstVarRel * (xmag + kTiny) || fabs(vy) <= kConstVarRel * (ymag + kTiny)) fix = true;
+  const double r = safe_pearson(cov, vx, vy);
+  if (!isfinite(r) || fabs(r) > 1.0) fix = true;
+  flag = fix;
+  return fix ? dnan() : r;
+}
+
+FCB_DEV void dmma_f64(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+}  // namespace fcb

@@ -27,417 +27,10 @@
 
 #include <algorithm>
 
-#include "fcb_common.cuh"
+#include "corr_common.cuh"
 #include "fcb_kernels.h"
 
 namespace fcb {
-
-constexpr double kBigPos = 1e300;
-constexpr double kCancelRatio = 3.0;
-constexpr double kConstVarRel = 1e-10;
-constexpr double kTiny = 1e-300;
-constexpr int kTwoPassKahanT = 2048;
-
-struct Kahan {
-  double s = 0.0, c = 0.0;
-  FCB_DEV void add(double x) {
-    const double y = x - c;
-    const double t = s + y;
-    c = (t - s) - y;
-    s = t;
-  }
-  FCB_DEV void merge(const Kahan& o) {
-    add(o.s);
-    add(-o.c);
-  }
-};
-
-FCB_DEV double dnan() { return __longlong_as_double(0x7ff8000000000000ll); }
-
-FCB_DEV double safe_pearson(double sxy, double sxx, double syy) {
-  if (!(sxx > 0.0 && syy > 0.0) || !isfinite(sxx) || !isfinite(syy) || !isfinite(sxy)) return dnan();
-  const double r = (sxy / sqrt(sxx)) / sqrt(syy);
-  return isfinite(r) ? r : dnan();
-}
-
-// Decide from the centred moment sums of one pair whether the Gram value is
-// trustworthy; returns NaN + flag when the pair must go to the fallback.
-FCB_DEV double finalize_pair(double n, double sx, double sy, double sxy, double sx2, double sy2, double mux,
-                             double muy, bool& flag) {
-  flag = false;
-  if (n < 2.0) return dnan();
-  const double cov = sxy - sx * sy / n;
-  const double vx = sx2 - sx * sx / n;
-  const double vy = sy2 - sy * sy / n;
-  // uncentred sums of the reference's one-pass Gram, reconstructed
-  const double sxr = sx + n * mux;
-  const double syr = sy + n * muy;
-  const double sx2r = sx2 + 2.0 * mux * sx + n * mux * mux;
-  const double sy2r = sy2 + 2.0 * muy * sy + n * muy * muy;
-  bool fix = (fabs(sxr * syr / n) > kCancelRatio * fabs(cov)) ||
-             (fabs(sxr * sxr / n) > kCancelRatio * fabs(vx)) ||
-             (fabs(syr * syr / n) > kCancelRatio * fabs(vy));
-  const double xmag = fmax(fabs(sx2r), fabs(sxr * sxr / n));
-  const double ymag = fmax(fabs(sy2r), fabs(syr * syr / n));
-  if (fabs(vx) <= kConstVarRel * (xmag + kTiny) || fabs(vy) <= kConstVarRel * (ymag + kTiny)) fix = true;
-  const double r = safe_pearson(cov, vx, vy);
-  if (!isfinite(r) || fabs(r) > 1.0) fix = true;
-  flag = fix;
-  return fix ? dnan() : r;
-}
-
-// ---------------------------------------------------------------------------
-// stock_corr
-// ---------------------------------------------------------------------------
-
-// (T,N) row-major -> column-major Xraw/Xc/Mc (N, Tp), zero padded, tiled.
-template <typename TIN>
-__global__ void k_sc_transpose(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, int T, int N, int Tp,
-                               double* __restrict__ Xraw, double* __restrict__ Mc) {
-  __shared__ double tx[32][33];
-  __shared__ double tm[32][33];
-  const int t0 = blockIdx.x * 32, i0 = blockIdx.y * 32;
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int t = t0 + r, i = i0 + threadIdx.x;
-    double v = 0.0, m = 0.0;
-    if (t < T && i < N) {
-      const size_t e = static_cast<size_t>(t) * N + i;
-      const double x = static_cast<double>(X[e]);
-      const bool ok = finite_f64(x) && (mask == nullptr || mask[e] != 0);
-      v = ok ? x : 0.0;
-      m = ok ? 1.0 : 0.0;
-    }
-    tx[r][threadIdx.x] = v;
-    tm[r][threadIdx.x] = m;
-  }
-  __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int i = i0 + r, t = t0 + threadIdx.x;
-    if (i < N && t < Tp) {
-      Xraw[static_cast<size_t>(i) * Tp + t] = tx[threadIdx.x][r];
-      Mc[static_cast<size_t>(i) * Tp + t] = tm[threadIdx.x][r];
-    }
-  }
-}
-
-// One warp per column: serial Kahan mean in row order, extrema, centred
-// copy Xc = valid ? x - mu : 0, centred sum of squares for the diagonal.
-__global__ void k_sc_colstats(const double* __restrict__ Xraw, const double* __restrict__ Mc, int T, int N, int Tp,
-                              double* __restrict__ Xc, ColStat* __restrict__ st) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= N) return;
-  const double* x = Xraw + static_cast<size_t>(w) * Tp;
-  const double* m = Mc + static_cast<size_t>(w) * Tp;
-  Kahan k;
-  double cnt = 0.0, mn = kBigPos, mx = -kBigPos, mna = kBigPos, mxa = 0.0;
-  for (int t0 = 0; t0 < T; t0 += 32) {
-    const int t = t0 + lane;
-    const double xv = (t < T) ? x[t] : 0.0;
-    const bool ok = (t < T) && m[t] != 0.0;
-    const unsigned vb = __ballot_sync(kFull, ok);
-    // serial Kahan in row order: lane 0 consumes the 32 values in order
-    for (int l = 0; l < 32; ++l) {
-      const double v = __shfl_sync(kFull, xv, l);
-      if ((vb >> l) & 1u) k.add(v);
-    }
-    if (ok) {
-      cnt += 1.0;
-      mn = fmin(mn, xv);
-      mx = fmax(mx, xv);
-      const double ax = fabs(xv);
-      mxa = fmax(mxa, ax);
-      if (ax != 0.0) mna = fmin(mna, ax);
-    }
-  }
-  cnt = warp_sum(cnt);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mn = fmin(mn, __shfl_xor_sync(kFull, mn, o));
-    mx = fmax(mx, __shfl_xor_sync(kFull, mx, o));
-    mna = fmin(mna, __shfl_xor_sync(kFull, mna, o));
-    mxa = fmax(mxa, __shfl_xor_sync(kFull, mxa, o));
-  }
-  const double mu = cnt > 0.0 ? k.s / cnt : 0.0;
-  double s2 = 0.0, s1 = 0.0;
-  for (int t = lane; t < Tp; t += 32) {
-    const bool ok = (t < T) && m[t] != 0.0;
-    const double d = ok ? x[t] - mu : 0.0;
-    Xc[static_cast<size_t>(w) * Tp + t] = d;
-    s2 += d * d;
-    s1 += d;
-  }
-  s2 = warp_sum(s2);
-  s1 = warp_sum(s1);
-  if (lane == 0) {
-    ColStat c;
-    c.count = cnt;
-    c.mean = mu;
-    c.min = mn;
-    c.max = mx;
-    c.min_abs = mna;
-    c.max_abs = mxa;
-    c.s2 = s2;
-    c.s1 = s1;
-    st[w] = c;
-  }
-}
-
-// Domain check + full-validity over the column stats (single block).
-__global__ void k_sc_summary(const ColStat* __restrict__ st, int N, int T, double* __restrict__ out3) {
-  double mxa = 0.0, mna = kBigPos;
-  int full = 1;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    mxa = fmax(mxa, st[i].max_abs);
-    mna = fmin(mna, st[i].min_abs);
-    if (st[i].count < static_cast<double>(T)) full = 0;
-  }
-  __shared__ double smx[32], smn[32];
-  __shared__ int sf[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mxa = fmax(mxa, __shfl_xor_sync(kFull, mxa, o));
-    mna = fmin(mna, __shfl_xor_sync(kFull, mna, o));
-    full = min(full, __shfl_xor_sync(kFull, full, o));
-  }
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    smx[w] = mxa;
-    smn[w] = mna;
-    sf[w] = full;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < (blockDim.x + 31) / 32; ++i) {
-      mxa = fmax(mxa, smx[i]);
-      mna = fmin(mna, smn[i]);
-      full = min(full, sf[i]);
-    }
-    out3[0] = mxa;
-    out3[1] = mna;
-    out3[2] = full;
-  }
-}
-
-// Upper-triangle 32x32 tiles; 256 threads, 2x2 cells per thread; six
-// accumulators per cell; 32-wide k tiles staged in shared memory.
-constexpr int kScTile = 32, kScK = 32;
-
-FCB_DEV void tri_tile(int b, int nt, int& ib, int& jb) {
-  int lo = 0, hi = nt - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) / 2;
-    const long long pm = static_cast<long long>(mid) * nt - static_cast<long long>(mid) * (mid - 1) / 2;
-    if (pm <= b) lo = mid; else hi = mid - 1;
-  }
-  ib = lo;
-  const long long p = static_cast<long long>(ib) * nt - static_cast<long long>(ib) * (ib - 1) / 2;
-  jb = ib + static_cast<int>(b - p);
-}
-
-__global__ void __launch_bounds__(256, 2)
-    k_sc_gram(const double* __restrict__ Xc, const double* __restrict__ Mc, const ColStat* __restrict__ st, int N,
-              int Tp, int nt, double* __restrict__ out, int* __restrict__ fb_list, int* __restrict__ fb_count,
-              int full) {
-  __shared__ double Ax[kScTile][kScK + 1], Am[kScTile][kScK + 1], Bx[kScTile][kScK + 1], Bm[kScTile][kScK + 1];
-  int ib, jb;
-  tri_tile(blockIdx.x, nt, ib, jb);
-  const int i0 = ib * kScTile, j0 = jb * kScTile;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  double acc[4][6], part[4][6];
-#pragma unroll
-  for (int c = 0; c < 4; ++c)
-#pragma unroll
-    for (int q = 0; q < 6; ++q) acc[c][q] = 0.0;
-  for (int k0 = 0; k0 < Tp; k0 += kScK) {
-    for (int e = threadIdx.x; e < kScTile * kScK; e += 256) {
-      const int r = e / kScK, kk = e % kScK;
-      const int gi = i0 + r, gj = j0 + r;
-      Ax[r][kk] = gi < N ? Xc[static_cast<size_t>(gi) * Tp + k0 + kk] : 0.0;
-      Am[r][kk] = gi < N ? Mc[static_cast<size_t>(gi) * Tp + k0 + kk] : 0.0;
-      Bx[r][kk] = gj < N ? Xc[static_cast<size_t>(gj) * Tp + k0 + kk] : 0.0;
-      Bm[r][kk] = gj < N ? Mc[static_cast<size_t>(gj) * Tp + k0 + kk] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-      for (int q = 0; q < 6; ++q) part[c][q] = 0.0;
-#pragma unroll 4
-    for (int kk = 0; kk < kScK; ++kk) {
-      const double ax0 = Ax[ty * 2][kk], ax1 = Ax[ty * 2 + 1][kk];
-      const double am0 = Am[ty * 2][kk], am1 = Am[ty * 2 + 1][kk];
-      const double bx0 = Bx[tx * 2][kk], bx1 = Bx[tx * 2 + 1][kk];
-      const double bm0 = Bm[tx * 2][kk], bm1 = Bm[tx * 2 + 1][kk];
-      const double axs[2] = {ax0, ax1}, ams[2] = {am0, am1}, bxs[2] = {bx0, bx1}, bms[2] = {bm0, bm1};
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const int c = a * 2 + b;
-          const double jx = axs[a] * bms[b];
-          const double jy = ams[a] * bxs[b];
-          part[c][0] = fma(ams[a], bms[b], part[c][0]);
-          part[c][1] += jx;
-          part[c][2] += jy;
-          part[c][3] = fma(axs[a], bxs[b], part[c][3]);
-          part[c][4] = fma(axs[a], jx, part[c][4]);
-          part[c][5] = fma(bxs[b], jy, part[c][5]);
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-      for (int q = 0; q < 6; ++q) acc[c][q] += part[c][q];
-    __syncthreads();
-  }
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const int i = i0 + ty * 2 + a, j = j0 + tx * 2 + b;
-      if (i >= N || j >= N || i > j) continue;
-      const double* q = acc[a * 2 + b];
-      double r;
-      bool flag = false;
-      if (i == j) {
-        // diagonal: 1.0 iff the column's centred sum of squares is usable
-        const ColStat& s = st[i];
-        r = (s.count >= 2.0 && s.min != s.max && s.s2 > 0.0 && isfinite(s.s2)) ? 1.0 : dnan();
-      } else {
-        r = finalize_pair(q[0], q[1], q[2], q[3], q[4], q[5], st[i].mean, st[j].mean, flag);
-        if (!flag && q[0] >= 2.0) {
-          // an exact-constant column on the joint set has zero centred
-          // variance; the gate above catches it, min==max settles it
-        }
-      }
-      out[static_cast<size_t>(i) * N + j] = r;
-      out[static_cast<size_t>(j) * N + i] = r;
-      if (flag) {
-        const int slot = atomicAdd(fb_count, 1);
-        fb_list[slot] = i * N + j;  // N*N <= INT32_MAX
-      }
-    }
-  (void)full;
-}
-
-// Two-pass Pearson of one pair over its joint valid dates, serial in date
-// order (the Kahan-mean two-pass reference's exact sequence of operations).
-// One thread per pair: the dates are read kU at a time, all loads issued
-// before they are used, so each step does not wait on its own loads; the
-// values are then consumed in date order.
-template <int kU>
-FCB_DEV double two_pass_serial(const double* __restrict__ xi, const double* __restrict__ mi,
-                               const double* __restrict__ xj, const double* __restrict__ mj, int T) {
-  double n = 0.0, mnx = kBigPos, mxx = -kBigPos, mny = kBigPos, mxy = -kBigPos;
-  Kahan kx, ky;
-  for (int t0 = 0; t0 < T; t0 += kU) {
-    double a[kU], b[kU], x[kU], y[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int t = t0 + u;
-      const bool in = t < T;
-      a[u] = in ? mi[t] : 0.0;
-      b[u] = in ? mj[t] : 0.0;
-      x[u] = in ? xi[t] : 0.0;
-      y[u] = in ? xj[t] : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      if (a[u] != 0.0 && b[u] != 0.0) {
-        n += 1.0;
-        kx.add(x[u]);
-        ky.add(y[u]);
-        mnx = fmin(mnx, x[u]);
-        mxx = fmax(mxx, x[u]);
-        mny = fmin(mny, y[u]);
-        mxy = fmax(mxy, y[u]);
-      }
-    }
-  }
-  if (n < 2.0) return dnan();
-  if (mnx == mxx || mny == mxy) return dnan();
-  const double mx = kx.s / n, my = ky.s / n;
-  const bool kahan = T > kTwoPassKahanT;
-  Kahan ka, kb, kc;
-  double sxx = 0.0, syy = 0.0, sxy = 0.0;
-  for (int t0 = 0; t0 < T; t0 += kU) {
-    double a[kU], b[kU], x[kU], y[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int t = t0 + u;
-      const bool in = t < T;
-      a[u] = in ? mi[t] : 0.0;
-      b[u] = in ? mj[t] : 0.0;
-      x[u] = in ? xi[t] : 0.0;
-      y[u] = in ? xj[t] : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      if (a[u] != 0.0 && b[u] != 0.0) {
-        const double dx = x[u] - mx, dy = y[u] - my;
-        if (kahan) {
-          ka.add(dx * dx);
-          kb.add(dy * dy);
-          kc.add(dx * dy);
-        } else {
-          sxx += dx * dx;
-          syy += dy * dy;
-          sxy += dx * dy;
-        }
-      }
-    }
-  }
-  if (kahan) {
-    sxx = ka.s - ka.c;
-    syy = kb.s - kb.c;
-    sxy = kc.s - kc.c;
-  }
-  return safe_pearson(sxy, sxx, syy);
-}
-
-__global__ void k_sc_fallback(const double* __restrict__ Xraw, const double* __restrict__ Mc, int T, int N, int Tp,
-                              const int* __restrict__ fb_list, const int* __restrict__ fb_count,
-                              double* __restrict__ out) {
-  const int cnt = *fb_count;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
-    const int cell = fb_list[k];
-    const int i = cell / N, j = cell % N;
-    const double r = two_pass_serial<8>(Xraw + static_cast<size_t>(i) * Tp, Mc + static_cast<size_t>(i) * Tp,
-                                        Xraw + static_cast<size_t>(j) * Tp, Mc + static_cast<size_t>(j) * Tp, T);
-    out[static_cast<size_t>(i) * N + j] = r;
-    out[static_cast<size_t>(j) * N + i] = r;
-  }
-}
-
-cudaError_t launch_stock_corr_prep(const void* X, int dtype, const uint8_t* mask, int T, int N, int Tp,
-                                   double* Xraw, double* Xc, double* Mc, ColStat* st, double* summary,
-                                   cudaStream_t s) {
-  dim3 grid((Tp + 31) / 32, (N + 31) / 32), block(32, 8);
-  if (dtype == 0)
-    k_sc_transpose<float><<<grid, block, 0, s>>>(static_cast<const float*>(X), mask, T, N, Tp, Xraw, Mc);
-  else
-    k_sc_transpose<double><<<grid, block, 0, s>>>(static_cast<const double*>(X), mask, T, N, Tp, Xraw, Mc);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_sc_colstats<<<(N * 32 + 255) / 256, 256, 0, s>>>(Xraw, Mc, T, N, Tp, Xc, st);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_sc_summary<<<1, 1024, 0, s>>>(st, N, T, summary);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_stock_corr_gram(const double* Xraw, const double* Xc, const double* Mc, const ColStat* st, int T,
-                                   int N, int Tp, double* out, int* fb_list, int* fb_count, cudaStream_t s) {
-  const int nt = (N + kScTile - 1) / kScTile;
-  const long long tiles = static_cast<long long>(nt) * (nt + 1) / 2;
-  k_sc_gram<<<static_cast<unsigned>(tiles), 256, 0, s>>>(Xc, Mc, st, N, Tp, nt, out, fb_list, fb_count, 0);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  // grid-stride over the device-side fallback count (no host round trip)
-  k_sc_fallback<<<148 * 4, 128, 0, s>>>(Xraw, Mc, T, N, Tp, fb_list, fb_count, out);
-  return cudaGetLastError();
-}
 
 // Correlation domain extremes over the valid cells of a factor_corr panel.
 // Non-negative doubles order like their bit patterns, so the block results
@@ -716,12 +309,6 @@ __host__ __device__ inline size_t fc_mma_raw_offset(int Fp, int units_per_block)
   const size_t red = static_cast<size_t>(units_per_block) * kFcMmaGroup * 4 * 64;
   return ((stage > red ? stage : red) + 1) / 2 * 2;  // 16-byte aligned
 }
-FCB_DEV void dmma_f64(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
 // Asynchronous global -> shared copies of single elements (cp.async, L1
 // allocating); each thread waits for its own groups, a barrier publishes them.
 template <int BYTES>

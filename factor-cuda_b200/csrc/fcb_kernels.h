@@ -53,6 +53,27 @@ struct RankIcArgs {
 struct ColStat {  // one stock_corr column
   double count, mean, min, max, min_abs, max_abs, s2, s1;
 };
+// stock_corr: what the device knows of the whole panel (zeroed first).
+struct ScSummary {
+  unsigned long long max_abs;      // bits of the largest |x| over the valid cells
+  unsigned long long min_abs_inv;  // inverted bits of the smallest nonzero |x| (0: none)
+  int masked;                      // some cell is invalid
+  int flagged;                     // pairs sent to the two-pass fallback
+};
+struct ScWork {
+  double *xraw, *xc;  // (N,Tp) column-major values, as they are and centred; Tp = T rounded to 32
+  void* masks;        // sc_masks_bytes: validity bits, date lists
+  double2* ab;        // sc_pairs_bytes: pair sums
+  ColStat* st;        // [N]
+  ScSummary* summary;
+  int* fb_list;       // [N (N-1) / 2]
+};
+size_t sc_masks_bytes(int T, int N);
+size_t sc_pairs_bytes(int N);
+// (N,N) correlations of a (T,N) panel into out (untouched when the panel is
+// out of the domain, see the summary).
+cudaError_t launch_stock_corr(const void* X, int dtype, const uint8_t* mask, int T, int N, const ScWork& w, double* out,
+                              cudaStream_t s);
 struct FcColPart {
   double count, s, c, min, max;
 };
@@ -158,16 +179,11 @@ cudaError_t launch_corr_fp32(const PrecOperands& op, const int2* tiles, int ntil
                              cudaStream_t s);
 
 // corr_kernels.cu
-cudaError_t launch_stock_corr_prep(const void* X, int dtype, const uint8_t* mask, int T, int N, int Tp,
-                                   double* Xraw, double* Xc, double* Mc, ColStat* st, double* summary,
-                                   cudaStream_t s);
 // max |x| and min nonzero |x| over the valid cells (finite, mask true) of a
 // factor_corr panel, as IEEE bit patterns in ext[0] / ext[1] (0 and +inf when
 // no cell is valid).  planes = 0: (R,F) rows; planes = 1: F planes of R rows.
 cudaError_t launch_corr_domain(const void* X, int dtype, const uint8_t* mask, long long R, int F, int planes,
                                unsigned long long* ext, cudaStream_t s);
-cudaError_t launch_stock_corr_gram(const double* Xraw, const double* Xc, const double* Mc, const ColStat* st, int T,
-                                   int N, int Tp, double* out, int* fb_list, int* fb_count, cudaStream_t s);
 size_t fc_gram_smem(int Fp, int tasks_per_block, int elem_bytes);
 // Work split of the Gram pass for Fp (factors rounded to 4): tiles or tile
 // units in all, per block (blockIdx.y), and the blocks along y.

@@ -1,0 +1,641 @@
+// stock_corr.cu -- FP64 pairwise-complete Pearson of every pair of columns of
+// a (T,N) panel (the drop-in path), for sm_100a.
+//
+// A pair's six moment sums run over the dates on which both columns are
+// valid.  Only one of them, sum x'y' of column-centred values (0 where
+// invalid), is a matrix product; it runs on the FP64 tensor cores
+// (k_sc_gram).  The other five are cheaper than products:
+//   * n is a population count of the AND of two validity bitmasks;
+//   * sum x' and sum x'^2 over the other column's valid dates are the column's
+//     totals less the dates that the other column misses.  A column misses few
+//     dates as a rule, so k_sc_pairsum adds up short lists: one CTA keeps the
+//     centred values of 16 columns in shared memory ([date][16]) and walks
+//     every column's list of missing dates (of valid dates where more than a
+//     quarter is missing).  Where what is taken away is more than three
+//     quarters of the column's sum of squares, the pair's sums are formed over
+//     the joint dates directly, so that the subtraction costs at most two bits.
+// Steps: column statistics (compensated mean, extrema; replaces
+// stock_corr_gpu's col_stats_kernel, src/stock_corr.cu:73-116, and the
+// demean_kernel's mean, :244-261), column-major copies and bitmasks, lists,
+// pair sums, Gram pass with the finalize and its gates
+// (src/stock_corr_impl.cuh:102-132), and the two-pass fallback of the flagged
+// pairs (two_pass_centered, src/stock_corr_impl.cuh:150-201; _two_pass_corr,
+// fc/_cpu_core.py:111-137).
+// The domain check and the full-validity flag stay on the device: the later
+// kernels return at once when the panel is out of the domain, and the host
+// reads the summary once, at the end.
+#include <algorithm>
+
+#include "corr_common.cuh"
+#include "fcb_kernels.h"
+
+namespace fcb {
+namespace {
+
+constexpr int kScRows = 16;      // columns of one k_sc_pairsum CTA
+constexpr int kScChunk = 1664;   // dates it holds at a time (208 KB)
+constexpr int kScTile = 64;      // k_sc_gram tile
+constexpr int kScK = 32;         // dates per stage
+constexpr int kScPitch = kScK + 4;  // doubles per staged row: fragment loads of 4 rows x 4 dates are conflict-free
+constexpr int kScBlock = 5120;   // columns whose pair sums are held at a time
+
+FCB_DEV bool out_of_domain(const ScSummary* s) {
+  const double mx = __longlong_as_double(static_cast<long long>(s->max_abs));
+  const double mn = __longlong_as_double(static_cast<long long>(~s->min_abs_inv));
+  return mx > 1e150 || mn < 1e-150;  // (no valid nonzero cell: mn is a NaN)
+}
+
+FCB_DEV bool sc_valid(double v, const uint8_t* mask, size_t e) {
+  return finite_f64(v) && (mask == nullptr || mask[e] != 0);
+}
+
+// ---------------------------------------------------------------------------
+// column statistics
+// ---------------------------------------------------------------------------
+// 32 columns per CTA, lane = column (coalesced rows); warp w takes every 32nd
+// date with its own compensated sum, and the 32 partials merge in order.  (One
+// serial compensated sum per column costs four dependent FP64 adds, about 120
+// clocks, per date: 80 us for 1218 dates.)  The mean is the shift of the
+// centred values; the fallback forms its own means.
+constexpr int kStWarps = 32;
+template <typename TIN>
+__global__ void __launch_bounds__(32 * kStWarps) k_sc_colstats(const TIN* __restrict__ X, const uint8_t* __restrict__ mask,
+                                                               int T, int N, ColStat* __restrict__ st,
+                                                               ScSummary* __restrict__ sum) {
+  __shared__ double ps[kStWarps][32], pc[kStWarps][32], pmn[kStWarps][32], pmx[kStWarps][32], pna[kStWarps][32];
+  __shared__ int pn[kStWarps][32];
+  const int lane = static_cast<int>(threadIdx.x & 31), w = static_cast<int>(threadIdx.x >> 5);
+  const int i = blockIdx.x * 32 + lane;
+  Kahan k;
+  int cnt = 0;
+  double mn = kBigPos, mx = -kBigPos, mna = kBigPos;
+  if (i < N) {
+#pragma unroll 4
+    for (int t = w; t < T; t += kStWarps) {
+      const size_t e = static_cast<size_t>(t) * N + i;
+      const double v = static_cast<double>(X[e]);
+      if (sc_valid(v, mask, e)) {
+        k.add(v);
+        ++cnt;
+        mn = fmin(mn, v);
+        mx = fmax(mx, v);
+        if (v != 0.0) mna = fmin(mna, fabs(v));
+      }
+    }
+  }
+  ps[w][lane] = k.s;
+  pc[w][lane] = k.c;
+  pn[w][lane] = cnt;
+  pmn[w][lane] = mn;
+  pmx[w][lane] = mx;
+  pna[w][lane] = mna;
+  __syncthreads();
+  if (w != 0) return;
+  for (int q = 1; q < kStWarps; ++q) {
+    k.add(ps[q][lane]);
+    k.add(-pc[q][lane]);
+    cnt += pn[q][lane];
+    mn = fmin(mn, pmn[q][lane]);
+    mx = fmax(mx, pmx[q][lane]);
+    mna = fmin(mna, pna[q][lane]);
+  }
+  const double mxa = cnt > 0 ? fmax(fabs(mn), fabs(mx)) : 0.0;
+  if (i < N) {
+    ColStat c;
+    c.count = static_cast<double>(cnt);
+    c.mean = cnt > 0 ? k.s / static_cast<double>(cnt) : 0.0;
+    c.min = mn;
+    c.max = mx;
+    c.min_abs = mna;
+    c.max_abs = mxa;
+    c.s2 = 0.0;
+    c.s1 = 0.0;
+    st[i] = c;
+  }
+  // non-negative doubles order like their bit patterns
+  unsigned long long a = static_cast<unsigned long long>(__double_as_longlong(mxa));
+  unsigned long long z = mna < kBigPos ? ~static_cast<unsigned long long>(__double_as_longlong(mna)) : 0ull;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long a2 = __shfl_xor_sync(kFull, a, o), z2 = __shfl_xor_sync(kFull, z, o);
+    a = a2 > a ? a2 : a;
+    z = z2 > z ? z2 : z;
+  }
+  const bool part = __any_sync(kFull, i < N && cnt < T);
+  if (lane == 0) {
+    atomicMax(&sum->max_abs, a);
+    atomicMax(&sum->min_abs_inv, z);
+    if (part) atomicExch(&sum->masked, 1);
+  }
+}
+
+// (T,N) row-major -> column-major Xraw, Xc (N,Tp) (0 where invalid or past T)
+// and validity bits (N, Tp/32).
+template <typename TIN>
+__global__ void k_sc_transpose(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, int T, int N, int Tp,
+                               const ColStat* __restrict__ st, double* __restrict__ Xraw, double* __restrict__ Xc,
+                               uint32_t* __restrict__ bits) {
+  __shared__ double tx[32][33];
+  __shared__ uint8_t tm[32][33];
+  const int t0 = blockIdx.x * 32, i0 = blockIdx.y * 32;
+  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+    const int t = t0 + r, i = i0 + threadIdx.x;
+    double v = 0.0;
+    bool ok = false;
+    if (t < T && i < N) {
+      const size_t e = static_cast<size_t>(t) * N + i;
+      v = static_cast<double>(X[e]);
+      ok = sc_valid(v, mask, e);
+    }
+    tx[r][threadIdx.x] = ok ? v : 0.0;
+    tm[r][threadIdx.x] = ok ? 1 : 0;
+  }
+  __syncthreads();
+  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+    const int i = i0 + r;
+    if (i >= N) continue;  // uniform across the warp
+    const double v = tx[threadIdx.x][r];
+    const bool ok = tm[threadIdx.x][r] != 0;
+    const size_t e = static_cast<size_t>(i) * Tp + t0 + threadIdx.x;
+    Xraw[e] = v;
+    Xc[e] = ok ? v - st[i].mean : 0.0;
+    const unsigned b = __ballot_sync(kFull, ok);
+    if (threadIdx.x == 0) bits[static_cast<size_t>(i) * (Tp / 32) + blockIdx.x] = b;
+  }
+}
+
+// One warp per column: sums of the centred values and their squares, and the
+// column's date list -- missing dates when they are at most a quarter (invert
+// = 1), valid dates otherwise.  Entries are dates within their chunk, each
+// chunk's run padded to eight with the chunk's number of dates (a row of
+// zeros); ptr[c] is where chunk c starts.
+__global__ void k_sc_lists(const double* __restrict__ Xc, const uint32_t* __restrict__ bits, int T, int N, int Tp,
+                           int nchunk, int lcap, ColStat* __restrict__ st, uint16_t* __restrict__ list,
+                           int* __restrict__ ptr, int* __restrict__ invert) {
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (w >= N) return;
+  double s2 = 0.0, s1 = 0.0;
+  for (int t = lane; t < Tp; t += 32) {
+    const double d = Xc[static_cast<size_t>(w) * Tp + t];
+    s2 += d * d;
+    s1 += d;
+  }
+  s2 = warp_sum(s2);
+  s1 = warp_sum(s1);
+  const int missing = T - static_cast<int>(st[w].count);
+  const bool inv = 4ll * missing <= T;
+  if (lane == 0) {
+    st[w].s2 = s2;
+    st[w].s1 = s1;
+    invert[w] = inv ? 1 : 0;
+  }
+  uint16_t* out = list + static_cast<size_t>(w) * lcap;
+  int* p = ptr + static_cast<size_t>(w) * (nchunk + 1);
+  const uint32_t* b = bits + static_cast<size_t>(w) * (Tp / 32);
+  int pos = 0;
+  for (int c = 0; c < nchunk; ++c) {
+    if (lane == 0) p[c] = pos;
+    const int t1 = min(T, (c + 1) * kScChunk);
+    for (int t0 = c * kScChunk; t0 < t1; t0 += 32) {
+      uint32_t m = b[t0 / 32];
+      if (inv) m = ~m;
+      if (t1 - t0 < 32) m &= (1u << (t1 - t0)) - 1u;
+      if ((m >> lane) & 1u) out[pos + __popc(m & lanemask_lt())] = static_cast<uint16_t>(t0 - c * kScChunk + lane);
+      pos += __popc(m);
+    }
+    const int pad = (8 - (pos & 7)) & 7;
+    if (lane < pad) out[pos + lane] = static_cast<uint16_t>(t1 - c * kScChunk);
+    pos += pad;
+  }
+  if (lane == 0) p[nchunk] = pos;
+}
+
+// ---------------------------------------------------------------------------
+// pair sums: AB[(j - ja) * ld + (i - ia)] = (sum x'_i, sum x'_i^2) over the
+// valid dates of column j
+// ---------------------------------------------------------------------------
+// A half-warp takes one column j at a time: lane = column i.  A list entry
+// costs one 128-byte shared-memory row and two FP64 instructions per lane.
+// Chunk c of the dates; the sums of earlier chunks wait in AB.
+template <typename TIN>
+__global__ void __launch_bounds__(1024, 1)
+    k_sc_pairsum(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, const double* __restrict__ Xc,
+                 const uint32_t* __restrict__ bits, const ColStat* __restrict__ st, const uint16_t* __restrict__ list,
+                 const int* __restrict__ ptr, const int* __restrict__ invert, int T, int N, int Tp, int nchunk,
+                 int lcap, int c, int ia, int ib, int ja, int jb, int ld, double2* __restrict__ AB,
+                 const ScSummary* __restrict__ sum) {
+  if (sum->masked == 0 || out_of_domain(sum)) return;  // a full panel needs no pair sums
+  extern __shared__ __align__(16) double xs[];         // [tn + 1][kScRows], the last row zero
+  const int t0 = c * kScChunk, tn = min(T - t0, kScChunk);
+  const int i0 = ia + static_cast<int>(blockIdx.x) * kScRows;
+  for (int e = threadIdx.x; e < tn * kScRows; e += blockDim.x) {
+    const int i = i0 + (e % kScRows);
+    double v = 0.0;
+    if (i < ib) {
+      const size_t at = static_cast<size_t>(t0 + e / kScRows) * N + i;
+      const double x = static_cast<double>(X[at]);
+      if (sc_valid(x, mask, at)) v = x - st[i].mean;
+    }
+    xs[e] = v;
+  }
+  // the padding entries' row
+  if (threadIdx.x < kScRows) xs[tn * kScRows + threadIdx.x] = 0.0;
+  __syncthreads();
+  const int lane = threadIdx.x & 15, i = i0 + lane;
+  const int hw = static_cast<int>(threadIdx.x >> 4), nhw = static_cast<int>(blockDim.x >> 4);
+  const double* col = xs + lane;
+  const double s1 = i < ib ? st[i].s1 : 0.0, s2 = i < ib ? st[i].s2 : 0.0;
+  for (int j = ja + static_cast<int>(blockIdx.y) * nhw + hw; j < jb; j += nhw * static_cast<int>(gridDim.y)) {
+    const int* p = ptr + static_cast<size_t>(j) * (nchunk + 1) + c;
+    const uint4* l = reinterpret_cast<const uint4*>(list + static_cast<size_t>(j) * lcap);
+    double a0 = 0.0, a1 = 0.0, q0 = 0.0, q1 = 0.0;
+    const int k0 = p[0] >> 3, k1 = p[1] >> 3;
+    uint4 next = k0 < k1 ? __ldg(l + k0) : make_uint4(0u, 0u, 0u, 0u);
+    for (int k = k0; k < k1; ++k) {
+      const uint4 v = next;
+      if (k + 1 < k1) next = __ldg(l + k + 1);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const double x = col[(w[u] & 0xFFFFu) * kScRows];
+        const double y = col[(w[u] >> 16) * kScRows];
+        a0 += x;
+        q0 = fma(x, x, q0);
+        a1 += y;
+        q1 = fma(y, y, q1);
+      }
+    }
+    if (i >= ib) continue;
+    double a = a0 + a1, q = q0 + q1;
+    double2* o = AB + static_cast<size_t>(j - ja) * ld + (i - ia);
+    if (c > 0) {
+      const double2 e = *o;
+      a += e.x;
+      q += e.y;
+    }
+    if (c == nchunk - 1 && invert[j] != 0) {
+      if (q > 0.75 * s2) {
+        // little is left of the column: form the sums over the joint dates
+        a = q = 0.0;
+        for (int t = 0; t < T; ++t)
+          if ((bits[static_cast<size_t>(j) * (Tp / 32) + (t >> 5)] >> (t & 31)) & 1u) {
+            const double x = Xc[static_cast<size_t>(i) * Tp + t];
+            a += x;
+            q = fma(x, x, q);
+          }
+      } else {
+        a = s1 - a;
+        q = s2 - q;
+      }
+    }
+    *o = make_double2(a, q);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Gram pass
+// ---------------------------------------------------------------------------
+FCB_DEV void tri_tile(int b, int nt, int& ib, int& jb) {
+  int lo = 0, hi = nt - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    const long long pm = static_cast<long long>(mid) * nt - static_cast<long long>(mid) * (mid - 1) / 2;
+    if (pm <= b) lo = mid; else hi = mid - 1;
+  }
+  ib = lo;
+  const long long p = static_cast<long long>(ib) * nt - static_cast<long long>(ib) * (ib - 1) / 2;
+  jb = ib + static_cast<int>(b - p);
+}
+
+FCB_DEV void cp_async16(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+
+// One stage: 32 dates of the tile's two sets of 64 columns, and their bits.
+struct ScStage {
+  double a[kScTile][kScPitch], b[kScTile][kScPitch];
+  uint32_t wa[kScTile], wb[kScTile];
+};
+// The tile's products and counts, for the finalize.
+struct ScProducts {
+  double xy[kScTile][kScTile + 1];
+  uint32_t n[kScTile][kScTile + 1];
+};
+
+// 64 x 64 tiles of columns [ia, ib) x [ja, jb) (the same range: the upper
+// triangle of tiles); four warps of 32 x 32, 4 x 4 FP64 matrix instructions
+// per four dates and warp against eight fragment loads.  The FP64 tensor
+// pipe bounds it: one product instead of the six masked sums per pair and
+// date (eight FP64 instructions) that it formed before.
+__global__ void __launch_bounds__(128, 3)
+    k_sc_gram(const double* __restrict__ Xc, const uint32_t* __restrict__ bits, const ColStat* __restrict__ st, int T,
+              int N, int Tp, int ia, int ib, int ja, int jb, const double2* __restrict__ ABij,
+              const double2* __restrict__ ABji, double* __restrict__ out, int* __restrict__ fb_list,
+              ScSummary* __restrict__ sum) {
+  if (out_of_domain(sum)) return;
+  extern __shared__ __align__(16) uint8_t smem[];
+  ScStage* stage = reinterpret_cast<ScStage*>(smem);
+  const bool full = sum->masked == 0;
+  int bi, bj;
+  if (ia == ja) {
+    tri_tile(blockIdx.x, (ib - ia + kScTile - 1) / kScTile, bi, bj);
+  } else {
+    const int nj = (jb - ja + kScTile - 1) / kScTile;
+    bi = static_cast<int>(blockIdx.x) / nj;
+    bj = static_cast<int>(blockIdx.x) % nj;
+  }
+  const int i0 = ia + bi * kScTile, j0 = ja + bj * kScTile;
+  const int tid = static_cast<int>(threadIdx.x), lane = tid & 31, wr = (tid >> 6) * 32, wc = ((tid >> 5) & 1) * 32;
+  const int W = Tp / 32, r = lane >> 2, kq = lane & 3;
+  auto load = [&](int s, int kc) {
+    ScStage& S = stage[s];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = tid + q * 128, row = e >> 4, at = (e & 15) * 2;
+      const int gi = i0 + row, gj = j0 + row;
+      cp_async16(smem_u32(&S.a[row][at]), Xc + static_cast<size_t>(gi < ib ? gi : ia) * Tp + kc * kScK + at, gi < ib);
+      cp_async16(smem_u32(&S.b[row][at]), Xc + static_cast<size_t>(gj < jb ? gj : ja) * Tp + kc * kScK + at, gj < jb);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (!full) {
+      const int row = tid & 63;
+      const int g = tid < 64 ? i0 + row : j0 + row, end = tid < 64 ? ib : jb;
+      (tid < 64 ? S.wa : S.wb)[row] = g < end ? bits[static_cast<size_t>(g) * W + kc] : 0u;
+    }
+  };
+  double acc[4][4][2];
+  uint32_t n[4][4][2];
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      acc[m][c][0] = acc[m][c][1] = 0.0;
+      n[m][c][0] = n[m][c][1] = 0u;
+    }
+  load(0, 0);
+  for (int kc = 0; kc < W; ++kc) {
+    if (kc + 1 < W) {
+      load((kc + 1) & 1, kc + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const ScStage& S = stage[kc & 1];
+#pragma unroll
+    for (int k = 0; k < kScK; k += 4) {
+      double a[4], b[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        a[m] = S.a[wr + m * 8 + r][k + kq];
+        b[m] = S.b[wc + m * 8 + r][k + kq];
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) dmma_f64(acc[m][c], a[m], b[c]);
+    }
+    if (!full) {
+      uint32_t wb[4][2];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        wb[c][0] = S.wb[wc + c * 8 + 2 * kq];
+        wb[c][1] = S.wb[wc + c * 8 + 2 * kq + 1];
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const uint32_t wa = S.wa[wr + m * 8 + r];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          n[m][c][0] += __popc(wa & wb[c][0]);
+          n[m][c][1] += __popc(wa & wb[c][1]);
+        }
+      }
+    }
+    __syncthreads();  // the stage is refilled two steps on
+  }
+  ScProducts& P = *reinterpret_cast<ScProducts*>(smem);
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        P.xy[wr + m * 8 + r][wc + c * 8 + 2 * kq + e] = acc[m][c][e];
+        P.n[wr + m * 8 + r][wc + c * 8 + 2 * kq + e] = full ? static_cast<uint32_t>(T) : n[m][c][e];
+      }
+  __syncthreads();
+  // a warp finishes 8 x 4 pairs at a time: whole sectors of both triangles
+  const int ldi = ib - ia, ldj = jb - ja;
+#pragma unroll 1
+  for (int q = tid >> 5; q < (kScTile / 8) * (kScTile / 4); q += 4) {
+    const int li = (q >> 4) * 8 + (lane & 7), lj = (q & 15) * 4 + (lane >> 3);
+    const int i = i0 + li, j = j0 + lj;
+    if (i >= ib || j >= jb || i > j) continue;
+    double v;
+    bool flag = false;
+    const ColStat& si = st[i];
+    if (i == j) {
+      // diagonal: 1.0 iff the column's centred sum of squares is usable
+      v = (si.count >= 2.0 && si.min != si.max && si.s2 > 0.0 && isfinite(si.s2)) ? 1.0 : dnan();
+    } else {
+      const ColStat& sj = st[j];
+      const double2 x = full ? make_double2(si.s1, si.s2) : ABij[static_cast<size_t>(j - ja) * ldi + (i - ia)];
+      const double2 y = full ? make_double2(sj.s1, sj.s2) : ABji[static_cast<size_t>(i - ia) * ldj + (j - ja)];
+      v = finalize_pair(static_cast<double>(P.n[li][lj]), x.x, y.x, P.xy[li][lj], x.y, y.y, si.mean, sj.mean, flag);
+    }
+    out[static_cast<size_t>(i) * N + j] = v;
+    out[static_cast<size_t>(j) * N + i] = v;
+    if (flag) fb_list[atomicAdd(&sum->flagged, 1)] = i * N + j;  // N*N <= INT32_MAX
+  }
+}
+
+// ---------------------------------------------------------------------------
+// two-pass fallback of the flagged pairs
+// ---------------------------------------------------------------------------
+// A sum with its rounding errors (two-sum): s + c is the sum to about twice
+// the precision.
+struct TwoSum {
+  double s = 0.0, c = 0.0;
+  FCB_DEV void add(double x) {
+    const double t = s + x, b = t - s;
+    c += (s - (t - b)) + (x - b);
+    s = t;
+  }
+  FCB_DEV double value() const { return s + c; }
+  // the warp's total, the same in every lane
+  FCB_DEV void warp_total() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double s2 = __shfl_xor_sync(kFull, s, o), c2 = __shfl_xor_sync(kFull, c, o);
+      c += c2;
+      add(s2);
+    }
+  }
+};
+
+// One warp per pair, a lane every 32nd date: means from sums carried to twice
+// the precision (the mean two-pass reference's compensated sums, without
+// their serial chain: four dependent FP64 adds, 120 clocks, per date, and
+// 672 us for the 6400 flagged pairs of 1218 x 2000), then the centred second
+// pass (compensated above T = 2048).
+__global__ void __launch_bounds__(128) k_sc_fallback(const double* __restrict__ Xraw, const uint32_t* __restrict__ bits,
+                                                     int T, int N, int Tp, const int* __restrict__ fb_list,
+                                                     const ScSummary* __restrict__ sum, double* __restrict__ out) {
+  if (out_of_domain(sum)) return;
+  const int cnt = sum->flagged, W = Tp / 32, lane = static_cast<int>(threadIdx.x & 31);
+  const int nw = static_cast<int>(gridDim.x * blockDim.x) >> 5;
+  for (int g = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < cnt; g += nw) {
+    const int cell = fb_list[g], i = cell / N, j = cell % N;
+    const double* xi = Xraw + static_cast<size_t>(i) * Tp + lane;
+    const double* xj = Xraw + static_cast<size_t>(j) * Tp + lane;
+    const uint32_t* bi = bits + static_cast<size_t>(i) * W;
+    const uint32_t* bj = bits + static_cast<size_t>(j) * W;
+    int n = 0;
+    double mnx = kBigPos, mxx = -kBigPos, mny = kBigPos, mxy = -kBigPos;
+    TwoSum kx, ky;
+#pragma unroll 4
+    for (int w = 0; w < W; ++w) {
+      const uint32_t m = __ldg(bi + w) & __ldg(bj + w);
+      const double x = __ldg(xi + w * 32), y = __ldg(xj + w * 32);
+      n += __popc(m);
+      if ((m >> lane) & 1u) {
+        kx.add(x);
+        ky.add(y);
+        mnx = fmin(mnx, x);
+        mxx = fmax(mxx, x);
+        mny = fmin(mny, y);
+        mxy = fmax(mxy, y);
+      }
+    }
+    kx.warp_total();
+    ky.warp_total();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      mnx = fmin(mnx, __shfl_xor_sync(kFull, mnx, o));
+      mxx = fmax(mxx, __shfl_xor_sync(kFull, mxx, o));
+      mny = fmin(mny, __shfl_xor_sync(kFull, mny, o));
+      mxy = fmax(mxy, __shfl_xor_sync(kFull, mxy, o));
+    }
+    double v = dnan();
+    if (n >= 2 && mnx != mxx && mny != mxy) {  // uniform across the warp
+      const double mx = kx.value() / n, my = ky.value() / n;
+      double sxx = 0.0, syy = 0.0, sxy = 0.0;
+      if (T > kTwoPassKahanT) {
+        TwoSum ka, kb, kc;
+#pragma unroll 4
+        for (int w = 0; w < W; ++w)
+          if (((__ldg(bi + w) & __ldg(bj + w)) >> lane) & 1u) {
+            const double dx = __ldg(xi + w * 32) - mx, dy = __ldg(xj + w * 32) - my;
+            ka.add(dx * dx);
+            kb.add(dy * dy);
+            kc.add(dx * dy);
+          }
+        ka.warp_total();
+        kb.warp_total();
+        kc.warp_total();
+        sxx = ka.value();
+        syy = kb.value();
+        sxy = kc.value();
+      } else {
+#pragma unroll 4
+        for (int w = 0; w < W; ++w)
+          if (((__ldg(bi + w) & __ldg(bj + w)) >> lane) & 1u) {
+            const double dx = __ldg(xi + w * 32) - mx, dy = __ldg(xj + w * 32) - my;
+            sxx += dx * dx;
+            syy += dy * dy;
+            sxy += dx * dy;
+          }
+        sxx = warp_sum(sxx);
+        syy = warp_sum(syy);
+        sxy = warp_sum(sxy);
+      }
+      v = safe_pearson(sxy, sxx, syy);
+    }
+    if (lane == 0) {
+      out[static_cast<size_t>(i) * N + j] = v;
+      out[static_cast<size_t>(j) * N + i] = v;
+    }
+  }
+}
+
+int sc_chunks(int T) { return (T + kScChunk - 1) / kScChunk; }
+int sc_list_cap(int T) { return (T + 8 * sc_chunks(T) + 7) / 8 * 8; }  // (whole 16-byte groups)
+size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
+// columns of one block of pair sums: all of them, or equal blocks of whole tiles
+int sc_block(int N) {
+  const int nb = (N + kScBlock - 1) / kScBlock;
+  return nb <= 1 ? N : ((N + nb - 1) / nb + kScTile - 1) / kScTile * kScTile;
+}
+
+template <typename TIN>
+cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScWork& w, double* out, cudaStream_t s) {
+  const int Tp = (T + 31) / 32 * 32, nchunk = sc_chunks(T), lcap = sc_list_cap(T);
+  uint8_t* m = static_cast<uint8_t*>(w.masks);
+  uint32_t* bits = reinterpret_cast<uint32_t*>(m);
+  m += al256(static_cast<size_t>(N) * (Tp / 32) * 4);
+  uint16_t* list = reinterpret_cast<uint16_t*>(m);
+  m += al256(static_cast<size_t>(N) * lcap * 2);
+  int* ptr = reinterpret_cast<int*>(m);
+  m += al256(static_cast<size_t>(N) * (nchunk + 1) * 4);
+  int* invert = reinterpret_cast<int*>(m);
+  cudaError_t e = cudaMemsetAsync(w.summary, 0, sizeof(ScSummary), s);
+  if (e != cudaSuccess) return e;
+  k_sc_colstats<TIN><<<(N + 31) / 32, 32 * kStWarps, 0, s>>>(X, mask, T, N, w.st, w.summary);
+  k_sc_transpose<TIN><<<dim3(Tp / 32, (N + 31) / 32), dim3(32, 8), 0, s>>>(X, mask, T, N, Tp, w.st, w.xraw, w.xc, bits);
+  k_sc_lists<<<(N * 32 + 255) / 256, 256, 0, s>>>(w.xc, bits, T, N, Tp, nchunk, lcap, w.st, list, ptr, invert);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  const size_t psmem = static_cast<size_t>(std::min(T, kScChunk) + 1) * kScRows * 8;
+  const size_t gsmem = std::max(2 * sizeof(ScStage), sizeof(ScProducts));
+  e = cudaFuncSetAttribute(k_sc_pairsum<TIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(psmem));
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k_sc_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gsmem));
+  if (e != cudaSuccess) return e;
+  auto pairsum = [&](int ia, int ib, int ja, int jb, double2* ab) {
+    const int rows = (ib - ia + kScRows - 1) / kScRows, cols = (jb - ja + 63) / 64;
+    // a CTA per SM and row block; few row blocks share out the columns
+    const int split = std::max(1, std::min(cols, 148 / rows));
+    for (int c = 0; c < nchunk; ++c)
+      k_sc_pairsum<TIN><<<dim3(rows, split), 1024, psmem, s>>>(X, mask, w.xc, bits, w.st, list, ptr, invert, T, N, Tp,
+                                                               nchunk, lcap, c, ia, ib, ja, jb, ib - ia, ab, w.summary);
+  };
+  const int bs = sc_block(N);
+  for (int ia = 0; ia < N; ia += bs)
+    for (int ja = ia; ja < N; ja += bs) {
+      const int ib = std::min(N, ia + bs), jb = std::min(N, ja + bs);
+      const long long ti = (ib - ia + kScTile - 1) / kScTile, tj = (jb - ja + kScTile - 1) / kScTile;
+      double2* ab = w.ab;
+      double2* ba = ia == ja ? ab : ab + static_cast<size_t>(bs) * bs;
+      pairsum(ia, ib, ja, jb, ab);
+      if (ia != ja) pairsum(ja, jb, ia, ib, ba);
+      const long long tiles = ia == ja ? ti * (ti + 1) / 2 : ti * tj;
+      k_sc_gram<<<static_cast<unsigned>(tiles), 128, gsmem, s>>>(w.xc, bits, w.st, T, N, Tp, ia, ib, ja, jb, ab, ba, out,
+                                                                 w.fb_list, w.summary);
+      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+  // grid-stride over the device-side fallback count (no host round trip)
+  k_sc_fallback<<<148 * 8, 128, 0, s>>>(w.xraw, bits, T, N, Tp, w.fb_list, w.summary, out);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+size_t sc_masks_bytes(int T, int N) {
+  const size_t Tp = static_cast<size_t>((T + 31) / 32 * 32);
+  return al256(N * (Tp / 32) * 4) + al256(static_cast<size_t>(N) * sc_list_cap(T) * 2) +
+         al256(static_cast<size_t>(N) * (sc_chunks(T) + 1) * 4) + al256(static_cast<size_t>(N) * 4);
+}
+
+size_t sc_pairs_bytes(int N) {
+  const size_t bs = static_cast<size_t>(sc_block(N));
+  return bs * bs * sizeof(double2) * (bs < static_cast<size_t>(N) ? 2 : 1);
+}
+
+cudaError_t launch_stock_corr(const void* X, int dtype, const uint8_t* mask, int T, int N, const ScWork& w, double* out,
+                              cudaStream_t s) {
+  return dtype == 0 ? sc_launch(static_cast<const float*>(X), mask, T, N, w, out, s)
+                    : sc_launch(static_cast<const double*>(X), mask, T, N, w, out, s);
+}
+
+}  // namespace fcb

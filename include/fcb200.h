@@ -236,9 +236,9 @@ int fcb_dev_rolling_ic(const void* d_f, int f_dtype, const void* d_r, int r_dtyp
                        const uint8_t* d_rmask, int T, int N, int min_valid, double* d_ic, double* d_rank_f,
                        double* d_rank_r, void* stream);
 
-/* stock_corr into a device (N,N) f64 buffer.  Synchronises `stream` twice:
- * the domain check and the path flag are read on the host before the Gram
- * pass, and fallback_count after it.  Scratch from `ws` (required). */
+/* stock_corr into a device (N,N) f64 buffer (untouched on the domain error).
+ * Synchronises `stream` once, to read the domain check, the path flag and
+ * fallback_count.  Scratch from `ws` (required). */
 int fcb_dev_stock_corr(const void* d_x, int dtype, const uint8_t* d_mask, int T, int N, double* d_out,
                        int* selected_path, int* fallback_count, fcb_workspace* ws, void* stream);
 
