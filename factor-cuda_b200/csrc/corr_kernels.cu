@@ -1,22 +1,19 @@
-// corr_kernels.cu -- FP64 pairwise-complete Pearson correlations (drop-in path).
+// corr_kernels.cu -- FP64 pooled pairwise-complete Pearson of factors
+// (factor_corr, the drop-in path) and the correlation domain check.
 //
-// stock_corr (N,N) over t and factor_corr (F,F) over pooled (t,i) rows, with
-// the reference's numeric contract (|dr| <= 1e-12 against np.corrcoef on the
-// joint subset, serial-Kahan semantics on reduction-sensitive inputs):
+// factor_corr (F,F) pools the (t,i) rows of the panel, with the reference's
+// numeric contract (|dr| <= 1e-12 against np.corrcoef on the joint subset,
+// compensated sums on reduction-sensitive inputs):
 //
-//  1. column statistics: count, serial-Kahan mean in row order, min/max,
-//     |x| extrema for the domain check (stock_corr_gpu's col_stats_kernel,
-//     src/stock_corr.cu:73-116, with the demean_kernel's serial Kahan mean,
-//     :244-261);
+//  1. column statistics: count, Kahan mean, min / max;
 //  2. a Gram pass on column-centred values: n, sum x', sum y', sum x'y',
 //     sum x'^2, sum y'^2 over each pair's joint valid set (the six masked
-//     products of _masked_gemm_stats, fc/_cpu_core.py:139-169), accumulated
-//     hierarchically (per 32-wide k tile, then into the running total);
+//     products of _masked_gemm_stats, fc/_cpu_core.py:139-169);
 //  3. finalize: the cancellation gate of _gemm_cancel_mask (ratio 3 on the
 //     uncentred sums, reconstructed from the centred ones), |r|>1, the
 //     near-zero-variance gate of finalize_cell (src/stock_corr_impl.cuh:102-132);
 //     flagged pairs are recomputed by
-//  4. the two-pass fallback on the original values: Kahan mean in row order,
+//  4. the two-pass fallback on the original values: Kahan mean,
 //     exact-constant (min==max) gate, centred second pass (Kahan above T=2048),
 //     sequential (sxy/sqrt(sxx))/sqrt(syy) (two_pass_centered,
 //     src/stock_corr_impl.cuh:150-201; _two_pass_corr, fc/_cpu_core.py:111-137).

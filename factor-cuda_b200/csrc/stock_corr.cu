@@ -9,9 +9,10 @@
 //   * sum x' and sum x'^2 over the other column's valid dates are the column's
 //     totals less the dates that the other column misses.  A column misses few
 //     dates as a rule, so k_sc_pairsum adds up short lists: one CTA keeps the
-//     centred values of 16 columns in shared memory ([date][16]) and walks
-//     every column's list of missing dates (of valid dates where more than a
-//     quarter is missing).  Where what is taken away is more than three
+//     centred values of 16 columns in shared memory ([date][16], and the sums
+//     of every 32 dates) and walks every column's list of missing dates (of
+//     valid dates where more than a quarter is missing); 32 dates that are
+//     all on the list count as one entry.  Where what is taken away is more than three
 //     quarters of the column's sum of squares, the pair's sums are formed over
 //     the joint dates directly, so that the subtraction costs at most two bits.
 // Steps: column statistics (compensated mean, extrema; replaces
@@ -21,6 +22,12 @@
 // (src/stock_corr_impl.cuh:102-132), and the two-pass fallback of the flagged
 // pairs (two_pass_centered, src/stock_corr_impl.cuh:150-201; _two_pass_corr,
 // fc/_cpu_core.py:111-137).
+// Measured on a B200, 1218 x 2000 f32 masked (7 % missing, 6400 flagged pairs):
+// 2.71 ms -> 0.53 ms a call; k_sc_gram 243 us (from 1905; FP64 tensor pipe,
+// 150 us at its peak, and the finalize on the same pipe), k_sc_pairsum 116
+// (shared-memory bandwidth), k_sc_fallback 47 (from 672), statistics, copies
+// and lists 44 (from 103).  64 x 32 tiles, four CTAs per SM: 64 x 64 tiles take
+// 267-294 us, their last wave being nearly empty.
 // The domain check and the full-validity flag stay on the device: the later
 // kernels return at once when the panel is out of the domain, and the host
 // reads the summary once, at the end.
@@ -33,8 +40,8 @@ namespace fcb {
 namespace {
 
 constexpr int kScRows = 16;      // columns of one k_sc_pairsum CTA
-constexpr int kScChunk = 1664;   // dates it holds at a time (208 KB)
-constexpr int kScTile = 64;      // k_sc_gram tile
+constexpr int kScChunk = 1536;   // dates it holds at a time (192 KB, and 12 KB of sums)
+constexpr int kScTile = 64, kScTileJ = 32;  // k_sc_gram tile: rows, columns
 constexpr int kScK = 32;         // dates per stage
 constexpr int kScPitch = kScK + 4;  // doubles per staged row: fragment loads of 4 rows x 4 dates are conflict-free
 constexpr int kScBlock = 5120;   // columns whose pair sums are held at a time
@@ -45,15 +52,14 @@ FCB_DEV bool out_of_domain(const ScSummary* s) {
   return mx > 1e150 || mn < 1e-150;  // (no valid nonzero cell: mn is a NaN)
 }
 
-FCB_DEV bool sc_valid(double v, const uint8_t* mask, size_t e) {
-  return finite_f64(v) && (mask == nullptr || mask[e] != 0);
-}
+// The mask byte of a cell (1 without a mask); valid = finite and nonzero byte.
+FCB_DEV uint32_t sc_mask(const uint8_t* mask, size_t e) { return mask != nullptr ? __ldg(mask + e) : 1u; }
 
 // ---------------------------------------------------------------------------
 // column statistics
 // ---------------------------------------------------------------------------
 // 32 columns per CTA, lane = column (coalesced rows); warp w takes every 32nd
-// date with its own compensated sum, and the 32 partials merge in order.  (One
+// date with its own compensated sum, and the 32 partials merge pairwise.  (One
 // serial compensated sum per column costs four dependent FP64 adds, about 120
 // clocks, per date: 80 us for 1218 dates.)  The mean is the shift of the
 // centred values; the fallback forms its own means.
@@ -62,43 +68,64 @@ template <typename TIN>
 __global__ void __launch_bounds__(32 * kStWarps) k_sc_colstats(const TIN* __restrict__ X, const uint8_t* __restrict__ mask,
                                                                int T, int N, ColStat* __restrict__ st,
                                                                ScSummary* __restrict__ sum) {
-  __shared__ double ps[kStWarps][32], pc[kStWarps][32], pmn[kStWarps][32], pmx[kStWarps][32], pna[kStWarps][32];
-  __shared__ int pn[kStWarps][32];
+  constexpr int kHalf = kStWarps / 2;
+  __shared__ double ps[kHalf][32], pc[kHalf][32], pmn[kHalf][32], pmx[kHalf][32], pna[kHalf][32];
+  __shared__ int pn[kHalf][32];
   const int lane = static_cast<int>(threadIdx.x & 31), w = static_cast<int>(threadIdx.x >> 5);
   const int i = blockIdx.x * 32 + lane;
   Kahan k;
   int cnt = 0;
-  double mn = kBigPos, mx = -kBigPos, mna = kBigPos;
+  TIN lo = TIN(0), hi = TIN(0), near0 = TIN(0);  // extrema in the input type
   if (i < N) {
-#pragma unroll 4
-    for (int t = w; t < T; t += kStWarps) {
-      const size_t e = static_cast<size_t>(t) * N + i;
-      const double v = static_cast<double>(X[e]);
-      if (sc_valid(v, mask, e)) {
-        k.add(v);
-        ++cnt;
-        mn = fmin(mn, v);
-        mx = fmax(mx, v);
-        if (v != 0.0) mna = fmin(mna, fabs(v));
+    constexpr int U = 8;  // dates loaded ahead of their use
+    for (int t0 = w; t0 < T; t0 += U * kStWarps) {
+      TIN x[U];
+      uint32_t m[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int t = t0 + u * kStWarps;
+        const size_t e = static_cast<size_t>(t) * N + i;
+        x[u] = t < T ? __ldg(X + e) : TIN(0);
+        m[u] = t < T ? sc_mask(mask, e) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const TIN v = x[u];
+        if (m[u] != 0u && finite_f64(static_cast<double>(v))) {
+          k.add(static_cast<double>(v));
+          lo = cnt > 0 ? (v < lo ? v : lo) : v;
+          hi = cnt > 0 ? (v > hi ? v : hi) : v;
+          ++cnt;
+          const TIN av = v < TIN(0) ? -v : v;
+          if (av != TIN(0) && (near0 == TIN(0) || av < near0)) near0 = av;
+        }
       }
     }
   }
-  ps[w][lane] = k.s;
-  pc[w][lane] = k.c;
-  pn[w][lane] = cnt;
-  pmn[w][lane] = mn;
-  pmx[w][lane] = mx;
-  pna[w][lane] = mna;
-  __syncthreads();
-  if (w != 0) return;
-  for (int q = 1; q < kStWarps; ++q) {
-    k.add(ps[q][lane]);
-    k.add(-pc[q][lane]);
-    cnt += pn[q][lane];
-    mn = fmin(mn, pmn[q][lane]);
-    mx = fmax(mx, pmx[q][lane]);
-    mna = fmin(mna, pna[q][lane]);
+  double mn = cnt > 0 ? static_cast<double>(lo) : kBigPos, mx = cnt > 0 ? static_cast<double>(hi) : -kBigPos;
+  double mna = near0 != TIN(0) ? static_cast<double>(near0) : kBigPos;
+  // pairwise merge of the warps' partials
+  for (int h = kStWarps / 2; h > 0; h >>= 1) {
+    if (w >= h && w < 2 * h) {
+      ps[w - h][lane] = k.s;
+      pc[w - h][lane] = k.c;
+      pn[w - h][lane] = cnt;
+      pmn[w - h][lane] = mn;
+      pmx[w - h][lane] = mx;
+      pna[w - h][lane] = mna;
+    }
+    __syncthreads();
+    if (w < h) {
+      k.add(ps[w][lane]);
+      k.add(-pc[w][lane]);
+      cnt += pn[w][lane];
+      mn = fmin(mn, pmn[w][lane]);
+      mx = fmax(mx, pmx[w][lane]);
+      mna = fmin(mna, pna[w][lane]);
+    }
+    __syncthreads();
   }
+  if (w != 0) return;
   const double mxa = cnt > 0 ? fmax(fabs(mn), fabs(mx)) : 0.0;
   if (i < N) {
     ColStat c;
@@ -138,17 +165,22 @@ __global__ void k_sc_transpose(const TIN* __restrict__ X, const uint8_t* __restr
   __shared__ double tx[32][33];
   __shared__ uint8_t tm[32][33];
   const int t0 = blockIdx.x * 32, i0 = blockIdx.y * 32;
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int t = t0 + r, i = i0 + threadIdx.x;
-    double v = 0.0;
-    bool ok = false;
-    if (t < T && i < N) {
-      const size_t e = static_cast<size_t>(t) * N + i;
-      v = static_cast<double>(X[e]);
-      ok = sc_valid(v, mask, e);
-    }
-    tx[r][threadIdx.x] = ok ? v : 0.0;
-    tm[r][threadIdx.x] = ok ? 1 : 0;
+  TIN x[4];
+  uint32_t m[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {  // blockDim.y is 8
+    const int t = t0 + q * 8 + threadIdx.y, i = i0 + threadIdx.x;
+    const bool in = t < T && i < N;
+    const size_t e = static_cast<size_t>(t) * N + i;
+    x[q] = in ? __ldg(X + e) : TIN(0);
+    m[q] = in ? sc_mask(mask, e) : 0u;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const double v = static_cast<double>(x[q]);
+    const bool ok = m[q] != 0u && finite_f64(v);
+    tx[q * 8 + threadIdx.y][threadIdx.x] = ok ? v : 0.0;
+    tm[q * 8 + threadIdx.y][threadIdx.x] = ok ? 1 : 0;
   }
   __syncthreads();
   for (int r = threadIdx.y; r < 32; r += blockDim.y) {
@@ -165,10 +197,12 @@ __global__ void k_sc_transpose(const TIN* __restrict__ X, const uint8_t* __restr
 }
 
 // One warp per column: sums of the centred values and their squares, and the
-// column's date list -- missing dates when they are at most a quarter (invert
-// = 1), valid dates otherwise.  Entries are dates within their chunk, each
-// chunk's run padded to eight with the chunk's number of dates (a row of
-// zeros); ptr[c] is where chunk c starts.
+// column's list -- its missing dates when they are at most a quarter (invert =
+// 1), its valid dates otherwise.  Per chunk of dates two runs of entries: the
+// listed dates, then the aligned groups of 32 dates that are listed as a whole
+// (date and group numbers within the chunk), each run padded to eight with the
+// number of a row of zeros.  ptr[2c], ptr[2c + 1] are where chunk c's runs
+// start.
 __global__ void k_sc_lists(const double* __restrict__ Xc, const uint32_t* __restrict__ bits, int T, int N, int Tp,
                            int nchunk, int lcap, ColStat* __restrict__ st, uint16_t* __restrict__ list,
                            int* __restrict__ ptr, int* __restrict__ invert) {
@@ -176,6 +210,7 @@ __global__ void k_sc_lists(const double* __restrict__ Xc, const uint32_t* __rest
   const int lane = threadIdx.x & 31;
   if (w >= N) return;
   double s2 = 0.0, s1 = 0.0;
+#pragma unroll 4
   for (int t = lane; t < Tp; t += 32) {
     const double d = Xc[static_cast<size_t>(w) * Tp + t];
     s2 += d * d;
@@ -191,32 +226,53 @@ __global__ void k_sc_lists(const double* __restrict__ Xc, const uint32_t* __rest
     invert[w] = inv ? 1 : 0;
   }
   uint16_t* out = list + static_cast<size_t>(w) * lcap;
-  int* p = ptr + static_cast<size_t>(w) * (nchunk + 1);
+  int* p = ptr + static_cast<size_t>(w) * (2 * nchunk + 1);
   const uint32_t* b = bits + static_cast<size_t>(w) * (Tp / 32);
   int pos = 0;
+  auto pad_to = [&](int zero_row) {
+    const int pad = (8 - (pos & 7)) & 7;
+    if (lane < pad) out[pos + lane] = static_cast<uint16_t>(zero_row);
+    pos += pad;
+  };
   for (int c = 0; c < nchunk; ++c) {
-    if (lane == 0) p[c] = pos;
-    const int t1 = min(T, (c + 1) * kScChunk);
-    for (int t0 = c * kScChunk; t0 < t1; t0 += 32) {
-      uint32_t m = b[t0 / 32];
+    const int tn = min(T - c * kScChunk, kScChunk), nw = (tn + 31) / 32;
+    // a lane keeps the words lane, lane + 32 of the chunk (at most 48)
+    uint32_t word[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int k = q * 32 + lane;
+      uint32_t m = k < nw ? b[c * (kScChunk / 32) + k] : 0u;
       if (inv) m = ~m;
-      if (t1 - t0 < 32) m &= (1u << (t1 - t0)) - 1u;
-      if ((m >> lane) & 1u) out[pos + __popc(m & lanemask_lt())] = static_cast<uint16_t>(t0 - c * kScChunk + lane);
+      if (k == tn / 32) m &= (1u << (tn & 31)) - 1u;  // (the last, partial word)
+      word[q] = k < nw ? m : 0u;
+    }
+    if (lane == 0) p[2 * c] = pos;
+    for (int k = 0; k < nw; ++k) {
+      const uint32_t m = __shfl_sync(kFull, k < 32 ? word[0] : word[1], k & 31);
+      if (m == kFull) continue;
+      if ((m >> lane) & 1u) out[pos + __popc(m & lanemask_lt())] = static_cast<uint16_t>(32 * k + lane);
       pos += __popc(m);
     }
-    const int pad = (8 - (pos & 7)) & 7;
-    if (lane < pad) out[pos + lane] = static_cast<uint16_t>(t1 - c * kScChunk);
-    pos += pad;
+    pad_to(tn);
+    if (lane == 0) p[2 * c + 1] = pos;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const unsigned whole = __ballot_sync(kFull, word[q] == kFull);
+      if (word[q] == kFull) out[pos + __popc(whole & lanemask_lt())] = static_cast<uint16_t>(q * 32 + lane);
+      pos += __popc(whole);
+    }
+    pad_to(nw);
   }
-  if (lane == 0) p[nchunk] = pos;
+  if (lane == 0) p[2 * nchunk] = pos;
 }
 
 // ---------------------------------------------------------------------------
 // pair sums: AB[(j - ja) * ld + (i - ia)] = (sum x'_i, sum x'_i^2) over the
 // valid dates of column j
 // ---------------------------------------------------------------------------
-// A half-warp takes one column j at a time: lane = column i.  A list entry
-// costs one 128-byte shared-memory row and two FP64 instructions per lane.
+// A half-warp takes one column j at a time: lane = column i.  A listed date
+// costs one 128-byte shared-memory row and two FP64 instructions per lane, a
+// listed group of 32 dates twice the row.  Shared-memory bandwidth bounds it.
 // Chunk c of the dates; the sums of earlier chunks wait in AB.
 template <typename TIN>
 __global__ void __launch_bounds__(1024, 1)
@@ -226,35 +282,61 @@ __global__ void __launch_bounds__(1024, 1)
                  int lcap, int c, int ia, int ib, int ja, int jb, int ld, double2* __restrict__ AB,
                  const ScSummary* __restrict__ sum) {
   if (sum->masked == 0 || out_of_domain(sum)) return;  // a full panel needs no pair sums
-  extern __shared__ __align__(16) double xs[];         // [tn + 1][kScRows], the last row zero
-  const int t0 = c * kScChunk, tn = min(T - t0, kScChunk);
+  extern __shared__ __align__(16) double xs[];  // [tn + 1][kScRows] values, [nw + 1][kScRows] sums; last rows zero
+  const int t0 = c * kScChunk, tn = min(T - t0, kScChunk), nw = (tn + 31) / 32;
+  double2* gs = reinterpret_cast<double2*>(xs + static_cast<size_t>(tn + 1) * kScRows);
   const int i0 = ia + static_cast<int>(blockIdx.x) * kScRows;
-  for (int e = threadIdx.x; e < tn * kScRows; e += blockDim.x) {
-    const int i = i0 + (e % kScRows);
-    double v = 0.0;
-    if (i < ib) {
-      const size_t at = static_cast<size_t>(t0 + e / kScRows) * N + i;
-      const double x = static_cast<double>(X[at]);
-      if (sc_valid(x, mask, at)) v = x - st[i].mean;
+  {
+    const int li = static_cast<int>(threadIdx.x) % kScRows, i = i0 + li, step = static_cast<int>(blockDim.x) / kScRows;
+    const double mean = i < ib ? st[i].mean : 0.0;
+    constexpr int U = 8;  // dates loaded ahead of their use
+    for (int t1 = static_cast<int>(threadIdx.x) / kScRows; t1 < tn; t1 += U * step) {
+      TIN x[U];
+      uint32_t m[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int t = t1 + u * step;
+        const bool in = t < tn && i < ib;
+        const size_t at = static_cast<size_t>(t0 + t) * N + i;
+        x[u] = in ? __ldg(X + at) : TIN(0);
+        m[u] = in ? sc_mask(mask, at) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int t = t1 + u * step;
+        const double v = static_cast<double>(x[u]);
+        if (t < tn) xs[t * kScRows + li] = m[u] != 0u && finite_f64(v) ? v - mean : 0.0;
+      }
     }
-    xs[e] = v;
+    if (threadIdx.x < kScRows) xs[tn * kScRows + li] = 0.0;
   }
-  // the padding entries' row
-  if (threadIdx.x < kScRows) xs[tn * kScRows + threadIdx.x] = 0.0;
+  __syncthreads();
+  for (int e = static_cast<int>(threadIdx.x); e < (nw + 1) * kScRows; e += static_cast<int>(blockDim.x)) {
+    const int k = e / kScRows;
+    double a = 0.0, q = 0.0;
+    if (k < nw)
+      for (int t = 32 * k; t < min(tn, 32 * k + 32); ++t) {
+        const double x = xs[t * kScRows + e % kScRows];
+        a += x;
+        q = fma(x, x, q);
+      }
+    gs[e] = make_double2(a, q);
+  }
   __syncthreads();
   const int lane = threadIdx.x & 15, i = i0 + lane;
   const int hw = static_cast<int>(threadIdx.x >> 4), nhw = static_cast<int>(blockDim.x >> 4);
   const double* col = xs + lane;
+  const double2* gcol = gs + lane;
   const double s1 = i < ib ? st[i].s1 : 0.0, s2 = i < ib ? st[i].s2 : 0.0;
   for (int j = ja + static_cast<int>(blockIdx.y) * nhw + hw; j < jb; j += nhw * static_cast<int>(gridDim.y)) {
-    const int* p = ptr + static_cast<size_t>(j) * (nchunk + 1) + c;
+    const int* p = ptr + static_cast<size_t>(j) * (2 * nchunk + 1) + 2 * c;
     const uint4* l = reinterpret_cast<const uint4*>(list + static_cast<size_t>(j) * lcap);
+    const int k0 = p[0] >> 3, k1 = p[1] >> 3, k2 = p[2] >> 3;
     double a0 = 0.0, a1 = 0.0, q0 = 0.0, q1 = 0.0;
-    const int k0 = p[0] >> 3, k1 = p[1] >> 3;
-    uint4 next = k0 < k1 ? __ldg(l + k0) : make_uint4(0u, 0u, 0u, 0u);
+    uint4 next = k0 < k2 ? __ldg(l + k0) : make_uint4(0u, 0u, 0u, 0u);
     for (int k = k0; k < k1; ++k) {
       const uint4 v = next;
-      if (k + 1 < k1) next = __ldg(l + k + 1);
+      if (k + 1 < k2) next = __ldg(l + k + 1);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -264,6 +346,20 @@ __global__ void __launch_bounds__(1024, 1)
         q0 = fma(x, x, q0);
         a1 += y;
         q1 = fma(y, y, q1);
+      }
+    }
+    for (int k = k1; k < k2; ++k) {
+      const uint4 v = next;
+      if (k + 1 < k2) next = __ldg(l + k + 1);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const double2 x = gcol[(w[u] & 0xFFFFu) * kScRows];
+        const double2 y = gcol[(w[u] >> 16) * kScRows];
+        a0 += x.x;
+        q0 += x.y;
+        a1 += y.x;
+        q1 += y.y;
       }
     }
     if (i >= ib) continue;
@@ -296,39 +392,41 @@ __global__ void __launch_bounds__(1024, 1)
 // ---------------------------------------------------------------------------
 // Gram pass
 // ---------------------------------------------------------------------------
-FCB_DEV void tri_tile(int b, int nt, int& ib, int& jb) {
-  int lo = 0, hi = nt - 1;
+// Tile b of the row-major list of tiles on or above the diagonal: row block ib
+// has the nj - 2 ib column blocks from 2 ib on (64-row blocks, 32-column
+// blocks).
+FCB_DEV void tri_tile(int b, int ni, int nj, int& ib, int& jb) {
+  int lo = 0, hi = ni - 1;
+  auto first = [&](int r) { return static_cast<long long>(r) * nj - static_cast<long long>(r) * (r - 1); };
   while (lo < hi) {
     const int mid = (lo + hi + 1) / 2;
-    const long long pm = static_cast<long long>(mid) * nt - static_cast<long long>(mid) * (mid - 1) / 2;
-    if (pm <= b) lo = mid; else hi = mid - 1;
+    if (first(mid) <= b) lo = mid; else hi = mid - 1;
   }
   ib = lo;
-  const long long p = static_cast<long long>(ib) * nt - static_cast<long long>(ib) * (ib - 1) / 2;
-  jb = ib + static_cast<int>(b - p);
+  jb = 2 * ib + static_cast<int>(b - first(ib));
 }
 
 FCB_DEV void cp_async16(uint32_t dst, const void* src, bool in) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
 }
 
-// One stage: 32 dates of the tile's two sets of 64 columns, and their bits.
+// One stage: 32 dates of the tile's two sets of columns, and their bits.
 struct ScStage {
-  double a[kScTile][kScPitch], b[kScTile][kScPitch];
-  uint32_t wa[kScTile], wb[kScTile];
+  double a[kScTile][kScPitch], b[kScTileJ][kScPitch];
+  uint32_t wa[kScTile], wb[kScTileJ];
 };
 // The tile's products and counts, for the finalize.
 struct ScProducts {
-  double xy[kScTile][kScTile + 1];
-  uint32_t n[kScTile][kScTile + 1];
+  double xy[kScTile][kScTileJ + 1];
+  uint32_t n[kScTile][kScTileJ + 1];
 };
 
-// 64 x 64 tiles of columns [ia, ib) x [ja, jb) (the same range: the upper
-// triangle of tiles); four warps of 32 x 32, 4 x 4 FP64 matrix instructions
-// per four dates and warp against eight fragment loads.  The FP64 tensor
+// 64 x 32 tiles of columns [ia, ib) x [ja, jb) (the same range: the tiles on
+// and above the diagonal); eight warps of 16 x 16, 2 x 2 FP64 matrix
+// instructions per four dates and warp against four fragment loads.  The FP64 tensor
 // pipe bounds it: one product instead of the six masked sums per pair and
 // date (eight FP64 instructions) that it formed before.
-__global__ void __launch_bounds__(128, 3)
+__global__ void __launch_bounds__(256, 4)
     k_sc_gram(const double* __restrict__ Xc, const uint32_t* __restrict__ bits, const ColStat* __restrict__ st, int T,
               int N, int Tp, int ia, int ib, int ja, int jb, const double2* __restrict__ ABij,
               const double2* __restrict__ ABji, double* __restrict__ out, int* __restrict__ fb_list,
@@ -339,37 +437,38 @@ __global__ void __launch_bounds__(128, 3)
   const bool full = sum->masked == 0;
   int bi, bj;
   if (ia == ja) {
-    tri_tile(blockIdx.x, (ib - ia + kScTile - 1) / kScTile, bi, bj);
+    tri_tile(blockIdx.x, (ib - ia + kScTile - 1) / kScTile, (ib - ia + kScTileJ - 1) / kScTileJ, bi, bj);
   } else {
-    const int nj = (jb - ja + kScTile - 1) / kScTile;
+    const int nj = (jb - ja + kScTileJ - 1) / kScTileJ;
     bi = static_cast<int>(blockIdx.x) / nj;
     bj = static_cast<int>(blockIdx.x) % nj;
   }
-  const int i0 = ia + bi * kScTile, j0 = ja + bj * kScTile;
-  const int tid = static_cast<int>(threadIdx.x), lane = tid & 31, wr = (tid >> 6) * 32, wc = ((tid >> 5) & 1) * 32;
+  const int i0 = ia + bi * kScTile, j0 = ja + bj * kScTileJ;
+  const int tid = static_cast<int>(threadIdx.x), lane = tid & 31, wr = (tid >> 6) * 16, wc = ((tid >> 5) & 1) * 16;
   const int W = Tp / 32, r = lane >> 2, kq = lane & 3;
   auto load = [&](int s, int kc) {
     ScStage& S = stage[s];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = tid + q * 128, row = e >> 4, at = (e & 15) * 2;
-      const int gi = i0 + row, gj = j0 + row;
-      cp_async16(smem_u32(&S.a[row][at]), Xc + static_cast<size_t>(gi < ib ? gi : ia) * Tp + kc * kScK + at, gi < ib);
-      cp_async16(smem_u32(&S.b[row][at]), Xc + static_cast<size_t>(gj < jb ? gj : ja) * Tp + kc * kScK + at, gj < jb);
+    for (int q = 0; q < 6; ++q) {
+      const int e = tid + q * 256, at = (e & 15) * 2;
+      const int row = (e >> 4) - (q < 4 ? 0 : kScTile), g = (q < 4 ? i0 : j0) + row;
+      const int end = q < 4 ? ib : jb, any = q < 4 ? ia : ja;
+      cp_async16(smem_u32(q < 4 ? &S.a[row][at] : &S.b[row][at]),
+                 Xc + static_cast<size_t>(g < end ? g : any) * Tp + kc * kScK + at, g < end);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    if (!full) {
-      const int row = tid & 63;
-      const int g = tid < 64 ? i0 + row : j0 + row, end = tid < 64 ? ib : jb;
-      (tid < 64 ? S.wa : S.wb)[row] = g < end ? bits[static_cast<size_t>(g) * W + kc] : 0u;
+    if (!full && tid < kScTile + kScTileJ) {
+      const bool left = tid < kScTile;
+      const int row = left ? tid : tid - kScTile, g = (left ? i0 : j0) + row;
+      (left ? S.wa : S.wb)[row] = g < (left ? ib : jb) ? bits[static_cast<size_t>(g) * W + kc] : 0u;
     }
   };
-  double acc[4][4][2];
-  uint32_t n[4][4][2];
+  double acc[2][2][2];
+  uint32_t n[2][2][2];
 #pragma unroll
-  for (int m = 0; m < 4; ++m)
+  for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < 2; ++c) {
       acc[m][c][0] = acc[m][c][1] = 0.0;
       n[m][c][0] = n[m][c][1] = 0u;
     }
@@ -385,29 +484,28 @@ __global__ void __launch_bounds__(128, 3)
     const ScStage& S = stage[kc & 1];
 #pragma unroll
     for (int k = 0; k < kScK; k += 4) {
-      double a[4], b[4];
+      double a[2], b[2];
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        a[m] = S.a[wr + m * 8 + r][k + kq];
-        b[m] = S.b[wc + m * 8 + r][k + kq];
-      }
+      for (int m = 0; m < 2; ++m) a[m] = S.a[wr + m * 8 + r][k + kq];
 #pragma unroll
-      for (int m = 0; m < 4; ++m)
+      for (int c = 0; c < 2; ++c) b[c] = S.b[wc + c * 8 + r][k + kq];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) dmma_f64(acc[m][c], a[m], b[c]);
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) dmma_f64(acc[m][c], a[m], b[c]);
     }
     if (!full) {
-      uint32_t wb[4][2];
+      uint32_t wb[2][2];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < 2; ++c) {
         wb[c][0] = S.wb[wc + c * 8 + 2 * kq];
         wb[c][1] = S.wb[wc + c * 8 + 2 * kq + 1];
       }
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
+      for (int m = 0; m < 2; ++m) {
         const uint32_t wa = S.wa[wr + m * 8 + r];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < 2; ++c) {
           n[m][c][0] += __popc(wa & wb[c][0]);
           n[m][c][1] += __popc(wa & wb[c][1]);
         }
@@ -417,9 +515,9 @@ __global__ void __launch_bounds__(128, 3)
   }
   ScProducts& P = *reinterpret_cast<ScProducts*>(smem);
 #pragma unroll
-  for (int m = 0; m < 4; ++m)
+  for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
+    for (int c = 0; c < 2; ++c)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         P.xy[wr + m * 8 + r][wc + c * 8 + 2 * kq + e] = acc[m][c][e];
@@ -429,8 +527,8 @@ __global__ void __launch_bounds__(128, 3)
   // a warp finishes 8 x 4 pairs at a time: whole sectors of both triangles
   const int ldi = ib - ia, ldj = jb - ja;
 #pragma unroll 1
-  for (int q = tid >> 5; q < (kScTile / 8) * (kScTile / 4); q += 4) {
-    const int li = (q >> 4) * 8 + (lane & 7), lj = (q & 15) * 4 + (lane >> 3);
+  for (int q = tid >> 5; q < (kScTile / 8) * (kScTileJ / 4); q += 8) {
+    const int li = (q >> 3) * 8 + (lane & 7), lj = (q & 7) * 4 + (lane >> 3);
     const int i = i0 + li, j = j0 + lj;
     if (i >= ib || j >= jb || i > j) continue;
     double v;
@@ -493,33 +591,33 @@ __global__ void __launch_bounds__(128) k_sc_fallback(const double* __restrict__ 
     const uint32_t* bi = bits + static_cast<size_t>(i) * W;
     const uint32_t* bj = bits + static_cast<size_t>(j) * W;
     int n = 0;
-    double mnx = kBigPos, mxx = -kBigPos, mny = kBigPos, mxy = -kBigPos;
+    // a column is constant on the joint dates when all its values equal the
+    // first (bit patterns: a column of both zeros has no variance either)
+    unsigned long long dx0 = 0ull, dy0 = 0ull;
+    long long x0 = 0, y0 = 0;
     TwoSum kx, ky;
 #pragma unroll 4
     for (int w = 0; w < W; ++w) {
       const uint32_t m = __ldg(bi + w) & __ldg(bj + w);
       const double x = __ldg(xi + w * 32), y = __ldg(xj + w * 32);
+      const long long xb = __double_as_longlong(x), yb = __double_as_longlong(y);
+      if (n == 0 && m != 0u) {  // uniform across the warp
+        x0 = __shfl_sync(kFull, xb, __ffs(m) - 1);
+        y0 = __shfl_sync(kFull, yb, __ffs(m) - 1);
+      }
       n += __popc(m);
       if ((m >> lane) & 1u) {
         kx.add(x);
         ky.add(y);
-        mnx = fmin(mnx, x);
-        mxx = fmax(mxx, x);
-        mny = fmin(mny, y);
-        mxy = fmax(mxy, y);
+        dx0 |= static_cast<unsigned long long>(xb ^ x0);
+        dy0 |= static_cast<unsigned long long>(yb ^ y0);
       }
     }
     kx.warp_total();
     ky.warp_total();
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      mnx = fmin(mnx, __shfl_xor_sync(kFull, mnx, o));
-      mxx = fmax(mxx, __shfl_xor_sync(kFull, mxx, o));
-      mny = fmin(mny, __shfl_xor_sync(kFull, mny, o));
-      mxy = fmax(mxy, __shfl_xor_sync(kFull, mxy, o));
-    }
+    const bool varies = __any_sync(kFull, dx0 != 0ull) && __any_sync(kFull, dy0 != 0ull);
     double v = dnan();
-    if (n >= 2 && mnx != mxx && mny != mxy) {  // uniform across the warp
+    if (n >= 2 && varies) {  // uniform across the warp
       const double mx = kx.value() / n, my = ky.value() / n;
       double sxx = 0.0, syy = 0.0, sxy = 0.0;
       if (T > kTwoPassKahanT) {
@@ -561,7 +659,7 @@ __global__ void __launch_bounds__(128) k_sc_fallback(const double* __restrict__ 
 }
 
 int sc_chunks(int T) { return (T + kScChunk - 1) / kScChunk; }
-int sc_list_cap(int T) { return (T + 8 * sc_chunks(T) + 7) / 8 * 8; }  // (whole 16-byte groups)
+int sc_list_cap(int T) { return (T + 16 * sc_chunks(T) + 7) / 8 * 8; }  // whole 16-byte groups, two padded runs a chunk
 size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 // columns of one block of pair sums: all of them, or equal blocks of whole tiles
 int sc_block(int N) {
@@ -578,7 +676,7 @@ cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScW
   uint16_t* list = reinterpret_cast<uint16_t*>(m);
   m += al256(static_cast<size_t>(N) * lcap * 2);
   int* ptr = reinterpret_cast<int*>(m);
-  m += al256(static_cast<size_t>(N) * (nchunk + 1) * 4);
+  m += al256(static_cast<size_t>(N) * (2 * nchunk + 1) * 4);
   int* invert = reinterpret_cast<int*>(m);
   cudaError_t e = cudaMemsetAsync(w.summary, 0, sizeof(ScSummary), s);
   if (e != cudaSuccess) return e;
@@ -586,7 +684,8 @@ cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScW
   k_sc_transpose<TIN><<<dim3(Tp / 32, (N + 31) / 32), dim3(32, 8), 0, s>>>(X, mask, T, N, Tp, w.st, w.xraw, w.xc, bits);
   k_sc_lists<<<(N * 32 + 255) / 256, 256, 0, s>>>(w.xc, bits, T, N, Tp, nchunk, lcap, w.st, list, ptr, invert);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  const size_t psmem = static_cast<size_t>(std::min(T, kScChunk) + 1) * kScRows * 8;
+  const int tc = std::min(T, kScChunk);
+  const size_t psmem = (static_cast<size_t>(tc + 1) * 8 + static_cast<size_t>((tc + 31) / 32 + 1) * 16) * kScRows;
   const size_t gsmem = std::max(2 * sizeof(ScStage), sizeof(ScProducts));
   e = cudaFuncSetAttribute(k_sc_pairsum<TIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(psmem));
   if (e != cudaSuccess) return e;
@@ -604,13 +703,13 @@ cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScW
   for (int ia = 0; ia < N; ia += bs)
     for (int ja = ia; ja < N; ja += bs) {
       const int ib = std::min(N, ia + bs), jb = std::min(N, ja + bs);
-      const long long ti = (ib - ia + kScTile - 1) / kScTile, tj = (jb - ja + kScTile - 1) / kScTile;
+      const long long ti = (ib - ia + kScTile - 1) / kScTile, tj = (jb - ja + kScTileJ - 1) / kScTileJ;
       double2* ab = w.ab;
       double2* ba = ia == ja ? ab : ab + static_cast<size_t>(bs) * bs;
       pairsum(ia, ib, ja, jb, ab);
       if (ia != ja) pairsum(ja, jb, ia, ib, ba);
-      const long long tiles = ia == ja ? ti * (ti + 1) / 2 : ti * tj;
-      k_sc_gram<<<static_cast<unsigned>(tiles), 128, gsmem, s>>>(w.xc, bits, w.st, T, N, Tp, ia, ib, ja, jb, ab, ba, out,
+      const long long tiles = ia == ja ? ti * tj - ti * (ti - 1) : ti * tj;
+      k_sc_gram<<<static_cast<unsigned>(tiles), 256, gsmem, s>>>(w.xc, bits, w.st, T, N, Tp, ia, ib, ja, jb, ab, ba, out,
                                                                  w.fb_list, w.summary);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
@@ -624,7 +723,7 @@ cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScW
 size_t sc_masks_bytes(int T, int N) {
   const size_t Tp = static_cast<size_t>((T + 31) / 32 * 32);
   return al256(N * (Tp / 32) * 4) + al256(static_cast<size_t>(N) * sc_list_cap(T) * 2) +
-         al256(static_cast<size_t>(N) * (sc_chunks(T) + 1) * 4) + al256(static_cast<size_t>(N) * 4);
+         al256(static_cast<size_t>(N) * (2 * sc_chunks(T) + 1) * 4) + al256(static_cast<size_t>(N) * 4);
 }
 
 size_t sc_pairs_bytes(int N) {
