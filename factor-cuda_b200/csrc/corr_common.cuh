@@ -34,12 +34,19 @@ FCB_DEV double safe_pearson(double sxy, double sxx, double syy) {
   return isfinite(r) ? r : dnan();
 }
 
-// Decide from the centred moment sums of one pair whether the Gram value is
-// trustworthy; returns NaN + flag when the pair must go to the fallback.
-FCB_DEV double finalize_pair(double n, double sx, double sy, double sxy, double sx2, double sy2, double mux,
-                             double muy, bool& flag) {
-  flag = false;
-  if (n < 2.0) return dnan();
+// One pair from its centred moment sums (x' = x - mux).  gate: the reference's
+// cancellation gate on the uncentred sums (reconstructed) fails.  redo: the
+// value must come from the two-pass recomputation.  A gated pair's value is
+// kept when the centred sums carry it at full precision: the joint means lie
+// within two standard deviations of the shifts, and the shifts within 1e6 of
+// them from zero (beyond, the rounding of the two-pass mean itself shows).
+struct PairResult {
+  double r;
+  bool gate, redo;
+};
+FCB_DEV PairResult finalize_pair(double n, double sx, double sy, double sxy, double sx2, double sy2, double mux,
+                                 double muy) {
+  if (n < 2.0) return PairResult{dnan(), false, false};
   const double rn = 1.0 / n, mx = sx * rn, my = sy * rn;  // one division for all
   const double cov = fma(-mx, sy, sxy);
   const double vx = fma(-mx, sx, sx2);
@@ -50,15 +57,17 @@ FCB_DEV double finalize_pair(double n, double sx, double sy, double sxy, double 
   const double sx2r = sx2 + 2.0 * mux * sx + n * mux * mux;
   const double sy2r = sy2 + 2.0 * muy * sy + n * muy * muy;
   const double qxx = sxr * sxr * rn, qyy = syr * syr * rn;
-  bool fix = (fabs(sxr * syr * rn) > kCancelRatio * fabs(cov)) || (fabs(qxx) > kCancelRatio * fabs(vx)) ||
-             (fabs(qyy) > kCancelRatio * fabs(vy));
+  const bool gate = (fabs(sxr * syr * rn) > kCancelRatio * fabs(cov)) || (fabs(qxx) > kCancelRatio * fabs(vx)) ||
+                    (fabs(qyy) > kCancelRatio * fabs(vy));
   const double xmag = fmax(fabs(sx2r), fabs(qxx));
   const double ymag = fmax(fabs(sy2r), fabs(qyy));
-  if (fabs(vx) <= kConstVarRel * (xmag + kTiny) || fabs(vy) <= kConstVarRel * (ymag + kTiny)) fix = true;
   const double r = safe_pearson(cov, vx, vy);
-  if (!isfinite(r) || fabs(r) > 1.0) fix = true;
-  flag = fix;
-  return fix ? dnan() : r;
+  const bool degenerate = fabs(vx) <= kConstVarRel * (xmag + kTiny) || fabs(vy) <= kConstVarRel * (ymag + kTiny) ||
+                          !isfinite(r) || fabs(r) > 1.0;
+  const bool near = mx * sx <= 4.0 * vx && my * sy <= 4.0 * vy;
+  const bool small = n * mux * mux <= 1e12 * vx && n * muy * muy <= 1e12 * vy;
+  const bool redo = degenerate || !near || (gate && !small);
+  return PairResult{redo ? dnan() : r, gate || degenerate, redo};
 }
 
 FCB_DEV void dmma_f64(double (&d)[2], double a, double b) {

@@ -105,13 +105,14 @@ FCB_DEV Blk launch_blk() {
   return Blk{static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.y), static_cast<int>(gridDim.x)};
 }
 
-// Per-block column partials over a contiguous row range: count, Kahan sum,
+// Per-block column partials over a contiguous range of the sampled rows (every
+// ms-th; R, sr and the mask index count in sampled rows): count, Kahan sum,
 // min, max.  Rows are visited in increasing order within each thread's
 // strided slice; partials are merged in a fixed order by k_fc_colfinal.
-template <typename TIN, bool UNIT_ROWS>
+template <typename TIN>
 FCB_DEV void fc_colpart_body(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, long long R, int F,
-                             long long sr, long long sf, long long rows_per_block, FcColPart* __restrict__ part,
-                             const Blk bk) {
+                             long long sr, long long sf, long long ms, long long rows_per_block,
+                             FcColPart* __restrict__ part, const Blk bk) {
   const long long r0 = bk.x * rows_per_block;
   const long long r1 = min(R, r0 + rows_per_block);
   for (int f = threadIdx.y; f < F; f += blockDim.y) {
@@ -130,8 +131,8 @@ FCB_DEV void fc_colpart_body(const TIN* __restrict__ X, const uint8_t* __restric
       for (int u = 0; u < kU; ++u) {
         const long long r = rb + static_cast<long long>(u) * blockDim.x;
         ok[u] = r < r1;
-        xv[u] = ok[u] ? col[UNIT_ROWS ? r : r * sr] : TIN(0);
-        ok[u] = ok[u] && (mask == nullptr || mask[r] != 0);
+        xv[u] = ok[u] ? col[r * sr] : TIN(0);
+        ok[u] = ok[u] && (mask == nullptr || mask[r * ms] != 0);
       }
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
@@ -173,10 +174,11 @@ FCB_DEV void fc_colpart_body(const TIN* __restrict__ X, const uint8_t* __restric
   }
 }
 
-template <typename TIN, bool UNIT_ROWS>
+template <typename TIN>
 __global__ void k_fc_colpart(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, long long R, int F,
-                             long long sr, long long sf, long long rows_per_block, FcColPart* __restrict__ part) {
-  fc_colpart_body<TIN, UNIT_ROWS>(X, mask, R, F, sr, sf, rows_per_block, part, launch_blk());
+                             long long sr, long long sf, long long ms, long long rows_per_block,
+                             FcColPart* __restrict__ part) {
+  fc_colpart_body<TIN>(X, mask, R, F, sr, sf, ms, rows_per_block, part, launch_blk());
 }
 
 // One warp per column: lane l merges partials l, l+32, ... in order, then a
@@ -671,7 +673,7 @@ FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int
   if (e >= F * F) return;  // whole warps exit together
   const int i = e / F, j = e % F;
   if (i > j) return;
-  double q[6] = {0, 0, 0, 0, 0, 0};
+  double q[6] = {0, 0, 0, 0, 0, 0}, tot[2] = {0, 0};  // tot: sums of squares of each factor's own rows
   // q: n, sx (x'_i m_j), sy (m_i x'_j), sxy, sx2 (x'^2_i m_j), sy2 (m_i x'^2_j)
   for (int b = lane; b < nblk; b += 32) {
     const double* P = part + static_cast<size_t>(b) * 4 * Fp * Fp;
@@ -681,6 +683,8 @@ FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int
     q[3] += P[(3 * Fp + i) * Fp + j];
     q[4] += P[(2 * Fp + i) * Fp + j];
     q[5] += P[(2 * Fp + j) * Fp + i];
+    tot[0] += P[(2 * Fp + i) * Fp + i];
+    tot[1] += P[(2 * Fp + j) * Fp + j];
   }
   for (int o = 1; o < 32; o <<= 1) {
 #pragma unroll
@@ -688,21 +692,37 @@ FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int
       const double v = __shfl_down_sync(kFull, q[k], o);
       if ((lane & (2 * o - 1)) == 0) q[k] += v;
     }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const double v = __shfl_down_sync(kFull, tot[k], o);
+      if ((lane & (2 * o - 1)) == 0) tot[k] += v;
+    }
   }
   if (lane != 0) return;
-  double r;
-  bool flag = false;
+  PairResult p{dnan(), false, false};
+  const double mui = st[i].mean, muj = st[j].mean;
   if (i == j) {
-    const FcColStat& s = st[i];
-    const double v = q[4] - q[1] * q[1] / fmax(q[0], 1.0);
-    r = (s.count >= 2.0 && s.min != s.max && v > 0.0 && isfinite(v)) ? 1.0 : dnan();
+    // 1.0 iff the column is not constant and its centred sum of squares is
+    // positive and finite; the two-pass recomputation settles a column whose
+    // sums leave that open
+    if (q[0] >= 2.0) {
+      const double mx = q[1] / q[0], v = fma(-mx, q[1], q[4]), m = mx + mui;
+      p.redo = !(v > kConstVarRel * (fmax(fabs(q[4]), q[0] * m * m) + kTiny)) || !isfinite(v);
+      p.r = p.redo ? dnan() : 1.0;
+    }
   } else {
-    r = finalize_pair(q[0], q[1], q[2], q[3], q[4], q[5], st[i].mean, st[j].mean, flag);
+    p = finalize_pair(q[0], q[1], q[2], q[3], q[4], q[5], mui, muj);
+    // the register form's sums are totals less the rows that the other factor
+    // misses: where little is left of a total, its rounding shows
+    if (F <= kFcRegMaxF && (tot[0] * 0.25 > q[4] || tot[1] * 0.25 > q[5])) {
+      p.redo = q[0] >= 2.0;
+      p.r = dnan();
+    }
   }
-  out[i * F + j] = r;
-  out[j * F + i] = r;
-  if (flags != nullptr) flags[i * F + j] = flag ? 1 : 0;
-  if (flag) {
+  out[i * F + j] = p.r;
+  out[j * F + i] = p.r;
+  if (flags != nullptr) flags[i * F + j] = p.gate || (p.redo && i != j) ? 1 : 0;
+  if (p.redo) {
     const int slot = atomicAdd(fb_count, 1);
     fb_list[slot] = e;
   }
@@ -835,7 +855,8 @@ FCB_DEV void fc_fallback_body(const TIN* __restrict__ X, const uint8_t* __restri
     __syncthreads();
   }
   if (tid == 0) {
-    const double r = safe_pearson(sh[4][0] - sh[5][0], sh[0][0] - sh[1][0], sh[2][0] - sh[3][0]);
+    double r = safe_pearson(sh[4][0] - sh[5][0], sh[0][0] - sh[1][0], sh[2][0] - sh[3][0]);
+    if (i == j && isfinite(r)) r = 1.0;
     (void)nn;
     out[i * F + j] = r;
     out[j * F + i] = r;
@@ -1144,7 +1165,8 @@ FCB_DEV void fc_fb_final_body(int F, int nblk, const int* __restrict__ fb_list, 
   if (lane != 0) return;
   const int e = fb_list[slot];
   const int i = e / F, j = e % F;
-  const double r = safe_pearson(c.s - c.c, a.s - a.c, b.s - b.c);
+  double r = safe_pearson(c.s - c.c, a.s - a.c, b.s - b.c);
+  if (i == j && isfinite(r)) r = 1.0;
   out[i * F + j] = r;
   out[j * F + i] = r;
 }
@@ -1156,13 +1178,13 @@ __global__ void k_fc_fb_final(int F, int nblk, const int* __restrict__ fb_list, 
 }
 
 size_t fc_fb_part_doubles(long long R, int F) {
-  const int maxpairs = F * (F - 1) / 2 > 0 ? F * (F - 1) / 2 : 1;
+  const int maxpairs = F * (F + 1) / 2;
   const int nblk = fc_fb_nblk(R, F);
   return static_cast<size_t>(maxpairs) * nblk * kFbP1 + static_cast<size_t>(maxpairs) * 4;
 }
 
 int fc_fb_nblk(long long R, int F) {
-  const int maxpairs = F * (F - 1) / 2 > 0 ? F * (F - 1) / 2 : 1;
+  const int maxpairs = F * (F + 1) / 2;
   long long nb = R / 32768;
   nb = std::min<long long>(nb, kFcFbMaxNblk);
   nb = std::min<long long>(nb, 65536 / maxpairs);
@@ -1195,49 +1217,49 @@ cudaError_t launch_factor_corr_strided(const void* X, int dtype, const uint8_t* 
   (void)tb;
   int tasks_total = 0, tasks_per_block = 0, ytiles = 0;
   fc_gram_plan(Fp, &tasks_total, &tasks_per_block, &ytiles);
-  const long long rpb_cols = (R + w.nblk_cols - 1) / w.nblk_cols;
+  // column statistics of the sampled rows
+  const long long ms = fc_col_stride(R), rs = (R + ms - 1) / ms;
+  const long long rpb_cols = (rs + w.nblk_cols - 1) / w.nblk_cols;
   const long long rpb_gram = (R + w.nblk_gram - 1) / w.nblk_gram;
   dim3 cb(32, 8);
-  // factor planes (rows at unit stride) take the instantiation without the row-stride product
-  if (dtype == 0 && sr == 1)
-    k_fc_colpart<float, true><<<w.nblk_cols, cb, 0, s>>>(static_cast<const float*>(X), mask, R, F, sr, sf, rpb_cols,
-                                                         w.colpart);
-  else if (dtype == 0)
-    k_fc_colpart<float, false><<<w.nblk_cols, cb, 0, s>>>(static_cast<const float*>(X), mask, R, F, sr, sf,
-                                                          rpb_cols, w.colpart);
-  else if (sr == 1)
-    k_fc_colpart<double, true><<<w.nblk_cols, cb, 0, s>>>(static_cast<const double*>(X), mask, R, F, sr, sf,
-                                                          rpb_cols, w.colpart);
+  if (dtype == 0)
+    k_fc_colpart<float><<<w.nblk_cols, cb, 0, s>>>(static_cast<const float*>(X), mask, rs, F, sr * ms, sf, ms, rpb_cols,
+                                                   w.colpart);
   else
-    k_fc_colpart<double, false><<<w.nblk_cols, cb, 0, s>>>(static_cast<const double*>(X), mask, R, F, sr, sf,
-                                                           rpb_cols, w.colpart);
+    k_fc_colpart<double><<<w.nblk_cols, cb, 0, s>>>(static_cast<const double*>(X), mask, rs, F, sr * ms, sf, ms,
+                                                    rpb_cols, w.colpart);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_fc_colfinal<<<(F * 32 + 127) / 128, 128, 0, s>>>(w.colpart, w.nblk_cols, F, w.colstat);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  const size_t smem = fc_gram_smem(Fp, tasks_per_block, dtype == 0 ? 4 : 8);
-  dim3 gg(w.nblk_gram, ytiles);
-  auto gram = [&](auto kernel, const auto* x) -> cudaError_t {
-    const cudaError_t ge =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (ge != cudaSuccess) return ge;
-    kernel<<<gg, 256, smem, s>>>(x, mask, R, F, sr, sf, Fp, rpb_gram, w.colstat, tasks_total, tasks_per_block, w.gram);
-    return cudaSuccess;
-  };
-  const bool mma = fc_gram_use_mma(Fp);
-  if (dtype == 0)
-    e = mma ? gram(k_fc_gram<float, true>, static_cast<const float*>(X))
-            : gram(k_fc_gram<float, false>, static_cast<const float*>(X));
-  else
-    e = mma ? gram(k_fc_gram<double, true>, static_cast<const double*>(X))
-            : gram(k_fc_gram<double, false>, static_cast<const double*>(X));
-  if (e != cudaSuccess) return e;
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (F <= kFcRegMaxF) {
+    e = launch_fc_gram_reg(X, dtype, mask, R, F, sr, sf, Fp, rpb_gram, w.nblk_gram, w.colstat, w.gram, s);
+    if (e != cudaSuccess) return e;
+  } else {
+    const size_t smem = fc_gram_smem(Fp, tasks_per_block, dtype == 0 ? 4 : 8);
+    dim3 gg(w.nblk_gram, ytiles);
+    auto gram = [&](auto kernel, const auto* x) -> cudaError_t {
+      const cudaError_t ge =
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      if (ge != cudaSuccess) return ge;
+      kernel<<<gg, 256, smem, s>>>(x, mask, R, F, sr, sf, Fp, rpb_gram, w.colstat, tasks_total, tasks_per_block, w.gram);
+      return cudaSuccess;
+    };
+    const bool mma = fc_gram_use_mma(Fp);
+    if (dtype == 0)
+      e = mma ? gram(k_fc_gram<float, true>, static_cast<const float*>(X))
+              : gram(k_fc_gram<float, false>, static_cast<const float*>(X));
+    else
+      e = mma ? gram(k_fc_gram<double, true>, static_cast<const double*>(X))
+              : gram(k_fc_gram<double, false>, static_cast<const double*>(X));
+    if (e != cudaSuccess) return e;
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
   if ((e = cudaMemsetAsync(w.fb_count, 0, sizeof(int), s)) != cudaSuccess) return e;
   k_fc_final<<<(F * F * 32 + 255) / 256, 256, 0, s>>>(w.gram, w.nblk_gram, F, Fp, w.colstat, out, w.fb_list,
                                                       w.fb_count, flags);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  const int maxpairs = F * (F - 1) / 2 > 0 ? F * (F - 1) / 2 : 1;
+  const int maxpairs = F * (F + 1) / 2;
   const int nblk = fc_fb_nblk(R, F);
   if (w.fb_part != nullptr && R >= 4096 && nblk > 1) {
     // large pools, caller-provided partials: rows split over nblk blocks per pair
@@ -1311,8 +1333,9 @@ template <typename TIN>
 __global__ void k_fcb_colpart(const FcBatchPanel* __restrict__ P, const int* __restrict__ off, int np) {
   const FcbAt a = fcb_at(P, off, np);
   const FcBatchPanel& q = *a.q;
-  fc_colpart_body<TIN, true>(static_cast<const TIN*>(q.X), q.mask, q.R, q.F, 1, q.R, q.rpb_cols, q.w.colpart,
-                             Blk{a.local, 0, q.w.nblk_cols});
+  const long long ms = fc_col_stride(q.R);
+  fc_colpart_body<TIN>(static_cast<const TIN*>(q.X), q.mask, (q.R + ms - 1) / ms, q.F, ms, q.R, ms, q.rpb_cols,
+                       q.w.colpart, Blk{a.local, 0, q.w.nblk_cols});
 }
 
 __global__ void k_fcb_colfinal(const FcBatchPanel* __restrict__ P, const int* __restrict__ off, int np) {
@@ -1395,9 +1418,10 @@ FcBatchPanel fc_batch_panel(const void* X, const uint8_t* mask, long long R, int
   const int tb = q.Fp / 4;
   (void)tb;
   fc_gram_plan(q.Fp, &q.tasks_total, &q.tasks_per_block, &q.ytiles);
-  q.rpb_cols = (R + w.nblk_cols - 1) / w.nblk_cols;
+  const long long ms = fc_col_stride(R);
+  q.rpb_cols = ((R + ms - 1) / ms + w.nblk_cols - 1) / w.nblk_cols;
   q.rpb_gram = (R + w.nblk_gram - 1) / w.nblk_gram;
-  q.maxpairs = F * (F - 1) / 2 > 0 ? F * (F - 1) / 2 : 1;
+  q.maxpairs = F * (F + 1) / 2;
   q.fb_nblk = fc_fb_nblk(R, F);
   // the same choice of fallback as launch_factor_corr_strided
   q.large = (w.fb_part != nullptr && R >= 4096 && q.fb_nblk > 1) ? 1 : 0;
@@ -1408,7 +1432,9 @@ FcBatchPanel fc_batch_panel(const void* X, const uint8_t* mask, long long R, int
 void fc_batch_grids(const FcBatchPanel& q, int (&blocks)[kFcbGrids]) {
   blocks[kFcbCols] = q.w.nblk_cols;
   blocks[kFcbColFinal] = (q.F * 32 + 127) / 128;
-  blocks[kFcbGram] = q.w.nblk_gram * q.ytiles;
+  for (int k = kFcbReg; k < kFcbGrids; ++k) blocks[k] = 0;
+  blocks[kFcbGram] = q.F <= kFcRegMaxF ? 0 : q.w.nblk_gram * q.ytiles;
+  if (q.F <= kFcRegMaxF) blocks[kFcbReg + fc_reg_kind(q.F)] = q.w.nblk_gram;
   blocks[kFcbFinal] = (q.F * q.F * 32 + 255) / 256;
   blocks[kFcbFbPass] = q.large ? q.fb_ysl * q.fb_nblk : 0;
   blocks[kFcbFbPair] = q.large ? (q.maxpairs * 32 + 127) / 128 : 0;
@@ -1444,6 +1470,10 @@ cudaError_t launch_factor_corr_batch(const FcBatchPanel* d_panels, int np, const
     }
     if (chk() != cudaSuccess) return e;
   }
+  for (int k = 0; k < kFcbGrids - kFcbReg; ++k)
+    if (total[kFcbReg + k] > 0 &&
+        (e = launch_fc_gram_reg_batch(k, dtype, d_panels, off(kFcbReg + k), np, total[kFcbReg + k], s)) != cudaSuccess)
+      return e;
   if (total[kFcbFinal] > 0) {
     k_fcb_final<<<total[kFcbFinal], 256, 0, s>>>(d_panels, off(kFcbFinal), np);
     if (chk() != cudaSuccess) return e;

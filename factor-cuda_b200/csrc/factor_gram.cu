@@ -1,0 +1,333 @@
+// factor_gram.cu -- Gram pass of factor_corr for up to 12 factors, in
+// registers, for sm_100a.
+//
+// A pooled row of F factor values adds one rank-1 update to the F x F moment
+// sums.  A thread takes one row at a time and keeps the F (F + 1) / 2 sums of
+// x'_i x'_j (x' = value minus the factor's shift, 0 where invalid) and the F
+// sums of x'_i in registers: no staging, and one FP64 FMA per pair and row,
+// which is what bounds the pass.  The masked sums of a pair (i, j) -- the rows
+// n, sum x'_i and sum x'_i^2 where j is valid too -- are the totals less the
+// rows on which j is missing.  Rows with no valid factor add nothing, and rows
+// with all of them need no correction; the others (one in ten at 12 factors
+// with 1 % missing cells) go on a queue per warp in shared memory, and the warp
+// adds up a full queue list by list: lanes own (i, j) pairs and walk the rows
+// that miss j.  All sums are formed in a fixed order.
+// Per block the same partials come out as from the staged pass
+// (fc_gram_body): P[product][i][j] with product 0 n, 1 sum x'_i over rows where
+// j is valid, 2 sum x'_i^2 likewise, 3 sum x'_i x'_j.
+#include "corr_common.cuh"
+#include "fcb_kernels.h"
+
+namespace fcb {
+namespace {
+
+constexpr int kRegThreads = 128, kRegWarps = kRegThreads / 32;
+constexpr int kQueue = 96;   // rows a warp's queue holds: flushed from 64 on, 32 arrive at a time
+
+template <int FP>
+struct RegShape {
+  static constexpr int kPairs = FP * (FP + 1) / 2, kSums = kPairs + FP;
+};
+
+// One warp's shared memory.
+template <int FP>
+struct RegWarp {
+  double row[kQueue][FP];   // centred values, 0 where invalid
+  uint32_t valid[kQueue];
+  uint8_t list[FP][kQueue]; // queued rows that miss factor j
+  double cx[FP][FP], cq[FP][FP];  // [j][i]: sum x'_i, sum x'_i^2 over the rows that miss j
+  uint32_t cn[FP][FP];            // rows where i is valid and j is not
+  uint32_t miss[FP];              // rows (with some valid factor) that miss j
+};
+
+// Sums of M values over the warp's lanes, spread over the lanes: each step
+// trades one half of the values for the other lanes' share of the other half.
+// On return a lane holds the totals of values base .. base + len - 1 in v[0 ..].
+template <int M, int O, int FULL>
+FCB_DEV void spread_sums(double (&v)[FULL], int& base, int& len) {
+  if constexpr (O > 0) {
+    constexpr int H = (M + 1) / 2;
+    const bool up = (lane_id() & O) != 0;
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+      const double hi = H + k < M ? v[H + k] : 0.0, lo = v[k];
+      const double other = __shfl_xor_sync(kFull, up ? lo : hi, O);
+      v[k] = (up ? hi : lo) + other;
+    }
+    base += up ? H : 0;
+    len = up ? max(0, len - H) : min(len, H);
+    spread_sums<H, O / 2, FULL>(v, base, len);
+  }
+}
+template <int M>
+constexpr int spread_len() {
+  int m = M;
+  for (int o = 16; o > 0; o >>= 1) m = (m + 1) / 2;
+  return m;
+}
+
+// Adds the queued rows to the warp's corrections.
+template <int FP>
+FCB_DEV void flush_queue(RegWarp<FP>& w, int n, int F) {
+  const int lane = static_cast<int>(lane_id());
+  __syncwarp();
+  int len[FP];
+#pragma unroll
+  for (int j = 0; j < FP; ++j) {
+    len[j] = 0;
+    for (int q = 0; q < n; q += 32) {
+      const bool m = q + lane < n && !((w.valid[q + lane] >> j) & 1u) && j < F;
+      const unsigned b = __ballot_sync(kFull, m);
+      if (m) w.list[j][len[j] + __popc(b & lanemask_lt())] = static_cast<uint8_t>(q + lane);
+      len[j] += __popc(b);
+    }
+    if (lane == 0) w.miss[j] += static_cast<uint32_t>(len[j]);
+  }
+  __syncwarp();
+  for (int e = lane; e < FP * FP; e += 32) {
+    const int j = e / FP, i = e % FP;
+    int nj = 0;
+#pragma unroll
+    for (int q = 0; q < FP; ++q) nj = q == j ? len[q] : nj;
+    double a = 0.0, q2 = 0.0;
+    uint32_t c = 0u;
+    for (int k = 0; k < nj; ++k) {
+      const int r = w.list[j][k];
+      const double x = w.row[r][i];
+      a += x;
+      q2 = fma(x, x, q2);
+      c += (w.valid[r] >> i) & 1u;
+    }
+    w.cx[j][i] += a;
+    w.cq[j][i] += q2;
+    w.cn[j][i] += c;
+  }
+  __syncwarp();
+}
+
+// Row values of a thread: element (r, f) at X[r * sr + f * sf].
+template <typename TIN, int FP, bool ROWS>
+struct RowLoad {
+  TIN x[FP];
+  uint32_t mask;
+  FCB_DEV void get(const TIN* __restrict__ X, const uint8_t* __restrict__ m, long long r, long long r1, int F,
+                   long long sf) {
+    mask = 0u;
+#pragma unroll
+    for (int f = 0; f < FP; ++f) x[f] = TIN(0);
+    if (r >= r1) return;
+    mask = m != nullptr ? __ldg(m + r) : 1u;
+    if (ROWS) {
+      const TIN* p = X + r * F;
+      constexpr int VL = 16 / static_cast<int>(sizeof(TIN));  // values per 16 bytes
+      if (FP % VL == 0 && F == FP && (reinterpret_cast<uintptr_t>(X) & 15u) == 0) {
+#pragma unroll
+        for (int f = 0; f < FP; f += VL) {
+          const uint4 q = __ldg(reinterpret_cast<const uint4*>(p + f));
+          if constexpr (sizeof(TIN) == 4) {
+            x[f] = __uint_as_float(q.x);
+            x[f + 1] = __uint_as_float(q.y);
+            x[f + 2] = __uint_as_float(q.z);
+            x[f + 3] = __uint_as_float(q.w);
+          } else {
+            x[f] = __hiloint2double(static_cast<int>(q.y), static_cast<int>(q.x));
+            x[f + 1] = __hiloint2double(static_cast<int>(q.w), static_cast<int>(q.z));
+          }
+        }
+      } else {
+#pragma unroll
+        for (int f = 0; f < FP; ++f)
+          if (f < F) x[f] = __ldg(p + f);
+      }
+    } else {
+#pragma unroll
+      for (int f = 0; f < FP; ++f)
+        if (f < F) x[f] = __ldg(X + f * sf + r);
+    }
+  }
+};
+
+// Rows [bx * rows_per_block, ...) of the pool into part + bx * 4 Fp^2.
+template <typename TIN, int FP, bool ROWS>
+FCB_DEV void gram_reg_body(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, long long R, int F,
+                           long long sf, int Fp, long long rows_per_block, const FcColStat* __restrict__ st,
+                           double* __restrict__ part, int bx, uint8_t* smem) {
+  using S = RegShape<FP>;
+  RegWarp<FP>* warps = reinterpret_cast<RegWarp<FP>*>(smem);
+  const int tid = static_cast<int>(threadIdx.x), lane = tid & 31, wi = tid >> 5;
+  RegWarp<FP>& w = warps[wi];
+  for (int e = lane; e < FP * FP; e += 32) {
+    (&w.cx[0][0])[e] = 0.0;
+    (&w.cq[0][0])[e] = 0.0;
+    (&w.cn[0][0])[e] = 0u;
+    if (e < FP) w.miss[e] = 0u;
+  }
+  const uint32_t all = (1u << F) - 1u;
+  double shift[FP];
+#pragma unroll
+  for (int f = 0; f < FP; ++f) shift[f] = f < F ? st[f].mean : 0.0;
+  double acc[S::kSums];
+#pragma unroll
+  for (int k = 0; k < S::kSums; ++k) acc[k] = 0.0;
+  uint32_t rows = 0u;  // rows with some valid factor (this warp's, uniform)
+  int queued = 0;
+  const long long r0 = bx * rows_per_block, r1 = min(R, r0 + rows_per_block);
+  RowLoad<TIN, FP, ROWS> next;
+  next.get(X, mask, r0 + tid, r1, F, sf);
+  for (long long rb = r0; rb < r1; rb += kRegThreads) {
+    const RowLoad<TIN, FP, ROWS> cur = next;
+    if (rb + kRegThreads < r1) next.get(X, mask, rb + kRegThreads + tid, r1, F, sf);
+    uint32_t v = 0u;
+    double x[FP];
+#pragma unroll
+    for (int f = 0; f < FP; ++f) {
+      const bool ok = f < F && cur.mask != 0u && KeyOf<TIN>::finite(cur.x[f]);
+      x[f] = ok ? static_cast<double>(cur.x[f]) - shift[f] : 0.0;
+      v |= ok ? 1u << f : 0u;
+    }
+    const unsigned some = __ballot_sync(kFull, v != 0u);
+    rows += __popc(some);
+    if (some == 0u) continue;  // uniform across the warp
+#pragma unroll
+    for (int i = 0, k = 0; i < FP; ++i)
+#pragma unroll
+      for (int j = i; j < FP; ++j, ++k) acc[k] = fma(x[i], x[j], acc[k]);
+#pragma unroll
+    for (int f = 0; f < FP; ++f) acc[S::kPairs + f] += x[f];
+    const unsigned q = __ballot_sync(kFull, v != 0u && v != all);
+    if (q != 0u) {
+      if ((q >> lane) & 1u) {
+        const int at = queued + __popc(q & lanemask_lt());
+#pragma unroll
+        for (int f = 0; f < FP; ++f) w.row[at][f] = x[f];
+        w.valid[at] = v;
+      }
+      queued += __popc(q);
+      if (queued > kQueue - 32) {
+        flush_queue<FP>(w, queued, F);
+        queued = 0;
+      }
+    }
+  }
+  flush_queue<FP>(w, queued, F);
+  // the warps' sums meet in shared memory, in warp order
+  constexpr int L = spread_len<S::kSums>(), TS = S::kSums + 1;
+  double* t0 = reinterpret_cast<double*>(smem + kRegWarps * sizeof(RegWarp<FP>));
+  int base = 0, len = S::kSums;
+  spread_sums<S::kSums, 16, S::kSums>(acc, base, len);
+#pragma unroll
+  for (int k = 0; k < L; ++k)
+    if (k < len) t0[wi * TS + base + k] = acc[k];
+  if (lane == 0) t0[wi * TS + S::kSums] = static_cast<double>(rows);
+  __syncthreads();
+  double* P = part + static_cast<size_t>(bx) * 4 * Fp * Fp;
+  for (int e = tid; e < Fp * Fp; e += kRegThreads) {
+    const int i = e / Fp, j = e % Fp;
+    double n = 0.0, sx = 0.0, sx2 = 0.0, sxy = 0.0;
+    if (i < F && j < F) {
+      const int a = i < j ? i : j, b = i < j ? j : i;
+      const int kij = a * FP - a * (a - 1) / 2 + (b - a), kii = i * FP - i * (i - 1) / 2;
+      for (int q = 0; q < kRegWarps; ++q) {
+        const RegWarp<FP>& u = warps[q];
+        const double* t = t0 + q * TS;
+        n += t[S::kSums] - static_cast<double>(u.miss[i]) - static_cast<double>(u.cn[j][i]);
+        sxy += t[kij];
+        sx += t[S::kPairs + i] - u.cx[j][i];
+        sx2 += t[kii] - u.cq[j][i];
+      }
+    }
+    P[(0 * Fp + i) * Fp + j] = n;
+    P[(1 * Fp + i) * Fp + j] = sx;
+    P[(2 * Fp + i) * Fp + j] = sx2;
+    P[(3 * Fp + i) * Fp + j] = sxy;
+  }
+}
+
+template <int FP>
+constexpr size_t reg_smem() {
+  using S = RegShape<FP>;
+  return kRegWarps * (sizeof(RegWarp<FP>) + (S::kSums + 1) * sizeof(double));
+}
+
+template <typename TIN, int FP, bool ROWS>
+__global__ void __launch_bounds__(kRegThreads, 2)
+    k_fc_gram_reg(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, long long R, int F, long long sf, int Fp,
+                  long long rows_per_block, const FcColStat* __restrict__ st, double* __restrict__ part) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  gram_reg_body<TIN, FP, ROWS>(X, mask, R, F, sf, Fp, rows_per_block, st, part, blockIdx.x, smem);
+}
+
+// Many factor-plane panels: a block finds its panel by binary search.
+template <typename TIN, int FP>
+__global__ void __launch_bounds__(kRegThreads, 2)
+    k_fcb_gram_reg(const FcBatchPanel* __restrict__ P, const int* __restrict__ off, int np) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int b = static_cast<int>(blockIdx.x);
+  int lo = 0, hi = np - 1;  // largest p with off[p] <= b
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (off[mid] <= b) lo = mid; else hi = mid - 1;
+  }
+  const FcBatchPanel& q = P[lo];
+  gram_reg_body<TIN, FP, false>(static_cast<const TIN*>(q.X), q.mask, q.R, q.F, q.R, q.Fp, q.rpb_gram, q.w.colstat,
+                                q.w.gram, b - off[lo], smem);
+}
+
+template <typename TIN, int FP>
+cudaError_t reg_launch(const TIN* X, const uint8_t* mask, long long R, int F, bool rows, long long sf, int Fp,
+                       long long rpb, int nblk, const FcColStat* st, double* part, cudaStream_t s) {
+  auto go = [&](auto kernel) -> cudaError_t {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(reg_smem<FP>()));
+    if (e != cudaSuccess) return e;
+    kernel<<<nblk, kRegThreads, reg_smem<FP>(), s>>>(X, mask, R, F, sf, Fp, rpb, st, part);
+    return cudaGetLastError();
+  };
+  return rows ? go(k_fc_gram_reg<TIN, FP, true>) : go(k_fc_gram_reg<TIN, FP, false>);
+}
+
+template <typename TIN>
+cudaError_t reg_by_width(const TIN* X, const uint8_t* mask, long long R, int F, bool rows, long long sf, int Fp,
+                         long long rpb, int nblk, const FcColStat* st, double* part, cudaStream_t s) {
+  if (F <= 4) return reg_launch<TIN, 4>(X, mask, R, F, rows, sf, Fp, rpb, nblk, st, part, s);
+  if (F <= 6) return reg_launch<TIN, 6>(X, mask, R, F, rows, sf, Fp, rpb, nblk, st, part, s);
+  if (F <= 8) return reg_launch<TIN, 8>(X, mask, R, F, rows, sf, Fp, rpb, nblk, st, part, s);
+  if (F <= 10) return reg_launch<TIN, 10>(X, mask, R, F, rows, sf, Fp, rpb, nblk, st, part, s);
+  return reg_launch<TIN, 12>(X, mask, R, F, rows, sf, Fp, rpb, nblk, st, part, s);
+}
+
+}  // namespace
+
+cudaError_t launch_fc_gram_reg(const void* X, int dtype, const uint8_t* mask, long long R, int F, long long sr,
+                               long long sf, int Fp, long long rows_per_block, int nblk, const FcColStat* st,
+                               double* part, cudaStream_t s) {
+  if (F > kFcRegMaxF || !((sr == F && sf == 1) || sr == 1)) return cudaErrorInvalidValue;
+  const bool rows = sr != 1 || sf == 1;  // (one factor: both layouts are the same)
+  return dtype == 0 ? reg_by_width(static_cast<const float*>(X), mask, R, F, rows, sf, Fp, rows_per_block, nblk, st,
+                                   part, s)
+                    : reg_by_width(static_cast<const double*>(X), mask, R, F, rows, sf, Fp, rows_per_block, nblk, st,
+                                   part, s);
+}
+
+int fc_reg_kind(int F) { return F <= 4 ? 0 : F <= 6 ? 1 : F <= 8 ? 2 : F <= 10 ? 3 : 4; }
+
+cudaError_t launch_fc_gram_reg_batch(int kind, int dtype, const FcBatchPanel* panels, const int* off, int np, int blocks,
+                                     cudaStream_t s) {
+  auto go = [&](auto kernel, size_t smem) -> cudaError_t {
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    kernel<<<blocks, kRegThreads, smem, s>>>(panels, off, np);
+    return cudaGetLastError();
+  };
+  const bool f32 = dtype == 0;
+  switch (kind) {
+    case 0: return f32 ? go(k_fcb_gram_reg<float, 4>, reg_smem<4>()) : go(k_fcb_gram_reg<double, 4>, reg_smem<4>());
+    case 1: return f32 ? go(k_fcb_gram_reg<float, 6>, reg_smem<6>()) : go(k_fcb_gram_reg<double, 6>, reg_smem<6>());
+    case 2: return f32 ? go(k_fcb_gram_reg<float, 8>, reg_smem<8>()) : go(k_fcb_gram_reg<double, 8>, reg_smem<8>());
+    case 3: return f32 ? go(k_fcb_gram_reg<float, 10>, reg_smem<10>()) : go(k_fcb_gram_reg<double, 10>, reg_smem<10>());
+    default: return f32 ? go(k_fcb_gram_reg<float, 12>, reg_smem<12>()) : go(k_fcb_gram_reg<double, 12>, reg_smem<12>());
+  }
+}
+
+}  // namespace fcb

@@ -58,7 +58,8 @@ struct ScSummary {
   unsigned long long max_abs;      // bits of the largest |x| over the valid cells
   unsigned long long min_abs_inv;  // inverted bits of the smallest nonzero |x| (0: none)
   int masked;                      // some cell is invalid
-  int flagged;                     // pairs sent to the two-pass fallback
+  int flagged;                     // pairs that the two-pass fallback recomputes
+  int gated;                       // pairs that fail the cancellation gate
 };
 struct ScWork {
   double *xraw, *xc;  // (N,Tp) column-major values, as they are and centred; Tp = T rounded to 32
@@ -89,14 +90,26 @@ struct FcWork {
   int* fb_count;       // [1]
   double* fb_part;     // fc_fb_part_doubles(R, F) doubles, or nullptr (single-block fallback)
 };
-// Row blocks of factor_corr's Gram pass: narrow panels (F <= 32) use enough
-// blocks to fill the SMs several times over (their staging tile is small);
-// the same count everywhere keeps single-panel and batched results identical.
+// Up to this many factors the Gram pass keeps its sums in registers
+// (factor_gram.cu).
+constexpr int kFcRegMaxF = 12;
+// Row blocks of factor_corr's Gram pass: two per SM for the register form (a
+// block's final reduction costs as much as about ten of its rows per thread);
+// staged panels of F <= 32 fill the SMs several times over (their tile is
+// small).  The same count everywhere keeps single-panel and batched results
+// identical.
 inline int fc_gram_blocks(long long R, int F) {
-  const long long cap = F <= 32 ? 888 : 148;
+  const long long cap = F <= kFcRegMaxF ? 296 : F <= 32 ? 888 : 148;
   long long nb = R / 1024;
   if (nb < 1) nb = 1;
   return static_cast<int>(nb < cap ? nb : cap);
+}
+// Column statistics come from a sample of the rows (every fc_col_stride-th, at
+// most about 16384): the mean is only the shift of the centred sums.
+__host__ __device__ inline long long fc_col_stride(long long R) { return R / 16384 > 1 ? R / 16384 : 1; }
+inline int fc_col_blocks(long long R) {
+  const long long rows = (R + fc_col_stride(R) - 1) / fc_col_stride(R), nb = rows / 128;
+  return static_cast<int>(nb < 1 ? 1 : nb < 148 ? nb : 148);
 }
 // Row blocks per flagged pair of the multi-block fallback (at most
 // kFcFbMaxNblk), and the partials buffer it needs (doubles): kFcFbPartDoubles
@@ -121,7 +134,7 @@ struct FcBatchPanel {
 };
 // Kinds of batched grid (prefix offsets are kept per kind).
 constexpr int kFcbCols = 0, kFcbColFinal = 1, kFcbGram = 2, kFcbFinal = 3, kFcbFbPass = 4, kFcbFbPair = 5,
-              kFcbSmall = 6, kFcbGrids = 7;
+              kFcbSmall = 6, kFcbReg = 7, kFcbGrids = 12;  // kFcbReg: the register form, one kind per fc_reg_kind
 FcBatchPanel fc_batch_panel(const void* X, const uint8_t* mask, long long R, int F, const FcWork& w, double* out);
 // Blocks the panel contributes to each kind of batched grid.
 void fc_batch_grids(const FcBatchPanel& q, int (&blocks)[kFcbGrids]);
@@ -131,7 +144,16 @@ void fc_batch_grids(const FcBatchPanel& q, int (&blocks)[kFcbGrids]);
 cudaError_t launch_factor_corr_batch(const FcBatchPanel* d_panels, int np, const int* d_off, const int* total,
                                      int dtype, size_t gram_smem, cudaStream_t s);
 
-// rank_kernels.cu
+// factor_gram.cu: the register form of the Gram pass, F <= kFcRegMaxF, (T,N,F)
+// rows (sr = F, sf = 1) or factor planes (sr = 1); partials as the staged form's.
+cudaError_t launch_fc_gram_reg(const void* X, int dtype, const uint8_t* mask, long long R, int F, long long sr,
+                               long long sf, int Fp, long long rows_per_block, int nblk, const FcColStat* st,
+                               double* part, cudaStream_t s);
+int fc_reg_kind(int F);  // 0..4: the width its panel runs at
+cudaError_t launch_fc_gram_reg_batch(int kind, int dtype, const FcBatchPanel* panels, const int* off, int np, int blocks,
+                                     cudaStream_t s);
+
+// rank_plane.cu, rank_kernels.cu
 cudaError_t launch_cs_rank(const float* X, const uint8_t* mask, int T, int N, int desc, float* out,
                            int* status, cudaStream_t st);
 cudaError_t launch_param_scan(const float* X, const uint8_t* mask, int T, int N, ScanOut outs, int* status,

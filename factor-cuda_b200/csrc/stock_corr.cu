@@ -526,13 +526,13 @@ __global__ void __launch_bounds__(256, 4)
   __syncthreads();
   // a warp finishes 8 x 4 pairs at a time: whole sectors of both triangles
   const int ldi = ib - ia, ldj = jb - ja;
+  int gated = 0;
 #pragma unroll 1
   for (int q = tid >> 5; q < (kScTile / 8) * (kScTileJ / 4); q += 8) {
     const int li = (q >> 3) * 8 + (lane & 7), lj = (q & 7) * 4 + (lane >> 3);
     const int i = i0 + li, j = j0 + lj;
     if (i >= ib || j >= jb || i > j) continue;
     double v;
-    bool flag = false;
     const ColStat& si = st[i];
     if (i == j) {
       // diagonal: 1.0 iff the column's centred sum of squares is usable
@@ -541,12 +541,17 @@ __global__ void __launch_bounds__(256, 4)
       const ColStat& sj = st[j];
       const double2 x = full ? make_double2(si.s1, si.s2) : ABij[static_cast<size_t>(j - ja) * ldi + (i - ia)];
       const double2 y = full ? make_double2(sj.s1, sj.s2) : ABji[static_cast<size_t>(i - ia) * ldj + (j - ja)];
-      v = finalize_pair(static_cast<double>(P.n[li][lj]), x.x, y.x, P.xy[li][lj], x.y, y.y, si.mean, sj.mean, flag);
+      const PairResult p =
+          finalize_pair(static_cast<double>(P.n[li][lj]), x.x, y.x, P.xy[li][lj], x.y, y.y, si.mean, sj.mean);
+      v = p.r;
+      gated += p.gate || p.redo ? 1 : 0;
+      if (p.redo) fb_list[atomicAdd(&sum->flagged, 1)] = i * N + j;  // N*N <= INT32_MAX
     }
     out[static_cast<size_t>(i) * N + j] = v;
     out[static_cast<size_t>(j) * N + i] = v;
-    if (flag) fb_list[atomicAdd(&sum->flagged, 1)] = i * N + j;  // N*N <= INT32_MAX
   }
+  gated = __reduce_add_sync(kFull, gated);
+  if (lane == 0 && gated != 0) atomicAdd(&sum->gated, gated);
 }
 
 // ---------------------------------------------------------------------------
