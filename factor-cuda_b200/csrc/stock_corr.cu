@@ -23,11 +23,13 @@
 // pairs (two_pass_centered, src/stock_corr_impl.cuh:150-201; _two_pass_corr,
 // fc/_cpu_core.py:111-137).
 // Measured on a B200, 1218 x 2000 f32 masked (7 % missing, 6400 flagged pairs):
-// 2.71 ms -> 0.53 ms a call; k_sc_gram 243 us (from 1905; FP64 tensor pipe,
-// 150 us at its peak, and the finalize on the same pipe), k_sc_pairsum 116
-// (shared-memory bandwidth), k_sc_fallback 47 (from 672), statistics, copies
-// and lists 44 (from 103).  64 x 32 tiles, four CTAs per SM: 64 x 64 tiles take
-// 267-294 us, their last wave being nearly empty.
+// 2.71 ms -> 0.43 ms a call; k_sc_gram 229 us (from 1905; FP64 tensor pipe,
+// 150 us at its peak, and the finalize on the same pipe), k_sc_pairsum 123
+// (shared-memory bandwidth), statistics, copies and lists 43 (from 103).
+// 64 x 32 tiles, four CTAs per SM: 64 x 64 tiles take 267-294 us, their last
+// wave being nearly empty.  Against 80-bit sums the rms error of a correlation
+// is 2.6e-17 (2.8e-17 with the six products): every long sum is a sum of short
+// ones, single chains over all dates gave 1.1e-16.
 // The domain check and the full-validity flag stay on the device: the later
 // kernels return at once when the panel is out of the domain, and the host
 // reads the summary once, at the end.
@@ -43,7 +45,6 @@ constexpr int kScRows = 16;      // columns of one k_sc_pairsum CTA
 constexpr int kScChunk = 1536;   // dates it holds at a time (192 KB, and 12 KB of sums)
 constexpr int kScTile = 64, kScTileJ = 32;  // k_sc_gram tile: rows, columns
 constexpr int kScK = 32;         // dates per stage
-constexpr int kScPitch = kScK + 4;  // doubles per staged row: fragment loads of 4 rows x 4 dates are conflict-free
 constexpr int kScBlock = 5120;   // columns whose pair sums are held at a time
 
 FCB_DEV bool out_of_domain(const ScSummary* s) {
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(1024, 1)
     const int* p = ptr + static_cast<size_t>(j) * (2 * nchunk + 1) + 2 * c;
     const uint4* l = reinterpret_cast<const uint4*>(list + static_cast<size_t>(j) * lcap);
     const int k0 = p[0] >> 3, k1 = p[1] >> 3, k2 = p[2] >> 3;
-    double a0 = 0.0, a1 = 0.0, q0 = 0.0, q1 = 0.0;
+    double a0 = 0.0, a1 = 0.0, q0 = 0.0, q1 = 0.0, a = 0.0, q = 0.0;
     uint4 next = k0 < k2 ? __ldg(l + k0) : make_uint4(0u, 0u, 0u, 0u);
     for (int k = k0; k < k1; ++k) {
       const uint4 v = next;
@@ -346,6 +347,11 @@ __global__ void __launch_bounds__(1024, 1)
         q0 = fma(x, x, q0);
         a1 += y;
         q1 = fma(y, y, q1);
+      }
+      if (((k - k0) & 3) == 3) {  // long lists: short chains round less
+        a += a0 + a1;
+        q += q0 + q1;
+        a0 = a1 = q0 = q1 = 0.0;
       }
     }
     for (int k = k1; k < k2; ++k) {
@@ -363,7 +369,8 @@ __global__ void __launch_bounds__(1024, 1)
       }
     }
     if (i >= ib) continue;
-    double a = a0 + a1, q = q0 + q1;
+    a += a0 + a1;
+    q += q0 + q1;
     double2* o = AB + static_cast<size_t>(j - ja) * ld + (i - ia);
     if (c > 0) {
       const double2 e = *o;
@@ -412,13 +419,19 @@ FCB_DEV void cp_async16(uint32_t dst, const void* src, bool in) {
 
 // One stage: 32 dates of the tile's two sets of columns, and their bits.
 struct ScStage {
-  double a[kScTile][kScPitch], b[kScTileJ][kScPitch];
-  uint32_t wa[kScTile], wb[kScTileJ];
+  double a[kScTile][kScK], b[kScTileJ][kScK];
 };
-// The tile's products and counts, for the finalize.
+// Where date t of a staged row lies. Odd rows have their halves swapped, so
+// that the 8 threads of a 16-byte load phase (2 rows x 8 dates) meet every bank
+// once.
+FCB_DEV int sc_at(int row, int t) { return t ^ ((row & 1) << 3); }
+// The tile's products and counts, for the finalize, and the bits that are
+// counted.
+constexpr int kScWords = 48;
 struct ScProducts {
   double xy[kScTile][kScTileJ + 1];
   uint32_t n[kScTile][kScTileJ + 1];
+  uint32_t w[kScTile + kScTileJ][kScWords + 1];  // words of 32 dates each
 };
 
 // 64 x 32 tiles of columns [ia, ib) x [ja, jb) (the same range: the tiles on
@@ -446,71 +459,61 @@ __global__ void __launch_bounds__(256, 4)
   const int i0 = ia + bi * kScTile, j0 = ja + bj * kScTileJ;
   const int tid = static_cast<int>(threadIdx.x), lane = tid & 31, wr = (tid >> 6) * 16, wc = ((tid >> 5) & 1) * 16;
   const int W = Tp / 32, r = lane >> 2, kq = lane & 3;
-  auto load = [&](int s, int kc) {
-    ScStage& S = stage[s];
+  // Six 16-byte pieces a thread and stage: rows 16 apart, the first four of the
+  // tile's rows. Rows past the end are zero.
+  const int lrow = tid >> 4, lt = (tid & 15) * 2;
+  const double* src = Xc + lt;
+  auto load = [&](int s) {
+    const uint32_t dst = smem_u32(&stage[s].a[lrow][sc_at(lrow, lt)]);
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-      const int e = tid + q * 256, at = (e & 15) * 2;
-      const int row = (e >> 4) - (q < 4 ? 0 : kScTile), g = (q < 4 ? i0 : j0) + row;
+      const int g = (q < 4 ? i0 : j0 - kScTile) + lrow + 16 * q;
       const int end = q < 4 ? ib : jb, any = q < 4 ? ia : ja;
-      cp_async16(smem_u32(q < 4 ? &S.a[row][at] : &S.b[row][at]),
-                 Xc + static_cast<size_t>(g < end ? g : any) * Tp + kc * kScK + at, g < end);
+      cp_async16(dst + q * 16 * kScK * sizeof(double), src + static_cast<size_t>(g < end ? g : any) * Tp, g < end);
     }
+    src += kScK;
     asm volatile("cp.async.commit_group;" ::: "memory");
-    if (!full && tid < kScTile + kScTileJ) {
-      const bool left = tid < kScTile;
-      const int row = left ? tid : tid - kScTile, g = (left ? i0 : j0) + row;
-      (left ? S.wa : S.wb)[row] = g < (left ? ib : jb) ? bits[static_cast<size_t>(g) * W + kc] : 0u;
-    }
   };
   double acc[2][2][2];
-  uint32_t n[2][2][2];
 #pragma unroll
   for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      acc[m][c][0] = acc[m][c][1] = 0.0;
-      n[m][c][0] = n[m][c][1] = 0u;
-    }
-  load(0, 0);
+    for (int c = 0; c < 2; ++c) acc[m][c][0] = acc[m][c][1] = 0.0;
+  load(0);
   for (int kc = 0; kc < W; ++kc) {
     if (kc + 1 < W) {
-      load((kc + 1) & 1, kc + 1);
+      load((kc + 1) & 1);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
     } else {
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
     const ScStage& S = stage[kc & 1];
+    // The stage's own sums, then one addition each: chains of 8 products round
+    // less than chains of T / 4.
+    double part[2][2][2] = {};
 #pragma unroll
-    for (int k = 0; k < kScK; k += 4) {
-      double a[2], b[2];
+    for (int k = 0; k < kScK; k += 8) {
+      double2 b[2];
 #pragma unroll
-      for (int m = 0; m < 2; ++m) a[m] = S.a[wr + m * 8 + r][k + kq];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) b[c] = S.b[wc + c * 8 + r][k + kq];
-#pragma unroll
-      for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int c = 0; c < 2; ++c) dmma_f64(acc[m][c], a[m], b[c]);
-    }
-    if (!full) {
-      uint32_t wb[2][2];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        wb[c][0] = S.wb[wc + c * 8 + 2 * kq];
-        wb[c][1] = S.wb[wc + c * 8 + 2 * kq + 1];
-      }
+      for (int c = 0; c < 2; ++c)
+        b[c] = *reinterpret_cast<const double2*>(&S.b[wc + c * 8 + r][sc_at(r, k + 2 * kq)]);
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
-        const uint32_t wa = S.wa[wr + m * 8 + r];
+        const double2 a = *reinterpret_cast<const double2*>(&S.a[wr + m * 8 + r][sc_at(r, k + 2 * kq)]);
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          n[m][c][0] += __popc(wa & wb[c][0]);
-          n[m][c][1] += __popc(wa & wb[c][1]);
-        }
+        for (int c = 0; c < 2; ++c) dmma_f64(part[m][c], a.x, b[c].x);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) dmma_f64(part[m][c], a.y, b[c].y);
       }
     }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        acc[m][c][0] += part[m][c][0];
+        acc[m][c][1] += part[m][c][1];
+      }
     __syncthreads();  // the stage is refilled two steps on
   }
   ScProducts& P = *reinterpret_cast<ScProducts*>(smem);
@@ -519,10 +522,36 @@ __global__ void __launch_bounds__(256, 4)
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        P.xy[wr + m * 8 + r][wc + c * 8 + 2 * kq + e] = acc[m][c][e];
-        P.n[wr + m * 8 + r][wc + c * 8 + 2 * kq + e] = full ? static_cast<uint32_t>(T) : n[m][c][e];
+      for (int e = 0; e < 2; ++e) P.xy[wr + m * 8 + r][wc + c * 8 + 2 * kq + e] = acc[m][c][e];
+  // The counts come after the products: both sets of sums do not fit the 64
+  // registers that 4 CTAs per SM leave a thread. Rows 2 rp, 2 rp + 1 and
+  // columns cp, cp + 8, cp + 16, cp + 24 are this thread's.
+  const int rp = (tid >> 3) * 2, cp = tid & 7;
+  uint32_t n[2][4] = {{0u, 0u, 0u, 0u}, {0u, 0u, 0u, 0u}};
+  for (int w0 = 0; w0 < W && !full; w0 += kScWords) {
+    const int nw = min(W - w0, kScWords);
+    __syncthreads();
+    for (int row = tid >> 3; row < kScTile + kScTileJ; row += 32) {
+      const bool left = row < kScTile;
+      const int g = left ? i0 + row : j0 + row - kScTile;
+      const bool in = g < (left ? ib : jb);
+      for (int w = cp; w < nw; w += 8) P.w[row][w] = in ? bits[static_cast<size_t>(g) * W + w0 + w] : 0u;
+    }
+    __syncthreads();
+    for (int w = 0; w < nw; ++w) {
+      const uint32_t x0 = P.w[rp][w], x1 = P.w[rp + 1][w];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const uint32_t y = P.w[kScTile + cp + 8 * c][w];
+        n[0][c] += __popc(x0 & y);
+        n[1][c] += __popc(x1 & y);
       }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) P.n[rp + m][cp + 8 * c] = full ? static_cast<uint32_t>(T) : n[m][c];
   __syncthreads();
   // a warp finishes 8 x 4 pairs at a time: whole sectors of both triangles
   const int ldi = ib - ia, ldj = jb - ja;
