@@ -649,7 +649,7 @@ extern "C" int fcb_batch_run_per_panel(fcb_batch* b, void* stream) {
       if (a.F >= 2 && ric_items_fit(a.N))
         FCB_BTRY(launch_rank_ic_items(a, b->preps[i], false, s));
       else
-        FCB_BTRY(launch_rank_ic<float, float>(a, b->d_status, s));
+        FCB_BTRY(launch_rank_ic<float, float>(a, s));
     } else {
       RankIcArgs<double, double> a{};
       a.X = static_cast<const double*>(q.X);
@@ -662,7 +662,7 @@ extern "C" int fcb_batch_run_per_panel(fcb_batch* b, void* stream) {
       a.min_valid = b->min_valid;
       a.ranks_out = q.ranks_out;
       a.ic_out = q.ic_out;
-      FCB_BTRY(launch_rank_ic<double, double>(a, b->d_status, s));
+      FCB_BTRY(launch_rank_ic<double, double>(a, s));
     }
     if (q.corr_out != nullptr) {
       const long long R = static_cast<long long>(q.T) * q.N;

@@ -493,7 +493,7 @@ extern "C" int fcb_dev_parameter_scan_f32(const float* d_x, const uint8_t* d_mas
 // rolling_ic (single factor) and the batched panel
 // ---------------------------------------------------------------------------
 template <typename TF, typename TR>
-static int run_rank_ic(const RankIcArgs<TF, TR>& a, int* dst, cudaStream_t s, fcb_workspace& ws) {
+static int run_rank_ic(const RankIcArgs<TF, TR>& a, cudaStream_t s, fcb_workspace& ws) {
   if constexpr (std::is_same<TF, float>::value && std::is_same<TR, float>::value) {
     if (a.F >= 2 && ric_items_fit(a.N) && a.rank_f_out == nullptr) {
       // several factors: returns prepared once per date, one CTA per (date, factor)
@@ -502,7 +502,7 @@ static int run_rank_ic(const RankIcArgs<TF, TR>& a, int* dst, cudaStream_t s, fc
       return rc(launch_rank_ic_items(a, ric_prep_carve(prep, a.T, a.N, a.F), false, s));
     }
   }
-  if (rank_ic_fits_smem<TF, TR>(a.N)) return rc(launch_rank_ic<TF, TR>(a, dst, s));
+  if (rank_ic_fits<TF, TR>(a.N)) return rc(launch_rank_ic<TF, TR>(a, s));
   const size_t bytes =
       rank_global_scratch(rank_global_bytes_per_date(2, a.N, a.F, sizeof(TF), sizeof(TR)), a.T);
   uint8_t* scr;
@@ -528,10 +528,10 @@ extern "C" int fcb_rolling_ic(const void* f, int fdt, const void* r, int rdt, co
   void *df, *dr;
   uint8_t *dfm = nullptr, *drm = nullptr;
   double *dic, *drf = nullptr, *drr = nullptr;
-  int* dst;
   FCB_TRY(ws.get(S_X, n * fsz, &df));
   FCB_TRY(ws.get(S_X2, n * rsz, &dr));
   FCB_TRY(ws.get(S_IC, static_cast<size_t>(T) * 8, &dic));
+  int* dst;  // the status word of the documented budget
   FCB_TRY(ws.get(S_STATUS, 64, &dst));
   if (fmask) FCB_TRY(ws.get(S_MASK, n, &dfm));
   if (rmask) FCB_TRY(ws.get(S_MASK2, n, &drm));
@@ -543,43 +543,36 @@ extern "C" int fcb_rolling_ic(const void* f, int fdt, const void* r, int rdt, co
   FCB_TRY(cudaMemcpyAsync(dr, r, n * rsz, cudaMemcpyHostToDevice, s));
   if (fmask) FCB_TRY(cudaMemcpyAsync(dfm, fmask, n, cudaMemcpyHostToDevice, s));
   if (rmask) FCB_TRY(cudaMemcpyAsync(drm, rmask, n, cudaMemcpyHostToDevice, s));
-  FCB_TRY(cudaMemsetAsync(dst, 0, sizeof(int), s));
   int e;
   if (fdt == FCB_DTYPE_F32 && rdt == FCB_DTYPE_F32)
     e = run_rank_ic(RankIcArgs<float, float>{static_cast<const float*>(df), static_cast<const float*>(dr), dfm, drm,
                                              1, T, N, min_valid, nullptr, dic, drf, drr},
-                    dst, s, ws);
+                    s, ws);
   else if (fdt == FCB_DTYPE_F32)
     e = run_rank_ic(RankIcArgs<float, double>{static_cast<const float*>(df), static_cast<const double*>(dr), dfm,
                                               drm, 1, T, N, min_valid, nullptr, dic, drf, drr},
-                    dst, s, ws);
+                    s, ws);
   else if (rdt == FCB_DTYPE_F32)
     e = run_rank_ic(RankIcArgs<double, float>{static_cast<const double*>(df), static_cast<const float*>(dr), dfm,
                                               drm, 1, T, N, min_valid, nullptr, dic, drf, drr},
-                    dst, s, ws);
+                    s, ws);
   else
     e = run_rank_ic(RankIcArgs<double, double>{static_cast<const double*>(df), static_cast<const double*>(dr),
                                                dfm, drm, 1, T, N, min_valid, nullptr, dic, drf, drr},
-                    dst, s, ws);
+                    s, ws);
   if (e != 0) return e;
-  int hst = 0;
   FCB_TRY(cudaMemcpyAsync(ic, dic, static_cast<size_t>(T) * 8, cudaMemcpyDeviceToHost, s));
   if (rank_f) {
     FCB_TRY(cudaMemcpyAsync(rank_f, drf, n * 8, cudaMemcpyDeviceToHost, s));
     FCB_TRY(cudaMemcpyAsync(rank_r, drr, n * 8, cudaMemcpyDeviceToHost, s));
   }
-  FCB_TRY(cudaMemcpyAsync(&hst, dst, sizeof(int), cudaMemcpyDeviceToHost, s));
   FCB_TRY(cudaStreamSynchronize(s));
-  return check_status(&hst);
+  return FCB_OK;
 }
 
 template <typename TF, typename TR>
 static int dev_rank_ic(const RankIcArgs<TF, TR>& a, cudaStream_t s) {
-  if (rank_ic_fits_smem<TF, TR>(a.N)) {
-    int* d_status;
-    FCB_TRY(dev_status_sink(&d_status));
-    return rc(launch_rank_ic<TF, TR>(a, d_status, s));
-  }
+  if (rank_ic_fits<TF, TR>(a.N)) return rc(launch_rank_ic<TF, TR>(a, s));
   const size_t bytes =
       rank_global_scratch(rank_global_bytes_per_date(2, a.N, a.F, sizeof(TF), sizeof(TR)), a.T);
   void* scr = nullptr;
@@ -636,8 +629,6 @@ extern "C" int fcb_dev_rank_ic_panel(const float* d_x, const float* d_r, const u
   const int chk = panel_args_check(d_x, d_r, d_ic, F, T, N, min_valid, method);
   if (chk != FCB_OK) return chk;
   if (method != 0) return FCB_ERR_UNSUPPORTED;  // learned: fcb_dev_rank_ic_panel_learned (needs a model)
-  int* d_status;
-  FCB_TRY(dev_status_sink(&d_status));
   RankIcArgs<float, float> a{d_x, d_r, d_fmask, d_rmask, F, T, N, min_valid, d_ranks, d_ic, nullptr, nullptr};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (F >= 2 && ric_items_fit(N)) {
@@ -648,7 +639,7 @@ extern "C" int fcb_dev_rank_ic_panel(const float* d_x, const float* d_r, const u
     FCB_TRY(scratch_free(prep, s));
     return rc(e);
   }
-  if (rank_ic_fits_smem<float, float>(N)) return rc(launch_rank_ic<float, float>(a, d_status, s));
+  if (rank_ic_fits<float, float>(N)) return rc(launch_rank_ic<float, float>(a, s));
   // global-memory path; scratch is stream-ordered (no host synchronisation)
   const size_t bytes = rank_global_scratch(rank_global_bytes_per_date(2, N, F, 4, 4), T);
   void* scr = nullptr;
@@ -718,7 +709,7 @@ extern "C" int fcb_rank_ic_panel(const float* x, const float* r, const uint8_t* 
   const int nchunk = static_cast<int>(chunk_tc.size());
   // learned splitters need a shared-memory kernel; wider sections are ranked
   // by the global-memory radix path (identical results)
-  const bool learned = (method == 1) && (F >= 2 ? ric_items_fit(N) : rank_ic_fits_smem<float, float>(N));
+  const bool learned = (method == 1) && (F >= 2 ? ric_items_fit(N) : rank_ic_learned_fits(N));
   const bool need_ranks = ranks != nullptr || learned;
   float* dx[NB];
   float* dr[NB];
@@ -791,7 +782,7 @@ extern "C" int fcb_rank_ic_panel(const float* x, const float* r, const uint8_t* 
     } else {
       RankIcArgs<float, float> a{dx[j], dr[j], dfm[j], drm[j], F, tc, N, min_valid, drk[j], dic + t0, nullptr, nullptr};
       a.ic_ld = T;
-      const int e = run_rank_ic(a, dst, s_c, ws);
+      const int e = run_rank_ic(a, s_c, ws);
       if (e != 0) return e;
     }
     if (learned) {
@@ -1186,10 +1177,10 @@ extern "C" int fcb_memory_budget(int op, int dtype, int T, int N, int F, int fla
       const int fsz = dtype == FCB_DTYPE_F64 ? 8 : 4, rsz = (flags & FCB_BUDGET_R_F64) ? 8 : 4;
       b = slot_bytes(n * fsz) + slot_bytes(n * rsz) + slot_bytes(static_cast<size_t>(T) * 8) + 64 +
           (m1 ? slot_bytes(n) : 0) + (m2 ? slot_bytes(n) : 0) + (ranks ? 2 * slot_bytes(n * 8) : 0);
-      const bool fits = (fsz == 4 && rsz == 4)   ? rank_ic_fits_smem<float, float>(N)
-                        : (fsz == 4)             ? rank_ic_fits_smem<float, double>(N)
-                        : (rsz == 4)             ? rank_ic_fits_smem<double, float>(N)
-                                                 : rank_ic_fits_smem<double, double>(N);
+      const bool fits = (fsz == 4 && rsz == 4)   ? rank_ic_fits<float, float>(N)
+                        : (fsz == 4)             ? rank_ic_fits<float, double>(N)
+                        : (rsz == 4)             ? rank_ic_fits<double, float>(N)
+                                                 : rank_ic_fits<double, double>(N);
       if (!fits) b += slot_bytes(rank_global_scratch(rank_global_bytes_per_date(2, N, 1, fsz, rsz), T));
       break;
     }
@@ -1244,7 +1235,7 @@ extern "C" int fcb_memory_budget(int op, int dtype, int T, int N, int F, int fla
                (ranks ? slot_bytes(cn * F * 4) : 0));
       if (F >= 2 && ric_items_fit(N))
         b += slot_bytes(ric_prep_bytes(Tc, N, F));
-      else if (!rank_ic_fits_smem<float, float>(N))
+      else if (!rank_ic_fits<float, float>(N))
         b += slot_bytes(rank_global_scratch(rank_global_bytes_per_date(2, N, F, 4, 4), Tc));
       break;
     }

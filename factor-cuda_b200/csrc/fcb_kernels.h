@@ -158,11 +158,15 @@ cudaError_t launch_cs_rank(const float* X, const uint8_t* mask, int T, int N, in
                            int* status, cudaStream_t st);
 cudaError_t launch_param_scan(const float* X, const uint8_t* mask, int T, int N, ScanOut outs, int* status,
                               cudaStream_t st);
-template <typename TF, typename TR>
-size_t rank_ic_smem(int N);
-template <typename TF, typename TR>
-cudaError_t launch_rank_ic(const RankIcArgs<TF, TR>& a, int* status, cudaStream_t st);
+size_t rank_ic_learned_smem(int N);
 cudaError_t launch_rank_ic_learned(const RankIcArgs<float, float>& a, int* status, cudaStream_t st);
+
+// rank_ic_pair.cu: rank + IC of one factor row against one returns row per CTA
+// (any F); true when its shared-memory kernel takes N for these dtypes.
+template <typename TF, typename TR>
+bool rank_ic_fits(int N);
+template <typename TF, typename TR>
+cudaError_t launch_rank_ic(const RankIcArgs<TF, TR>& a, cudaStream_t st);
 
 // cdf_mlp.cu
 size_t cdf_train_smem();
@@ -274,10 +278,9 @@ cudaError_t launch_param_scan_global(const float* X, const uint8_t* mask, int T,
                                      uint8_t* scratch, size_t bytes, cudaStream_t s);
 template <typename TF, typename TR>
 cudaError_t launch_rank_ic_global(const RankIcArgs<TF, TR>& a, uint8_t* scratch, size_t bytes, cudaStream_t s);
-// True when the shared-memory rank+IC kernel takes N for these dtypes.
-template <typename TF, typename TR>
-inline bool rank_ic_fits_smem(int N) {
-  return N <= kSmemRankCap && rank_ic_smem<TF, TR>(N) <= kMaxSmemPerBlock;
+// True when the one-factor learned kernel takes N.
+inline bool rank_ic_learned_fits(int N) {
+  return N <= kSmemRankCap && rank_ic_learned_smem(N) <= kMaxSmemPerBlock;
 }
 inline size_t rank_global_scratch(size_t per_date, int T) {
   size_t b = per_date * static_cast<size_t>(T);

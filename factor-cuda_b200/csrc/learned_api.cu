@@ -263,7 +263,8 @@ int fcb::rank_ic_learned_ld(const float* d_x, const float* d_r, const uint8_t* d
     FCB_TRY(scratch_free(prep, stream));
     return rc(e);
   }
-  if (rank_ic_fits_smem<float, float>(N)) return rc(launch_rank_ic_learned(a, d_status, stream));
+  if (!learned && rank_ic_fits<float, float>(N)) return rc(launch_rank_ic<float, float>(a, stream));
+  if (learned && rank_ic_learned_fits(N)) return rc(launch_rank_ic_learned(a, d_status, stream));
   // too wide for the shared-memory kernel: the global-memory radix path ranks
   // the section (identical results); statistics read outcome 0 (not learned)
   if (d_stats != nullptr)

@@ -432,15 +432,7 @@ constexpr int cap_of() { return NT * 16; }
 
 static int pick_nt(int n) { return n <= 4096 ? 256 : (n <= 8192 ? 512 : 1024); }
 
-template <typename TF, typename TR>
-size_t rank_ic_smem(int N) {
-  constexpr int KSZ = (sizeof(TF) > sizeof(TR)) ? int(sizeof(TF)) : int(sizeof(TR));
-  return RankIcLayout(N, KSZ, SortScratch<1024>::bytes).total;
-}
-template size_t rank_ic_smem<float, float>(int);
-template size_t rank_ic_smem<float, double>(int);
-template size_t rank_ic_smem<double, float>(int);
-template size_t rank_ic_smem<double, double>(int);
+size_t rank_ic_learned_smem(int N) { return RankIcLayout(N, 4, SortScratch<1024>::bytes).total; }
 
 template <int NT, typename TF, typename TR, bool LEARNED>
 static cudaError_t launch_rank_ic_nt(const RankIcArgs<TF, TR>& a, int* status, cudaStream_t st) {
@@ -454,16 +446,6 @@ static cudaError_t launch_rank_ic_nt(const RankIcArgs<TF, TR>& a, int* status, c
   return cudaGetLastError();
 }
 
-template <typename TF, typename TR>
-cudaError_t launch_rank_ic(const RankIcArgs<TF, TR>& a, int* status, cudaStream_t st) {
-  if (a.N > kSmemRankCap) return cudaErrorInvalidValue;
-  switch (pick_nt(a.N)) {
-    case 256: return launch_rank_ic_nt<256, TF, TR, false>(a, status, st);
-    case 512: return launch_rank_ic_nt<512, TF, TR, false>(a, status, st);
-    default: return launch_rank_ic_nt<1024, TF, TR, false>(a, status, st);
-  }
-}
-
 cudaError_t launch_rank_ic_learned(const RankIcArgs<float, float>& a, int* status, cudaStream_t st) {
   if (a.N > kSmemRankCap || a.cdf_table == nullptr || a.cdf_zrange == nullptr) return cudaErrorInvalidValue;
   switch (pick_nt(a.N)) {
@@ -472,10 +454,6 @@ cudaError_t launch_rank_ic_learned(const RankIcArgs<float, float>& a, int* statu
     default: return launch_rank_ic_nt<1024, float, float, true>(a, status, st);
   }
 }
-template cudaError_t launch_rank_ic<float, float>(const RankIcArgs<float, float>&, int*, cudaStream_t);
-template cudaError_t launch_rank_ic<float, double>(const RankIcArgs<float, double>&, int*, cudaStream_t);
-template cudaError_t launch_rank_ic<double, float>(const RankIcArgs<double, float>&, int*, cudaStream_t);
-template cudaError_t launch_rank_ic<double, double>(const RankIcArgs<double, double>&, int*, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // persistent batch launchers

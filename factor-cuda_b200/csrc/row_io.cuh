@@ -138,8 +138,9 @@ FCB_DEV int compact_bases(uint32_t flags, int (&base)[V], unsigned long long* sc
 // per position with room to spare.
 __host__ __device__ inline int mark_words(int n) { return n / 16 + 2; }
 
-// Shared-memory layout of the radix-sorted forms (bytes; every region 16-aligned).
-template <int NT>
+// Shared-memory layout of the radix-sorted forms (bytes; every region 16-aligned)
+// with keys of K bytes.
+template <int NT, int K = 4>
 struct SortedLayout {
   size_t red, dw, dw2, scratch, k0, k1, i0, i1, total;
   __host__ __device__ explicit SortedLayout(int n) {
@@ -148,8 +149,8 @@ struct SortedLayout {
     dw = o; o = al16(o + size_t(mark_words(n)) * 4);   // two bitmaps over positions
     dw2 = o; o = al16(o + size_t(mark_words(n)) * 4);  // for the kernels' own use
     scratch = o; o = al16(o + SortScratch<NT>::bytes);
-    k0 = o; o = al16(o + size_t(n) * 4 + 16);
-    k1 = o; o = al16(o + size_t(n) * 4 + 16);
+    k0 = o; o = al16(o + size_t(n) * K + 16);
+    k1 = o; o = al16(o + size_t(n) * K + 16);
     i0 = o; o = al16(o + size_t(n) * 2 + 16);
     i1 = o; o = al16(o + size_t(n) * 2 + 16);
     total = o;

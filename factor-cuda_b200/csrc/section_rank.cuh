@@ -123,6 +123,7 @@ struct SpreadTotals {
   int m;           // valid cells
   bool heavy;      // some bucket is above kSpreadHeavy
   uint32_t range;  // largest valid key less the smallest
+  uint32_t largest;  // largest bucket: no value is shared by more cells
 };
 
 // Counters -> packed (start | size << 16) per bucket.  Thread t takes the P
@@ -268,7 +269,7 @@ FCB_DEV bool spread_place(uint32_t (&key)[4 * V], const SpreadLayout<NT, V>& L, 
   if (kmin == kInvalidKey32) {  // no valid cell
     T.m = 0;
     T.heavy = false;
-    T.range = 0u;
+    T.range = T.largest = 0u;
 #pragma unroll
     for (int c = 0; c < C; ++c) W[c] = 0u;
     if (tid < 4) reinterpret_cast<unsigned long long*>(sm + L.mem)[tid] = ~0ull;
@@ -322,6 +323,7 @@ FCB_DEV bool spread_place(uint32_t (&key)[4 * V], const SpreadLayout<NT, V>& L, 
     return false;
   }
   T.heavy = ct.largest > kSpreadHeavy;
+  T.largest = ct.largest;
   scatter_cells<NT, V>(key, range, T.m, L, sm, W);
   return true;
 }
