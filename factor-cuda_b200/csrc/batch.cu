@@ -204,10 +204,13 @@ int occupancy(const fcb_batch& b, int k, int* occ) {
 // f32 panels: the kernel variant of a panel of width N under the current
 // configuration (a panel may be served by a wider variant than it needs).
 int variant_of(const fcb_batch& b, int N) {
-  if (N <= std::min(b.cfg.nt_small_max, ric_variant_cap(1))) return N <= ric_variant_cap(0) ? 0 : 1;
-  if (N <= std::min(b.cfg.nt_mid_max, ric_variant_cap(3))) return N <= ric_variant_cap(2) ? 2 : 3;
-  if (N <= ric_variant_cap(4)) return 4;
-  return 5;
+  int k = 0;
+  for (; k < kRicVariants - 1; ++k) {
+    const int cap = ric_variant_cap(k);
+    const int limit = cap <= 2048 ? b.cfg.nt_small_max : cap <= 5120 ? b.cfg.nt_mid_max : cap;
+    if (N <= cap && N <= limit) break;
+  }
+  return k;
 }
 
 // f32 panels: per variant, the panel descriptors (order 1: widest work

@@ -22,7 +22,7 @@ constexpr int kRadix = 1 << kRadixBits;
 // Shared-memory words the sorter needs besides the key/index buffers.
 template <int NT>
 struct SortScratch {
-  static_assert(NT >= 256 && NT % 32 == 0, "one thread per digit is needed");
+  static_assert(NT % 32 == 0, "whole warps");
   static constexpr int NW = NT / 32;
   static constexpr size_t hist_bytes = size_t(NW) * kRadix * sizeof(uint16_t);
   static constexpr size_t base_bytes = size_t(kRadix) * sizeof(uint32_t);
@@ -108,21 +108,31 @@ FCB_DEV void radix_pass(const K* __restrict__ ks, const uint16_t* __restrict__ i
     }
   }
   __syncthreads();
-  uint32_t tot = 0;
-  if (threadIdx.x < kRadix) {
-    const int d = threadIdx.x;
-    uint32_t run = 0;
+  constexpr int DPT = (kRadix + NT - 1) / NT;  // digits per thread
+  uint32_t tot[DPT], all = 0;
 #pragma unroll
-    for (int ww = 0; ww < NW; ++ww) {
-      const uint32_t c = whist[ww * kRadix + d];
-      whist[ww * kRadix + d] = static_cast<uint16_t>(run);
-      run += c;
+  for (int q = 0; q < DPT; ++q) {
+    tot[q] = 0;
+    const int d = threadIdx.x * DPT + q;
+    if (d < kRadix) {
+      uint32_t run = 0;
+#pragma unroll
+      for (int ww = 0; ww < NW; ++ww) {
+        const uint32_t c = whist[ww * kRadix + d];
+        whist[ww * kRadix + d] = static_cast<uint16_t>(run);
+        run += c;
+      }
+      tot[q] = run;
     }
-    tot = run;
+    all += tot[q];
   }
   uint32_t total;
-  const uint32_t ex = block_exclusive_sum(tot, scan, total);
-  if (threadIdx.x < kRadix) dbase[threadIdx.x] = ex;
+  uint32_t ex = block_exclusive_sum(all, scan, total);
+#pragma unroll
+  for (int q = 0; q < DPT; ++q) {
+    if (threadIdx.x * DPT + q < kRadix) dbase[threadIdx.x * DPT + q] = ex;
+    ex += tot[q];
+  }
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < MAXIPT; ++k) {

@@ -240,7 +240,7 @@ bool ric_items_fit(int N);
 // Batched form: the panels of one size variant (variant v serves N up to
 // ric_variant_cap(v)) in one returns launch and one rank launch; items are a
 // panel's dates (returns pass) or its (date, factor) sections, in panel order.
-constexpr int kRicVariants = 6;
+constexpr int kRicVariants = 9;
 int ric_variant_cap(int variant);
 struct RicPanel {
   RankIcArgs<float, float> a;

@@ -748,18 +748,21 @@ cudaError_t ric_batch_launch(const RicBatchVariant& v, cudaStream_t st) {
 }  // namespace
 
 int ric_variant_cap(int variant) {
-  static const int caps[kRicVariants] = {1024, 2048, 3072, 5120, 8192, 16384};
+  static const int caps[kRicVariants] = {512, 768, 1024, 1536, 2048, 3072, 5120, 8192, 16384};
   return (variant >= 0 && variant < kRicVariants) ? caps[variant] : 0;
 }
 
 cudaError_t launch_rank_ic_items_batch(int variant, const RicBatchVariant& v, cudaStream_t st) {
   if (v.np < 1 || v.items < 1 || v.maxN > ric_variant_cap(variant)) return cudaErrorInvalidValue;
   switch (variant) {
-    case 0: return ric_batch_launch<256, 1>(v, st);
-    case 1: return ric_batch_launch<256, 2>(v, st);
-    case 2: return ric_batch_launch<384, 2>(v, st);
-    case 3: return ric_batch_launch<448, 3>(v, st);
-    case 4: return ric_batch_launch<512, 4>(v, st);
+    case 0: return ric_batch_launch<128, 1>(v, st);
+    case 1: return ric_batch_launch<192, 1>(v, st);
+    case 2: return ric_batch_launch<256, 1>(v, st);
+    case 3: return ric_batch_launch<192, 2>(v, st);
+    case 4: return ric_batch_launch<256, 2>(v, st);
+    case 5: return ric_batch_launch<256, 3>(v, st);
+    case 6: return ric_batch_launch<448, 3>(v, st);
+    case 7: return ric_batch_launch<512, 4>(v, st);
     default: return ric_batch_launch<1024, 4>(v, st);
   }
 }
@@ -769,14 +772,9 @@ bool ric_items_fit(int N) { return N >= 1 && N <= kSmemRankCap; }
 cudaError_t launch_rank_ic_items(const RankIcArgs<float, float>& a, RicPrep rp, bool learned, cudaStream_t st) {
   if (!ric_items_fit(a.N) || a.rank_f_out != nullptr || a.rank_r_out != nullptr) return cudaErrorInvalidValue;
   if (learned && (a.cdf_table == nullptr || a.cdf_zrange == nullptr)) return cudaErrorInvalidValue;
-  if (a.N <= 1024) return ric_launch<256, 1>(a, rp, learned, st);
-  if (a.N <= 2048) return ric_launch<256, 2>(a, rp, learned, st);
-  if (a.N <= 3072) return ric_launch<384, 2>(a, rp, learned, st);
-  if (a.N <= 4096) return ric_launch<512, 2>(a, rp, learned, st);
-  if (a.N <= 5376) return ric_launch<448, 3>(a, rp, learned, st);
-  if (a.N <= 6144) return ric_launch<512, 3>(a, rp, learned, st);
-  if (a.N <= 8192) return ric_launch<512, 4>(a, rp, learned, st);
-  return ric_launch<1024, 4>(a, rp, learned, st);
+  return section_shape(a.N, [&](auto shape) {
+    return ric_launch<decltype(shape)::kThreads, decltype(shape)::kVectors>(a, rp, learned, st);
+  });
 }
 
 }  // namespace fcb

@@ -354,30 +354,15 @@ cudaError_t pair_launch(const PairArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// Fewer sections than SMs: the most threads a section can use.
-constexpr int kFewSections = 148;
-
-// Block shapes by width, four cells a thread and vector.  Wide keys' radix form
-// takes 20 bytes a cell: from 5376 cells on one CTA fills an SM, which then
-// should have 1024 threads.
+// Wide keys' radix form takes 20 bytes a cell: from 5377 cells on one CTA fills
+// an SM, which then should have 1024 threads.
 template <bool WIDE>
 cudaError_t pair_by_width(const PairArgs& a, cudaStream_t st) {
-  const int N = a.N;
-  if (static_cast<long long>(a.T) * a.F <= kFewSections && N > 1024) {
-    if (N <= 4096) return pair_launch<1024, 1, WIDE>(a, st);
-    if (N <= 8192) return pair_launch<1024, 2, WIDE>(a, st);
-    return pair_launch<1024, 4, WIDE>(a, st);
-  }
-  if (N <= 1024) return pair_launch<256, 1, WIDE>(a, st);
-  if (N <= 2048) return pair_launch<256, 2, WIDE>(a, st);
-  if (N <= 4096) return pair_launch<512, 2, WIDE>(a, st);
-  if (N <= 5376) return pair_launch<448, 3, WIDE>(a, st);
-  if constexpr (WIDE) {
-    if (N <= 8192) return pair_launch<1024, 2, WIDE>(a, st);
-  } else {
-    if (N <= 8192) return pair_launch<512, 4, WIDE>(a, st);
-  }
-  return pair_launch<1024, 4, WIDE>(a, st);
+  auto go = [&](auto shape) {
+    return pair_launch<decltype(shape)::kThreads, decltype(shape)::kVectors, WIDE>(a, st);
+  };
+  const bool few = static_cast<long long>(a.T) * a.F <= kFewSections || (WIDE && a.N > 5376);
+  return few ? section_shape_few(a.N, go) : section_shape(a.N, go);
 }
 }  // namespace
 

@@ -363,51 +363,26 @@ cudaError_t pscan_launch(const float* X, const uint8_t* mask, int T, int N, Scan
 }  // namespace
 
 
-// Up to one date per SM the CTAs do not share SMs: wider CTAs shorten each
-// (one date of 5000 takes 17 us a call, most of it on the host).  Above that,
-// the narrowest CTA whose registers hold the row, two or more per SM:
-// at N = 5000 448 x 3 vectors takes 47 us per 1218 dates (the bare kernel)
-// against 51 for 512 x 3, 58 for 256 x 5 and 78 for 1024 x 2.
-constexpr int kFewDates = 148;
-
 // The per-date rank kernels stage nothing through mbarriers, so `status` has
 // nothing to report; it is kept for the callers' uniform interface.
 cudaError_t launch_cs_rank(const float* X, const uint8_t* mask, int T, int N, int desc, float* out, int* status,
                            cudaStream_t st) {
   (void)status;
   if (N < 1 || N > kSmemRankCap) return cudaErrorInvalidValue;
-  if (T <= kFewDates) {
-    if (N <= 4096) return csr_launch<1024, 1>(X, mask, T, N, desc, out, st);
-    if (N <= 8192) return csr_launch<1024, 2>(X, mask, T, N, desc, out, st);
-    return csr_launch<1024, 4>(X, mask, T, N, desc, out, st);
-  }
-  if (N <= 1024) return csr_launch<256, 1>(X, mask, T, N, desc, out, st);
-  if (N <= 2048) return csr_launch<256, 2>(X, mask, T, N, desc, out, st);
-  if (N <= 3072) return csr_launch<384, 2>(X, mask, T, N, desc, out, st);
-  if (N <= 4096) return csr_launch<512, 2>(X, mask, T, N, desc, out, st);
-  if (N <= 5376) return csr_launch<448, 3>(X, mask, T, N, desc, out, st);
-  if (N <= 6144) return csr_launch<512, 3>(X, mask, T, N, desc, out, st);
-  if (N <= 8192) return csr_launch<512, 4>(X, mask, T, N, desc, out, st);
-  return csr_launch<1024, 4>(X, mask, T, N, desc, out, st);
+  auto go = [&](auto shape) {
+    return csr_launch<decltype(shape)::kThreads, decltype(shape)::kVectors>(X, mask, T, N, desc, out, st);
+  };
+  return T <= kFewSections ? section_shape_few(N, go) : section_shape(N, go);
 }
 
 cudaError_t launch_param_scan(const float* X, const uint8_t* mask, int T, int N, ScanOut outs, int* status,
                               cudaStream_t st) {
   (void)status;
   if (N < 1 || N > kSmemRankCap) return cudaErrorInvalidValue;
-  if (T <= kFewDates) {
-    if (N <= 4096) return pscan_launch<1024, 1>(X, mask, T, N, outs, st);
-    if (N <= 8192) return pscan_launch<1024, 2>(X, mask, T, N, outs, st);
-    return pscan_launch<1024, 4>(X, mask, T, N, outs, st);
-  }
-  if (N <= 1024) return pscan_launch<256, 1>(X, mask, T, N, outs, st);
-  if (N <= 2048) return pscan_launch<256, 2>(X, mask, T, N, outs, st);
-  if (N <= 3072) return pscan_launch<384, 2>(X, mask, T, N, outs, st);
-  if (N <= 4096) return pscan_launch<512, 2>(X, mask, T, N, outs, st);
-  if (N <= 5376) return pscan_launch<448, 3>(X, mask, T, N, outs, st);
-  if (N <= 6144) return pscan_launch<512, 3>(X, mask, T, N, outs, st);
-  if (N <= 8192) return pscan_launch<512, 4>(X, mask, T, N, outs, st);
-  return pscan_launch<1024, 4>(X, mask, T, N, outs, st);
+  auto go = [&](auto shape) {
+    return pscan_launch<decltype(shape)::kThreads, decltype(shape)::kVectors>(X, mask, T, N, outs, st);
+  };
+  return T <= kFewSections ? section_shape_few(N, go) : section_shape(N, go);
 }
 
 

@@ -47,6 +47,47 @@ constexpr uint32_t kSpreadHeavy = 16;
 // fraction of it is a cluster far narrower than its range.
 constexpr uint32_t kSpreadBinShare = 8;
 
+// One block shape: NT threads with V vectors of four cells each.
+template <int NT, int V>
+struct SectionShape {
+  static constexpr int kThreads = NT, kVectors = V, kCap = 4 * NT * V;
+};
+
+// Calls go(SectionShape<NT, V>{}) with the block shape for sections of N cells,
+// many of them.  A section takes the same time however many of its block's
+// cells it fills, and two vectors of four cells pay from 1025 cells on: in
+// units of cells, rank + IC takes 71 ps per cell of capacity at 256 threads x 1
+// vector, 74 at 512 cells, 95 at 1024 x 4.  2 M cells x 8 factors as sections of
+// 250, 500, 768, 1500 and 2500: 0.72 ms -> 0.23, 0.38 -> 0.22, 0.26 -> 0.20,
+// 0.24 -> 0.20, 0.24 -> 0.19, against shapes of 256 x 1 and 2 and 384 x 2 alone.
+template <typename Go>
+auto section_shape(int N, Go&& go) {
+  if (N <= 256) return go(SectionShape<64, 1>{});
+  if (N <= 512) return go(SectionShape<128, 1>{});
+  if (N <= 768) return go(SectionShape<192, 1>{});
+  if (N <= 1024) return go(SectionShape<256, 1>{});
+  if (N <= 1536) return go(SectionShape<192, 2>{});
+  if (N <= 2048) return go(SectionShape<256, 2>{});
+  if (N <= 2560) return go(SectionShape<320, 2>{});
+  if (N <= 3072) return go(SectionShape<256, 3>{});
+  if (N <= 4096) return go(SectionShape<512, 2>{});
+  if (N <= 5376) return go(SectionShape<448, 3>{});
+  if (N <= 6144) return go(SectionShape<512, 3>{});
+  if (N <= 8192) return go(SectionShape<512, 4>{});
+  return go(SectionShape<1024, 4>{});
+}
+
+// Up to one section per SM the CTAs do not share SMs: wider CTAs shorten each
+// (one date of 5000 takes 17 us a call, most of it on the host).
+constexpr int kFewSections = 148;
+template <typename Go>
+auto section_shape_few(int N, Go&& go) {
+  if (N <= 1024) return section_shape(N, go);
+  if (N <= 4096) return go(SectionShape<1024, 1>{});
+  if (N <= 8192) return go(SectionShape<1024, 2>{});
+  return go(SectionShape<1024, 4>{});
+}
+
 template <int NT, int V>
 struct SpreadLayout {
   static constexpr int K = 2 * NT;  // bins: two per thread
