@@ -2,10 +2,11 @@
 //
 // Rank + IC of f32 panels: the per-(date, factor) kernels of the single-panel
 // entry points in batched form.  Panels are grouped by the kernel variant
-// their width needs (N up to 1024 / 2048 / 3072 / 5120 / 8192 / 16384; how far
-// the narrow and the middle ones reach is tunable), and each variant is one
+// their width needs (ric_variant_cap: N up to 512 ... 16384; how far the narrow
+// and the middle ones reach is tunable), and each variant is one
 // returns-preparation launch over all its panels' dates and one rank launch
-// over all their (date, factor) sections -- the same device bodies, so results
+// over all their (date, factor) sections (the preparations run ahead on a
+// branch of their own) -- the same device bodies, so results
 // are those of the single-panel calls bit for bit.  A panel's CDF model changes
 // nothing here: the value-spread buckets rank its sections faster than the
 // model's do, with the same results.
@@ -104,7 +105,7 @@ struct fcb_batch {
   size_t cls_smem[kClasses] = {};
   double cls_work[kClasses] = {};
   cudaStream_t s[kClasses] = {};
-  cudaEvent_t ev_fork = nullptr, ev_join[kClasses] = {}, ev_t0 = nullptr, ev_t1 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join[kClasses] = {}, ev_prep[kRicVariants] = {}, ev_t0 = nullptr, ev_t1 = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   bool dirty = true;
@@ -139,6 +140,10 @@ struct fcb_batch {
       if (ev_join[k] != nullptr) cudaEventDestroy(ev_join[k]);
       s[k] = nullptr;
       ev_join[k] = nullptr;
+    }
+    for (int k = 0; k < kRicVariants; ++k) {
+      if (ev_prep[k] != nullptr) cudaEventDestroy(ev_prep[k]);
+      ev_prep[k] = nullptr;
     }
     if (ev_fork != nullptr) cudaEventDestroy(ev_fork);
     if (ev_t0 != nullptr) cudaEventDestroy(ev_t0);
@@ -352,7 +357,11 @@ int enqueue(fcb_batch& b, cudaStream_t s0) {
   for (int k = 1; k < kClasses; ++k) FCB_BTRY(cudaStreamWaitEvent(b.s[k], b.ev_fork, 0));
   for (int k = 0; k < kRicVariants && b.dtx == FCB_DTYPE_F32; ++k) {
     if (b.var[k].np == 0) continue;
+    // the short returns passes fill the tails of the rank launches before theirs
     cudaStream_t st = (b.cfg.concurrent && k > 0) ? b.s[std::min(k, kClasses - 1)] : s0;
+    FCB_BTRY(launch_rank_ic_prep_batch(k, b.var[k], b.s[1]));
+    FCB_BTRY(cudaEventRecord(b.ev_prep[k], b.s[1]));
+    FCB_BTRY(cudaStreamWaitEvent(st, b.ev_prep[k], 0));
     FCB_BTRY(launch_rank_ic_items_batch(k, b.var[k], st));
   }
   for (int k = 0; k < kClasses && b.dtx != FCB_DTYPE_F32; ++k) {
@@ -509,6 +518,8 @@ extern "C" int fcb_batch_create(const fcb_panel* panels, int npanels, int dtype_
     e = cudaStreamCreateWithFlags(&b->s[k], cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join[k], cudaEventDisableTiming);
   }
+  for (int k = 0; k < kRicVariants && e == cudaSuccess; ++k)
+    e = cudaEventCreateWithFlags(&b->ev_prep[k], cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev_t0);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev_t1);

@@ -252,6 +252,7 @@ struct RicBatchVariant {
   const int* off_items;    // device, exclusive prefix of the panels' T*F (np entries)
   int np, dates, items, maxN;
 };
+cudaError_t launch_rank_ic_prep_batch(int variant, const RicBatchVariant& v, cudaStream_t st);
 cudaError_t launch_rank_ic_items_batch(int variant, const RicBatchVariant& v, cudaStream_t st);
 // Rank + IC of F >= 1 f32 factor panels against one f32 returns panel: the
 // returns pass, then one CTA per (date, factor) -- value-spread buckets, or

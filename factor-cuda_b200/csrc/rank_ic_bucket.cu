@@ -734,16 +734,31 @@ RicPrep ric_prep_carve(void* base, int T, int N, int F) {
 
 namespace {
 template <int NT, int V>
-cudaError_t ric_batch_launch(const RicBatchVariant& v, cudaStream_t st) {
+cudaError_t ric_batch_launch(const RicBatchVariant& v, bool prep, cudaStream_t st) {
   const size_t smem = ric_smem<NT, V>(v.maxN);
   if (smem > kMaxSmemPerBlock || v.maxN > 4 * NT * V) return cudaErrorInvalidValue;
-  cudaError_t e = set_smem(k_ric_prep_batch<NT, V>, smem);
+  const cudaError_t e = prep ? set_smem(k_ric_prep_batch<NT, V>, smem) : set_smem(k_ric_items_batch<NT, V>, smem);
   if (e != cudaSuccess) return e;
-  k_ric_prep_batch<NT, V><<<v.dates, NT, smem, st>>>(v.panels, v.off_dates, v.np);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = set_smem(k_ric_items_batch<NT, V>, smem)) != cudaSuccess) return e;
-  k_ric_items_batch<NT, V><<<v.items, NT, smem, st>>>(v.panels, v.off_items, v.np);
+  if (prep)
+    k_ric_prep_batch<NT, V><<<v.dates, NT, smem, st>>>(v.panels, v.off_dates, v.np);
+  else
+    k_ric_items_batch<NT, V><<<v.items, NT, smem, st>>>(v.panels, v.off_items, v.np);
   return cudaGetLastError();
+}
+
+cudaError_t ric_batch(int variant, const RicBatchVariant& v, bool prep, cudaStream_t st) {
+  if (v.np < 1 || v.items < 1 || v.maxN > ric_variant_cap(variant)) return cudaErrorInvalidValue;
+  switch (variant) {
+    case 0: return ric_batch_launch<128, 1>(v, prep, st);
+    case 1: return ric_batch_launch<192, 1>(v, prep, st);
+    case 2: return ric_batch_launch<256, 1>(v, prep, st);
+    case 3: return ric_batch_launch<192, 2>(v, prep, st);
+    case 4: return ric_batch_launch<256, 2>(v, prep, st);
+    case 5: return ric_batch_launch<256, 3>(v, prep, st);
+    case 6: return ric_batch_launch<448, 3>(v, prep, st);
+    case 7: return ric_batch_launch<512, 4>(v, prep, st);
+    default: return ric_batch_launch<1024, 4>(v, prep, st);
+  }
 }
 }  // namespace
 
@@ -752,19 +767,11 @@ int ric_variant_cap(int variant) {
   return (variant >= 0 && variant < kRicVariants) ? caps[variant] : 0;
 }
 
+cudaError_t launch_rank_ic_prep_batch(int variant, const RicBatchVariant& v, cudaStream_t st) {
+  return ric_batch(variant, v, true, st);
+}
 cudaError_t launch_rank_ic_items_batch(int variant, const RicBatchVariant& v, cudaStream_t st) {
-  if (v.np < 1 || v.items < 1 || v.maxN > ric_variant_cap(variant)) return cudaErrorInvalidValue;
-  switch (variant) {
-    case 0: return ric_batch_launch<128, 1>(v, st);
-    case 1: return ric_batch_launch<192, 1>(v, st);
-    case 2: return ric_batch_launch<256, 1>(v, st);
-    case 3: return ric_batch_launch<192, 2>(v, st);
-    case 4: return ric_batch_launch<256, 2>(v, st);
-    case 5: return ric_batch_launch<256, 3>(v, st);
-    case 6: return ric_batch_launch<448, 3>(v, st);
-    case 7: return ric_batch_launch<512, 4>(v, st);
-    default: return ric_batch_launch<1024, 4>(v, st);
-  }
+  return ric_batch(variant, v, false, st);
 }
 
 bool ric_items_fit(int N) { return N >= 1 && N <= kSmemRankCap; }
