@@ -105,47 +105,81 @@ FCB_DEV void flush_queue(RegWarp<FP>& w, int n, int F) {
   __syncwarp();
 }
 
-// Row values of a thread: element (r, f) at X[r * sr + f * sf].
+// The rows of a warp's next kStages - 1 steps are on their way to shared memory
+// (cp.async) while it works on the current ones: two warps per SM quadrant hide
+// no memory latency by themselves.  A lane copies and reads its own row only, so
+// no barrier is needed.  Element (r, f) is X[r * sr + f * sf].
+constexpr int kStages = 4;
+
 template <typename TIN, int FP, bool ROWS>
-struct RowLoad {
-  TIN x[FP];
-  uint32_t mask;
-  FCB_DEV void get(const TIN* __restrict__ X, const uint8_t* __restrict__ m, long long r, long long r1, int F,
-                   long long sf) {
-    mask = 0u;
+struct RowRing {
+  static constexpr int VL = 16 / static_cast<int>(sizeof(TIN));  // values per 16 bytes
+  static constexpr bool kWhole = ROWS && FP % VL == 0;           // 16-byte pieces when F == FP and X is aligned
+  static constexpr size_t kStage = size_t(32) * FP * sizeof(TIN), kBytes = kStages * kStage;
+  const TIN* X;
+  long long sf, r1;
+  int F;
+  bool pieces;
+  uint8_t* mem;  // this lane's first piece or value of stage 0
+
+  FCB_DEV RowRing(const TIN* X_, long long sf_, long long r1_, int F_, uint8_t* ring)
+      : X(X_), sf(sf_), r1(r1_), F(F_) {
+    pieces = kWhole && F == FP && (reinterpret_cast<uintptr_t>(X) & 15u) == 0;
+    mem = ring + lane_id() * (pieces ? 16u : static_cast<unsigned>(sizeof(TIN)));
+  }
+  // Row r into stage s (nothing beyond the last row: its values are not used).
+  FCB_DEV void fetch(int s, long long r) {
+    if (r < r1) {
+      const uint32_t dst = smem_u32(mem + s * kStage);
+      if (kWhole && pieces) {
+        const TIN* p = X + r * F;
 #pragma unroll
-    for (int f = 0; f < FP; ++f) x[f] = TIN(0);
-    if (r >= r1) return;
-    mask = m != nullptr ? __ldg(m + r) : 1u;
-    if (ROWS) {
-      const TIN* p = X + r * F;
-      constexpr int VL = 16 / static_cast<int>(sizeof(TIN));  // values per 16 bytes
-      if (FP % VL == 0 && F == FP && (reinterpret_cast<uintptr_t>(X) & 15u) == 0) {
-#pragma unroll
-        for (int f = 0; f < FP; f += VL) {
-          const uint4 q = __ldg(reinterpret_cast<const uint4*>(p + f));
-          if constexpr (sizeof(TIN) == 4) {
-            x[f] = __uint_as_float(q.x);
-            x[f + 1] = __uint_as_float(q.y);
-            x[f + 2] = __uint_as_float(q.z);
-            x[f + 3] = __uint_as_float(q.w);
-          } else {
-            x[f] = __hiloint2double(static_cast<int>(q.y), static_cast<int>(q.x));
-            x[f + 1] = __hiloint2double(static_cast<int>(q.w), static_cast<int>(q.z));
-          }
-        }
+        for (int c = 0; c < FP / VL; ++c)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + c * 512), "l"(p + c * VL) : "memory");
       } else {
+        const TIN* p = ROWS ? X + r * F : X + r;
 #pragma unroll
         for (int f = 0; f < FP; ++f)
-          if (f < F) x[f] = __ldg(p + f);
+          if (f < F)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                             dst + f * 32 * static_cast<int>(sizeof(TIN))),
+                         "l"(p + (ROWS ? static_cast<long long>(f) : f * sf)), "n"(sizeof(TIN))
+                         : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // The values of the oldest row in flight, which is in stage s.
+  FCB_DEV void take(int s, TIN (&x)[FP]) const {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    const uint8_t* src = mem + s * kStage;
+    if (kWhole && pieces) {
+#pragma unroll
+      for (int f = 0; f < FP; f += VL) {
+        const uint4 q = *reinterpret_cast<const uint4*>(src + f / VL * 512);
+        if constexpr (sizeof(TIN) == 4) {
+          x[f] = __uint_as_float(q.x);
+          if (f + 1 < FP) x[f + 1] = __uint_as_float(q.y);
+          if (f + 2 < FP) x[f + 2] = __uint_as_float(q.z);
+          if (f + 3 < FP) x[f + 3] = __uint_as_float(q.w);
+        } else {
+          x[f] = __hiloint2double(static_cast<int>(q.y), static_cast<int>(q.x));
+          if (f + 1 < FP) x[f + 1] = __hiloint2double(static_cast<int>(q.w), static_cast<int>(q.z));
+        }
       }
     } else {
 #pragma unroll
       for (int f = 0; f < FP; ++f)
-        if (f < F) x[f] = __ldg(X + f * sf + r);
+        x[f] = f < F ? *reinterpret_cast<const TIN*>(src + f * 32 * sizeof(TIN)) : TIN(0);
     }
   }
 };
+
+// The warps' queues and their sums, before the rings.
+template <int FP>
+__host__ __device__ constexpr size_t reg_sums_bytes() {
+  return (kRegWarps * (sizeof(RegWarp<FP>) + (RegShape<FP>::kSums + 1) * sizeof(double)) + 15) / 16 * 16;
+}
 
 // Rows [bx * rows_per_block, ...) of the pool into part + bx * 4 Fp^2.
 template <typename TIN, int FP, bool ROWS>
@@ -172,18 +206,29 @@ FCB_DEV void gram_reg_body(const TIN* __restrict__ X, const uint8_t* __restrict_
   uint32_t rows = 0u;  // rows with some valid factor (this warp's, uniform)
   int queued = 0;
   const long long r0 = bx * rows_per_block, r1 = min(R, r0 + rows_per_block);
-  RowLoad<TIN, FP, ROWS> next;
-  next.get(X, mask, r0 + tid, r1, F, sf);
+  RowRing<TIN, FP, ROWS> ring(X, sf, r1, F,
+                              smem + reg_sums_bytes<FP>() + wi * RowRing<TIN, FP, ROWS>::kBytes);
+  auto mask_of = [&](long long r) { return r < r1 ? (mask != nullptr ? __ldg(mask + r) : 1u) : 0u; };
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) ring.fetch(s, r0 + tid + s * kRegThreads);
+  uint32_t next_mask = mask_of(r0 + tid);
+  int stage = 0;
   for (long long rb = r0; rb < r1; rb += kRegThreads) {
-    const RowLoad<TIN, FP, ROWS> cur = next;
-    if (rb + kRegThreads < r1) next.get(X, mask, rb + kRegThreads + tid, r1, F, sf);
+    const uint32_t cur_mask = next_mask;
+    next_mask = mask_of(rb + kRegThreads + tid);
     uint32_t v = 0u;
     double x[FP];
+    {
+      TIN raw[FP];
+      ring.take(stage, raw);
+      ring.fetch((stage + kStages - 1) % kStages, rb + tid + (kStages - 1) * kRegThreads);
+      stage = (stage + 1) % kStages;
 #pragma unroll
-    for (int f = 0; f < FP; ++f) {
-      const bool ok = f < F && cur.mask != 0u && KeyOf<TIN>::finite(cur.x[f]);
-      x[f] = ok ? static_cast<double>(cur.x[f]) - shift[f] : 0.0;
-      v |= ok ? 1u << f : 0u;
+      for (int f = 0; f < FP; ++f) {
+        const bool ok = f < F && cur_mask != 0u && KeyOf<TIN>::finite(raw[f]);
+        x[f] = ok ? static_cast<double>(raw[f]) - shift[f] : 0.0;
+        v |= ok ? 1u << f : 0u;
+      }
     }
     const unsigned some = __ballot_sync(kFull, v != 0u);
     rows += __popc(some);
@@ -243,10 +288,9 @@ FCB_DEV void gram_reg_body(const TIN* __restrict__ X, const uint8_t* __restrict_
   }
 }
 
-template <int FP>
+template <typename TIN, int FP>
 constexpr size_t reg_smem() {
-  using S = RegShape<FP>;
-  return kRegWarps * (sizeof(RegWarp<FP>) + (S::kSums + 1) * sizeof(double));
+  return reg_sums_bytes<FP>() + kRegWarps * RowRing<TIN, FP, true>::kBytes;
 }
 
 template <typename TIN, int FP, bool ROWS>
@@ -278,9 +322,9 @@ cudaError_t reg_launch(const TIN* X, const uint8_t* mask, long long R, int F, bo
                        long long rpb, int nblk, const FcColStat* st, double* part, cudaStream_t s) {
   auto go = [&](auto kernel) -> cudaError_t {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(reg_smem<FP>()));
+                                               static_cast<int>(reg_smem<TIN, FP>()));
     if (e != cudaSuccess) return e;
-    kernel<<<nblk, kRegThreads, reg_smem<FP>(), s>>>(X, mask, R, F, sf, Fp, rpb, st, part);
+    kernel<<<nblk, kRegThreads, reg_smem<TIN, FP>(), s>>>(X, mask, R, F, sf, Fp, rpb, st, part);
     return cudaGetLastError();
   };
   return rows ? go(k_fc_gram_reg<TIN, FP, true>) : go(k_fc_gram_reg<TIN, FP, false>);
@@ -322,11 +366,11 @@ cudaError_t launch_fc_gram_reg_batch(int kind, int dtype, const FcBatchPanel* pa
   };
   const bool f32 = dtype == 0;
   switch (kind) {
-    case 0: return f32 ? go(k_fcb_gram_reg<float, 4>, reg_smem<4>()) : go(k_fcb_gram_reg<double, 4>, reg_smem<4>());
-    case 1: return f32 ? go(k_fcb_gram_reg<float, 6>, reg_smem<6>()) : go(k_fcb_gram_reg<double, 6>, reg_smem<6>());
-    case 2: return f32 ? go(k_fcb_gram_reg<float, 8>, reg_smem<8>()) : go(k_fcb_gram_reg<double, 8>, reg_smem<8>());
-    case 3: return f32 ? go(k_fcb_gram_reg<float, 10>, reg_smem<10>()) : go(k_fcb_gram_reg<double, 10>, reg_smem<10>());
-    default: return f32 ? go(k_fcb_gram_reg<float, 12>, reg_smem<12>()) : go(k_fcb_gram_reg<double, 12>, reg_smem<12>());
+    case 0: return f32 ? go(k_fcb_gram_reg<float, 4>, reg_smem<float, 4>()) : go(k_fcb_gram_reg<double, 4>, reg_smem<double, 4>());
+    case 1: return f32 ? go(k_fcb_gram_reg<float, 6>, reg_smem<float, 6>()) : go(k_fcb_gram_reg<double, 6>, reg_smem<double, 6>());
+    case 2: return f32 ? go(k_fcb_gram_reg<float, 8>, reg_smem<float, 8>()) : go(k_fcb_gram_reg<double, 8>, reg_smem<double, 8>());
+    case 3: return f32 ? go(k_fcb_gram_reg<float, 10>, reg_smem<float, 10>()) : go(k_fcb_gram_reg<double, 10>, reg_smem<double, 10>());
+    default: return f32 ? go(k_fcb_gram_reg<float, 12>, reg_smem<float, 12>()) : go(k_fcb_gram_reg<double, 12>, reg_smem<double, 12>());
   }
 }
 
