@@ -10,8 +10,8 @@
 // rows on which j is missing.  Rows with no valid factor add nothing, and rows
 // with all of them need no correction; the others (one in ten at 12 factors
 // with 1 % missing cells) go on a queue per warp in shared memory, and the warp
-// adds up a full queue list by list: lanes own (i, j) pairs and walk the rows
-// that miss j.  All sums are formed in a fixed order.
+// adds a full queue to the sums of the factors that its rows miss.  All sums
+// are formed in a fixed order.
 // Per block the same partials come out as from the staged pass
 // (fc_gram_body): P[product][i][j] with product 0 n, 1 sum x'_i over rows where
 // j is valid, 2 sum x'_i^2 likewise, 3 sum x'_i x'_j.
@@ -32,12 +32,10 @@ struct RegShape {
 // One warp's shared memory.
 template <int FP>
 struct RegWarp {
-  double row[kQueue][FP];   // centred values, 0 where invalid
+  double2 row[kQueue][FP / 2];  // centred values, 0 where invalid
+  double2 c[2][FP][FP];         // [half][j][i]: sum x'_i, sum x'_i^2 over the rows that miss j
+  uint32_t cn[2][FP][FP];       // rows where i is valid and j is not; [j][j]: rows that miss j
   uint32_t valid[kQueue];
-  uint8_t list[FP][kQueue]; // queued rows that miss factor j
-  double cx[FP][FP], cq[FP][FP];  // [j][i]: sum x'_i, sum x'_i^2 over the rows that miss j
-  uint32_t cn[FP][FP];            // rows where i is valid and j is not
-  uint32_t miss[FP];              // rows (with some valid factor) that miss j
 };
 
 // Sums of M values over the warp's lanes, spread over the lanes: each step
@@ -66,41 +64,33 @@ constexpr int spread_len() {
   return m;
 }
 
-// Adds the queued rows to the warp's corrections.
+// Adds the n queued rows to the warp's corrections: each half-warp takes every
+// other row, lane i the factor i, and adds it to the sums of the factors that
+// the row misses (one, as a rule).
 template <int FP>
-FCB_DEV void flush_queue(RegWarp<FP>& w, int n, int F) {
-  const int lane = static_cast<int>(lane_id());
+FCB_DEV void flush_queue(RegWarp<FP>& w, int n, uint32_t all) {
+  const int h = static_cast<int>(lane_id() >> 4), i = static_cast<int>(lane_id() & 15u);
   __syncwarp();
-  int len[FP];
-#pragma unroll
-  for (int j = 0; j < FP; ++j) {
-    len[j] = 0;
-    for (int q = 0; q < n; q += 32) {
-      const bool m = q + lane < n && !((w.valid[q + lane] >> j) & 1u) && j < F;
-      const unsigned b = __ballot_sync(kFull, m);
-      if (m) w.list[j][len[j] + __popc(b & lanemask_lt())] = static_cast<uint8_t>(q + lane);
-      len[j] += __popc(b);
+  if (i < FP) {
+    const double* rows = reinterpret_cast<const double*>(w.row);
+    uint32_t valid = h < n ? w.valid[h] : all;
+    double x = h < n ? rows[h * FP + i] : 0.0;
+    for (int r = h; r < n; r += 2) {
+      const uint32_t v = valid;
+      const double y = x;
+      if (r + 2 < n) {
+        valid = w.valid[r + 2];
+        x = rows[(r + 2) * FP + i];
+      }
+      for (uint32_t m = all & ~v; m != 0u; m &= m - 1u) {
+        const int j = __ffs(m) - 1;
+        double2 c = w.c[h][j][i];
+        c.x += y;
+        c.y = fma(y, y, c.y);
+        w.c[h][j][i] = c;
+        w.cn[h][j][i] += i == j ? 1u : (v >> i) & 1u;
+      }
     }
-    if (lane == 0) w.miss[j] += static_cast<uint32_t>(len[j]);
-  }
-  __syncwarp();
-  for (int e = lane; e < FP * FP; e += 32) {
-    const int j = e / FP, i = e % FP;
-    int nj = 0;
-#pragma unroll
-    for (int q = 0; q < FP; ++q) nj = q == j ? len[q] : nj;
-    double a = 0.0, q2 = 0.0;
-    uint32_t c = 0u;
-    for (int k = 0; k < nj; ++k) {
-      const int r = w.list[j][k];
-      const double x = w.row[r][i];
-      a += x;
-      q2 = fma(x, x, q2);
-      c += (w.valid[r] >> i) & 1u;
-    }
-    w.cx[j][i] += a;
-    w.cq[j][i] += q2;
-    w.cn[j][i] += c;
   }
   __syncwarp();
 }
@@ -181,6 +171,9 @@ __host__ __device__ constexpr size_t reg_sums_bytes() {
   return (kRegWarps * (sizeof(RegWarp<FP>) + (RegShape<FP>::kSums + 1) * sizeof(double)) + 15) / 16 * 16;
 }
 
+FCB_DEV bool row_finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+FCB_DEV bool row_finite(double x) { return KeyOf<double>::finite(x); }
+
 // Rows [bx * rows_per_block, ...) of the pool into part + bx * 4 Fp^2.
 template <typename TIN, int FP, bool ROWS>
 FCB_DEV void gram_reg_body(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, long long R, int F,
@@ -190,11 +183,9 @@ FCB_DEV void gram_reg_body(const TIN* __restrict__ X, const uint8_t* __restrict_
   RegWarp<FP>* warps = reinterpret_cast<RegWarp<FP>*>(smem);
   const int tid = static_cast<int>(threadIdx.x), lane = tid & 31, wi = tid >> 5;
   RegWarp<FP>& w = warps[wi];
-  for (int e = lane; e < FP * FP; e += 32) {
-    (&w.cx[0][0])[e] = 0.0;
-    (&w.cq[0][0])[e] = 0.0;
-    (&w.cn[0][0])[e] = 0u;
-    if (e < FP) w.miss[e] = 0u;
+  for (int e = lane; e < 2 * FP * FP; e += 32) {
+    (&w.c[0][0][0])[e] = make_double2(0.0, 0.0);
+    (&w.cn[0][0][0])[e] = 0u;
   }
   const uint32_t all = (1u << F) - 1u;
   double shift[FP];
@@ -225,7 +216,7 @@ FCB_DEV void gram_reg_body(const TIN* __restrict__ X, const uint8_t* __restrict_
       stage = (stage + 1) % kStages;
 #pragma unroll
       for (int f = 0; f < FP; ++f) {
-        const bool ok = f < F && cur_mask != 0u && KeyOf<TIN>::finite(raw[f]);
+        const bool ok = f < F && cur_mask != 0u && row_finite(raw[f]);
         x[f] = ok ? static_cast<double>(raw[f]) - shift[f] : 0.0;
         v |= ok ? 1u << f : 0u;
       }
@@ -244,17 +235,17 @@ FCB_DEV void gram_reg_body(const TIN* __restrict__ X, const uint8_t* __restrict_
       if ((q >> lane) & 1u) {
         const int at = queued + __popc(q & lanemask_lt());
 #pragma unroll
-        for (int f = 0; f < FP; ++f) w.row[at][f] = x[f];
+        for (int f = 0; f < FP; f += 2) w.row[at][f / 2] = make_double2(x[f], x[f + 1]);
         w.valid[at] = v;
       }
       queued += __popc(q);
       if (queued > kQueue - 32) {
-        flush_queue<FP>(w, queued, F);
+        flush_queue<FP>(w, queued, all);
         queued = 0;
       }
     }
   }
-  flush_queue<FP>(w, queued, F);
+  flush_queue<FP>(w, queued, all);
   // the warps' sums meet in shared memory, in warp order
   constexpr int L = spread_len<S::kSums>(), TS = S::kSums + 1;
   double* t0 = reinterpret_cast<double*>(smem + kRegWarps * sizeof(RegWarp<FP>));
@@ -275,10 +266,11 @@ FCB_DEV void gram_reg_body(const TIN* __restrict__ X, const uint8_t* __restrict_
       for (int q = 0; q < kRegWarps; ++q) {
         const RegWarp<FP>& u = warps[q];
         const double* t = t0 + q * TS;
-        n += t[S::kSums] - static_cast<double>(u.miss[i]) - static_cast<double>(u.cn[j][i]);
+        n += t[S::kSums] - static_cast<double>(u.cn[0][i][i] + u.cn[1][i][i]);
+        if (i != j) n -= static_cast<double>(u.cn[0][j][i] + u.cn[1][j][i]);
         sxy += t[kij];
-        sx += t[S::kPairs + i] - u.cx[j][i];
-        sx2 += t[kii] - u.cq[j][i];
+        sx += t[S::kPairs + i] - (u.c[0][j][i].x + u.c[1][j][i].x);
+        sx2 += t[kii] - (u.c[0][j][i].y + u.c[1][j][i].y);
       }
     }
     P[(0 * Fp + i) * Fp + j] = n;
