@@ -309,6 +309,7 @@ extern "C" int fcb_dev_cs_rank_f32(const float* d_x, const uint8_t* d_mask, int 
   if (N > (1 << 24)) return FCB_ERR_CAP2;
   if (static_cast<long long>(T) * N > INT32_MAX) return FCB_ERR_CAP3;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (N > kSmemRankCap && N <= kSliceMaxN) return rc(launch_cs_rank_slices(d_x, d_mask, T, N, desc, d_out, s));
   if (N > kSmemRankCap) {
     // global-memory path; scratch is stream-ordered (no host synchronisation)
     const size_t bytes = rank_global_scratch(rank_global_bytes_per_date(0, N, 1, 4, 4), T);

@@ -161,6 +161,11 @@ cudaError_t launch_param_scan(const float* X, const uint8_t* mask, int T, int N,
 size_t rank_ic_learned_smem(int N);
 cudaError_t launch_rank_ic_learned(const RankIcArgs<float, float>& a, int* status, cudaStream_t st);
 
+// rank_slices.cu: cs_rank of rows above kSmemRankCap, without scratch.
+constexpr int kSliceMaxN = 65536;
+cudaError_t launch_cs_rank_slices(const float* X, const uint8_t* mask, int T, int N, int desc, float* out,
+                                  cudaStream_t st);
+
 // rank_ic_pair.cu: rank + IC of one factor row against one returns row per CTA
 // (any F); true when its shared-memory kernel takes N for these dtypes.
 template <typename TF, typename TR>
