@@ -9,11 +9,11 @@
 // which every CTA finds for itself: any parting gives the same ranks, it only
 // decides how even the slices are.  A slice that holds more cells than a CTA
 // takes (a much repeated value, a sample that does not show the row) is worked
-// off in parts.
+// off in parts, cut at the median of the cells that it could hold.
 //
 // Measured on a B200, against one CTA per row that sorts it in global memory:
-// 4 x 16500 151 -> 26 us, 61 x 20000 182 -> 50, 64 x 40000 340 -> 147, 500 x
-// 17000 594 -> 282.  Rows of a few values only gain at few dates (16 x 20000 111
+// 4 x 16500 151 -> 26 us, 61 x 20000 182 -> 50, 64 x 40000 340 -> 148, 500 x
+// 17000 594 -> 275.  Rows of a few values only gain at few dates (16 x 20000 111
 // -> 55 us) and lose 5 % at 500 x 17000.  What bounds it is instruction issue:
 // ranking the slice, and reading the row R times at about 12 instructions per
 // cell and slice, which is why the form ends at kSliceMaxN; beyond,
@@ -30,10 +30,11 @@ namespace {
 constexpr int kSlNT = 512, kSlV = 2, kSlWarps = kSlNT / 32;
 constexpr int kSlCap = 4 * kSlNT * kSlV;  // cells a CTA ranks at a time
 // Cells of a slice on average.  With s sampled cells a slice, its size varies by
-// 1 / sqrt(s): 12 % at 24576 cells, 24 % at 65536, and the cap stands at least
-// 3 sigma above the mean.  (61 x 20000: 58 us at 2304, 50 at 2900; but 30 x
-// 65000 147 and 581, some slices being worked off in parts.)
-constexpr int slice_mean(int N) { return N <= 24576 ? 2900 : 2304; }
+// 1 / sqrt(s), 16 % at 32768 cells; one above the cap costs its CTA two more
+// passes over the row.  (61 x 20000: 58 us at 2304, 50 at 2900, or 60 where one
+// slice comes out above the cap, one call in ten; 64 x 40000 147 and 133-153;
+// 30 x 65000 149 at 2304.)
+constexpr int slice_mean(int N) { return N <= 32768 ? 2900 : 2304; }
 constexpr int kSlTile = 4 * kSlNT;        // cells per step over the row
 constexpr int kSlSample = 16;             // sampled cells per lane
 
@@ -73,21 +74,17 @@ struct SliceRow {
   }
 };
 
-// Valid cells with a <= key < b.  wt: 32 words; ends with a barrier.
-__device__ __noinline__ uint32_t slice_count(const SliceRow& row, uint32_t a, uint32_t b, uint32_t* wt) {
-  uint32_t n = 0u;
-  for (int i0 = 4 * static_cast<int>(threadIdx.x); i0 < row.N; i0 += kSlTile) {
-    uint32_t k[4];
-    row.four(i0, k);
+// The key of 0-based rank `rank` among a warp's samples, `rank` being below
+// their number: the largest v with no more than `rank` keys below it.
+FCB_DEV uint32_t sample_rank(const uint32_t (&k)[kSlSample], uint32_t rank) {
+  uint32_t v = 0u;
+  for (uint32_t bit = 0x80000000u; bit != 0u; bit >>= 1) {
+    uint32_t c = 0u;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) n += k[q] - a < b - a ? 1u : 0u;
+    for (int q = 0; q < kSlSample; ++q) c += k[q] < (v | bit) ? 1u : 0u;
+    if (__reduce_add_sync(kFull, c) <= rank) v |= bit;
   }
-  n = __reduce_add_sync(kFull, n);
-  if (lane_id() == 0) wt[threadIdx.x >> 5] = n;
-  __syncthreads();
-  n = warps_sum<kSlWarps>(wt);
-  __syncthreads();
-  return n;
+  return v;
 }
 
 enum class Take { kFirst, kList, kTies };
@@ -187,7 +184,7 @@ __global__ void __launch_bounds__(kSlNT, kSmThreads / kSlNT)
   const SpreadLayout<kSlNT, kSlV> L(kSlCap);
   uint32_t* cols = reinterpret_cast<uint32_t*>(sm + S.col);
   uint32_t* keys = reinterpret_cast<uint32_t*>(sm + L.mem);  // read out before the buckets are filled
-  uint32_t* wt = reinterpret_cast<uint32_t*>(sm + S.wt);     // [0, 96) counts, [96, 98) the slice's ends
+  uint32_t* wt = reinterpret_cast<uint32_t*>(sm + S.wt);     // [0, 96) counts, [96, 99) the slice's ends and a cut
   const int t = static_cast<int>(blockIdx.x) / R, r = static_cast<int>(blockIdx.x) % R;
   const int tid = static_cast<int>(threadIdx.x), wi = tid >> 5, lane = tid & 31;
   const size_t at = static_cast<size_t>(t) * N;
@@ -206,36 +203,32 @@ __global__ void __launch_bounds__(kSlNT, kSmThreads / kSlNT)
         ms += k[q] != kInvalidKey32 ? 1u : 0u;
       }
       ms = __reduce_add_sync(kFull, ms);
-      const uint32_t rank = ms * static_cast<uint32_t>(r + wi) / static_cast<uint32_t>(R);
-      for (uint32_t bit = 0x80000000u; bit != 0u; bit >>= 1) {  // the largest v with no more than `rank` keys below
-        uint32_t c = 0u;
-#pragma unroll
-        for (int q = 0; q < kSlSample; ++q) c += k[q] < (v | bit) ? 1u : 0u;
-        if (__reduce_add_sync(kFull, c) <= rank) v |= bit;
-      }
+      // (no valid sample: the first slice takes all cells)
+      v = sample_rank(k, ms * static_cast<uint32_t>(r + wi) / static_cast<uint32_t>(R));
     }
     if (lane == 0) wt[96 + wi] = v;
   }
   __syncthreads();
-  const uint32_t start = wt[96], end = wt[97];
-  uint32_t a = start;
-  uint32_t b = end, below = 0u;
+  uint32_t a = wt[96], below = 0u;
+  const uint32_t end = wt[97];
+  uint32_t b = end;
   uint32_t n = slice_collect<Take::kFirst>(row, a, b, keys, cols, 0u, out, wt, r, R, below);
   for (;;) {  // uniform: the slice, as a rule in one part
     if (n > kSlCap) {
       if (b - a == 1u) {  // one value: ranked by column
         below += slice_collect<Take::kTies>(row, a, b, keys, cols, below, out, wt, r, R, below);
       } else {
-        if (b == end && a == start) {  // a sampled value: much repeated, perhaps
-          b = a + 1u;
-        } else {  // the largest part that fits
-          uint32_t lo = a + 1u, hi = b;  // [a, lo) fits or is one value; [a, hi) does not fit
-          while (hi - lo > 1u) {
-            const uint32_t mid = lo + (hi - lo) / 2u;
-            if (slice_count(row, a, mid, wt) <= kSlCap) lo = mid; else hi = mid;
-          }
-          b = lo;
+        // up to the median of the full list; a value that fills half of it is
+        // thereby taken alone
+        if (wi == 0) {
+          uint32_t k[kSlSample];
+#pragma unroll
+          for (int q = 0; q < kSlSample; ++q) k[q] = keys[(q * 32 + lane) * (kSlCap / (32 * kSlSample))];
+          const uint32_t v = sample_rank(k, 16 * kSlSample);
+          if (lane == 0) wt[98] = max(v, a + 1u);
         }
+        __syncthreads();
+        b = wt[98];
         n = slice_collect<Take::kList>(row, a, b, keys, cols, 0u, out, wt, r, R, below);
         continue;
       }
