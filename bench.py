@@ -698,30 +698,30 @@ def bench_batch(dev, steps=5, warmup=2, tune_cache=None, cpu_sample=True):
                torch.equal(torch.nan_to_num(c, nan=7.0), torch.nan_to_num(p["corr"], nan=7.0)) and
                torch.equal(r.view(torch.int32), p["ranks"][:, :3].view(torch.int32))
                for a, c, r, p in zip(ic_g, corr_g, rk_g, panels))
-    def variant(n):  # the f32 kernel variant a panel of width n runs in (fcb200.h, batched panels)
-        if n <= min(cfg["nt_small_max"], 2048):
-            return 0
-        if n <= min(cfg["nt_mid_max"], 5120):
-            return 1
-        return 2 if n <= 8192 else 3
+    def variant(n):  # the f32 kernel variant a panel of width n runs in (batch.cu, variant_of)
+        caps = (512, 768, 1024, 1536, 2048, 3072, 5120, 8192)
+        for k, cap in enumerate(caps):
+            limit = cfg["nt_small_max"] if cap <= 2048 else cfg["nt_mid_max"] if cap <= 5120 else cap
+            if n <= min(cap, limit):
+                return k
+        return len(caps)
     variants = sorted({variant(p["X"].shape[2]) for p in panels})
     res = {"workload": "64 uneven panels (N ~ U[300,6000], T ~ U[250,2500], F=8, gaps ~ U[0,0.2]): "
                        "cs_rank + rolling_ic(30) + factor_corr per panel",
            "cells": cells, "unit": "Gelem/s",
-           # kernels: per kernel variant, the returns pass, the rank pass over all its
-           # panels and the pass over the sections the learned buckets handed back; for all
-           # panels together, factor_corr's column pass + merge, Gram pass + finalize and the
-           # four fallback kernels (every pool here has 4096 rows or more; they exit at once
-           # when no pair is flagged); the per-panel arm runs, for each panel, those three
-           # rank kernels and the eight factor_corr kernels
+           # kernels: per kernel variant, the returns pass and the rank pass over all its
+           # panels; for all panels together, factor_corr's column pass + merge, Gram pass +
+           # finalize and the four fallback kernels (every pool here has 4096 rows or more;
+           # they exit at once when no pair is flagged); the per-panel arm runs, for each
+           # panel, those two rank kernels and the eight factor_corr kernels
            "method": "learned splitters, one CdfModel (F=8) fitted on panel 0 and shared by every panel",
            "fit_ms": fit_ms,
            "graph": {"ms": ms_graph, "value": cells / (ms_graph / 1e3) / 1e9,
-                     "kernels_per_replay": 3 * len(variants) + 8},
+                     "kernels_per_replay": 2 * len(variants) + 8},
            "graph_radix": {"ms": ms_graph_rx, "value": cells / (ms_graph_rx / 1e3) / 1e9},
            "learned_speedup_vs_radix_graph": ms_graph_rx / ms_graph,
            "per_panel": {"ms": ms_pp, "value": cells / (ms_pp / 1e3) / 1e9,
-                         "kernels_per_step": sum((3 if p["X"].shape[0] >= 2 else 1) + 8 for p in panels)},
+                         "kernels_per_step": sum((2 if p["X"].shape[0] >= 2 else 1) + 8 for p in panels)},
            "speedup_graph_vs_per_panel": ms_pp / ms_graph,
            "bit_exact_graph_vs_per_panel": bool(same),
            "autotune": {"config": cfg, "tuned_ms": tuned_ms, "tuning_s": tune_s, "from_cache": cached}}

@@ -169,14 +169,15 @@ int class_of(const fcb_batch& b, int N) {
 // returns sort) -- what the queue order and the concurrent grid split use.
 double item_work(const fcb_panel& p) { return static_cast<double>(p.N) * (p.F + 1); }
 
-template <typename TF, typename TR>
+// f64 panels: the kernel arguments of every panel.
 int upload_args(fcb_batch& b) {
-  std::vector<RankIcArgs<TF, TR>> a(b.p.size());
+  std::vector<RankIcArgs<double, double>> a(b.p.size());
   for (size_t i = 0; i < b.p.size(); ++i) {
     const fcb_panel& q = b.p[i];
-    RankIcArgs<TF, TR> r{};
-    r.X = static_cast<const TF*>(q.X);
-    r.R = static_cast<const TR*>(q.R);
+    RankIcArgs<double, double>& r = a[i];
+    r = RankIcArgs<double, double>{};
+    r.X = static_cast<const double*>(q.X);
+    r.R = static_cast<const double*>(q.R);
     r.fmask = q.fmask;
     r.rmask = q.rmask;
     r.F = q.F;
@@ -185,25 +186,17 @@ int upload_args(fcb_batch& b) {
     r.min_valid = b.min_valid;
     r.ranks_out = q.ranks_out;
     r.ic_out = q.ic_out;
-    if (q.model != nullptr) {
-      r.cdf_table = q.model->table[q.model->cur];
-      r.cdf_zrange = q.model->zrange[q.model->cur];
-    }
-    r.learn_cap = b.cfg.learn_cap > 0 ? b.cfg.learn_cap : kLearnCapDefault;
-    r.ic_ld = 0;
-    a[i] = r;
   }
-  const size_t bytes = a.size() * sizeof(RankIcArgs<TF, TR>);
+  const size_t bytes = a.size() * sizeof(a[0]);
   if (b.d_args == nullptr) FCB_BTRY(cudaMalloc(&b.d_args, bytes));
   b.args_bytes = bytes;
   FCB_BTRY(cudaMemcpy(b.d_args, a.data(), bytes, cudaMemcpyHostToDevice));
   return FCB_OK;
 }
 
-template <typename TF, typename TR>
-int occupancy(const fcb_batch& b, int k, int* occ) {
-  return rcode(launch_rank_ic_batch<TF, TR>(kClassNt[k], b.learned, static_cast<const RankIcArgs<TF, TR>*>(b.d_args),
-                                            nullptr, 0, nullptr, 0, b.cls_smem[k], nullptr, nullptr, occ));
+int occupancy(const fcb_batch& b, int nt, size_t smem, int* occ) {
+  return rcode(launch_rank_ic_batch(nt, static_cast<const RankIcArgs<double, double>*>(b.d_args), nullptr, 0, nullptr, 0,
+                                    smem, nullptr, nullptr, occ));
 }
 
 // f32 panels: the kernel variant of a panel of width N under the current
@@ -334,11 +327,10 @@ int plan(fcb_batch& b) {
   for (int k = 0; k < kClasses; ++k) {
     b.cls_grid[k] = 0;
     if (b.cls_cnt[k] == 0) continue;
-    b.cls_smem[k] = (b.dtx == FCB_DTYPE_F32) ? rank_ic_batch_smem<float, float>(kClassNt[k], b.cls_maxN[k])
-                                             : rank_ic_batch_smem<double, double>(kClassNt[k], b.cls_maxN[k]);
+    b.cls_smem[k] = rank_ic_batch_smem(kClassNt[k], b.cls_maxN[k]);
     if (b.cls_smem[k] > kMaxSmemPerBlock) return FCB_ERR_UNSUPPORTED;
     int occ = 0;
-    const int r = (b.dtx == FCB_DTYPE_F32) ? occupancy<float, float>(b, k, &occ) : occupancy<double, double>(b, k, &occ);
+    const int r = occupancy(b, kClassNt[k], b.cls_smem[k], &occ);
     if (r != FCB_OK) return r;
     if (occ < 1) return FCB_ERR_UNSUPPORTED;
     if (b.cfg.ctas_per_sm > 0) occ = std::min(occ, b.cfg.ctas_per_sm);
@@ -368,10 +360,8 @@ int enqueue(fcb_batch& b, cudaStream_t s0) {
     if (b.cls_cnt[k] == 0) continue;
     cudaStream_t st = (b.cfg.concurrent && k > 0) ? b.s[k] : s0;
     const int2* items = b.d_items + b.cls_off[k];
-    FCB_BTRY(launch_rank_ic_batch<double, double>(kClassNt[k], false,
-                                                  static_cast<const RankIcArgs<double, double>*>(b.d_args), items,
-                                                  b.cls_cnt[k], b.d_ctr + k, b.cls_grid[k], b.cls_smem[k],
-                                                  b.d_status, st, nullptr));
+    FCB_BTRY(launch_rank_ic_batch(kClassNt[k], static_cast<const RankIcArgs<double, double>*>(b.d_args), items,
+                                  b.cls_cnt[k], b.d_ctr + k, b.cls_grid[k], b.cls_smem[k], b.d_status, st, nullptr));
   }
   // factor_corr of every panel: one batched launch per kernel kind, on the
   // last branch, alongside the rank + IC kernels (it reads only the factor
@@ -390,7 +380,7 @@ int build_graph(fcb_batch& b) {
   b.drop_graph();
   int r = plan(b);
   if (r != FCB_OK) return r;
-  if (b.dtx != FCB_DTYPE_F32 && (r = upload_args<double, double>(b)) != FCB_OK) return r;
+  if (b.dtx != FCB_DTYPE_F32 && (r = upload_args(b)) != FCB_OK) return r;
   FCB_BTRY(cudaStreamBeginCapture(b.s[0], cudaStreamCaptureModeRelaxed));
   r = enqueue(b, b.s[0]);
   cudaGraph_t g = nullptr;
@@ -416,15 +406,8 @@ int bind_device(const fcb_batch& b) {
 // shared memory sized for sections of N cells (0 when it does not fit).
 int occ_at(const fcb_batch& b, int nt, int N, int* occ) {
   *occ = 0;
-  const size_t smem = (b.dtx == FCB_DTYPE_F32) ? rank_ic_batch_smem<float, float>(nt, N)
-                                               : rank_ic_batch_smem<double, double>(nt, N);
-  if (smem > kMaxSmemPerBlock) return FCB_OK;
-  if (b.dtx == FCB_DTYPE_F32)
-    return rcode(launch_rank_ic_batch<float, float>(nt, b.learned,
-                                                    static_cast<const RankIcArgs<float, float>*>(b.d_args), nullptr,
-                                                    0, nullptr, 0, smem, nullptr, nullptr, occ));
-  return rcode(launch_rank_ic_batch<double, double>(nt, false, static_cast<const RankIcArgs<double, double>*>(b.d_args),
-                                                    nullptr, 0, nullptr, 0, smem, nullptr, nullptr, occ));
+  const size_t smem = rank_ic_batch_smem(nt, N);
+  return smem > kMaxSmemPerBlock ? FCB_OK : occupancy(b, nt, smem, occ);
 }
 
 // Class boundaries worth measuring: for each occupancy level block size nt
@@ -485,7 +468,7 @@ extern "C" int fcb_batch_create(const fcb_panel* panels, int npanels, int dtype_
     if (q.N > kSmemRankCap) return FCB_ERR_UNSUPPORTED;
     // the cross-section must fit one CTA's shared memory (largest block size)
     if (dtype_x == FCB_DTYPE_F32 ? !ric_items_fit(q.N)
-                                 : rank_ic_batch_smem<double, double>(1024, q.N) > kMaxSmemPerBlock)
+                                 : rank_ic_batch_smem(1024, q.N) > kMaxSmemPerBlock)
       return FCB_ERR_UNSUPPORTED;
     if (q.corr_out != nullptr && q.F > 128) return FCB_ERR_CAP3;
     if (q.model != nullptr) {
@@ -605,7 +588,7 @@ extern "C" int fcb_batch_create(const fcb_panel* panels, int npanels, int dtype_
       c8 += al(ric_prep_bytes(b->p[i].T, b->p[i].N, b->p[i].F));
     }
   } else {
-    const int r = upload_args<double, double>(*b);
+    const int r = upload_args(*b);
     if (r != FCB_OK) return fail(r);
   }
   *out = b;

@@ -5,14 +5,17 @@
 // numeric contract (|dr| <= 1e-12 against np.corrcoef on the joint subset,
 // compensated sums on reduction-sensitive inputs):
 //
-//  1. column statistics: count, Kahan mean, min / max;
-//  2. a Gram pass on column-centred values: n, sum x', sum y', sum x'y',
+//  1. column statistics of a sample of the rows: the Kahan mean is the shift of
+//     the sums (any shift near the mean serves);
+//  2. a Gram pass on shifted values (in registers up to 12 factors,
+//     factor_gram.cu): n, sum x', sum y', sum x'y',
 //     sum x'^2, sum y'^2 over each pair's joint valid set (the six masked
 //     products of _masked_gemm_stats, fc/_cpu_core.py:139-169);
 //  3. finalize: the cancellation gate of _gemm_cancel_mask (ratio 3 on the
 //     uncentred sums, reconstructed from the centred ones), |r|>1, the
 //     near-zero-variance gate of finalize_cell (src/stock_corr_impl.cuh:102-132);
-//     flagged pairs are recomputed by
+//     pairs whose shifted sums do not carry the value at full precision are
+//     recomputed by
 //  4. the two-pass fallback on the original values: Kahan mean,
 //     exact-constant (min==max) gate, centred second pass (Kahan above T=2048),
 //     sequential (sxy/sqrt(sxx))/sqrt(syy) (two_pass_centered,

@@ -15,6 +15,14 @@
 // Per block the same partials come out as from the staged pass
 // (fc_gram_body): P[product][i][j] with product 0 n, 1 sum x'_i over rows where
 // j is valid, 2 sum x'_i^2 likewise, 3 sum x'_i x'_j.
+//
+// Measured on a B200, 6.1 M rows x 12 factors f32 with a mask and 1 % missing
+// cells: 143 us (the staged pass took 673; memory alone 46, the FP64 sums 35),
+// factor_corr 1405 -> 217 us a call with the sampled shift and the two-pass
+// recomputation kept for sums that fall short.  What bounds it is the issue of
+// 300 instructions per 32 rows (102 FP64; the rest converts, tests and selects)
+// and the queue, at 8 warps per SM of 255 registers: the 90 sums of a thread
+// leave room for no more.
 #include "corr_common.cuh"
 #include "fcb_kernels.h"
 
@@ -22,7 +30,7 @@ namespace fcb {
 namespace {
 
 constexpr int kRegThreads = 128, kRegWarps = kRegThreads / 32;
-constexpr int kQueue = 96;   // rows a warp's queue holds: flushed from 64 on, 32 arrive at a time
+constexpr int kQueue = 96;   // rows a warp's queue holds: flushed above 64, up to 32 arrive at a time
 
 template <int FP>
 struct RegShape {

@@ -26,9 +26,8 @@ struct ScanOut {
 
 // Default largest bucket the learned rank path ranks itself.  A bucket of b
 // cells costs each of its cells b comparisons; above the cap the section goes
-// to the radix kernel, whose single-section latency is far larger (C2: cap 64
-// sent one section in 14616 there and took 1.215 ms per step, cap 256 none
-// and 1.195 ms).
+// to the plain kernel after the learned one (at 1218 x 5000 x 12 a cap of 64
+// sent one section in 14616 there, 256 none).
 constexpr int kLearnCapDefault = 256;
 
 template <typename TF, typename TR>
@@ -153,7 +152,7 @@ int fc_reg_kind(int F);  // 0..4: the width its panel runs at
 cudaError_t launch_fc_gram_reg_batch(int kind, int dtype, const FcBatchPanel* panels, const int* off, int np, int blocks,
                                      cudaStream_t s);
 
-// rank_plane.cu, rank_kernels.cu
+// rank_plane.cu; rank_kernels.cu (one factor with learned splitters)
 cudaError_t launch_cs_rank(const float* X, const uint8_t* mask, int T, int N, int desc, float* out,
                            int* status, cudaStream_t st);
 cudaError_t launch_param_scan(const float* X, const uint8_t* mask, int T, int N, ScanOut outs, int* status,
@@ -295,14 +294,11 @@ inline size_t rank_global_scratch(size_t per_date, int T) {
   return b + 8192;
 }
 
-// Persistent rank+IC over (panel, date) items; nt in {256, 512, 1024}.  With
+// Persistent rank+IC over f64 (panel, date) items; nt in {256, 512, 1024}.  With
 // occ != nullptr nothing is launched: *occ receives the CTAs per SM that fit.
-template <typename TF, typename TR>
 size_t rank_ic_batch_smem(int nt, int maxN);
-template <typename TF, typename TR>
-cudaError_t launch_rank_ic_batch(int nt, bool learned, const RankIcArgs<TF, TR>* panels, const int2* items,
-                                 int nitems, int* counter, int grid, size_t smem, int* status, cudaStream_t st,
-                                 int* occ);
+cudaError_t launch_rank_ic_batch(int nt, const RankIcArgs<double, double>* panels, const int2* items, int nitems,
+                                 int* counter, int grid, size_t smem, int* status, cudaStream_t st, int* occ);
 // factor_corr precision form (fc_tc.cu): BF16x3 tcgen05 moment products over
 // the R pooled rows, split over one CTA per SM, FP64 finalize.  F <= kFcTcMaxF;
 // element (r, f) at X[r*sr + f*sf]; work: fc_tc_work_bytes(F) bytes.

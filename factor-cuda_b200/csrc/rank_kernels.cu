@@ -1,8 +1,8 @@
 // rank_kernels.cu -- per-date in-shared-memory rank kernels for sm_100a.
 //
-//  (cs_rank and parameter_scan of one plane: k_csr / k_pscan in
-//   rank_ic_bucket.cu.)
-//  k_rank_ic      one CTA per date, looping over F factor panels: the forward
+//  k_rank_ic, k_rank_ic_batch
+//                 one CTA per date, looping over F factor panels (one factor
+//                 with learned splitters; the f64 batch): the forward
 //                 returns are sorted once per date, each factor is sorted once;
 //                 cs_rank ranks (own valid set) and the joint-set ranks of the
 //                 Spearman IC come from prefix counts over the two sorted
@@ -434,44 +434,41 @@ static int pick_nt(int n) { return n <= 4096 ? 256 : (n <= 8192 ? 512 : 1024); }
 
 size_t rank_ic_learned_smem(int N) { return RankIcLayout(N, 4, SortScratch<1024>::bytes).total; }
 
-template <int NT, typename TF, typename TR, bool LEARNED>
-static cudaError_t launch_rank_ic_nt(const RankIcArgs<TF, TR>& a, int* status, cudaStream_t st) {
-  constexpr int KSZ = (sizeof(TF) > sizeof(TR)) ? int(sizeof(TF)) : int(sizeof(TR));
-  const size_t smem = RankIcLayout(a.N, KSZ, SortScratch<NT>::bytes).total;
+template <int NT>
+static cudaError_t launch_learned_nt(const RankIcArgs<float, float>& a, int* status, cudaStream_t st) {
+  auto* k = k_rank_ic<NT, 16, float, float, true>;
+  const size_t smem = RankIcLayout(a.N, 4, SortScratch<NT>::bytes).total;
   if (smem > kMaxSmemPerBlock) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(k_rank_ic<NT, 16, TF, TR, LEARNED>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
-  k_rank_ic<NT, 16, TF, TR, LEARNED><<<a.T, NT, smem, st>>>(a, status);
+  k<<<a.T, NT, smem, st>>>(a, status);
   return cudaGetLastError();
 }
 
 cudaError_t launch_rank_ic_learned(const RankIcArgs<float, float>& a, int* status, cudaStream_t st) {
   if (a.N > kSmemRankCap || a.cdf_table == nullptr || a.cdf_zrange == nullptr) return cudaErrorInvalidValue;
   switch (pick_nt(a.N)) {
-    case 256: return launch_rank_ic_nt<256, float, float, true>(a, status, st);
-    case 512: return launch_rank_ic_nt<512, float, float, true>(a, status, st);
-    default: return launch_rank_ic_nt<1024, float, float, true>(a, status, st);
+    case 256: return launch_learned_nt<256>(a, status, st);
+    case 512: return launch_learned_nt<512>(a, status, st);
+    default: return launch_learned_nt<1024>(a, status, st);
   }
 }
 
 // ---------------------------------------------------------------------------
 // persistent batch launchers
 // ---------------------------------------------------------------------------
-template <typename TF, typename TR>
 size_t rank_ic_batch_smem(int nt, int maxN) {
-  constexpr int KSZ = (sizeof(TF) > sizeof(TR)) ? int(sizeof(TF)) : int(sizeof(TR));
   switch (nt) {
-    case 256: return RankIcLayout(maxN, KSZ, SortScratch<256>::bytes).total;
-    case 512: return RankIcLayout(maxN, KSZ, SortScratch<512>::bytes).total;
-    default: return RankIcLayout(maxN, KSZ, SortScratch<1024>::bytes).total;
+    case 256: return RankIcLayout(maxN, 8, SortScratch<256>::bytes).total;
+    case 512: return RankIcLayout(maxN, 8, SortScratch<512>::bytes).total;
+    default: return RankIcLayout(maxN, 8, SortScratch<1024>::bytes).total;
   }
 }
 
-template <int NT, typename TF, typename TR, bool LEARNED>
-static cudaError_t batch_nt(const RankIcArgs<TF, TR>* panels, const int2* items, int nitems, int* counter,
+template <int NT>
+static cudaError_t batch_nt(const RankIcArgs<double, double>* panels, const int2* items, int nitems, int* counter,
                             int grid, size_t smem, int* status, cudaStream_t st, int* occ) {
-  auto* k = k_rank_ic_batch<NT, 16, TF, TR, LEARNED>;
+  auto* k = k_rank_ic_batch<NT, 16, double, double, false>;
   if (smem > kMaxSmemPerBlock) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
@@ -480,32 +477,13 @@ static cudaError_t batch_nt(const RankIcArgs<TF, TR>* panels, const int2* items,
   return cudaGetLastError();
 }
 
-template <typename TF, typename TR>
-cudaError_t launch_rank_ic_batch(int nt, bool learned, const RankIcArgs<TF, TR>* panels, const int2* items,
-                                 int nitems, int* counter, int grid, size_t smem, int* status, cudaStream_t st,
-                                 int* occ) {
-  if (learned) {
-    if constexpr (std::is_same<TF, float>::value && std::is_same<TR, float>::value) {
-      switch (nt) {
-        case 256: return batch_nt<256, TF, TR, true>(panels, items, nitems, counter, grid, smem, status, st, occ);
-        case 512: return batch_nt<512, TF, TR, true>(panels, items, nitems, counter, grid, smem, status, st, occ);
-        default: return batch_nt<1024, TF, TR, true>(panels, items, nitems, counter, grid, smem, status, st, occ);
-      }
-    } else {
-      return cudaErrorInvalidValue;
-    }
-  }
+cudaError_t launch_rank_ic_batch(int nt, const RankIcArgs<double, double>* panels, const int2* items, int nitems,
+                                 int* counter, int grid, size_t smem, int* status, cudaStream_t st, int* occ) {
   switch (nt) {
-    case 256: return batch_nt<256, TF, TR, false>(panels, items, nitems, counter, grid, smem, status, st, occ);
-    case 512: return batch_nt<512, TF, TR, false>(panels, items, nitems, counter, grid, smem, status, st, occ);
-    default: return batch_nt<1024, TF, TR, false>(panels, items, nitems, counter, grid, smem, status, st, occ);
+    case 256: return batch_nt<256>(panels, items, nitems, counter, grid, smem, status, st, occ);
+    case 512: return batch_nt<512>(panels, items, nitems, counter, grid, smem, status, st, occ);
+    default: return batch_nt<1024>(panels, items, nitems, counter, grid, smem, status, st, occ);
   }
 }
-template size_t rank_ic_batch_smem<float, float>(int, int);
-template size_t rank_ic_batch_smem<double, double>(int, int);
-template cudaError_t launch_rank_ic_batch<float, float>(int, bool, const RankIcArgs<float, float>*, const int2*, int,
-                                                         int*, int, size_t, int*, cudaStream_t, int*);
-template cudaError_t launch_rank_ic_batch<double, double>(int, bool, const RankIcArgs<double, double>*, const int2*,
-                                                           int, int*, int, size_t, int*, cudaStream_t, int*);
 
 }  // namespace fcb

@@ -148,8 +148,9 @@ int fcb_rolling_ic(const void* f, int f_dtype, const void* r, int r_dtype, const
 /* ---------------------------------------------------------- correlation ---
  * (F,F) pooled pairwise-complete Pearson of a (T,N,F) panel over (t,i) rows,
  * mask (T,N) broadcast to every factor.  x is f32 or f64.  fallback_out
- * (NULL = off) receives F*F bytes, 1 where the pair was recomputed by the
- * two-pass compensated fallback.
+ * (NULL = off) receives F*F bytes, 1 where the pair fails the cancellation
+ * gate (its value comes from centred sums or, where these fall short, from the
+ * two-pass compensated recomputation).
  * Replaces factor_corr_gpu (src/factor_corr.cuh:46-49).
  * Returns -1 null/dim, -2 T*N > INT32_MAX, -3 F > 128. */
 int fcb_factor_corr(const void* x, int dtype, const uint8_t* mask, int T, int N, int F, double* out,
@@ -165,7 +166,7 @@ int fcb_dev_factor_corr(const void* d_x, int dtype, const uint8_t* d_mask, int T
 
 /* (N,N) pairwise-complete Pearson of a (T,N) panel over t.  selected_path
  * (NULL = off): 0 fully valid panel, 1 masked panel; fallback_count: pairs
- * recomputed by the two-pass fallback.
+ * that fail the cancellation gate (as fallback_out above).
  * Replaces stock_corr_gpu (src/stock_corr.cuh:66-68).
  * Returns -1 null/dim, -2 T*N > INT32_MAX, -3 N*N > INT32_MAX,
  * -4 domain (max|x| > 1e150 or a nonzero |x| < 1e-150 on a valid cell). */
