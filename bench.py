@@ -415,8 +415,7 @@ def run_b200(args, rank, world):
 # of each kernel at T=600: dram__bytes_read.sum + dram__bytes_write.sum.
 # Traffic grows with the number of dates at fixed N and F, so the bench's step
 # is that times T.
-TRAFFIC_PER_DATE = {"learned": (156.591104e6 + 88.684544e6 + 18.057728e6) / 600,
-                    "radix": (156.073472e6 + 86.176000e6 + 18.057728e6) / 600}
+TRAFFIC_PER_DATE = dict.fromkeys(("learned", "radix"), (156.102144e6 + 108.951808e6 + 15.078656e6) / 600)
 
 
 def transfer_floor(h2d_bytes, d2h_bytes, dev, reps=3):

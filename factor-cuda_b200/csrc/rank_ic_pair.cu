@@ -17,6 +17,14 @@
 //
 // Crowded rows are radix-sorted in shared memory (pair_radix).
 //
+// Measured on a B200, against two radix sorts per date in 512-thread CTAs:
+// 1218 x 5000 f32 391 -> 129 us, f64 1108 -> 176, 250 x 500 f64 45 -> 23 (the
+// kernel 13.5); integers against returns rounded to 1e-4 252 -> 213, f64 587 ->
+// 397.  What bounds it is instruction issue (64 k warp instructions per date of
+// 5000 at 54 % of the slots).  Full keys of f64 ties read from global memory by
+// every comparison took 1662 us on a plane with 3 % zeros, from shared memory 461
+// (the radix form 1098).
+//
 // Semantics: rolling_ic_gpu (src/rolling_ic.cu:306-540) / np_rolling_ic
 // (fc/_cpu_core.py:271-293); ties rank by column, a pair that is constant on
 // either side over the joint set has no IC.

@@ -55,11 +55,12 @@ struct SectionShape {
 
 // Calls go(SectionShape<NT, V>{}) with the block shape for sections of N cells,
 // many of them.  A section takes the same time however many of its block's
-// cells it fills, and two vectors of four cells pay from 1025 cells on: in
-// units of cells, rank + IC takes 71 ps per cell of capacity at 256 threads x 1
-// vector, 74 at 512 cells, 95 at 1024 x 4.  2 M cells x 8 factors as sections of
-// 250, 500, 768, 1500 and 2500: 0.72 ms -> 0.23, 0.38 -> 0.22, 0.26 -> 0.20,
-// 0.24 -> 0.20, 0.24 -> 0.19, against shapes of 256 x 1 and 2 and 384 x 2 alone.
+// cells it fills (rank + IC: 12 to 14 ps per cell of capacity, whatever the
+// shape), so the shapes follow the width closely.  2 M cells x 8 factors as
+// sections of 250, 500, 768, 1500 and 2500 cells: 0.72 ms -> 0.23, 0.38 -> 0.22,
+// 0.26 -> 0.20, 0.24 -> 0.20, 0.24 -> 0.19, against shapes of 256 x 1, 256 x 2
+// and 384 x 2 alone.  At 5000 cells 448 x 3 takes 47 us per 1218 dates of
+// cs_rank, 512 x 3 51, 256 x 5 58 and 1024 x 2 78.
 template <typename Go>
 auto section_shape(int N, Go&& go) {
   if (N <= 256) return go(SectionShape<64, 1>{});
