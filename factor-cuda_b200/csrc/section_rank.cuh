@@ -44,7 +44,9 @@ constexpr uint32_t kSpreadMaxEqualPairs = 8;
 // threads, whose warps would wait for the longest loop.
 constexpr uint32_t kSpreadHeavy = 16;
 // A section whose bins hold, by the mean over its cells, more than this
-// fraction of it is a cluster far narrower than its range.
+// fraction of it is a cluster far narrower than its range.  (Above 1024 cells:
+// the few bins of a narrow block hold as much of an ordinary section, whose keys
+// lie within a few exponents, and there the counting pass costs little.)
 constexpr uint32_t kSpreadBinShare = 8;
 
 // One block shape: NT threads with V vectors of four cells each.
@@ -344,7 +346,7 @@ FCB_DEV bool spread_place(uint32_t (&key)[4 * V], const SpreadLayout<NT, V>& L, 
     const uint32_t ex = warps_before<NW>(red + 96) + inc - w0 - w1;
     T.m = static_cast<int>(warps_sum<NW>(red + 96)) - K;
     const uint32_t m = static_cast<uint32_t>(T.m);
-    if (m > 256u && warps_sum<NW>(red + 192) > m * m / kSpreadBinShare) {
+    if (m > 1024u && warps_sum<NW>(red + 192) > m * m / kSpreadBinShare) {
       __syncthreads();  // the caller reuses the shared memory
       return false;
     }
