@@ -19,7 +19,7 @@
 //
 // Measured on a B200, against two radix sorts per date in 512-thread CTAs:
 // 1218 x 5000 f32 391 -> 129 us, f64 1108 -> 176, 250 x 500 f64 45 -> 23 (the
-// kernel 13.5); integers against returns rounded to 1e-4 252 -> 213, f64 587 ->
+// kernel 13.1); integers against returns rounded to 1e-4 252 -> 213, f64 587 ->
 // 397.  What bounds it is instruction issue (64 k warp instructions per date of
 // 5000 at 54 % of the slots).  Full keys of f64 ties read from global memory by
 // every comparison took 1662 us on a plane with 3 % zeros, from shared memory 461

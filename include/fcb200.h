@@ -114,9 +114,9 @@ void fcb_host_free(void* p);
  * Replaces cs_rank_gpu (src/cross_sectional_rank.cuh:90-99).
  * Returns -1 null/dim, -2 N > 2^24, -3 T*N > INT32_MAX.
  * Every N up to the cap is served: sections that fit one CTA's shared memory
- * (N <= 16384 for cs_rank, parameter_scan and f32 rank + IC of several
- * factors; about 11000 f32 and 8192 f64 for single-factor rolling_ic) are
- * sorted there, wider ones by a
+ * (N <= 16384 for cs_rank, parameter_scan and f32 rank + IC; about 10100 for
+ * rolling_ic with an f64 side) are ranked there, cs_rank up to 65536 by slices
+ * of the value range, and wider ones by a
  * global-memory radix sort per date with the same results (scratch from the
  * workspace, or stream-ordered cudaMallocAsync for the fcb_dev_* variants). */
 int fcb_cs_rank_f32(const float* x, const uint8_t* mask, int T, int N, int descending, float* out,
@@ -258,8 +258,8 @@ int fcb_dev_corr_domain(const void* d_x, int dtype, const uint8_t* d_mask, int T
  * monotone CDF.  The learned rank path scatters each cross-section into
  * buckets by that CDF and ranks each bucket exactly; every date is checked
  * (strictly increasing (value, column) order over the whole output) and any
- * failure, bucket above `cap` or unusable scale falls back to the radix sort,
- * so ranks and IC are bit-identical to the radix path. */
+ * failure, bucket above `cap` or unusable scale falls back to the plain path,
+ * so ranks and IC are bit-identical to it. */
 #define FCB_CDF_PARAMS 1153
 #define FCB_CDF_KNOTS 1024
 typedef struct fcb_cdf_model fcb_cdf_model;
@@ -304,14 +304,14 @@ int fcb_cdf_grad(const float* params, const float* z, const float* u, int n, flo
  * d_stats (NULL = off) receives (F,T,4) ints: outcome (1 learned, 2 bucket overflow,
  * 3 order check rejected -- with several factors, a staged CDF table that
  * is not non-decreasing within [0, 1]; with one factor, the ranked keys out
- * of order --, 4 unusable scale; 2-4 fell back to radix), the largest
+ * of order --, 4 unusable scale; 2-4 fell back to the plain path), the largest
  * bucket, the sum of squared bucket sizes (the per-date comparison work; m
  * for perfectly even buckets of one) and m, the number of ranked cells.
  * Sections too wide for the shared-memory kernel are ranked by the
  * global-memory radix path (same results); their statistics read 0.  cap:
  * the largest bucket the learned kernel ranks itself; 0 = the default, 256
  * (a bucket of b cells costs each of its cells b comparisons, far less than
- * sending the section to the radix kernel). */
+ * sending the section to the plain kernel). */
 int fcb_dev_rank_ic_panel_learned(const float* d_x, const float* d_r, const uint8_t* d_fmask,
                                   const uint8_t* d_rmask, int F, int T, int N, int min_valid, float* d_ranks,
                                   double* d_ic, const fcb_cdf_model* model, int cap, int* d_stats, void* stream);
