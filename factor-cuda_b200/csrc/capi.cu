@@ -309,7 +309,13 @@ extern "C" int fcb_dev_cs_rank_f32(const float* d_x, const uint8_t* d_mask, int 
   if (N > (1 << 24)) return FCB_ERR_CAP2;
   if (static_cast<long long>(T) * N > INT32_MAX) return FCB_ERR_CAP3;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (N > kSmemRankCap && N <= kSliceMaxN) return rc(launch_cs_rank_slices(d_x, d_mask, T, N, desc, d_out, s));
+  // several CTAs read a row that others of them already write ranks of: the
+  // slices need x and out apart; in place the global-memory path sorts copies
+  const uintptr_t x0 = reinterpret_cast<uintptr_t>(d_x), o0 = reinterpret_cast<uintptr_t>(d_out);
+  const uintptr_t plane_bytes = static_cast<uintptr_t>(T) * N * 4;
+  const bool apart = x0 + plane_bytes <= o0 || o0 + plane_bytes <= x0;
+  if (N > kSmemRankCap && N <= kSliceMaxN && apart)
+    return rc(launch_cs_rank_slices(d_x, d_mask, T, N, desc, d_out, s));
   if (N > kSmemRankCap) {
     // global-memory path; scratch is stream-ordered (no host synchronisation)
     const size_t bytes = rank_global_scratch(rank_global_bytes_per_date(0, N, 1, 4, 4), T);
@@ -348,7 +354,10 @@ extern "C" int fcb_cs_rank_f32(const float* x, const uint8_t* mask, int T, int N
     const size_t bytes = rank_global_scratch(rank_global_bytes_per_date(0, N, 1, 4, 4), T);
     uint8_t* scr;
     FCB_TRY(ws.get(S_GSCR, bytes, &scr));
-    FCB_TRY(launch_cs_rank_global(dx, dm, T, N, desc, dout, scr, bytes, s));
+    if (N <= kSliceMaxN)
+      FCB_TRY(launch_cs_rank_slices(dx, dm, T, N, desc, dout, s));
+    else
+      FCB_TRY(launch_cs_rank_global(dx, dm, T, N, desc, dout, scr, bytes, s));
   } else {
     FCB_TRY(launch_cs_rank(dx, dm, T, N, desc, dout, dst, s));
   }

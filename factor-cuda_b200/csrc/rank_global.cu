@@ -521,7 +521,6 @@ size_t rank_global_bytes_per_date(int kind, int N, int F, int ksz_f, int ksz_r) 
 
 cudaError_t launch_cs_rank_global(const float* X, const uint8_t* mask, int T, int N, int desc, float* out,
                                   uint8_t* scratch, size_t bytes, cudaStream_t s) {
-  if (N <= kSliceMaxN) return launch_cs_rank_slices(X, mask, T, N, desc, out, s);
   const int Tc = chunk_dates(row_bytes(N, false), T, bytes);
   if (Tc < 1) return cudaErrorInvalidValue;
   const size_t n = static_cast<size_t>(Tc) * N;

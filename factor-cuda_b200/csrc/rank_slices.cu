@@ -19,6 +19,9 @@
 // cell and slice, which is why the form ends at kSliceMaxN; beyond,
 // rank_global.cu.
 //
+// The CTAs of a row read all of it while others write its ranks: out must not
+// overlap X.
+//
 // Semantics: cs_rank_gpu (src/cross_sectional_rank.cu:228-372).
 #include <algorithm>
 

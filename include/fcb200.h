@@ -220,7 +220,7 @@ int fcb_dev_status(void);
  * when it completed; the device stays usable either way.  Synchronous. */
 int fcb_selftest_bounded_wait(int arrive, int max_polls);
 
-/* cs_rank (asynchronous). */
+/* cs_rank (asynchronous); d_out may be d_x. */
 int fcb_dev_cs_rank_f32(const float* d_x, const uint8_t* d_mask, int T, int N, int descending, float* d_out,
                         void* stream);
 
