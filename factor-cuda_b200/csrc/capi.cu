@@ -350,14 +350,13 @@ extern "C" int fcb_cs_rank_f32(const float* x, const uint8_t* mask, int T, int N
   FCB_TRY(cudaMemcpyAsync(dx, x, n * 4, cudaMemcpyHostToDevice, s));
   if (mask != nullptr) FCB_TRY(cudaMemcpyAsync(dm, mask, n, cudaMemcpyHostToDevice, s));
   FCB_TRY(cudaMemsetAsync(dst, 0, sizeof(int), s));
-  if (N > kSmemRankCap) {
+  if (N > kSliceMaxN) {
     const size_t bytes = rank_global_scratch(rank_global_bytes_per_date(0, N, 1, 4, 4), T);
     uint8_t* scr;
     FCB_TRY(ws.get(S_GSCR, bytes, &scr));
-    if (N <= kSliceMaxN)
-      FCB_TRY(launch_cs_rank_slices(dx, dm, T, N, desc, dout, s));
-    else
-      FCB_TRY(launch_cs_rank_global(dx, dm, T, N, desc, dout, scr, bytes, s));
+    FCB_TRY(launch_cs_rank_global(dx, dm, T, N, desc, dout, scr, bytes, s));
+  } else if (N > kSmemRankCap) {
+    FCB_TRY(launch_cs_rank_slices(dx, dm, T, N, desc, dout, s));
   } else {
     FCB_TRY(launch_cs_rank(dx, dm, T, N, desc, dout, dst, s));
   }
@@ -1173,7 +1172,7 @@ extern "C" int fcb_memory_budget(int op, int dtype, int T, int N, int F, int fla
   switch (op) {
     case FCB_OP_CS_RANK:
       b = slot_bytes(n * 4) * 2 + 64 + (m1 ? slot_bytes(n) : 0);
-      if (N > kSmemRankCap) b += slot_bytes(rank_global_scratch(rank_global_bytes_per_date(0, N, 1, 4, 4), T));
+      if (N > kSliceMaxN) b += slot_bytes(rank_global_scratch(rank_global_bytes_per_date(0, N, 1, 4, 4), T));
       break;
     case FCB_OP_PARAMETER_SCAN: {
       const int groups = (flags >> 8) & 0xF;
