@@ -195,7 +195,7 @@ FCB_DEV uint32_t pair_positions(const PairRow row, int N, uint32_t (&key)[4 * V]
 }
 
 // Whether the row's cells in `joint` (some) all have the same value.  red: 128
-// words.
+// words.  Ends with a barrier.
 template <int NT, int V>
 __device__ __noinline__ bool pair_constant(const PairRow row, uint32_t joint, uint32_t* red) {
   unsigned long long lo = ~0ull, hi = 0ull;
@@ -219,6 +219,7 @@ __device__ __noinline__ bool pair_constant(const PairRow row, uint32_t joint, ui
     lo = min(lo, r[w]);
     hi = max(hi, r[32 + w]);
   }
+  __syncthreads();
   return lo == hi;
 }
 
@@ -280,9 +281,18 @@ __global__ void __launch_bounds__(NT, kSmThreads / NT) k_ic_pair(PairArgs a) {
 #pragma unroll
   for (int c = 0; c < C; ++c)
     if ((lone >> c) & 1u) mark_set(marks, W[c]);
+  const uint32_t nj = __reduce_add_sync(kFull, static_cast<uint32_t>(__popc(joint)));
+  if (lane_id() == 0) red[128 + wi] = nj;
   const bool any_drop = __syncthreads_or(dropped != 0u), any_lone = __syncthreads_or(lone != 0u);
   if (wi == 0 && any_lone) mark_prefix(marks, nbw);
   if (wi == 1 && any_drop) mark_prefix(drop, nbw);
+  const uint32_t m = warps_sum<NW>(red + 128);
+  bool some = m >= 2u && static_cast<int>(m) >= a.min_valid;
+  // a side can be constant on the joint set only when that is no larger than its
+  // largest group of ties may be; the rows are read again for it, so before any
+  // output (which may be written in their place)
+  if (some && m <= fties) some = !pair_constant<NT, V>(rf, joint, red);
+  if (some && m <= rties) some = !pair_constant<NT, V>(rr, joint, red);
   if (a.ranks_out != nullptr) {
     float v[C];
 #pragma unroll
@@ -325,19 +335,9 @@ __global__ void __launch_bounds__(NT, kSmThreads / NT) k_ic_pair(PairArgs a) {
   };
   unsigned long long* red64 = reinterpret_cast<unsigned long long*>(red);
   const unsigned long long wsum = warp_sum64(sum32);
-  const uint32_t nj = __reduce_add_sync(kFull, static_cast<uint32_t>(__popc(joint)));
-  if (lane_id() == 0) {
-    red64[wi] = wsum;
-    red[64 + wi] = nj;
-  }
+  if (lane_id() == 0) red64[wi] = wsum;
   __syncthreads();
-  const uint32_t m = warps_sum<NW>(red + 64);
   const unsigned long long sum = warp_sum64(lane_id() < NW ? red64[lane_id()] : 0ull);
-  bool some = m >= 2u && static_cast<int>(m) >= a.min_valid;
-  // a side can be constant on the joint set only when that is no larger than its
-  // largest group of ties may be
-  if (some && m <= fties) some = !pair_constant<NT, V>(rf, joint, red);
-  if (some && m <= rties) some = !pair_constant<NT, V>(rr, joint, red);
   if (threadIdx.x == 0)
     a.ic_out[static_cast<size_t>(f) * (a.ic_ld > 0 ? a.ic_ld : a.T) + t] =
         some ? spearman_from_sum(static_cast<long long>(m), static_cast<long long>(sum))
