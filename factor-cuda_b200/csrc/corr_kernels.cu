@@ -728,7 +728,7 @@ FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int
   }
   out[i * F + j] = p.r;
   out[j * F + i] = p.r;
-  if (flags != nullptr) flags[i * F + j] = p.gate || (p.redo && i != j) ? 1 : 0;
+  if (flags != nullptr) flags[i * F + j] = p.gate ? 1 : 0;
   if (p.redo) {
     const int slot = atomicAdd(fb_count, 1);
     fb_list[slot] = e;

@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(256, 4)
       const PairResult p =
           finalize_pair(static_cast<double>(P.n[li][lj]), x.x, y.x, P.xy[li][lj], x.y, y.y, si.mean, sj.mean);
       v = p.r;
-      gated += p.gate || p.redo ? 1 : 0;
+      gated += p.gate ? 1 : 0;
       if (p.redo) fb_list[atomicAdd(&sum->flagged, 1)] = i * N + j;  // N*N <= INT32_MAX
     }
     out[static_cast<size_t>(i) * N + j] = v;
