@@ -26,6 +26,7 @@
 #include <cmath>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "corr_common.cuh"
 #include "fcb_kernels.h"
@@ -109,21 +110,23 @@ FCB_DEV Blk launch_blk() {
 }
 
 // Per-block column partials over a contiguous range of the sampled rows (every
-// ms-th; R, sr and the mask index count in sampled rows): count, Kahan sum,
-// min, max.  Rows are visited in increasing order within each thread's
-// strided slice; partials are merged in a fixed order by k_fc_colfinal.
+// ms-th; R, sr and the mask index count in sampled rows; at most kFcColRows a
+// block): count and Kahan sum of each factor, and the rows with some valid
+// factor.  Rows are visited in increasing order within each thread's strided
+// slice; partials are merged in a fixed order by k_fc_colfinal.
 template <typename TIN>
 FCB_DEV void fc_colpart_body(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, long long R, int F,
                              long long sr, long long sf, long long ms, long long rows_per_block,
                              FcColPart* __restrict__ part, const Blk bk) {
+  __shared__ uint8_t some[kFcColRows];  // 1: some factor of the row is valid
+  const int tid = static_cast<int>(threadIdx.y * blockDim.x + threadIdx.x);
   const long long r0 = bk.x * rows_per_block;
   const long long r1 = min(R, r0 + rows_per_block);
+  for (int k = tid; k < kFcColRows; k += static_cast<int>(blockDim.x * blockDim.y)) some[k] = 0;
+  __syncthreads();
   for (int f = threadIdx.y; f < F; f += blockDim.y) {
     Kahan k;
-    // count, min and max in the input's own type (exact: the values are the
-    // same after the widening); only the Kahan sum needs FP64
     long long cnt_i = 0;
-    TIN mn_t = KeyOf<TIN>::max_finite(), mx_t = -KeyOf<TIN>::max_finite();
     const TIN* col = X + f * sf;
     // rows visited in the same order; kU loads in flight before they are added
     constexpr int kU = 8;
@@ -142,57 +145,40 @@ FCB_DEV void fc_colpart_body(const TIN* __restrict__ X, const uint8_t* __restric
         if (ok[u] && KeyOf<TIN>::finite(xv[u])) {
           ++cnt_i;
           k.add(static_cast<double>(xv[u]));
-          mn_t = xv[u] < mn_t ? xv[u] : mn_t;
-          mx_t = xv[u] > mx_t ? xv[u] : mx_t;
+          some[rb - r0 + static_cast<long long>(u) * blockDim.x] = 1;
         }
       }
     }
     double cnt = static_cast<double>(cnt_i);
-    double mn = cnt_i > 0 ? static_cast<double>(mn_t) : kBigPos;
-    double mx = cnt_i > 0 ? static_cast<double>(mx_t) : -kBigPos;
     // fixed-order warp merge (lanes are threadIdx.x within one warp row)
     for (int o = 1; o < 32; o <<= 1) {
       const double os = __shfl_down_sync(kFull, k.s, o), oc = __shfl_down_sync(kFull, k.c, o);
       const double on = __shfl_down_sync(kFull, cnt, o);
-      const double omn = __shfl_down_sync(kFull, mn, o), omx = __shfl_down_sync(kFull, mx, o);
       if ((threadIdx.x & (2 * o - 1)) == 0) {
         Kahan kk;
         kk.s = os;
         kk.c = oc;
         k.merge(kk);
         cnt += on;
-        mn = fmin(mn, omn);
-        mx = fmax(mx, omx);
       }
     }
-    if (threadIdx.x == 0) {
-      FcColPart p;
-      p.count = cnt;
-      p.s = k.s;
-      p.c = k.c;
-      p.min = mn;
-      p.max = mx;
-      part[static_cast<size_t>(bk.x) * F + f] = p;
-    }
+    if (threadIdx.x == 0) part[static_cast<size_t>(bk.x) * F + f] = FcColPart{cnt, k.s, k.c, 0.0};
+  }
+  __syncthreads();
+  if (threadIdx.y == 0) {
+    int n = 0;
+    for (int k = static_cast<int>(threadIdx.x); k < kFcColRows; k += 32) n += some[k];
+    n = __reduce_add_sync(kFull, n);
+    if (threadIdx.x == 0) part[static_cast<size_t>(bk.x) * F].rows = static_cast<double>(n);
   }
 }
 
-template <typename TIN>
-__global__ void k_fc_colpart(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, long long R, int F,
-                             long long sr, long long sf, long long ms, long long rows_per_block,
-                             FcColPart* __restrict__ part) {
-  fc_colpart_body<TIN>(X, mask, R, F, sr, sf, ms, rows_per_block, part, launch_blk());
-}
-
-// One warp per column: lane l merges partials l, l+32, ... in order, then a
+// One warp per column f: lane l merges partials l, l+32, ... in order, then a
 // fixed shuffle tree merges the lanes.
-FCB_DEV void fc_colfinal_body(const FcColPart* __restrict__ part, int nblk, int F, FcColStat* __restrict__ st,
-                              const Blk bk) {
-  const int f = (bk.x * blockDim.x + threadIdx.x) >> 5;
+FCB_DEV void fc_colfinal_warp(const FcColPart* part, int nblk, int F, FcColStat* __restrict__ st, int f) {
   const int lane = threadIdx.x & 31;
-  if (f >= F) return;  // whole warps exit together
   Kahan k;
-  double cnt = 0.0, mn = kBigPos, mx = -kBigPos;
+  double cnt = 0.0, rows = 0.0;
   for (int b = lane; b < nblk; b += 32) {
     const FcColPart& p = part[static_cast<size_t>(b) * F + f];
     Kahan o;
@@ -200,30 +186,45 @@ FCB_DEV void fc_colfinal_body(const FcColPart* __restrict__ part, int nblk, int 
     o.c = p.c;
     k.merge(o);
     cnt += p.count;
-    mn = fmin(mn, p.min);
-    mx = fmax(mx, p.max);
+    rows += p.rows;
   }
   for (int o = 1; o < 32; o <<= 1) {
     const double os = __shfl_down_sync(kFull, k.s, o), oc = __shfl_down_sync(kFull, k.c, o);
-    const double on = __shfl_down_sync(kFull, cnt, o);
-    const double omn = __shfl_down_sync(kFull, mn, o), omx = __shfl_down_sync(kFull, mx, o);
+    const double on = __shfl_down_sync(kFull, cnt, o), orows = __shfl_down_sync(kFull, rows, o);
     if ((lane & (2 * o - 1)) == 0) {
       Kahan kk;
       kk.s = os;
       kk.c = oc;
       k.merge(kk);
       cnt += on;
-      mn = fmin(mn, omn);
-      mx = fmax(mx, omx);
+      rows += orows;
     }
   }
-  if (lane != 0) return;
-  FcColStat s;
-  s.count = cnt;
-  s.mean = cnt > 0.0 ? k.s / cnt : 0.0;
-  s.min = mn;
-  s.max = mx;
-  st[f] = s;
+  if (lane == 0) st[f] = FcColStat{cnt, cnt > 0.0 ? k.s / cnt : 0.0, rows};
+}
+FCB_DEV void fc_colfinal_body(const FcColPart* __restrict__ part, int nblk, int F, FcColStat* __restrict__ st,
+                              const Blk bk) {
+  const int f = (bk.x * blockDim.x + threadIdx.x) >> 5;
+  if (f < F) fc_colfinal_warp(part, nblk, F, st, f);  // whole warps
+}
+
+// done (zero before): the last block to write its partials merges them as well
+// (a launch less, 2 to 3 us; few factors: its warps take them in turn), or null.
+template <typename TIN>
+__global__ void k_fc_colpart(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, long long R, int F,
+                             long long sr, long long sf, long long ms, long long rows_per_block,
+                             FcColPart* __restrict__ part, int* __restrict__ done, FcColStat* __restrict__ st) {
+  __shared__ bool last;
+  fc_colpart_body<TIN>(X, mask, R, F, sr, sf, ms, rows_per_block, part, launch_blk());
+  if (done == nullptr) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && threadIdx.y == 0) last = atomicAdd(done, 1) == static_cast<int>(gridDim.x) - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int f = static_cast<int>(threadIdx.y); f < F; f += static_cast<int>(blockDim.y))
+    fc_colfinal_warp(part, static_cast<int>(gridDim.x), F, st, f);
 }
 
 __global__ void k_fc_colfinal(const FcColPart* __restrict__ part, int nblk, int F, FcColStat* __restrict__ st) {
@@ -650,22 +651,28 @@ FCB_DEV void fc_gram_body(const TIN* __restrict__ X, const uint8_t* __restrict__
 }
 
 // Single panel: the path is chosen on the host (MMA = fc_gram_use_mma(Fp)), so
-// each instantiation holds one body.
-template <typename TIN, bool MMA>
+// each instantiation holds one body.  LOW: a panel of the register form's
+// widths, staged only if fc_staged says so; one wave of blocks goes through the
+// nblk row blocks.
+template <typename TIN, bool MMA, bool LOW>
 __global__ void __launch_bounds__(256, 3) k_fc_gram(const TIN* __restrict__ X, const uint8_t* __restrict__ mask,
                                                  long long R, int F, long long sr, long long sf, int Fp,
                                                  long long rows_per_block,
                                                  const FcColStat* __restrict__ st, int tasks_total,
-                                                 int tasks_per_block, double* __restrict__ part) {
-  if (MMA)
-    fc_gram_body_mma<TIN>(X, mask, R, F, sr, sf, Fp, rows_per_block, st, tasks_total, tasks_per_block, part,
-                          launch_blk());
-  else
-    fc_gram_body_fma<TIN>(X, mask, R, F, sr, sf, Fp, rows_per_block, st, tasks_total, tasks_per_block, part,
-                          launch_blk());
+                                                 int tasks_per_block, int nblk, double* __restrict__ part) {
+  if (LOW && !fc_staged(st, F)) return;
+  for (Blk bk = launch_blk(); bk.x < nblk; bk.x += static_cast<int>(gridDim.x)) {
+    if (MMA)
+      fc_gram_body_mma<TIN>(X, mask, R, F, sr, sf, Fp, rows_per_block, st, tasks_total, tasks_per_block, part, bk);
+    else
+      fc_gram_body_fma<TIN>(X, mask, R, F, sr, sf, Fp, rows_per_block, st, tasks_total, tasks_per_block, part, bk);
+    if (!LOW) break;
+    __syncthreads();  // the next block reuses the shared memory
+  }
 }
 
-// Sum the per-block Gram partials in block order, finalize each pair.
+// Sum the per-block Gram partials in block order (nblk of the staged form),
+// finalize each pair.
 // One warp per (i <= j) pair: lane l sums blocks l, l+32, ..., a fixed
 // shuffle tree sums the lanes, lane 0 finalizes.
 FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int Fp,
@@ -676,6 +683,8 @@ FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int
   if (e >= F * F) return;  // whole warps exit together
   const int i = e / F, j = e % F;
   if (i > j) return;
+  const bool reg = F <= kFcRegMaxF && !fc_staged(st, F);
+  if (reg) nblk = fc_reg_blocks(nblk);
   double q[6] = {0, 0, 0, 0, 0, 0}, tot[2] = {0, 0};  // tot: sums of squares of each factor's own rows
   // q: n, sx (x'_i m_j), sy (m_i x'_j), sxy, sx2 (x'^2_i m_j), sy2 (m_i x'^2_j)
   for (int b = lane; b < nblk; b += 32) {
@@ -716,11 +725,11 @@ FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int
   } else {
     p = finalize_pair(q[0], q[1], q[2], q[3], q[4], q[5], mui, muj);
     // The register form's sums are totals less the rows that the other factor
-    // misses: where less than three quarters are left, their rounding shows.
+    // misses: where less than half is left (an outlier among those rows, as a
+    // rule: see fc_staged), their rounding shows.
     // The staged form's longer chains lose more than the two-pass values of
     // gated pairs do (rms error 4.7e-18 against 2.7e-18 at 20 factors).
-    const bool again =
-        F <= kFcRegMaxF ? tot[0] * 0.75 > q[4] || tot[1] * 0.75 > q[5] : p.gate;
+    const bool again = reg ? tot[0] * 0.5 > q[4] || tot[1] * 0.5 > q[5] : p.gate;
     if (again) {
       p.redo = p.redo || q[0] >= 2.0;
       p.r = dnan();
@@ -1216,6 +1225,9 @@ void fc_gram_plan(int Fp, int* tasks_total, int* tasks_per_block, int* ytiles) {
   *ytiles = (*tasks_total + *tasks_per_block - 1) / *tasks_per_block;
 }
 
+// One wave of staged blocks (256 threads, at most 75 KB: three per SM).
+constexpr int kLowWave = 3 * 148;
+
 cudaError_t launch_factor_corr_strided(const void* X, int dtype, const uint8_t* mask, long long R, int F,
                                        long long sr, long long sf, FcWork& w, double* out, uint8_t* flags,
                                        cudaStream_t s) {
@@ -1228,41 +1240,49 @@ cudaError_t launch_factor_corr_strided(const void* X, int dtype, const uint8_t* 
   const long long ms = fc_col_stride(R), rs = (R + ms - 1) / ms;
   const long long rpb_cols = (rs + w.nblk_cols - 1) / w.nblk_cols;
   const long long rpb_gram = (R + w.nblk_gram - 1) / w.nblk_gram;
+  const int nreg = fc_reg_blocks(w.nblk_gram);
   dim3 cb(32, 8);
+  cudaError_t e = cudaMemsetAsync(w.fb_count, 0, 2 * sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  int* done = F <= kFcRegMaxF ? w.fb_count + 1 : nullptr;
   if (dtype == 0)
     k_fc_colpart<float><<<w.nblk_cols, cb, 0, s>>>(static_cast<const float*>(X), mask, rs, F, sr * ms, sf, ms, rpb_cols,
-                                                   w.colpart);
+                                                   w.colpart, done, w.colstat);
   else
     k_fc_colpart<double><<<w.nblk_cols, cb, 0, s>>>(static_cast<const double*>(X), mask, rs, F, sr * ms, sf, ms,
-                                                    rpb_cols, w.colpart);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_fc_colfinal<<<(F * 32 + 127) / 128, 128, 0, s>>>(w.colpart, w.nblk_cols, F, w.colstat);
+                                                    rpb_cols, w.colpart, done, w.colstat);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (done == nullptr) {
+    k_fc_colfinal<<<(F * 32 + 127) / 128, 128, 0, s>>>(w.colpart, w.nblk_cols, F, w.colstat);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
   if (F <= kFcRegMaxF) {
-    e = launch_fc_gram_reg(X, dtype, mask, R, F, sr, sf, Fp, rpb_gram, w.nblk_gram, w.colstat, w.gram, s);
+    e = launch_fc_gram_reg(X, dtype, mask, R, F, sr, sf, Fp, (R + nreg - 1) / nreg, nreg, w.colstat, w.gram, s);
     if (e != cudaSuccess) return e;
-  } else {
+  }
+  {
     const size_t smem = fc_gram_smem(Fp, tasks_per_block, dtype == 0 ? 4 : 8);
-    dim3 gg(w.nblk_gram, ytiles);
+    const dim3 gg(F <= kFcRegMaxF ? std::min(w.nblk_gram, kLowWave) : w.nblk_gram, ytiles);
     auto gram = [&](auto kernel, const auto* x) -> cudaError_t {
       const cudaError_t ge =
           cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
       if (ge != cudaSuccess) return ge;
-      kernel<<<gg, 256, smem, s>>>(x, mask, R, F, sr, sf, Fp, rpb_gram, w.colstat, tasks_total, tasks_per_block, w.gram);
+      kernel<<<gg, 256, smem, s>>>(x, mask, R, F, sr, sf, Fp, rpb_gram, w.colstat, tasks_total, tasks_per_block,
+                                   w.nblk_gram, w.gram);
       return cudaSuccess;
     };
-    const bool mma = fc_gram_use_mma(Fp);
-    if (dtype == 0)
-      e = mma ? gram(k_fc_gram<float, true>, static_cast<const float*>(X))
-              : gram(k_fc_gram<float, false>, static_cast<const float*>(X));
-    else
-      e = mma ? gram(k_fc_gram<double, true>, static_cast<const double*>(X))
-              : gram(k_fc_gram<double, false>, static_cast<const double*>(X));
+    auto by_width = [&](auto low, const auto* x) -> cudaError_t {
+      using TIN = std::remove_cv_t<std::remove_pointer_t<decltype(x)>>;
+      constexpr bool kLow = decltype(low)::value;
+      return fc_gram_use_mma(Fp) ? gram(k_fc_gram<TIN, true, kLow>, x) : gram(k_fc_gram<TIN, false, kLow>, x);
+    };
+    auto by_form = [&](const auto* x) {
+      return F <= kFcRegMaxF ? by_width(std::true_type{}, x) : by_width(std::false_type{}, x);
+    };
+    e = dtype == 0 ? by_form(static_cast<const float*>(X)) : by_form(static_cast<const double*>(X));
     if (e != cudaSuccess) return e;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
-  if ((e = cudaMemsetAsync(w.fb_count, 0, sizeof(int), s)) != cudaSuccess) return e;
   k_fc_final<<<(F * F * 32 + 255) / 256, 256, 0, s>>>(w.gram, w.nblk_gram, F, Fp, w.colstat, out, w.fb_list,
                                                       w.fb_count, flags);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -1362,6 +1382,30 @@ __global__ void __launch_bounds__(256, 3) k_fcb_gram(const FcBatchPanel* __restr
                     Blk{a.local % q.w.nblk_gram, a.local / q.w.nblk_gram, q.w.nblk_gram});
 }
 
+// The staged pass of the panels of the register form's widths that need it
+// (fc_staged): one wave of blocks goes through the panels, whose tests its
+// threads make in parallel, and shares out the row blocks of each such panel.
+template <typename TIN>
+__global__ void __launch_bounds__(256, 3) k_fcb_gram_low(const FcBatchPanel* __restrict__ P, int np) {
+  __shared__ uint8_t low[256];
+  for (int p0 = 0; p0 < np; p0 += 256) {
+    const int p = p0 + static_cast<int>(threadIdx.x);
+    low[threadIdx.x] = p < np && P[p].F <= kFcRegMaxF && fc_staged(P[p].w.colstat, P[p].F) ? 1 : 0;
+    __syncthreads();
+    for (int k = 0; k < min(256, np - p0); ++k) {
+      if (low[k] == 0) continue;  // uniform
+      const FcBatchPanel& q = P[p0 + k];
+      for (int b = static_cast<int>(blockIdx.x); b < q.w.nblk_gram * q.ytiles; b += static_cast<int>(gridDim.x)) {
+        fc_gram_body<TIN>(static_cast<const TIN*>(q.X), q.mask, q.R, q.F, 1, q.R, q.Fp, q.rpb_gram, q.w.colstat,
+                          q.tasks_total, q.tasks_per_block, q.w.gram,
+                          Blk{b % q.w.nblk_gram, b / q.w.nblk_gram, q.w.nblk_gram});
+        __syncthreads();
+      }
+    }
+    __syncthreads();
+  }
+}
+
 __global__ void k_fcb_final(const FcBatchPanel* __restrict__ P, const int* __restrict__ off, int np) {
   const FcbAt a = fcb_at(P, off, np);
   const FcBatchPanel& q = *a.q;
@@ -1428,6 +1472,8 @@ FcBatchPanel fc_batch_panel(const void* X, const uint8_t* mask, long long R, int
   const long long ms = fc_col_stride(R);
   q.rpb_cols = ((R + ms - 1) / ms + w.nblk_cols - 1) / w.nblk_cols;
   q.rpb_gram = (R + w.nblk_gram - 1) / w.nblk_gram;
+  const int nreg = fc_reg_blocks(w.nblk_gram);
+  q.rpb_reg = (R + nreg - 1) / nreg;
   q.maxpairs = F * (F + 1) / 2;
   q.fb_nblk = fc_fb_nblk(R, F);
   // the same choice of fallback as launch_factor_corr_strided
@@ -1439,9 +1485,10 @@ FcBatchPanel fc_batch_panel(const void* X, const uint8_t* mask, long long R, int
 void fc_batch_grids(const FcBatchPanel& q, int (&blocks)[kFcbGrids]) {
   blocks[kFcbCols] = q.w.nblk_cols;
   blocks[kFcbColFinal] = (q.F * 32 + 127) / 128;
-  for (int k = kFcbReg; k < kFcbGrids; ++k) blocks[k] = 0;
-  blocks[kFcbGram] = q.F <= kFcRegMaxF ? 0 : q.w.nblk_gram * q.ytiles;
-  if (q.F <= kFcRegMaxF) blocks[kFcbReg + fc_reg_kind(q.F)] = q.w.nblk_gram;
+  for (int k = 0; k < kFcRegKinds; ++k) blocks[kFcbReg + k] = 0;
+  blocks[q.F <= kFcRegMaxF ? kFcbLow : kFcbGram] = q.w.nblk_gram * q.ytiles;
+  blocks[q.F <= kFcRegMaxF ? kFcbGram : kFcbLow] = 0;
+  if (q.F <= kFcRegMaxF) blocks[kFcbReg + fc_reg_kind(q.F)] = fc_reg_blocks(q.w.nblk_gram);
   blocks[kFcbFinal] = (q.F * q.F * 32 + 255) / 256;
   blocks[kFcbFbPass] = q.large ? q.fb_ysl * q.fb_nblk : 0;
   blocks[kFcbFbPair] = q.large ? (q.maxpairs * 32 + 127) / 128 : 0;
@@ -1463,21 +1510,23 @@ cudaError_t launch_factor_corr_batch(const FcBatchPanel* d_panels, int np, const
     k_fcb_colfinal<<<total[kFcbColFinal], 128, 0, s>>>(d_panels, off(kFcbColFinal), np);
     if (chk() != cudaSuccess) return e;
   }
-  if (total[kFcbGram] > 0) {
-    if (f32) {
-      if ((e = cudaFuncSetAttribute(k_fcb_gram<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(gram_smem))) != cudaSuccess)
-        return e;
-      k_fcb_gram<float><<<total[kFcbGram], 256, gram_smem, s>>>(d_panels, off(kFcbGram), np);
-    } else {
-      if ((e = cudaFuncSetAttribute(k_fcb_gram<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(gram_smem))) != cudaSuccess)
-        return e;
-      k_fcb_gram<double><<<total[kFcbGram], 256, gram_smem, s>>>(d_panels, off(kFcbGram), np);
-    }
-    if (chk() != cudaSuccess) return e;
+  auto staged = [&](auto* kernel, int grid, auto... args) -> cudaError_t {
+    const cudaError_t r =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gram_smem));
+    if (r != cudaSuccess) return r;
+    kernel<<<grid, 256, gram_smem, s>>>(d_panels, args...);
+    return cudaGetLastError();
+  };
+  if (total[kFcbGram] > 0 &&
+      (e = f32 ? staged(k_fcb_gram<float>, total[kFcbGram], off(kFcbGram), np)
+               : staged(k_fcb_gram<double>, total[kFcbGram], off(kFcbGram), np)) != cudaSuccess)
+    return e;
+  if (total[kFcbLow] > 0) {
+    const int grid = std::min(total[kFcbLow], kLowWave);
+    if ((e = f32 ? staged(k_fcb_gram_low<float>, grid, np) : staged(k_fcb_gram_low<double>, grid, np)) != cudaSuccess)
+      return e;
   }
-  for (int k = 0; k < kFcbGrids - kFcbReg; ++k)
+  for (int k = 0; k < kFcRegKinds; ++k)
     if (total[kFcbReg + k] > 0 &&
         (e = launch_fc_gram_reg_batch(k, dtype, d_panels, off(kFcbReg + k), np, total[kFcbReg + k], s)) != cudaSuccess)
       return e;

@@ -74,11 +74,13 @@ size_t sc_pairs_bytes(int N);
 // out of the domain, see the summary).
 cudaError_t launch_stock_corr(const void* X, int dtype, const uint8_t* mask, int T, int N, const ScWork& w, double* out,
                               cudaStream_t s);
+// Column statistics of the sampled rows.  rows: those with some valid factor
+// (in the entries of factor 0).
 struct FcColPart {
-  double count, s, c, min, max;
+  double count, s, c, rows;
 };
 struct FcColStat {
-  double count, mean, min, max;
+  double count, mean, rows;
 };
 struct FcWork {
   int nblk_cols, nblk_gram;
@@ -86,26 +88,29 @@ struct FcWork {
   FcColStat* colstat;  // [F]
   double* gram;        // [nblk_gram][4][Fp][Fp]
   int* fb_list;        // [F*F]
-  int* fb_count;       // [1]
+  int* fb_count;       // [2]: flagged pairs; column blocks that are done
   double* fb_part;     // fc_fb_part_doubles(R, F) doubles, or nullptr (single-block fallback)
 };
 // Up to this many factors the Gram pass keeps its sums in registers
 // (factor_gram.cu).
 constexpr int kFcRegMaxF = 12;
-// Row blocks of factor_corr's Gram pass: two per SM for the register form (a
-// block's final reduction costs as much as about ten of its rows per thread);
-// staged panels of F <= 32 fill the SMs several times over (their tile is
-// small).  The same count everywhere keeps single-panel and batched results
+// Row blocks of factor_corr's Gram pass: staged panels of F <= 32 fill the SMs
+// several times over (their tile is small); the register form takes two per SM
+// of them (a block's final reduction costs as much as about ten of its rows per
+// thread).  The same count everywhere keeps single-panel and batched results
 // identical.
 inline int fc_gram_blocks(long long R, int F) {
-  const long long cap = F <= kFcRegMaxF ? 296 : F <= 32 ? 888 : 148;
+  const long long cap = F <= 32 ? 888 : 148;
   long long nb = R / 1024;
   if (nb < 1) nb = 1;
   return static_cast<int>(nb < cap ? nb : cap);
 }
+__host__ __device__ inline int fc_reg_blocks(int gram_blocks) { return gram_blocks < 296 ? gram_blocks : 296; }
 // Column statistics come from a sample of the rows (every fc_col_stride-th, at
 // most about 16384): the mean is only the shift of the centred sums.
 __host__ __device__ inline long long fc_col_stride(long long R) { return R / 16384 > 1 ? R / 16384 : 1; }
+// (at most kFcColRows sampled rows a block)
+constexpr int kFcColRows = 256;
 inline int fc_col_blocks(long long R) {
   const long long rows = (R + fc_col_stride(R) - 1) / fc_col_stride(R), nb = rows / 128;
   return static_cast<int>(nb < 1 ? 1 : nb < 148 ? nb : 148);
@@ -124,7 +129,7 @@ struct FcBatchPanel {
   const uint8_t* mask;
   long long R;
   int F, Fp;
-  long long rpb_cols, rpb_gram;   // rows per column / Gram block
+  long long rpb_cols, rpb_gram, rpb_reg;  // rows per column / staged / register Gram block
   int tasks_total, tasks_per_block, ytiles;
   int maxpairs, fb_nblk, fb_ysl;  // flagged-pair slots, fallback row blocks, pair slots per row block
   int large;                      // 1: multi-block fallback, 0: one block per flagged pair
@@ -133,11 +138,12 @@ struct FcBatchPanel {
 };
 // Kinds of batched grid (prefix offsets are kept per kind).
 constexpr int kFcbCols = 0, kFcbColFinal = 1, kFcbGram = 2, kFcbFinal = 3, kFcbFbPass = 4, kFcbFbPair = 5,
-              kFcbSmall = 6, kFcbReg = 7, kFcbGrids = 12;  // kFcbReg: the register form, one kind per fc_reg_kind
+              kFcbSmall = 6, kFcbReg = 7, kFcRegKinds = 5,  // kFcbReg: the register form, one kind per fc_reg_kind
+              kFcbLow = kFcbReg + kFcRegKinds, kFcbGrids = kFcbLow + 1;  // kFcbLow: its panels, staged (fc_staged)
 FcBatchPanel fc_batch_panel(const void* X, const uint8_t* mask, long long R, int F, const FcWork& w, double* out);
 // Blocks the panel contributes to each kind of batched grid.
 void fc_batch_grids(const FcBatchPanel& q, int (&blocks)[kFcbGrids]);
-// Up to nine launches for every panel: d_off holds kFcbGrids runs of np + 1
+// Up to ten launches for every panel: d_off holds kFcbGrids runs of np + 1
 // prefix offsets, total the grid sizes (host), gram_smem the largest Gram
 // staging of the panels; results equal launch_factor_corr_strided's per panel.
 cudaError_t launch_factor_corr_batch(const FcBatchPanel* d_panels, int np, const int* d_off, const int* total,

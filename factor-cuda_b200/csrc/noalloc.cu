@@ -37,7 +37,7 @@ constexpr size_t kOffColStat = al256(kOffColPart + size_t(kColBlocks) * kMaxF * 
 constexpr size_t kOffGram = al256(kOffColStat + size_t(kMaxF) * sizeof(fcb::FcColStat));
 constexpr size_t kOffFbList = al256(kOffGram + size_t(kGramBlocks) * 4 * kMaxFp * kMaxFp * sizeof(double));
 constexpr size_t kOffFbCount = al256(kOffFbList + size_t(kMaxF) * kMaxF * sizeof(int));
-constexpr size_t kOffFbPart = al256(kOffFbCount + sizeof(int));
+constexpr size_t kOffFbPart = al256(kOffFbCount + 2 * sizeof(int));
 constexpr size_t kFbPartDoubles =
     size_t(kMaxPairs) * fcb::kFcFbMaxNblk * fcb::kFcFbPartDoubles + size_t(kMaxPairs) * 4;
 constexpr size_t kFcNoallocScratchBytes = al256(kOffFbPart + kFbPartDoubles * sizeof(double));
