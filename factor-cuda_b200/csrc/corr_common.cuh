@@ -3,7 +3,6 @@
 #pragma once
 
 #include "fcb_common.cuh"
-#include "fcb_kernels.h"
 
 namespace fcb {
 
@@ -69,25 +68,6 @@ FCB_DEV PairResult finalize_pair(double n, double sx, double sy, double sxy, dou
   const bool small = n * mux * mux <= 1e12 * vx && n * muy * muy <= 1e12 * vy;
   const bool redo = degenerate || !near || (gate && !small);
   return PairResult{redo ? dnan() : r, gate || degenerate, redo};
-}
-
-// Up to kFcRegMaxF factors: whether the Gram pass takes the staged form after
-// all, by the sampled rows with some valid factor.  Every cell that such a row
-// misses costs the register form a trip through its queue, and a pair's sums
-// lose digits as the rows that the other factor misses are taken away.  With
-// every cell missing alike the two forms meet at 12 to 15 % (1218 x 5000 x 12:
-// 656 us at 10 % and 878 at 15 % against 820 staged; x 5: 340 and 452 against
-// 390), so staged above 10 %, or where a factor has less than two thirds of the
-// rows: of the others, any two share at least half of either's rows.
-FCB_DEV bool fc_staged(const FcColStat* st, int F) {
-  const double rows = st[0].rows;
-  double missing = 0.0;
-  bool low = false;
-  for (int f = 0; f < F; ++f) {
-    missing += rows - st[f].count;
-    low = low || 3.0 * st[f].count < 2.0 * rows;
-  }
-  return low || 10.0 * missing > F * rows;
 }
 
 FCB_DEV void dmma_f64(double (&d)[2], double a, double b) {

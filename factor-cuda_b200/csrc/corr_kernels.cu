@@ -174,8 +174,10 @@ FCB_DEV void fc_colpart_body(const TIN* __restrict__ X, const uint8_t* __restric
 }
 
 // One warp per column f: lane l merges partials l, l+32, ... in order, then a
-// fixed shuffle tree merges the lanes.
-FCB_DEV void fc_colfinal_warp(const FcColPart* part, int nblk, int F, FcColStat* __restrict__ st, int f) {
+// fixed shuffle tree merges the lanes.  fc_sh: count of each factor (up to
+// kFcRegMaxF), then the rows.
+FCB_DEV void fc_colfinal_warp(const FcColPart* part, int nblk, int F, FcColStat* __restrict__ st, int f,
+                              double (&fc_sh)[kFcRegMaxF + 1]) {
   const int lane = threadIdx.x & 31;
   Kahan k;
   double cnt = 0.0, rows = 0.0;
@@ -200,16 +202,48 @@ FCB_DEV void fc_colfinal_warp(const FcColPart* part, int nblk, int F, FcColStat*
       rows += orows;
     }
   }
-  if (lane == 0) st[f] = FcColStat{cnt, cnt > 0.0 ? k.s / cnt : 0.0, rows};
+  if (lane != 0) return;
+  st[f].count = cnt;
+  st[f].mean = cnt > 0.0 ? k.s / cnt : 0.0;
+  if (F <= kFcRegMaxF) {
+    fc_sh[f] = cnt;
+    if (f == 0) fc_sh[kFcRegMaxF] = rows;
+  }
 }
-FCB_DEV void fc_colfinal_body(const FcColPart* __restrict__ part, int nblk, int F, FcColStat* __restrict__ st,
-                              const Blk bk) {
-  const int f = (bk.x * blockDim.x + threadIdx.x) >> 5;
-  if (f < F) fc_colfinal_warp(part, nblk, F, st, f);  // whole warps
+
+// Up to kFcRegMaxF factors: whether the Gram pass takes the staged form after
+// all, by the sampled rows with some valid factor.  Every cell that such a row
+// misses costs the register form a trip through its queue, and a pair's sums
+// lose digits as the rows that the other factor misses are taken away.  With
+// every cell missing alike the two forms meet at 12 to 15 % (1218 x 5000 x 12:
+// 656 us a call at 10 % and 878 at 15 % against 715 staged; x 5: 340 and 452
+// against 390), so staged above 10 %, or where a factor has less than two
+// thirds of the rows: of the others, any two share at least half of either's
+// rows.
+FCB_DEV bool fc_stage_rule(const double (&fc_sh)[kFcRegMaxF + 1], int F) {
+  const double rows = fc_sh[kFcRegMaxF];
+  double missing = 0.0;
+  bool low = false;
+  for (int f = 0; f < F; ++f) {
+    missing += rows - fc_sh[f];
+    low = low || 3.0 * fc_sh[f] < 2.0 * rows;
+  }
+  return low || 10.0 * missing > F * rows;
+}
+
+// Up to kFcRegMaxF factors one block takes all.
+FCB_DEV void fc_colfinal_body(const FcColPart* part, int nblk, int F, FcColStat* __restrict__ st, const Blk bk) {
+  __shared__ double fc_sh[kFcRegMaxF + 1];
+  const int tid = static_cast<int>(threadIdx.y * blockDim.x + threadIdx.x), nt = static_cast<int>(blockDim.x * blockDim.y);
+  for (int f = (bk.x * nt + tid) >> 5; f < F; f += F <= kFcRegMaxF ? nt >> 5 : F)
+    fc_colfinal_warp(part, nblk, F, st, f, fc_sh);
+  if (F > kFcRegMaxF) return;
+  __syncthreads();
+  if (tid == 0) st[0].staged = fc_stage_rule(fc_sh, F) ? 1 : 0;
 }
 
 // done (zero before): the last block to write its partials merges them as well
-// (a launch less, 2 to 3 us; few factors: its warps take them in turn), or null.
+// (few factors, a warp each: a launch less), or null.
 template <typename TIN>
 __global__ void k_fc_colpart(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, long long R, int F,
                              long long sr, long long sf, long long ms, long long rows_per_block,
@@ -223,8 +257,7 @@ __global__ void k_fc_colpart(const TIN* __restrict__ X, const uint8_t* __restric
   __syncthreads();
   if (!last) return;
   __threadfence();
-  for (int f = static_cast<int>(threadIdx.y); f < F; f += static_cast<int>(blockDim.y))
-    fc_colfinal_warp(part, static_cast<int>(gridDim.x), F, st, f);
+  fc_colfinal_body(part, static_cast<int>(gridDim.x), F, st, Blk{0, 0, 1});
 }
 
 __global__ void k_fc_colfinal(const FcColPart* __restrict__ part, int nblk, int F, FcColStat* __restrict__ st) {
@@ -652,7 +685,7 @@ FCB_DEV void fc_gram_body(const TIN* __restrict__ X, const uint8_t* __restrict__
 
 // Single panel: the path is chosen on the host (MMA = fc_gram_use_mma(Fp)), so
 // each instantiation holds one body.  LOW: a panel of the register form's
-// widths, staged only if fc_staged says so; one wave of blocks goes through the
+// widths, staged only by fc_stage_rule; one wave of blocks goes through the
 // nblk row blocks.
 template <typename TIN, bool MMA, bool LOW>
 __global__ void __launch_bounds__(256, 3) k_fc_gram(const TIN* __restrict__ X, const uint8_t* __restrict__ mask,
@@ -660,7 +693,7 @@ __global__ void __launch_bounds__(256, 3) k_fc_gram(const TIN* __restrict__ X, c
                                                  long long rows_per_block,
                                                  const FcColStat* __restrict__ st, int tasks_total,
                                                  int tasks_per_block, int nblk, double* __restrict__ part) {
-  if (LOW && !fc_staged(st, F)) return;
+  if (LOW && st[0].staged == 0) return;
   for (Blk bk = launch_blk(); bk.x < nblk; bk.x += static_cast<int>(gridDim.x)) {
     if (MMA)
       fc_gram_body_mma<TIN>(X, mask, R, F, sr, sf, Fp, rows_per_block, st, tasks_total, tasks_per_block, part, bk);
@@ -683,7 +716,7 @@ FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int
   if (e >= F * F) return;  // whole warps exit together
   const int i = e / F, j = e % F;
   if (i > j) return;
-  const bool reg = F <= kFcRegMaxF && !fc_staged(st, F);
+  const bool reg = F <= kFcRegMaxF && st[0].staged == 0;
   if (reg) nblk = fc_reg_blocks(nblk);
   double q[6] = {0, 0, 0, 0, 0, 0}, tot[2] = {0, 0};  // tot: sums of squares of each factor's own rows
   // q: n, sx (x'_i m_j), sy (m_i x'_j), sxy, sx2 (x'^2_i m_j), sy2 (m_i x'^2_j)
@@ -726,7 +759,7 @@ FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int
     p = finalize_pair(q[0], q[1], q[2], q[3], q[4], q[5], mui, muj);
     // The register form's sums are totals less the rows that the other factor
     // misses: where less than half is left (an outlier among those rows, as a
-    // rule: see fc_staged), their rounding shows.
+    // rule: see fc_stage_rule), their rounding shows.
     // The staged form's longer chains lose more than the two-pass values of
     // gated pairs do (rms error 4.7e-18 against 2.7e-18 at 20 factors).
     const bool again = reg ? tot[0] * 0.5 > q[4] || tot[1] * 0.5 > q[5] : p.gate;
@@ -1241,7 +1274,7 @@ cudaError_t launch_factor_corr_strided(const void* X, int dtype, const uint8_t* 
   const long long rpb_cols = (rs + w.nblk_cols - 1) / w.nblk_cols;
   const long long rpb_gram = (R + w.nblk_gram - 1) / w.nblk_gram;
   const int nreg = fc_reg_blocks(w.nblk_gram);
-  dim3 cb(32, 8);
+  const dim3 cb(32, std::max(8, std::min(F, kFcRegMaxF)));
   cudaError_t e = cudaMemsetAsync(w.fb_count, 0, 2 * sizeof(int), s);
   if (e != cudaSuccess) return e;
   int* done = F <= kFcRegMaxF ? w.fb_count + 1 : nullptr;
@@ -1383,14 +1416,14 @@ __global__ void __launch_bounds__(256, 3) k_fcb_gram(const FcBatchPanel* __restr
 }
 
 // The staged pass of the panels of the register form's widths that need it
-// (fc_staged): one wave of blocks goes through the panels, whose tests its
+// (fc_stage_rule): one wave of blocks goes through the panels, whose tests its
 // threads make in parallel, and shares out the row blocks of each such panel.
 template <typename TIN>
 __global__ void __launch_bounds__(256, 3) k_fcb_gram_low(const FcBatchPanel* __restrict__ P, int np) {
   __shared__ uint8_t low[256];
   for (int p0 = 0; p0 < np; p0 += 256) {
     const int p = p0 + static_cast<int>(threadIdx.x);
-    low[threadIdx.x] = p < np && P[p].F <= kFcRegMaxF && fc_staged(P[p].w.colstat, P[p].F) ? 1 : 0;
+    low[threadIdx.x] = p < np && P[p].F <= kFcRegMaxF && P[p].w.colstat[0].staged != 0 ? 1 : 0;
     __syncthreads();
     for (int k = 0; k < min(256, np - p0); ++k) {
       if (low[k] == 0) continue;  // uniform
@@ -1484,7 +1517,7 @@ FcBatchPanel fc_batch_panel(const void* X, const uint8_t* mask, long long R, int
 
 void fc_batch_grids(const FcBatchPanel& q, int (&blocks)[kFcbGrids]) {
   blocks[kFcbCols] = q.w.nblk_cols;
-  blocks[kFcbColFinal] = (q.F * 32 + 127) / 128;
+  blocks[kFcbColFinal] = q.F <= kFcRegMaxF ? 1 : (q.F * 32 + 127) / 128;
   for (int k = 0; k < kFcRegKinds; ++k) blocks[kFcbReg + k] = 0;
   blocks[q.F <= kFcRegMaxF ? kFcbLow : kFcbGram] = q.w.nblk_gram * q.ytiles;
   blocks[q.F <= kFcRegMaxF ? kFcbGram : kFcbLow] = 0;

@@ -13,9 +13,8 @@
 // adds a full queue to the sums of the factors that its rows miss.  All sums
 // are formed in a fixed order.
 // Panels of which more than a few cells are missing take the staged pass
-// instead (fc_staged, decided on the device: both are launched, and one returns
-// at once; a call at 1218 x 5000 x 12 took 216 us without the choice and 221 with
-// it, and one with every cell missing at 70 % 5009 and 660).
+// instead (fc_stage_rule, decided on the device: both are launched, and one
+// returns at once).
 // Per block the same partials come out as from the staged pass
 // (fc_gram_body): P[product][i][j] with product 0 n, 1 sum x'_i over rows where
 // j is valid, 2 sum x'_i^2 likewise, 3 sum x'_i x'_j.
@@ -192,7 +191,7 @@ FCB_DEV void gram_reg_body(const TIN* __restrict__ X, const uint8_t* __restrict_
                            long long sf, int Fp, long long rows_per_block, const FcColStat* __restrict__ st,
                            double* __restrict__ part, int bx, uint8_t* smem) {
   using S = RegShape<FP>;
-  if (fc_staged(st, F)) return;  // uniform: the staged pass writes the partials
+  if (st[0].staged != 0) return;  // uniform: the staged pass writes the partials
   RegWarp<FP>* warps = reinterpret_cast<RegWarp<FP>*>(smem);
   const int tid = static_cast<int>(threadIdx.x), lane = tid & 31, wi = tid >> 5;
   RegWarp<FP>& w = warps[wi];

@@ -74,13 +74,14 @@ size_t sc_pairs_bytes(int N);
 // out of the domain, see the summary).
 cudaError_t launch_stock_corr(const void* X, int dtype, const uint8_t* mask, int T, int N, const ScWork& w, double* out,
                               cudaStream_t s);
-// Column statistics of the sampled rows.  rows: those with some valid factor
-// (in the entries of factor 0).
+// Column statistics of the sampled rows.  In the entries of factor 0: rows,
+// those with some valid factor; staged, the form of the Gram pass (fc_stage_rule).
 struct FcColPart {
   double count, s, c, rows;
 };
 struct FcColStat {
-  double count, mean, rows;
+  double count, mean;
+  int staged;
 };
 struct FcWork {
   int nblk_cols, nblk_gram;
@@ -139,7 +140,7 @@ struct FcBatchPanel {
 // Kinds of batched grid (prefix offsets are kept per kind).
 constexpr int kFcbCols = 0, kFcbColFinal = 1, kFcbGram = 2, kFcbFinal = 3, kFcbFbPass = 4, kFcbFbPair = 5,
               kFcbSmall = 6, kFcbReg = 7, kFcRegKinds = 5,  // kFcbReg: the register form, one kind per fc_reg_kind
-              kFcbLow = kFcbReg + kFcRegKinds, kFcbGrids = kFcbLow + 1;  // kFcbLow: its panels, staged (fc_staged)
+              kFcbLow = kFcbReg + kFcRegKinds, kFcbGrids = kFcbLow + 1;  // kFcbLow: its panels, staged (fc_stage_rule)
 FcBatchPanel fc_batch_panel(const void* X, const uint8_t* mask, long long R, int F, const FcWork& w, double* out);
 // Blocks the panel contributes to each kind of batched grid.
 void fc_batch_grids(const FcBatchPanel& q, int (&blocks)[kFcbGrids]);
