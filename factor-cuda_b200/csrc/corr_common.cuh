@@ -26,6 +26,34 @@ struct Kahan {
   }
 };
 
+// A sum with its rounding errors (two-sum): s + c is the sum to about twice
+// the precision.
+struct TwoSum {
+  double s = 0.0, c = 0.0;
+  FCB_DEV void add(double x) {
+    const double t = s + x, b = t - s;
+    c += (s - (t - b)) + (x - b);
+    s = t;
+  }
+  FCB_DEV double value() const { return s + c; }
+  // the sum less a * b, with one rounding of the size of the sum
+  FCB_DEV double less_product(double a, double b) const {
+    const double p = a * b, e = fma(a, b, -p);
+    TwoSum r = *this;
+    r.add(-p);
+    return r.s + (r.c - e);
+  }
+  // the warp's total, the same in every lane
+  FCB_DEV void warp_total() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double s2 = __shfl_xor_sync(kFull, s, o), c2 = __shfl_xor_sync(kFull, c, o);
+      c += c2;
+      add(s2);
+    }
+  }
+};
+
 FCB_DEV double dnan() { return __longlong_as_double(0x7ff8000000000000ll); }
 
 FCB_DEV double safe_pearson(double sxy, double sxx, double syy) {
@@ -44,13 +72,9 @@ struct PairResult {
   double r;
   bool gate, redo;
 };
-FCB_DEV PairResult finalize_pair(double n, double sx, double sy, double sxy, double sx2, double sy2, double mux,
-                                 double muy) {
-  if (n < 2.0) return PairResult{dnan(), false, false};
-  const double rn = 1.0 / n, mx = sx * rn, my = sy * rn;  // one division for all
-  const double cov = fma(-mx, sy, sxy);
-  const double vx = fma(-mx, sx, sx2);
-  const double vy = fma(-my, sy, sy2);
+// cov, vx, vy: the sums about the joint means (mx, my from the shifts, rn = 1 / n).
+FCB_DEV PairResult finalize_about_means(double n, double rn, double mx, double my, double sx, double sy, double cov,
+                                        double vx, double vy, double sx2, double sy2, double mux, double muy) {
   // uncentred sums of the reference's one-pass Gram, reconstructed
   const double sxr = sx + n * mux;
   const double syr = sy + n * muy;
@@ -68,6 +92,14 @@ FCB_DEV PairResult finalize_pair(double n, double sx, double sy, double sxy, dou
   const bool small = n * mux * mux <= 1e12 * vx && n * muy * muy <= 1e12 * vy;
   const bool redo = degenerate || !near || (gate && !small);
   return PairResult{redo ? dnan() : r, gate || degenerate, redo};
+}
+
+FCB_DEV PairResult finalize_pair(double n, double sx, double sy, double sxy, double sx2, double sy2, double mux,
+                                 double muy) {
+  if (n < 2.0) return PairResult{dnan(), false, false};
+  const double rn = 1.0 / n, mx = sx * rn, my = sy * rn;  // one division for all
+  return finalize_about_means(n, rn, mx, my, sx, sy, fma(-mx, sy, sxy), fma(-mx, sx, sx2), fma(-my, sy, sy2), sx2, sy2,
+                              mux, muy);
 }
 
 FCB_DEV void dmma_f64(double (&d)[2], double a, double b) {

@@ -586,27 +586,6 @@ __global__ void __launch_bounds__(256, 4)
 // ---------------------------------------------------------------------------
 // two-pass fallback of the flagged pairs
 // ---------------------------------------------------------------------------
-// A sum with its rounding errors (two-sum): s + c is the sum to about twice
-// the precision.
-struct TwoSum {
-  double s = 0.0, c = 0.0;
-  FCB_DEV void add(double x) {
-    const double t = s + x, b = t - s;
-    c += (s - (t - b)) + (x - b);
-    s = t;
-  }
-  FCB_DEV double value() const { return s + c; }
-  // the warp's total, the same in every lane
-  FCB_DEV void warp_total() {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double s2 = __shfl_xor_sync(kFull, s, o), c2 = __shfl_xor_sync(kFull, c, o);
-      c += c2;
-      add(s2);
-    }
-  }
-};
-
 // One warp per pair, a lane every 32nd date: means from sums carried to twice
 // the precision (the mean two-pass reference's compensated sums, without
 // their serial chain: four dependent FP64 adds, 120 clocks, per date, and

@@ -104,3 +104,18 @@ def test_batch_mixes_the_forms():
         one = run(X, m, 1)
         assert np.array_equal(p["corr"].cpu().numpy().view(np.uint64), one.view(np.uint64)), k
         assert corr_match(one, O.factor_corr(X, m)), k
+
+
+# A correlation near 0.9 takes five roundings of its own, 0.29 ulps rms each; each of its three sums is exact to its
+# last rounding and a third of one for the additions in the blocks: 0.65 and sqrt(1.5) * 0.39 = 0.48 ulps, 0.8 of
+# 1.1e-16 in all.  A tenth is left for the mean and the 264 pairs.
+@pytest.mark.parametrize("mean", [0.0, 5.0, 1000.0])
+def test_precision_of_larger_pools(mean):
+    sq = []
+    for seed in range(4):
+        r = np.random.default_rng(seed)
+        T, N, F = 200, 1000, 12
+        X = mean + np.sqrt(0.9) * r.standard_normal((T, N, 1)) + np.sqrt(0.1) * r.standard_normal((T, N, F))
+        err = (run(X, None, 0).astype(np.longdouble) - exact(X))[np.triu_indices(F, 1)]
+        sq.append(np.mean(err * err))
+    assert np.sqrt(np.mean(sq)) < 1e-16
