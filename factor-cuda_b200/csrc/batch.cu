@@ -518,7 +518,7 @@ extern "C" int fcb_batch_create(const fcb_panel* panels, int npanels, int dtype_
     const long long R = static_cast<long long>(q.T) * q.N;
     const int F = q.F, Fp = (F + 3) / 4 * 4;
     FcWork& w = b->fcw[i];
-    w.nblk_cols = fc_col_blocks(R);
+    w.nblk_cols = fc_col_blocks(R, F);
     w.nblk_gram = fc_gram_blocks(R, F);
     const size_t b_colpart = static_cast<size_t>(w.nblk_cols) * F * sizeof(FcColPart);
     const size_t b_colstat = static_cast<size_t>(F) * sizeof(FcColStat);

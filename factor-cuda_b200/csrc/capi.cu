@@ -939,7 +939,7 @@ extern "C" int fcb_dev_factor_corr(const void* d_x, int dtype, const uint8_t* d_
   const long long R = static_cast<long long>(T) * N;
   const int Fp = (F + 3) / 4 * 4;
   FcWork w{};
-  w.nblk_cols = fc_col_blocks(R);
+  w.nblk_cols = fc_col_blocks(R, F);
   w.nblk_gram = fc_gram_blocks(R, F);
   FCB_TRY(ws.get(S_FC_COLPART, static_cast<size_t>(w.nblk_cols) * F * sizeof(FcColPart), &w.colpart));
   FCB_TRY(ws.get(S_FC_COLSTAT, static_cast<size_t>(F) * sizeof(FcColStat), &w.colstat));
@@ -967,7 +967,7 @@ extern "C" int fcb_factor_corr(const void* x, int dtype, const uint8_t* mask, in
   const int Fp = (F + 3) / 4 * 4;
   const size_t esz = dtype == FCB_DTYPE_F32 ? 4 : 8;
   FcWork w{};
-  w.nblk_cols = fc_col_blocks(R);
+  w.nblk_cols = fc_col_blocks(R, F);
   w.nblk_gram = fc_gram_blocks(R, F);
   void* dx;
   uint8_t* dm = nullptr;
@@ -1145,7 +1145,7 @@ inline uint64_t slot_bytes(size_t b) { return b == 0 ? 16 : b; }
 uint64_t budget_dev_factor_corr(int dtype, long long R, int F) {
   (void)dtype;
   const int Fp = (F + 3) / 4 * 4;
-  const long long nbc = fc_col_blocks(R);
+  const long long nbc = fc_col_blocks(R, F);
   const long long nbg = fc_gram_blocks(R, F);
   return slot_bytes(static_cast<size_t>(nbc) * F * sizeof(FcColPart)) + slot_bytes(static_cast<size_t>(F) * sizeof(FcColStat)) +
          slot_bytes(static_cast<size_t>(nbg) * 4 * Fp * Fp * 8) + slot_bytes(static_cast<size_t>(F) * F * 4) + 64 +

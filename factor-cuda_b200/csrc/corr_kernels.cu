@@ -110,9 +110,8 @@ FCB_DEV Blk launch_blk() {
 }
 
 // Per-block column partials over a contiguous range of the sampled rows (every
-// ms-th; R, sr and the mask index count in sampled rows; at most kFcColRows a
-// block): count and Kahan sum of each factor, and the rows with some valid
-// factor.  Rows are visited in increasing order within each thread's strided
+// ms-th; R, sr and the mask index count in sampled rows): count and Kahan sum of
+// each factor and, up to kFcRegMaxF factors, the rows with some valid factor.  Rows are visited in increasing order within each thread's strided
 // slice; partials are merged in a fixed order by k_fc_colfinal.
 template <typename TIN>
 FCB_DEV void fc_colpart_body(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, long long R, int F,
@@ -145,7 +144,7 @@ FCB_DEV void fc_colpart_body(const TIN* __restrict__ X, const uint8_t* __restric
         if (ok[u] && KeyOf<TIN>::finite(xv[u])) {
           ++cnt_i;
           k.add(static_cast<double>(xv[u]));
-          some[rb - r0 + static_cast<long long>(u) * blockDim.x] = 1;
+          if (F <= kFcRegMaxF) some[rb - r0 + static_cast<long long>(u) * blockDim.x] = 1;
         }
       }
     }
@@ -1277,7 +1276,7 @@ cudaError_t launch_factor_corr_strided(const void* X, int dtype, const uint8_t* 
   int tasks_total = 0, tasks_per_block = 0, ytiles = 0;
   fc_gram_plan(Fp, &tasks_total, &tasks_per_block, &ytiles);
   // column statistics of the sampled rows
-  const long long ms = fc_col_stride(R), rs = (R + ms - 1) / ms;
+  const long long ms = fc_col_stride(R, F), rs = fc_col_rows(R, F);
   const long long rpb_cols = (rs + w.nblk_cols - 1) / w.nblk_cols;
   const long long rpb_gram = (R + w.nblk_gram - 1) / w.nblk_gram;
   const int nreg = fc_reg_blocks(w.nblk_gram);
@@ -1400,8 +1399,8 @@ template <typename TIN>
 __global__ void k_fcb_colpart(const FcBatchPanel* __restrict__ P, const int* __restrict__ off, int np) {
   const FcbAt a = fcb_at(P, off, np);
   const FcBatchPanel& q = *a.q;
-  const long long ms = fc_col_stride(q.R);
-  fc_colpart_body<TIN>(static_cast<const TIN*>(q.X), q.mask, (q.R + ms - 1) / ms, q.F, ms, q.R, ms, q.rpb_cols,
+  const long long ms = fc_col_stride(q.R, q.F);
+  fc_colpart_body<TIN>(static_cast<const TIN*>(q.X), q.mask, fc_col_rows(q.R, q.F), q.F, ms, q.R, ms, q.rpb_cols,
                        q.w.colpart, Blk{a.local, 0, q.w.nblk_cols});
 }
 
@@ -1509,8 +1508,7 @@ FcBatchPanel fc_batch_panel(const void* X, const uint8_t* mask, long long R, int
   const int tb = q.Fp / 4;
   (void)tb;
   fc_gram_plan(q.Fp, &q.tasks_total, &q.tasks_per_block, &q.ytiles);
-  const long long ms = fc_col_stride(R);
-  q.rpb_cols = ((R + ms - 1) / ms + w.nblk_cols - 1) / w.nblk_cols;
+  q.rpb_cols = (fc_col_rows(R, F) + w.nblk_cols - 1) / w.nblk_cols;
   q.rpb_gram = (R + w.nblk_gram - 1) / w.nblk_gram;
   const int nreg = fc_reg_blocks(w.nblk_gram);
   q.rpb_reg = (R + nreg - 1) / nreg;

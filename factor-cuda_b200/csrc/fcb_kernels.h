@@ -107,14 +107,26 @@ inline int fc_gram_blocks(long long R, int F) {
   return static_cast<int>(nb < cap ? nb : cap);
 }
 __host__ __device__ inline int fc_reg_blocks(int gram_blocks) { return gram_blocks < 296 ? gram_blocks : 296; }
-// Column statistics come from a sample of the rows (every fc_col_stride-th, at
-// most about 16384): the mean is only the shift of the centred sums.
-__host__ __device__ inline long long fc_col_stride(long long R) { return R / 16384 > 1 ? R / 16384 : 1; }
-// (at most kFcColRows sampled rows a block)
+// Column statistics come from a sample of the rows, every fc_col_stride-th: the
+// mean is only the shift of the centred sums.  Up to kFcRegMaxF factors about
+// 16384 rows, at most kFcColRows a block; above, where the Gram pass takes far
+// longer, 262144: f32 values less one shift end in the same bits, so that the
+// additions of a staged chain all round the same way and sum x' is off by a share
+// of the rows; in a covariance that counts with the shift's distance from the
+// mean (200 x 700 x 16 f32, independent factors: rms error 1.5e-18 with all rows,
+// 2.0e-18 with 16384).
 constexpr int kFcColRows = 256;
-inline int fc_col_blocks(long long R) {
-  const long long rows = (R + fc_col_stride(R) - 1) / fc_col_stride(R), nb = rows / 128;
-  return static_cast<int>(nb < 1 ? 1 : nb < 148 ? nb : 148);
+__host__ __device__ inline long long fc_col_stride(long long R, int F) {
+  const long long ms = R / (F <= kFcRegMaxF ? 16384 : 262144);
+  return ms > 1 ? ms : 1;
+}
+__host__ __device__ inline long long fc_col_rows(long long R, int F) {
+  const long long ms = fc_col_stride(R, F);
+  return (R + ms - 1) / ms;
+}
+inline int fc_col_blocks(long long R, int F) {
+  const long long nb = fc_col_rows(R, F) / 128, cap = F <= kFcRegMaxF ? 148 : 296;
+  return static_cast<int>(nb < 1 ? 1 : nb < cap ? nb : cap);
 }
 // Row blocks per flagged pair of the multi-block fallback (at most
 // kFcFbMaxNblk), and the partials buffer it needs (doubles): kFcFbPartDoubles

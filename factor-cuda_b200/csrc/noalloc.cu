@@ -72,7 +72,7 @@ extern "C" int fcb_dev_factor_corr_noalloc(const void* d_x, int dtype, const uin
   if (e != cudaSuccess) return static_cast<int>(e);
   const long long R = static_cast<long long>(T) * N;
   fcb::FcWork w{};
-  w.nblk_cols = fcb::fc_col_blocks(R);
+  w.nblk_cols = std::min(kColBlocks, fcb::fc_col_blocks(R, F));
   w.nblk_gram = static_cast<int>(std::min<long long>(kGramBlocks, std::max<long long>(1, R / 1024)));
   w.colpart = reinterpret_cast<fcb::FcColPart*>(base + kOffColPart);
   w.colstat = reinterpret_cast<fcb::FcColStat*>(base + kOffColStat);

@@ -119,3 +119,15 @@ def test_precision_of_larger_pools(mean):
         err = (run(X, None, 0).astype(np.longdouble) - exact(X))[np.triu_indices(F, 1)]
         sq.append(np.mean(err * err))
     assert np.sqrt(np.mean(sq)) < 1e-16
+
+
+# 140000 rows of 16 independent f32 factors, correlations near 3e-3.  A staged chain of up to 158 rows is 9 on average
+# and its additions are off by 0.29 ulps of that: 0.29 * 1.1e-16 * 9 / sqrt(140000) = 0.8e-18; twice that for the
+# matrix instruction's own additions, and a tenth for the 480 pairs.
+def test_precision_of_f32_staged_sums():
+    sq = []
+    for seed in range(4):
+        X = np.random.default_rng(seed).standard_normal((200, 700, 16)).astype(np.float32)
+        err = (run(X, None, 0).astype(np.longdouble) - exact(X))[np.triu_indices(16, 1)]
+        sq.append(np.mean(err * err))
+    assert np.sqrt(np.mean(sq)) < 1.75e-18
