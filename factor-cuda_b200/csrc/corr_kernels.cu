@@ -705,16 +705,19 @@ __global__ void __launch_bounds__(256, 3) k_fc_gram(const TIN* __restrict__ X, c
 
 // Sum the per-block Gram partials in block order (nblk of the staged form),
 // finalize each pair.
-// One warp per (i <= j) pair: lane l sums blocks l, l+32, ..., a fixed
-// shuffle tree sums the lanes, lane 0 finalizes.
+// Two warps per (i <= j) pair: lane l of 64 sums blocks l, l+64, ..., a fixed
+// shuffle tree sums a warp's lanes, the first warp's lane 0 adds the second's
+// totals and finalizes.  At most 256 threads a block.
+constexpr int kFinalThreads = 64;
 FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int Fp,
                            const FcColStat* __restrict__ st, double* __restrict__ out, int* __restrict__ fb_list,
                            int* __restrict__ fb_count, uint8_t* __restrict__ flags, const Blk bk) {
-  const int e = (bk.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (e >= F * F) return;  // whole warps exit together
+  __shared__ double second[256 / kFinalThreads][13];
+  const int e = (bk.x * blockDim.x + threadIdx.x) / kFinalThreads;
+  const int t = threadIdx.x % kFinalThreads;
   const int i = e / F, j = e % F;
-  if (i > j) return;
+  const bool act = e < F * F && i <= j;  // uniform across the pair's warps
+  if (!__syncthreads_or(act)) return;
   const bool reg = F <= kFcRegMaxF && st[0].staged == 0;
   if (reg) nblk = fc_reg_blocks(nblk);
   // n, sx (x'_i m_j), sy (m_i x'_j), sxy, sx2 (x'^2_i m_j), sy2 (m_i x'^2_j).  The
@@ -725,7 +728,7 @@ FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int
   TwoSum acc[5];
   double n = 0.0, tot[2] = {0.0, 0.0};  // tot: sums of squares of each factor's own rows
 #pragma unroll 4
-  for (int b = lane; b < nblk; b += 32) {
+  for (int b = act ? t : nblk; b < nblk; b += kFinalThreads) {
     const double* P = part + static_cast<size_t>(b) * 4 * Fp * Fp;
     n += P[(0 * Fp + i) * Fp + j];
     acc[0].add(P[(1 * Fp + i) * Fp + j]);
@@ -736,16 +739,34 @@ FCB_DEV void fc_final_body(const double* __restrict__ part, int nblk, int F, int
     tot[0] += P[(2 * Fp + i) * Fp + i];
     tot[1] += P[(2 * Fp + j) * Fp + j];
   }
-  double q[6];
-  q[0] = warp_sum(n);
+  n = warp_sum(n);
 #pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    acc[k].warp_total();
-    q[k + 1] = acc[k].value();
-  }
+  for (int k = 0; k < 5; ++k) acc[k].warp_total();
   tot[0] = warp_sum(tot[0]);
   tot[1] = warp_sum(tot[1]);
-  if (lane != 0) return;
+  double* o = second[threadIdx.x / kFinalThreads];
+  if (t == 32) {
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      o[2 * k] = acc[k].s;
+      o[2 * k + 1] = acc[k].c;
+    }
+    o[10] = n;
+    o[11] = tot[0];
+    o[12] = tot[1];
+  }
+  __syncthreads();
+  if (t != 0 || !act) return;
+  double q[6];
+  q[0] = n + o[10];
+  tot[0] += o[11];
+  tot[1] += o[12];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    acc[k].c += o[2 * k + 1];
+    acc[k].add(o[2 * k]);
+    q[k + 1] = acc[k].value();
+  }
   PairResult p{dnan(), false, false};
   const double mui = st[i].mean, muj = st[j].mean;
   if (i == j) {
@@ -1322,7 +1343,7 @@ cudaError_t launch_factor_corr_strided(const void* X, int dtype, const uint8_t* 
     if (e != cudaSuccess) return e;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
-  k_fc_final<<<(F * F * 32 + 63) / 64, 64, 0, s>>>(w.gram, w.nblk_gram, F, Fp, w.colstat, out, w.fb_list,
+  k_fc_final<<<F * F, kFinalThreads, 0, s>>>(w.gram, w.nblk_gram, F, Fp, w.colstat, out, w.fb_list,
                                                       w.fb_count, flags);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const int maxpairs = F * (F + 1) / 2;
@@ -1527,7 +1548,7 @@ void fc_batch_grids(const FcBatchPanel& q, int (&blocks)[kFcbGrids]) {
   blocks[q.F <= kFcRegMaxF ? kFcbLow : kFcbGram] = q.w.nblk_gram * q.ytiles;
   blocks[q.F <= kFcRegMaxF ? kFcbGram : kFcbLow] = 0;
   if (q.F <= kFcRegMaxF) blocks[kFcbReg + fc_reg_kind(q.F)] = fc_reg_blocks(q.w.nblk_gram);
-  blocks[kFcbFinal] = (q.F * q.F * 32 + 255) / 256;
+  blocks[kFcbFinal] = (q.F * q.F * kFinalThreads + 255) / 256;
   blocks[kFcbFbPass] = q.large ? q.fb_ysl * q.fb_nblk : 0;
   blocks[kFcbFbPair] = q.large ? (q.maxpairs * 32 + 127) / 128 : 0;
   blocks[kFcbSmall] = q.large ? 0 : q.maxpairs;
