@@ -59,6 +59,7 @@ struct ScSummary {
   int masked;                      // some cell is invalid
   int flagged;                     // pairs that the two-pass fallback recomputes
   int gated;                       // pairs that fail the cancellation gate
+  int direct;                      // pair sums to be formed over the joint dates (of one block of columns)
 };
 struct ScWork {
   double *xraw, *xc;  // (N,Tp) column-major values, as they are and centred; Tp = T rounded to 32

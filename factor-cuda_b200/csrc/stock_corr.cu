@@ -11,10 +11,11 @@
 //     dates as a rule, so k_sc_pairsum adds up short lists: one CTA keeps the
 //     centred values of 16 columns in shared memory ([date][16], and the sums
 //     of every 32 dates) and walks every column's list of missing dates (of
-//     valid dates where more than a quarter is missing); 32 dates that are
-//     all on the list count as one entry.  Where what is taken away is more than three
-//     quarters of the column's sum of squares, the pair's sums are formed over
-//     the joint dates directly, so that the subtraction costs at most two bits.
+//     valid dates where more than a sixth is missing); 32 dates that are
+//     all on the list count as one entry.  Where what is taken away is more than a
+//     quarter of the column's sum of squares (an outlier on a date that the other
+//     column misses, as a rule), the pair's sums are formed over the joint dates
+//     directly: the subtraction then rounds less than the sums do.
 // Steps: column statistics (compensated mean, extrema; replaces
 // stock_corr_gpu's col_stats_kernel, src/stock_corr.cu:73-116, and the
 // demean_kernel's mean, :244-261), column-major copies and bitmasks, lists,
@@ -46,6 +47,7 @@ constexpr int kScChunk = 1536;   // dates it holds at a time (192 KB, and 12 KB 
 constexpr int kScTile = 64, kScTileJ = 32;  // k_sc_gram tile: rows, columns
 constexpr int kScK = 32;         // dates per stage
 constexpr int kScBlock = 5120;   // columns whose pair sums are held at a time
+constexpr int kScDirect = 1 << 18;  // pair sums that k_sc_direct takes of them
 
 FCB_DEV bool out_of_domain(const ScSummary* s) {
   const double mx = __longlong_as_double(static_cast<long long>(s->max_abs));
@@ -198,7 +200,7 @@ __global__ void k_sc_transpose(const TIN* __restrict__ X, const uint8_t* __restr
 }
 
 // One warp per column: sums of the centred values and their squares, and the
-// column's list -- its missing dates when they are at most a quarter (invert =
+// column's list -- its missing dates when they are at most a sixth (invert =
 // 1), its valid dates otherwise.  Per chunk of dates two runs of entries: the
 // listed dates, then the aligned groups of 32 dates that are listed as a whole
 // (date and group numbers within the chunk), each run padded to eight with the
@@ -210,20 +212,20 @@ __global__ void k_sc_lists(const double* __restrict__ Xc, const uint32_t* __rest
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= N) return;
-  double s2 = 0.0, s1 = 0.0;
+  TwoSum s2, s1;  // the lists' sums are taken away from these
 #pragma unroll 4
   for (int t = lane; t < Tp; t += 32) {
     const double d = Xc[static_cast<size_t>(w) * Tp + t];
-    s2 += d * d;
-    s1 += d;
+    s2.add(d * d);
+    s1.add(d);
   }
-  s2 = warp_sum(s2);
-  s1 = warp_sum(s1);
+  s2.warp_total();
+  s1.warp_total();
   const int missing = T - static_cast<int>(st[w].count);
-  const bool inv = 4ll * missing <= T;
+  const bool inv = 6ll * missing <= T;
   if (lane == 0) {
-    st[w].s2 = s2;
-    st[w].s1 = s1;
+    st[w].s2 = s2.value();
+    st[w].s1 = s1.value();
     invert[w] = inv ? 1 : 0;
   }
   uint16_t* out = list + static_cast<size_t>(w) * lcap;
@@ -271,6 +273,39 @@ __global__ void k_sc_lists(const double* __restrict__ Xc, const uint32_t* __rest
 // pair sums: AB[(j - ja) * ld + (i - ia)] = (sum x'_i, sum x'_i^2) over the
 // valid dates of column j
 // ---------------------------------------------------------------------------
+// Sum and sum of squares of a column's centred values over the dates in `bits`,
+// by W lanes of a warp (mask `lanes`): a lane every W-th date, eight loads ahead
+// of their use.
+template <int W>
+FCB_DEV double2 joint_sums(const double* __restrict__ x, const uint32_t* __restrict__ bits, int T, int lane,
+                           uint32_t lanes) {
+  constexpr int U = 8;
+  double a[4] = {}, q[4] = {};
+  for (int t0 = lane; t0 < T; t0 += U * W) {
+    double v[U];
+    uint32_t b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + W * u;
+      b[u] = t < T ? __ldg(bits + (t >> 5)) >> (t & 31) : 0u;
+      v[u] = t < T ? __ldg(x + t) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const double d = (b[u] & 1u) != 0u ? v[u] : 0.0;
+      a[u & 3] += d;
+      q[u & 3] = fma(d, d, q[u & 3]);
+    }
+  }
+  double2 s = make_double2((a[0] + a[1]) + (a[2] + a[3]), (q[0] + q[1]) + (q[2] + q[3]));
+#pragma unroll
+  for (int o = W / 2; o > 0; o >>= 1) {
+    s.x += __shfl_xor_sync(lanes, s.x, o);
+    s.y += __shfl_xor_sync(lanes, s.y, o);
+  }
+  return s;
+}
+
 // A half-warp takes one column j at a time: lane = column i.  A listed date
 // costs one 128-byte shared-memory row and two FP64 instructions per lane, a
 // listed group of 32 dates twice the row.  Shared-memory bandwidth bounds it.
@@ -281,7 +316,7 @@ __global__ void __launch_bounds__(1024, 1)
                  const uint32_t* __restrict__ bits, const ColStat* __restrict__ st, const uint16_t* __restrict__ list,
                  const int* __restrict__ ptr, const int* __restrict__ invert, int T, int N, int Tp, int nchunk,
                  int lcap, int c, int ia, int ib, int ja, int jb, int ld, double2* __restrict__ AB,
-                 const ScSummary* __restrict__ sum) {
+                 int* __restrict__ direct_list, ScSummary* __restrict__ sum) {
   if (sum->masked == 0 || out_of_domain(sum)) return;  // a full panel needs no pair sums
   extern __shared__ __align__(16) double xs[];  // [tn + 1][kScRows] values, [nw + 1][kScRows] sums; last rows zero
   const int t0 = c * kScChunk, tn = min(T - t0, kScChunk), nw = (tn + 31) / 32;
@@ -325,6 +360,7 @@ __global__ void __launch_bounds__(1024, 1)
   }
   __syncthreads();
   const int lane = threadIdx.x & 15, i = i0 + lane;
+  const uint32_t half = 0xFFFFu << (threadIdx.x & 16);
   const int hw = static_cast<int>(threadIdx.x >> 4), nhw = static_cast<int>(blockDim.x >> 4);
   const double* col = xs + lane;
   const double2* gcol = gs + lane;
@@ -368,31 +404,52 @@ __global__ void __launch_bounds__(1024, 1)
         q1 += y.y;
       }
     }
-    if (i >= ib) continue;
     a += a0 + a1;
     q += q0 + q1;
     double2* o = AB + static_cast<size_t>(j - ja) * ld + (i - ia);
-    if (c > 0) {
+    if (c > 0 && i < ib) {
       const double2 e = *o;
       a += e.x;
       q += e.y;
     }
     if (c == nchunk - 1 && invert[j] != 0) {
-      if (q > 0.75 * s2) {
-        // little is left of the column: form the sums over the joint dates
-        a = q = 0.0;
-        for (int t = 0; t < T; ++t)
-          if ((bits[static_cast<size_t>(j) * (Tp / 32) + (t >> 5)] >> (t & 31)) & 1u) {
-            const double x = Xc[static_cast<size_t>(i) * Tp + t];
-            a += x;
-            q = fma(x, x, q);
-          }
-      } else {
-        a = s1 - a;
-        q = s2 - q;
+      // where a quarter of the squares or more would be taken away, the sums are
+      // formed over the joint dates: by k_sc_direct, or here when its list is full
+      bool here = false;
+      if (i < ib && q > 0.25 * s2) {
+        const int at = atomicAdd(&sum->direct, 1);
+        here = at >= kScDirect;
+        if (!here) direct_list[at] = (j - ja) * ld + (i - ia);
+      }
+      uint32_t direct = __ballot_sync(half, here) & half;
+      a = s1 - a;
+      q = s2 - q;
+      for (; direct != 0u; direct &= direct - 1u) {  // uniform across the half-warp
+        const int l = (__ffs(direct) - 1) & 15;
+        const double2 d = joint_sums<16>(Xc + static_cast<size_t>(i0 + l) * Tp,
+                                         bits + static_cast<size_t>(j) * (Tp / 32), T, lane, half);
+        if (lane == l) {
+          a = d.x;
+          q = d.y;
+        }
       }
     }
-    *o = make_double2(a, q);
+    if (i < ib) *o = make_double2(a, q);
+  }
+}
+
+// The listed pair sums over the joint dates, one warp each.  (One column's
+// outlier on a date that half of the others miss lists a thousand pairs of one
+// k_sc_pairsum CTA, 8 us each there: 1218 x 2000 587 us a call, and 442 so.)
+__global__ void __launch_bounds__(256) k_sc_direct(const double* __restrict__ Xc, const uint32_t* __restrict__ bits,
+                                                   int T, int Tp, int ia, int ja, int ld, const int* __restrict__ list,
+                                                   double2* __restrict__ AB, const ScSummary* __restrict__ sum) {
+  const int cnt = min(sum->direct, kScDirect), nw = static_cast<int>(gridDim.x * blockDim.x) >> 5;
+  for (int g = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < cnt; g += nw) {
+    const int e = list[g], j = ja + e / ld, i = ia + e % ld, lane = static_cast<int>(threadIdx.x & 31);
+    const double2 s = joint_sums<32>(Xc + static_cast<size_t>(i) * Tp, bits + static_cast<size_t>(j) * (Tp / 32), T,
+                                     lane, kFull);
+    if (lane == 0) AB[e] = s;
   }
 }
 
@@ -680,6 +737,12 @@ int sc_block(int N) {
   return nb <= 1 ? N : ((N + nb - 1) / nb + kScTile - 1) / kScTile * kScTile;
 }
 
+// entries of the list of direct pair sums
+int sc_direct_cap(int N) {
+  const long long bs = sc_block(N);
+  return static_cast<int>(std::min<long long>(bs * bs, kScDirect));
+}
+
 template <typename TIN>
 cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScWork& w, double* out, cudaStream_t s) {
   const int Tp = (T + 31) / 32 * 32, nchunk = sc_chunks(T), lcap = sc_list_cap(T);
@@ -691,6 +754,8 @@ cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScW
   int* ptr = reinterpret_cast<int*>(m);
   m += al256(static_cast<size_t>(N) * (2 * nchunk + 1) * 4);
   int* invert = reinterpret_cast<int*>(m);
+  m += al256(static_cast<size_t>(N) * 4);
+  int* direct_list = reinterpret_cast<int*>(m);
   cudaError_t e = cudaMemsetAsync(w.summary, 0, sizeof(ScSummary), s);
   if (e != cudaSuccess) return e;
   k_sc_colstats<TIN><<<(N + 31) / 32, 32 * kStWarps, 0, s>>>(X, mask, T, N, w.st, w.summary);
@@ -704,13 +769,22 @@ cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScW
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(k_sc_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gsmem));
   if (e != cudaSuccess) return e;
-  auto pairsum = [&](int ia, int ib, int ja, int jb, double2* ab) {
+  bool first = true;
+  auto pairsum = [&](int ia, int ib, int ja, int jb, double2* ab) -> cudaError_t {
+    if (!first) {
+      const cudaError_t r = cudaMemsetAsync(&w.summary->direct, 0, sizeof(int), s);
+      if (r != cudaSuccess) return r;
+    }
+    first = false;
     const int rows = (ib - ia + kScRows - 1) / kScRows, cols = (jb - ja + 63) / 64;
     // a CTA per SM and row block; few row blocks share out the columns
     const int split = std::max(1, std::min(cols, 148 / rows));
     for (int c = 0; c < nchunk; ++c)
       k_sc_pairsum<TIN><<<dim3(rows, split), 1024, psmem, s>>>(X, mask, w.xc, bits, w.st, list, ptr, invert, T, N, Tp,
-                                                               nchunk, lcap, c, ia, ib, ja, jb, ib - ia, ab, w.summary);
+                                                               nchunk, lcap, c, ia, ib, ja, jb, ib - ia, ab,
+                                                               direct_list, w.summary);
+    k_sc_direct<<<148 * 8, 256, 0, s>>>(w.xc, bits, T, Tp, ia, ja, ib - ia, direct_list, ab, w.summary);
+    return cudaGetLastError();
   };
   const int bs = sc_block(N);
   for (int ia = 0; ia < N; ia += bs)
@@ -719,8 +793,8 @@ cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScW
       const long long ti = (ib - ia + kScTile - 1) / kScTile, tj = (jb - ja + kScTileJ - 1) / kScTileJ;
       double2* ab = w.ab;
       double2* ba = ia == ja ? ab : ab + static_cast<size_t>(bs) * bs;
-      pairsum(ia, ib, ja, jb, ab);
-      if (ia != ja) pairsum(ja, jb, ia, ib, ba);
+      if ((e = pairsum(ia, ib, ja, jb, ab)) != cudaSuccess) return e;
+      if (ia != ja && (e = pairsum(ja, jb, ia, ib, ba)) != cudaSuccess) return e;
       const long long tiles = ia == ja ? ti * tj - ti * (ti - 1) : ti * tj;
       k_sc_gram<<<static_cast<unsigned>(tiles), 256, gsmem, s>>>(w.xc, bits, w.st, T, N, Tp, ia, ib, ja, jb, ab, ba, out,
                                                                  w.fb_list, w.summary);
@@ -736,7 +810,8 @@ cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScW
 size_t sc_masks_bytes(int T, int N) {
   const size_t Tp = static_cast<size_t>((T + 31) / 32 * 32);
   return al256(N * (Tp / 32) * 4) + al256(static_cast<size_t>(N) * sc_list_cap(T) * 2) +
-         al256(static_cast<size_t>(N) * (2 * sc_chunks(T) + 1) * 4) + al256(static_cast<size_t>(N) * 4);
+         al256(static_cast<size_t>(N) * (2 * sc_chunks(T) + 1) * 4) + al256(static_cast<size_t>(N) * 4) +
+         al256(static_cast<size_t>(sc_direct_cap(N)) * 4);
 }
 
 size_t sc_pairs_bytes(int N) {

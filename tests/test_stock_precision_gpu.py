@@ -1,0 +1,52 @@
+"""stock_corr against 80-bit sums where the way its moments are formed could
+show: columns that lose much of their squares to dates another column misses,
+long panels, means far from zero."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ULP = 1.11e-16  # of a correlation between 0.5 and 1
+
+
+def exact(X, m):
+    P, N = X.astype(np.longdouble), X.shape[1]
+    out = np.ones((N, N), np.longdouble)
+    for i in range(N):
+        for j in range(i + 1, N):
+            o = m[:, i] & m[:, j]
+            x, y = P[o, i] - P[o, i].mean(), P[o, j] - P[o, j].mean()
+            out[i, j] = (x * y).sum() / np.sqrt((x * x).sum()) / np.sqrt((y * y).sum())
+    return out
+
+
+def rms_error(X, m):
+    import torch
+
+    import fcb200
+    got = fcb200.stock_corr(torch.from_numpy(X).cuda(), torch.from_numpy(m).cuda()).cpu().numpy()
+    err = (got.astype(np.longdouble) - exact(X, m))[np.triu_indices(X.shape[1], 1)]
+    return float(np.sqrt(np.mean(err * err)))
+
+
+def common(T, N, seed):
+    r = np.random.default_rng(seed)
+    return r, 0.02 * (np.sqrt(0.9) * r.standard_normal((T, 1)) + np.sqrt(0.1) * r.standard_normal((T, N)))
+
+
+# A sum is formed of chains of 32 dates and T / 32 of those: 0.29 ulps rms a step, growing as the sum does, 1.0 ulp at
+# T = 1218 and 1.3 at 2040.  Three of them and the correlation's own roundings: 1.0 * sqrt(1.5) + 0.65 = 1.9 ulps and
+# 2.2.  A third is left for the subtraction of up to a quarter of the squares.
+@pytest.mark.parametrize("share", [0.2, 0.5, 0.7, 0.9])
+@pytest.mark.parametrize("T,ulps", [(120, 2.0), (1218, 2.5), (2040, 2.9)])
+def test_an_outlier_that_others_miss(T, ulps, share):
+    N = 48
+    r, X = common(T, N, T)
+    m = r.random((T, N)) < 0.93
+    amp = 0.02 * np.sqrt(share / (1 - share) * T)
+    for q in range(7):  # on date q + 3 every seventh column has an outlier, and the others miss the date
+        cols = np.arange(N) % 7 == q
+        X[q + 3, cols] = amp * np.sign(r.standard_normal(cols.sum()))
+        m[q + 3] = cols
+    # (the pairs of one group share their outlier: its product alone makes their correlation)
+    assert rms_error(X, m) < ulps * ULP
