@@ -310,7 +310,8 @@ FCB_DEV double2 joint_sums(const double* __restrict__ x, const uint32_t* __restr
 // costs one 128-byte shared-memory row and two FP64 instructions per lane, a
 // listed group of 32 dates twice the row.  Shared-memory bandwidth bounds it.
 // Chunk c of the dates; the sums of earlier chunks wait in AB.
-template <typename TIN>
+// LONG: the list's short chains are added to twice the precision (see k_sc_gram).
+template <typename TIN, bool LONG>
 __global__ void __launch_bounds__(1024, 1)
     k_sc_pairsum(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, const double* __restrict__ Xc,
                  const uint32_t* __restrict__ bits, const ColStat* __restrict__ st, const uint16_t* __restrict__ list,
@@ -369,7 +370,14 @@ __global__ void __launch_bounds__(1024, 1)
     const int* p = ptr + static_cast<size_t>(j) * (2 * nchunk + 1) + 2 * c;
     const uint4* l = reinterpret_cast<const uint4*>(list + static_cast<size_t>(j) * lcap);
     const int k0 = p[0] >> 3, k1 = p[1] >> 3, k2 = p[2] >> 3;
-    double a0 = 0.0, a1 = 0.0, q0 = 0.0, q1 = 0.0, a = 0.0, q = 0.0;
+    double a0 = 0.0, a1 = 0.0, q0 = 0.0, q1 = 0.0;
+    TwoSum ta, tq;
+    auto add_chains = [&](TwoSum& t, double x) {
+      if (LONG)
+        t.add(x);
+      else
+        t.s += x;
+    };
     uint4 next = k0 < k2 ? __ldg(l + k0) : make_uint4(0u, 0u, 0u, 0u);
     for (int k = k0; k < k1; ++k) {
       const uint4 v = next;
@@ -385,8 +393,8 @@ __global__ void __launch_bounds__(1024, 1)
         q1 = fma(y, y, q1);
       }
       if (((k - k0) & 3) == 3) {  // long lists: short chains round less
-        a += a0 + a1;
-        q += q0 + q1;
+        add_chains(ta, a0 + a1);
+        add_chains(tq, q0 + q1);
         a0 = a1 = q0 = q1 = 0.0;
       }
     }
@@ -403,9 +411,15 @@ __global__ void __launch_bounds__(1024, 1)
         a1 += y.x;
         q1 += y.y;
       }
+      if (LONG && ((k - k1) & 3) == 3) {
+        add_chains(ta, a0 + a1);
+        add_chains(tq, q0 + q1);
+        a0 = a1 = q0 = q1 = 0.0;
+      }
     }
-    a += a0 + a1;
-    q += q0 + q1;
+    add_chains(ta, a0 + a1);
+    add_chains(tq, q0 + q1);
+    double a = ta.value(), q = tq.value();
     double2* o = AB + static_cast<size_t>(j - ja) * ld + (i - ia);
     if (c > 0 && i < ib) {
       const double2 e = *o;
@@ -496,7 +510,13 @@ struct ScProducts {
 // instructions per four dates and warp against four fragment loads.  The FP64 tensor
 // pipe bounds it: one product instead of the six masked sums per pair and
 // date (eight FP64 instructions) that it formed before.
-__global__ void __launch_bounds__(256, 4)
+// LONG (above kTwoPassKahanT dates, where the two-pass sums of pairs that fail the
+// cancellation gate were compensated): the stages' sums are added to twice the
+// precision, 3 CTAs per SM.  (2500 dates, correlations near 0.9, means of 50
+// spreads: rms error 9e-17, 2.4e-16 with plain additions, 7.5e-17 by two passes;
+// 3000 x 1000 308 -> 342 us a call, the two passes 24.9 ms.)
+template <bool LONG>
+__global__ void __launch_bounds__(256, LONG ? 3 : 4)
     k_sc_gram(const double* __restrict__ Xc, const uint32_t* __restrict__ bits, const ColStat* __restrict__ st, int T,
               int N, int Tp, int ia, int ib, int ja, int jb, const double2* __restrict__ ABij,
               const double2* __restrict__ ABji, double* __restrict__ out, int* __restrict__ fb_list,
@@ -531,11 +551,7 @@ __global__ void __launch_bounds__(256, 4)
     src += kScK;
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  double acc[2][2][2];
-#pragma unroll
-  for (int m = 0; m < 2; ++m)
-#pragma unroll
-    for (int c = 0; c < 2; ++c) acc[m][c][0] = acc[m][c][1] = 0.0;
+  TwoSum acc[2][2][2];
   load(0);
   for (int kc = 0; kc < W; ++kc) {
     if (kc + 1 < W) {
@@ -567,10 +583,14 @@ __global__ void __launch_bounds__(256, 4)
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        acc[m][c][0] += part[m][c][0];
-        acc[m][c][1] += part[m][c][1];
-      }
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          if (LONG)
+            acc[m][c][e].add(part[m][c][e]);
+          else
+            acc[m][c][e].s += part[m][c][e];
+        }
     __syncthreads();  // the stage is refilled two steps on
   }
   ScProducts& P = *reinterpret_cast<ScProducts*>(smem);
@@ -579,7 +599,7 @@ __global__ void __launch_bounds__(256, 4)
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) P.xy[wr + m * 8 + r][wc + c * 8 + 2 * kq + e] = acc[m][c][e];
+      for (int e = 0; e < 2; ++e) P.xy[wr + m * 8 + r][wc + c * 8 + 2 * kq + e] = acc[m][c][e].value();
   // The counts come after the products: both sets of sums do not fit the 64
   // registers that 4 CTAs per SM leave a thread. Rows 2 rp, 2 rp + 1 and
   // columns cp, cp + 8, cp + 16, cp + 24 are this thread's.
@@ -765,9 +785,12 @@ cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScW
   const int tc = std::min(T, kScChunk);
   const size_t psmem = (static_cast<size_t>(tc + 1) * 8 + static_cast<size_t>((tc + 31) / 32 + 1) * 16) * kScRows;
   const size_t gsmem = std::max(2 * sizeof(ScStage), sizeof(ScProducts));
-  e = cudaFuncSetAttribute(k_sc_pairsum<TIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(psmem));
+  const bool lng = T > kTwoPassKahanT;
+  auto* k_pairsum = lng ? k_sc_pairsum<TIN, true> : k_sc_pairsum<TIN, false>;
+  auto* k_gram = lng ? k_sc_gram<true> : k_sc_gram<false>;
+  e = cudaFuncSetAttribute(k_pairsum, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(psmem));
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_sc_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gsmem));
+  e = cudaFuncSetAttribute(k_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gsmem));
   if (e != cudaSuccess) return e;
   bool first = true;
   auto pairsum = [&](int ia, int ib, int ja, int jb, double2* ab) -> cudaError_t {
@@ -780,9 +803,9 @@ cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScW
     // a CTA per SM and row block; few row blocks share out the columns
     const int split = std::max(1, std::min(cols, 148 / rows));
     for (int c = 0; c < nchunk; ++c)
-      k_sc_pairsum<TIN><<<dim3(rows, split), 1024, psmem, s>>>(X, mask, w.xc, bits, w.st, list, ptr, invert, T, N, Tp,
-                                                               nchunk, lcap, c, ia, ib, ja, jb, ib - ia, ab,
-                                                               direct_list, w.summary);
+      k_pairsum<<<dim3(rows, split), 1024, psmem, s>>>(X, mask, w.xc, bits, w.st, list, ptr, invert, T, N, Tp, nchunk,
+                                                       lcap, c, ia, ib, ja, jb, ib - ia, ab, direct_list,
+                                                       w.summary);
     k_sc_direct<<<148 * 8, 256, 0, s>>>(w.xc, bits, T, Tp, ia, ja, ib - ia, direct_list, ab, w.summary);
     return cudaGetLastError();
   };
@@ -796,7 +819,7 @@ cudaError_t sc_launch(const TIN* X, const uint8_t* mask, int T, int N, const ScW
       if ((e = pairsum(ia, ib, ja, jb, ab)) != cudaSuccess) return e;
       if (ia != ja && (e = pairsum(ja, jb, ia, ib, ba)) != cudaSuccess) return e;
       const long long tiles = ia == ja ? ti * tj - ti * (ti - 1) : ti * tj;
-      k_sc_gram<<<static_cast<unsigned>(tiles), 256, gsmem, s>>>(w.xc, bits, w.st, T, N, Tp, ia, ib, ja, jb, ab, ba, out,
+      k_gram<<<static_cast<unsigned>(tiles), 256, gsmem, s>>>(w.xc, bits, w.st, T, N, Tp, ia, ib, ja, jb, ab, ba, out,
                                                                  w.fb_list, w.summary);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }

@@ -50,3 +50,13 @@ def test_an_outlier_that_others_miss(T, ulps, share):
         m[q + 3] = cols
     # (the pairs of one group share their outlier: its product alone makes their correlation)
     assert rms_error(X, m) < ulps * ULP
+
+
+# Above 2048 dates the sums that a cancelling pair takes were compensated: their own error a third of an ulp, three of
+# them and the correlation's roundings sqrt(1.5) * 0.45 + 0.65 = 1.2 ulps; a tenth for the number of pairs.
+@pytest.mark.parametrize("miss", [0.0, 0.05, 0.2])
+@pytest.mark.parametrize("T", [2500, 4500])
+def test_means_far_from_zero_in_long_panels(T, miss):
+    N = 32
+    r, X = common(T, N, T)
+    assert rms_error(X + 1.0, r.random((T, N)) >= miss) < 1.3 * ULP
