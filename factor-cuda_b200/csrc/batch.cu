@@ -105,6 +105,7 @@ struct fcb_batch {
   size_t cls_smem[kClasses] = {};
   double cls_work[kClasses] = {};
   cudaStream_t s[kClasses] = {};
+  cudaStream_t vs[kRicVariants] = {};  // f32, concurrent: a branch for each variant (made when first used)
   cudaEvent_t ev_fork = nullptr, ev_join[kClasses] = {}, ev_prep[kRicVariants] = {}, ev_t0 = nullptr, ev_t1 = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -142,7 +143,9 @@ struct fcb_batch {
       ev_join[k] = nullptr;
     }
     for (int k = 0; k < kRicVariants; ++k) {
+      if (vs[k] != nullptr) cudaStreamDestroy(vs[k]);
       if (ev_prep[k] != nullptr) cudaEventDestroy(ev_prep[k]);
+      vs[k] = nullptr;
       ev_prep[k] = nullptr;
     }
     if (ev_fork != nullptr) cudaEventDestroy(ev_fork);
@@ -349,12 +352,19 @@ int enqueue(fcb_batch& b, cudaStream_t s0) {
   for (int k = 1; k < kClasses; ++k) FCB_BTRY(cudaStreamWaitEvent(b.s[k], b.ev_fork, 0));
   for (int k = 0; k < kRicVariants && b.dtx == FCB_DTYPE_F32; ++k) {
     if (b.var[k].np == 0) continue;
-    // the short returns passes fill the tails of the rank launches before theirs
-    cudaStream_t st = (b.cfg.concurrent && k > 0) ? b.s[std::min(k, kClasses - 1)] : s0;
-    FCB_BTRY(launch_rank_ic_prep_batch(k, b.var[k], b.s[1]));
-    FCB_BTRY(cudaEventRecord(b.ev_prep[k], b.s[1]));
-    FCB_BTRY(cudaStreamWaitEvent(st, b.ev_prep[k], 0));
-    FCB_BTRY(launch_rank_ic_items_batch(k, b.var[k], st));
+    if (b.cfg.concurrent) {  // side by side: both passes on the variant's branch
+      if (b.vs[k] == nullptr) FCB_BTRY(cudaStreamCreateWithFlags(&b.vs[k], cudaStreamNonBlocking));
+      FCB_BTRY(cudaStreamWaitEvent(b.vs[k], b.ev_fork, 0));
+      FCB_BTRY(launch_rank_ic_prep_batch(k, b.var[k], b.vs[k]));
+      FCB_BTRY(launch_rank_ic_items_batch(k, b.var[k], b.vs[k]));
+      FCB_BTRY(cudaEventRecord(b.ev_prep[k], b.vs[k]));
+      FCB_BTRY(cudaStreamWaitEvent(s0, b.ev_prep[k], 0));
+    } else {  // the short returns passes fill the tails of the rank launches before theirs
+      FCB_BTRY(launch_rank_ic_prep_batch(k, b.var[k], b.s[1]));
+      FCB_BTRY(cudaEventRecord(b.ev_prep[k], b.s[1]));
+      FCB_BTRY(cudaStreamWaitEvent(s0, b.ev_prep[k], 0));
+      FCB_BTRY(launch_rank_ic_items_batch(k, b.var[k], s0));
+    }
   }
   for (int k = 0; k < kClasses && b.dtx != FCB_DTYPE_F32; ++k) {
     if (b.cls_cnt[k] == 0) continue;
