@@ -314,7 +314,7 @@ extern "C" int fcb_dev_cs_rank_f32(const float* d_x, const uint8_t* d_mask, int 
   const uintptr_t x0 = reinterpret_cast<uintptr_t>(d_x), o0 = reinterpret_cast<uintptr_t>(d_out);
   const uintptr_t plane_bytes = static_cast<uintptr_t>(T) * N * 4;
   const bool apart = x0 + plane_bytes <= o0 || o0 + plane_bytes <= x0;
-  if (N > kSmemRankCap && N <= kSliceMaxN && apart)
+  if (cs_rank_by_slices(T, N) && apart)
     return rc(launch_cs_rank_slices(d_x, d_mask, T, N, desc, d_out, s));
   if (N > kSmemRankCap) {
     // global-memory path; scratch is stream-ordered (no host synchronisation)
@@ -350,7 +350,7 @@ extern "C" int fcb_cs_rank_f32(const float* x, const uint8_t* mask, int T, int N
   FCB_TRY(cudaMemcpyAsync(dx, x, n * 4, cudaMemcpyHostToDevice, s));
   if (mask != nullptr) FCB_TRY(cudaMemcpyAsync(dm, mask, n, cudaMemcpyHostToDevice, s));
   FCB_TRY(cudaMemsetAsync(dst, 0, sizeof(int), s));
-  if (N > kSliceMaxN) {
+  if (N > kSmemRankCap && !cs_rank_by_slices(T, N)) {
     const size_t bytes = rank_global_scratch(rank_global_bytes_per_date(0, N, 1, 4, 4), T);
     uint8_t* scr;
     FCB_TRY(ws.get(S_GSCR, bytes, &scr));
@@ -1172,7 +1172,8 @@ extern "C" int fcb_memory_budget(int op, int dtype, int T, int N, int F, int fla
   switch (op) {
     case FCB_OP_CS_RANK:
       b = slot_bytes(n * 4) * 2 + 64 + (m1 ? slot_bytes(n) : 0);
-      if (N > kSliceMaxN) b += slot_bytes(rank_global_scratch(rank_global_bytes_per_date(0, N, 1, 4, 4), T));
+      if (N > kSmemRankCap && !cs_rank_by_slices(T, N))
+        b += slot_bytes(rank_global_scratch(rank_global_bytes_per_date(0, N, 1, 4, 4), T));
       break;
     case FCB_OP_PARAMETER_SCAN: {
       const int groups = (flags >> 8) & 0xF;

@@ -180,8 +180,18 @@ cudaError_t launch_param_scan(const float* X, const uint8_t* mask, int T, int N,
 size_t rank_ic_learned_smem(int N);
 cudaError_t launch_rank_ic_learned(const RankIcArgs<float, float>& a, int* status, cudaStream_t st);
 
-// rank_slices.cu: cs_rank of rows above kSmemRankCap, without scratch.
+// rank_slices.cu: cs_rank of rows above kSmemRankCap, without scratch, for the
+// calls that cs_rank_by_slices names; the others, and those in place, sort in
+// global memory, one CTA a row.  A row costs the slices the reads of all its
+// slices, whatever its values, and the sort a pass for each digit in which its
+// values differ: full SMs of tied rows are sorted sooner (us, sort against slices,
+// values in 30 steps: 300 x 17000 227 / 168, 148 x 20000 98 / 105, 64 x 40000 172 /
+// 163, 148 x 40000 187 / 316, 64 x 60000 257 / 288; smooth: 469 / 165, 192 / 97,
+// 350 / 142, 384 / 329, 522 / 270).
 constexpr int kSliceMaxN = 65536;
+inline bool cs_rank_by_slices(int T, int N) {
+  return N > kSmemRankCap && (N <= 18432 || (T <= 64 && N <= 40960) || (T <= 32 && N <= kSliceMaxN));
+}
 cudaError_t launch_cs_rank_slices(const float* X, const uint8_t* mask, int T, int N, int desc, float* out,
                                   cudaStream_t st);
 

@@ -11,13 +11,19 @@
 // takes (a much repeated value, a sample that does not show the row) is worked
 // off in parts, cut at the median of the cells that it could hold.
 //
+// A row with few valid cells takes as many fewer slices.  Where a value repeats in
+// the sample so that slices would begin at it in vain, those only write their
+// share of the NaNs, and the last of them ranks the value's cells by column in a
+// second pass over the row; a slice of one value needs no ranking (its list is in
+// column order).
+//
 // Measured on a B200, against one CTA per row that sorts it in global memory:
-// 4 x 16500 151 -> 26 us, 61 x 20000 182 -> 50, 64 x 40000 340 -> 148, 500 x
-// 17000 594 -> 275.  Rows of a few values only gain at few dates (16 x 20000 111
-// -> 55 us) and lose 5 % at 500 x 17000.  What bounds it is instruction issue:
-// ranking the slice, and reading the row R times at about 12 instructions per
-// cell and slice, which is why the form ends at kSliceMaxN; beyond,
-// rank_global.cu.
+// 4 x 16500 151 -> 26 us, 61 x 20000 182 -> 53, 64 x 40000 350 -> 142, 500 x
+// 17000 633 -> 260; integers 0..6 64 x 40000 148 -> 116, 98 % of the cells
+// invalid 41 -> 48, one value 62 -> 80 (three passes; the sort
+// has nothing to do).  What bounds it is instruction issue: ranking the slice,
+// and reading the row R times at about 12 instructions per cell and slice;
+// cs_rank_by_slices says where the sort is taken instead.
 //
 // The CTAs of a row read all of it while others write its ranks: out must not
 // overlap X.
@@ -90,18 +96,33 @@ FCB_DEV uint32_t sample_rank(const uint32_t (&k)[kSlSample], uint32_t rank) {
   return v;
 }
 
-enum class Take { kFirst, kList, kTies };
+enum class Take { kFirst, kHeavy, kList, kTies };
+
+// NaN for the invalid cells of every R-th tile from r on.
+FCB_DEV void slice_nans(const SliceRow& row, float* out, int r, int R) {
+  for (int t0 = r * kSlTile; t0 < row.N; t0 += R * kSlTile) {
+    const int i0 = t0 + 4 * static_cast<int>(threadIdx.x);
+    uint32_t k[4];
+    row.four(i0, k);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (k[q] == kInvalidKey32 && i0 + q < row.N) out[i0 + q] = __uint_as_float(kQuietNanBits);
+  }
+}
 
 // The cells with a <= key < b in column order: their keys and columns into the
 // lists as far as these reach or (kTies) their ranks from first + 1 on into out.
-// Returns their number.  kFirst also counts the valid cells below a into
-// `below` and writes NaN for the invalid cells of every R-th tile from r on.
-// wt: 96 words; ends with a barrier.
+// Returns their number.  kFirst and kHeavy also count the valid cells below a
+// into `below` (kHeavy: below a - 1, and those equal to a - 1 into `ties`) and
+// write NaN for the invalid cells of every R-th tile from r on.  wt: 112 words
+// without [96, 101); ends with a barrier.
 template <Take TAKE>
 FCB_DEV uint32_t slice_collect(const SliceRow& row, uint32_t a, uint32_t b, uint32_t* keys, uint32_t* cols,
-                               uint32_t first, float* out, uint32_t* wt, int r, int R, uint32_t& below) {
+                               uint32_t first, float* out, uint32_t* wt, int r, int R, uint32_t& below,
+                               uint32_t& ties) {
+  constexpr bool kWhole = TAKE == Take::kFirst || TAKE == Take::kHeavy;
   const int wi = static_cast<int>(threadIdx.x >> 5);
-  uint32_t run = 0u, under = 0u;
+  uint32_t run = 0u, under = 0u, same = 0u;
   int buf = 0, tile = 0;
   uint32_t next[4];
   row.four(4 * static_cast<int>(threadIdx.x), next);
@@ -112,10 +133,11 @@ FCB_DEV uint32_t slice_collect(const SliceRow& row, uint32_t a, uint32_t b, uint
     for (int q = 0; q < 4; ++q) {
       k[q] = next[q];
       h += k[q] - a < b - a ? 1u : 0u;
-      if (TAKE == Take::kFirst) under += k[q] < a ? 1u : 0u;
+      if (kWhole) under += k[q] < a ? 1u : 0u;
+      if (TAKE == Take::kHeavy) same += k[q] == a - 1u ? 1u : 0u;
     }
     if (t0 + kSlTile < row.N) row.four(i0 + kSlTile, next);
-    if (TAKE == Take::kFirst) {
+    if (kWhole) {
       if (tile == r) {
 #pragma unroll
         for (int q = 0; q < 4; ++q)
@@ -140,12 +162,19 @@ FCB_DEV uint32_t slice_collect(const SliceRow& row, uint32_t a, uint32_t b, uint
         ++p;
       }
   }
-  if (TAKE == Take::kFirst) {
+  if (kWhole) {
     under = __reduce_add_sync(kFull, under);
-    if (lane_id() == 0) wt[64 + wi] = under;
+    same = __reduce_add_sync(kFull, same);
+    if (lane_id() == 0) {
+      wt[64 + wi] = under;
+      wt[80 + wi] = same;
+    }
   }
   __syncthreads();
-  if (TAKE == Take::kFirst) below = warps_sum<kSlWarps>(wt + 64);
+  if (kWhole) {
+    ties = warps_sum<kSlWarps>(wt + 80);
+    below = warps_sum<kSlWarps>(wt + 64) - ties;
+  }
   return run;
 }
 
@@ -187,39 +216,56 @@ __global__ void __launch_bounds__(kSlNT, kSmThreads / kSlNT)
   const SpreadLayout<kSlNT, kSlV> L(kSlCap);
   uint32_t* cols = reinterpret_cast<uint32_t*>(sm + S.col);
   uint32_t* keys = reinterpret_cast<uint32_t*>(sm + L.mem);  // read out before the buckets are filled
-  uint32_t* wt = reinterpret_cast<uint32_t*>(sm + S.wt);     // [0, 96) counts, [96, 99) the slice's ends and a cut
+  uint32_t* wt = reinterpret_cast<uint32_t*>(sm + S.wt);     // [0, 96) counts, [96, 101) the slice's ends, the slices and a cut
   const int t = static_cast<int>(blockIdx.x) / R, r = static_cast<int>(blockIdx.x) % R;
   const int tid = static_cast<int>(threadIdx.x), wi = tid >> 5, lane = tid & 31;
   const size_t at = static_cast<size_t>(t) * N;
   SliceRow row{X + at, mask != nullptr ? mask + at : nullptr, N, desc != 0, false};
   row.vec = (reinterpret_cast<uintptr_t>(row.x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(row.mask) & 3u) == 0;
   out += at;
-  if (wi < 2) {  // warp w: the key at which slice r + w begins
-    uint32_t k[kSlSample], v = 0u;
-    if (r + wi == R) {
-      v = kInvalidKey32;
-    } else if (r + wi > 0) {
-      uint32_t ms = 0u;
+  if (wi < 3) {  // warp w: the key at which slice r - 1 + w begins
+    uint32_t k[kSlSample], ms = 0u;
 #pragma unroll
-      for (int q = 0; q < kSlSample; ++q) {
-        k[q] = row.one(static_cast<int>(static_cast<long long>(q * 32 + lane) * N / (32 * kSlSample)));
-        ms += k[q] != kInvalidKey32 ? 1u : 0u;
-      }
-      ms = __reduce_add_sync(kFull, ms);
-      // (no valid sample: the first slice takes all cells)
-      v = sample_rank(k, ms * static_cast<uint32_t>(r + wi) / static_cast<uint32_t>(R));
+    for (int q = 0; q < kSlSample; ++q) {
+      k[q] = row.one(static_cast<int>(static_cast<long long>(q * 32 + lane) * N / (32 * kSlSample)));
+      ms += k[q] != kInvalidKey32 ? 1u : 0u;
     }
+    ms = __reduce_add_sync(kFull, ms);
+    // a row with few valid cells, by its sample and two standard deviations, takes
+    // as many fewer slices
+    const uint32_t valid = min(512u, ms + 2u * static_cast<uint32_t>(sqrtf(static_cast<float>(ms))) + 2u);
+    const int rows_slices = static_cast<int>((static_cast<uint32_t>(R) * valid + 511u) / 512u);
+    const int begin = r - 1 + wi;
+    uint32_t v = 0u;
+    if (begin >= rows_slices)
+      v = kInvalidKey32;
+    else if (begin > 0)  // (no valid sample: the first slice takes all cells)
+      v = sample_rank(k, ms * static_cast<uint32_t>(begin) / static_cast<uint32_t>(rows_slices));
     if (lane == 0) wt[96 + wi] = v;
+    if (lane == 0 && wi == 0) wt[99] = static_cast<uint32_t>(rows_slices);
   }
   __syncthreads();
-  uint32_t a = wt[96], below = 0u;
-  const uint32_t end = wt[97];
+  R = static_cast<int>(wt[99]);
+  if (r >= R) return;
+  uint32_t a = wt[97], below = 0u;
+  const uint32_t end = wt[98];
   uint32_t b = end;
-  uint32_t n = slice_collect<Take::kFirst>(row, a, b, keys, cols, 0u, out, wt, r, R, below);
+  if (a == b) {  // between two equal sampled cells: the last slice that begins at them has theirs
+    slice_nans(row, out, r, R);
+    return;
+  }
+  uint32_t n, ties = 0u;
+  if (r > 0 && wt[96] == a) {  // a value that fills a slice or more: by column, apart from the others
+    ++a;
+    n = slice_collect<Take::kHeavy>(row, a, b, keys, cols, 0u, out, wt, r, R, below, ties);
+    below += slice_collect<Take::kTies>(row, a - 1u, a, nullptr, nullptr, below, out, wt, r, R, below, ties);
+  } else {
+    n = slice_collect<Take::kFirst>(row, a, b, keys, cols, 0u, out, wt, r, R, below, ties);
+  }
   for (;;) {  // uniform: the slice, as a rule in one part
     if (n > kSlCap) {
       if (b - a == 1u) {  // one value: ranked by column
-        below += slice_collect<Take::kTies>(row, a, b, keys, cols, below, out, wt, r, R, below);
+        below += slice_collect<Take::kTies>(row, a, b, nullptr, nullptr, below, out, wt, r, R, below, ties);
       } else {
         // up to the median of the full list; a value that fills half of it is
         // thereby taken alone
@@ -228,23 +274,28 @@ __global__ void __launch_bounds__(kSlNT, kSmThreads / kSlNT)
 #pragma unroll
           for (int q = 0; q < kSlSample; ++q) k[q] = keys[(q * 32 + lane) * (kSlCap / (32 * kSlSample))];
           const uint32_t v = sample_rank(k, 16 * kSlSample);
-          if (lane == 0) wt[98] = max(v, a + 1u);
+          if (lane == 0) wt[100] = max(v, a + 1u);
         }
         __syncthreads();
-        b = wt[98];
-        n = slice_collect<Take::kList>(row, a, b, keys, cols, 0u, out, wt, r, R, below);
+        b = wt[100];
+        n = slice_collect<Take::kList>(row, a, b, keys, cols, 0u, out, wt, r, R, below, ties);
         continue;
       }
     } else {
       uint32_t key[C], W[C];
+      const uint32_t key0 = keys[0];
+      bool differs = false;
 #pragma unroll
       for (int c = 0; c < C; ++c) {
         const uint32_t i = cell_col<kSlNT>(c);
         key[c] = i < n ? keys[i] : kInvalidKey32;
+        differs = differs || (i < n && key[c] != key0);
       }
-      __syncthreads();  // the keys' place becomes the buckets'
       SpreadTotals T;
-      if (spread_place<kSlNT, kSlV>(key, L, sm, W, T)) {
+      if (!__syncthreads_or(differs)) {  // (the keys' place becomes the buckets')
+#pragma unroll
+        for (int c = 0; c < C; ++c) W[c] = cell_col<kSlNT>(c);  // one value: the list is in column order
+      } else if (spread_place<kSlNT, kSlV>(key, L, sm, W, T)) {
         spread_positions<kSlNT, kSlV, false>(L, sm, T.m, T.heavy, key, W);
       } else {
         uint32_t kk[C], w[C];
@@ -265,7 +316,7 @@ __global__ void __launch_bounds__(kSlNT, kSmThreads / kSlNT)
     if (b == end) break;
     a = b;
     b = end;
-    n = slice_collect<Take::kList>(row, a, b, keys, cols, 0u, out, wt, r, R, below);
+    n = slice_collect<Take::kList>(row, a, b, keys, cols, 0u, out, wt, r, R, below, ties);
   }
 }
 }  // namespace

@@ -115,8 +115,9 @@ void fcb_host_free(void* p);
  * Returns -1 null/dim, -2 N > 2^24, -3 T*N > INT32_MAX.
  * Every N up to the cap is served: sections that fit one CTA's shared memory
  * (N <= 16384 for cs_rank, parameter_scan and f32 rank + IC; about 10100 for
- * rolling_ic with an f64 side) are ranked there, cs_rank up to 65536 by slices
- * of the value range, and wider ones by a
+ * rolling_ic with an f64 side) are ranked there, cs_rank up to 18432 columns
+ * (40960 up to 64 dates, 65536 up to 32) by slices of the value range, and
+ * wider ones by a
  * global-memory radix sort per date with the same results (scratch from the
  * workspace, or stream-ordered cudaMallocAsync for the fcb_dev_* variants). */
 int fcb_cs_rank_f32(const float* x, const uint8_t* mask, int T, int N, int descending, float* out,

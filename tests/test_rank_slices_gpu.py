@@ -40,3 +40,40 @@ def test_cs_rank_wide_rows(N):
             for desc in (False, True):
                 got = fcb200.cross_sectional_rank(dX, dmm, descending=desc).cpu().numpy()
                 assert bitwise_f32(got, O.cs_rank(X[-T:], m, desc)), (N, T, m is None, desc)
+
+
+def repeated_rows(N, seed):
+    """Rows in which values fill slices: few values, one value with little beside it, few valid cells, and both sides
+    of each; the sample sees the value but not the cells around it, or does not see it."""
+    r = np.random.default_rng(seed)
+    z = r.standard_normal(N)
+    at = np.arange(512) * N // 512
+    rows = [np.full(N, 3.0), np.where(r.random(N) < 1e-3, z, 3.0), np.where(np.arange(N) < 5, -1.0, 3.0),
+            np.where(np.arange(N) > N - 6, 9.0, 3.0), r.integers(0, 7, N), (r.random(N) < 0.3).astype(float),
+            r.integers(0, 30, N), np.where(r.random(N) < 0.9, 0.0, z), np.where(r.random(N) < 0.2, 0.5, z),
+            np.where(r.random(N) < 0.98, np.nan, z), np.where(r.random(N) < 0.98, np.nan, 1.0), np.full(N, np.nan)]
+    hidden = np.full(N, np.nan)
+    hidden[at] = 1.0
+    rest = z.copy()
+    rest[at] = np.nan
+    one_seen = rest.copy()
+    one_seen[at[::100]] = 0.0
+    below = np.full(N, 2.0)
+    below[1::2] = -1.0
+    below[at] = 2.0
+    return np.array(rows + [hidden, rest, one_seen, below]).astype(np.float32)
+
+
+# each side of the lines at which the global sort takes over
+@pytest.mark.parametrize("N,T", [(16385, 16), (18432, 160), (18433, 160), (40960, 64), (40961, 64), (65535, 32)])
+def test_cs_rank_of_repeated_values(N, T):
+    import torch
+
+    import fcb200
+    X = np.tile(repeated_rows(N, N), (-(-T // 16), 1))[:T]
+    mask = np.random.default_rng(N + 2).random(X.shape) < 0.97
+    dX, dm = torch.from_numpy(X).cuda(), torch.from_numpy(mask).cuda()
+    for m, dmm in ((mask, dm), (None, None)):
+        for desc in (False, True):
+            got = fcb200.cross_sectional_rank(dX, dmm, descending=desc).cpu().numpy()
+            assert bitwise_f32(got, O.cs_rank(X, m, desc)), (N, T, m is None, desc)
