@@ -2,7 +2,8 @@
 //
 // One CTA sorts up to NT*MAXIPT (key, column) pairs held in shared memory.
 // Each 8-bit pass: every warp ranks a contiguous chunk of the input with
-// __match_any_sync (stable: lane order within a 32-wide step, steps in order),
+// __match_any_sync (stable: lane order within a 32-wide step, steps in order; eight
+// ballots instead take as long for many digits and twice as long for few),
 // per-warp digit counters are prefix-summed across warps and digits, and the
 // pairs are scattered to the alternate buffer.  Passes over digits on which
 // all keys agree are skipped (block-wide AND/OR of the keys).
@@ -79,7 +80,8 @@ FCB_DEV void radix_pass(const K* __restrict__ ks, const uint16_t* __restrict__ i
   const int ipt = per_warp >> 5;
   const int base = w * per_warp;
   uint16_t* wh = whist + w * kRadix;
-  for (int d = lane; d < kRadix; d += 32) wh[d] = 0;
+  static_assert(kRadix * sizeof(uint16_t) == 32 * sizeof(uint4), "16 bytes a lane");
+  reinterpret_cast<uint4*>(wh)[lane] = make_uint4(0u, 0u, 0u, 0u);
   __syncwarp();
   const unsigned lt = lanemask_lt();
 
@@ -90,13 +92,16 @@ FCB_DEV void radix_pass(const K* __restrict__ ks, const uint16_t* __restrict__ i
 #pragma unroll
   for (int k = 0; k < (MAXIPT + 1) / 2; ++k) loc[k] = 0;
 #pragma unroll
+  for (int k = 0; k < MAXIPT; ++k) {  // all loads before the first step, whose barriers they would wait at
+    const int pos = base + k * 32 + lane;
+    kreg[k] = k < ipt && pos < n ? ks[pos] : K(0);
+  }
+#pragma unroll
   for (int k = 0; k < MAXIPT; ++k) {
-    kreg[k] = K(0);
     if (k < ipt) {
       const int pos = base + k * 32 + lane;
       const bool v = pos < n;
-      const K key = v ? ks[pos] : K(0);
-      kreg[k] = key;
+      const K key = kreg[k];
       const uint32_t d = v ? static_cast<uint32_t>((key >> shift) & K(kRadix - 1)) : uint32_t(kRadix);
       const unsigned peers = __match_any_sync(kFull, d);
       const uint32_t r = __popc(peers & lt);
@@ -108,30 +113,37 @@ FCB_DEV void radix_pass(const K* __restrict__ ks, const uint16_t* __restrict__ i
     }
   }
   __syncthreads();
-  constexpr int DPT = (kRadix + NT - 1) / NT;  // digits per thread
-  uint32_t tot[DPT], all = 0;
+  // counts -> offsets before each warp, two digits to a word (a count is at most
+  // 16384), and each digit's first position
+  constexpr int WPT = (kRadix / 2 + NT - 1) / NT;  // words per thread
+  uint32_t* wh2 = reinterpret_cast<uint32_t*>(whist);
+  uint32_t tot[WPT], all = 0;
 #pragma unroll
-  for (int q = 0; q < DPT; ++q) {
+  for (int q = 0; q < WPT; ++q) {
     tot[q] = 0;
-    const int d = threadIdx.x * DPT + q;
-    if (d < kRadix) {
-      uint32_t run = 0;
+    const int d2 = threadIdx.x * WPT + q;
+    if (d2 < kRadix / 2) {
 #pragma unroll
       for (int ww = 0; ww < NW; ++ww) {
-        const uint32_t c = whist[ww * kRadix + d];
-        whist[ww * kRadix + d] = static_cast<uint16_t>(run);
-        run += c;
+        const uint32_t c = wh2[ww * (kRadix / 2) + d2];
+        wh2[ww * (kRadix / 2) + d2] = tot[q];
+        tot[q] += c;
       }
-      tot[q] = run;
     }
-    all += tot[q];
+    all += (tot[q] & 0xFFFFu) + (tot[q] >> 16);
   }
-  uint32_t total;
-  uint32_t ex = block_exclusive_sum(all, scan, total);
+  const uint32_t inc = warp_inclusive_sum(all);
+  if (lane == 31) scan[w] = inc;
+  __syncthreads();
+  uint32_t ex = __reduce_add_sync(kFull, lane < w ? scan[lane] : 0u) + inc - all;
 #pragma unroll
-  for (int q = 0; q < DPT; ++q) {
-    if (threadIdx.x * DPT + q < kRadix) dbase[threadIdx.x * DPT + q] = ex;
-    ex += tot[q];
+  for (int q = 0; q < WPT; ++q) {
+    const int d2 = threadIdx.x * WPT + q;
+    if (d2 < kRadix / 2) {
+      dbase[2 * d2] = ex;
+      dbase[2 * d2 + 1] = ex + (tot[q] & 0xFFFFu);
+    }
+    ex += (tot[q] & 0xFFFFu) + (tot[q] >> 16);
   }
   __syncthreads();
 #pragma unroll
@@ -150,21 +162,19 @@ FCB_DEV void radix_pass(const K* __restrict__ ks, const uint16_t* __restrict__ i
   __syncthreads();
 }
 
-// Sort n <= NT*MAXIPT pairs.  (k0,i0) hold the input; (k1,i1) are scratch of
-// the same size.  On return *kout/*iout point at whichever buffer holds the
-// sorted sequence.  `scratch` is SortScratch<NT>::bytes of 16-aligned shared
-// memory.  All threads of the block must call.
+// Sort n <= NT*MAXIPT pairs whose keys differ in the bits of `diff` (uniform).
+// (k0,i0) hold the input; (k1,i1) are scratch of the same size.  On return
+// *kout/*iout point at whichever buffer holds the sorted sequence.  `scratch` is
+// SortScratch<NT>::bytes of 16-aligned shared memory.  All threads of the block
+// must call.
 template <int NT, int MAXIPT, typename K>
-FCB_DEV void block_radix_sort(K* k0, uint16_t* i0, K* k1, uint16_t* i1, int n, uint8_t* scratch,
-                              K** kout, uint16_t** iout) {
+FCB_DEV void block_radix_sort_bits(K* k0, uint16_t* i0, K* k1, uint16_t* i1, int n, K diff, uint8_t* scratch,
+                                   K** kout, uint16_t** iout) {
   using S = SortScratch<NT>;
   uint16_t* whist = reinterpret_cast<uint16_t*>(scratch);
   uint32_t* dbase = reinterpret_cast<uint32_t*>(scratch + S::hist_bytes);
   unsigned long long* scan64 =
       reinterpret_cast<unsigned long long*>(scratch + S::hist_bytes + S::base_bytes);
-  K a, o;
-  block_and_or(k0, n, a, o, reinterpret_cast<K*>(scan64));
-  const K diff = a ^ o;
   K* ks = k0;
   K* kd = k1;
   uint16_t* is = i0;
@@ -179,6 +189,16 @@ FCB_DEV void block_radix_sort(K* k0, uint16_t* i0, K* k1, uint16_t* i1, int n, u
   }
   *kout = ks;
   *iout = is;
+}
+
+// The same of keys that only shared memory holds.
+template <int NT, int MAXIPT, typename K>
+FCB_DEV void block_radix_sort(K* k0, uint16_t* i0, K* k1, uint16_t* i1, int n, uint8_t* scratch,
+                              K** kout, uint16_t** iout) {
+  using S = SortScratch<NT>;
+  K a, o;
+  block_and_or(k0, n, a, o, reinterpret_cast<K*>(scratch + S::hist_bytes + S::base_bytes));
+  block_radix_sort_bits<NT, MAXIPT, K>(k0, i0, k1, i1, n, a ^ o, scratch, kout, iout);
 }
 
 // Order-preserving compaction: for each i in [0,n) with flag(i) true, writes

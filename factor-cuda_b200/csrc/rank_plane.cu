@@ -14,22 +14,52 @@
 // 1001 x 4733 (four groups) 190 -> 76.6 us, one date of 5000 31 -> 17 us.
 // What bounds them is instruction issue (about 140 instructions per cell at
 // 60 % of the issue slots; 8 HBM bytes per cell take a sixth of the time).  A
-// plane of nothing but ties pays for finding that out: cs_rank of integers
-// 0..6 takes 73 us against 56, of values rounded to 1e-2 130 against 103;
-// with 3 % zeros, or rounded to 1e-3, it takes 79 and 59 us against 175 and
-// 122.
+// plane of nothing but ties pays for finding that out, and sorts with two CTAs of
+// 448 threads per SM: cs_rank of integers 0..6 takes 64 us against 56, of values
+// rounded to 1e-1 and 1e-2 93 and 117 against 84 and 101, with 30 % zeros 153
+// against 141; with 3 % zeros, or rounded to 1e-3, 64 and 56 us against 174 and
+// 121.  (The keys go to the sort from registers; read and tested again they cost
+// 5 us more.)
 #include "section_rank.cuh"
 
 namespace fcb {
 namespace {
 
-// cs_rank by radix: valid = finite & mask; the valid cells are compacted in
-// column order, radix-sorted by key (of -x for descending), and each cell's
-// rank is its sorted position + 1.
+// compact_bases, and the bits in which the flagged cells' keys differ.  scratch:
+// 128 words.
 template <int NT, int V>
-__device__ __noinline__ void csr_radix(const float* __restrict__ X, const uint8_t* __restrict__ mask, int N, int desc,
-                                       float* __restrict__ out, uint8_t* sm) {
+FCB_DEV uint32_t compact_bits(const uint32_t (&key)[4 * V], uint32_t flags, int (&base)[V], int& m,
+                              unsigned long long* scratch) {
+  constexpr int NW = NT / 32;
+  uint32_t* red = reinterpret_cast<uint32_t*>(scratch + 33);  // past block_exclusive_sum's words
+  uint32_t all = 0xFFFFFFFFu, any = 0u;
+#pragma unroll
+  for (int c = 0; c < 4 * V; ++c)
+    if ((flags >> c) & 1u) {
+      all &= key[c];
+      any |= key[c];
+    }
+  all = __reduce_and_sync(kFull, all);
+  any = __reduce_or_sync(kFull, any);
+  if (lane_id() == 0) {
+    red[threadIdx.x >> 5] = all;
+    red[32 + (threadIdx.x >> 5)] = any;
+  }
+  m = compact_bases<NT, V>(flags, base, scratch);  // its barriers publish the words
+  return __reduce_and_sync(kFull, lane_id() < NW ? red[lane_id()] : 0xFFFFFFFFu) ^
+         __reduce_or_sync(kFull, lane_id() < NW ? red[32 + lane_id()] : 0u);
+}
+
+// cs_rank by radix: the valid cells (key <= range, as spread_place left them) are
+// compacted in column order, radix-sorted by key, and each cell's rank is its
+// sorted position + 1.  A section of one value is in order as it is.
+template <int NT, int V>
+__device__ __noinline__ void csr_radix(const uint32_t* keys, uint32_t range, int N, float* __restrict__ out,
+                                       uint8_t* sm) {
   constexpr int C = 4 * V;
+  uint32_t key[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) key[c] = keys[c];
   const SortedLayout<NT> L(N);
   unsigned long long* scan64 = reinterpret_cast<unsigned long long*>(sm + L.red);
   uint32_t* k0 = reinterpret_cast<uint32_t*>(sm + L.k0);
@@ -37,16 +67,23 @@ __device__ __noinline__ void csr_radix(const float* __restrict__ X, const uint8_
   uint16_t* i0 = reinterpret_cast<uint16_t*>(sm + L.i0);
   uint16_t* i1 = reinterpret_cast<uint16_t*>(sm + L.i1);
   const int tid = static_cast<int>(threadIdx.x);
-  const size_t row = static_cast<size_t>(blockIdx.x) * N;
-  float x[C];
-  uint32_t mk[C];
-  load_row_f32<NT, V, true>(X + row, N, x);
-  load_mask4<NT, V>(mask != nullptr ? mask + row : nullptr, N, mk);
+  const float qnan = __uint_as_float(kQuietNanBits);
   uint32_t valid = 0u;
 #pragma unroll
-  for (int c = 0; c < C; ++c) valid |= ((finite_f32(x[c]) && mk[c]) ? 1u : 0u) << c;
-  int base[V];
-  const int m = compact_bases<NT, V>(valid, base, scan64);
+  for (int c = 0; c < C; ++c) valid |= (key[c] <= range ? 1u : 0u) << c;
+  int base[V], m;
+  const uint32_t diff = compact_bits<NT, V>(key, valid, base, m, scan64);
+  float v[C];
+  if (diff == 0u || m < 2) {
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      int p = base[j];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[4 * j + k] = (valid >> (4 * j + k)) & 1u ? static_cast<float>(++p) : qnan;
+    }
+    store_row_f32v<NT, V>(out, N, v);
+    return;
+  }
 #pragma unroll
   for (int j = 0; j < V; ++j) {
     int p = base[j];
@@ -54,7 +91,7 @@ __device__ __noinline__ void csr_radix(const float* __restrict__ X, const uint8_
     for (int k = 0; k < 4; ++k) {
       const int c = 4 * j + k;
       if ((valid >> c) & 1u) {
-        k0[p] = key_f32(desc ? -x[c] : x[c]);
+        k0[p] = key[c];
         i0[p] = static_cast<uint16_t>(4 * (j * NT + tid) + k);
         ++p;
       }
@@ -63,19 +100,18 @@ __device__ __noinline__ void csr_radix(const float* __restrict__ X, const uint8_
   __syncthreads();
   uint32_t* ks;
   uint16_t* is;
-  block_radix_sort<NT, C, uint32_t>(k0, i0, k1, i1, m, sm + L.scratch, &ks, &is);
+  block_radix_sort_bits<NT, C, uint32_t>(k0, i0, k1, i1, m, diff, sm + L.scratch, &ks, &is);
   uint32_t* RK = (ks == k0) ? k1 : k0;
   for (int p = tid; p < m; p += NT) RK[is[p]] = static_cast<uint32_t>(p + 1);
   __syncthreads();
-  const float qnan = __uint_as_float(kQuietNanBits);
-  float v[C];
 #pragma unroll
   for (int c = 0; c < C; ++c)
     v[c] = ((valid >> c) & 1u) ? static_cast<float>(RK[4 * ((c >> 2) * NT + tid) + (c & 3)]) : qnan;
-  store_row_f32v<NT, V>(out + row, N, v);
+  store_row_f32v<NT, V>(out, N, v);
 }
 
-// parameter_scan by radix: one ascending sort of the finite cells serves all four
+// parameter_scan by radix, of the cells that spread_place left (out_of_mask: bit c,
+// cell c is finite but not in the mask): one ascending sort of the finite cells serves all four
 // groups (asc / desc x masked / unmasked).  With S the start and E the end of
 // a cell's tie group in sorted order, C the count of masked-valid cells before
 // a sorted position and m / mt the finite / masked-valid totals:
@@ -86,7 +122,7 @@ __device__ __noinline__ void csr_radix(const float* __restrict__ X, const uint8_
 // keys are then free for C and E), and the ascending and descending pairs of
 // ranks pass through one per-column buffer in turn.
 template <int NT, int V>
-__device__ __noinline__ void pscan_radix(const float* __restrict__ X, const uint8_t* __restrict__ mask, int N,
+__device__ __noinline__ void pscan_radix(const uint32_t* keys, uint32_t range, uint32_t out_of_mask, int N,
                                          const ScanOut& outs, uint8_t* sm) {
   constexpr int C = 4 * V;
   const SortedLayout<NT> L(N);
@@ -100,18 +136,14 @@ __device__ __noinline__ void pscan_radix(const float* __restrict__ X, const uint
   const int tid = static_cast<int>(threadIdx.x);
   const size_t row = static_cast<size_t>(blockIdx.x) * N;
   for (int k = tid; k < (N + 31) / 32 + 1; k += NT) bits[k] = 0u;
-  float x[C];
-  uint32_t mk[C];
-  load_row_f32<NT, V, true>(X + row, N, x);
-  load_mask4<NT, V>(mask != nullptr ? mask + row : nullptr, N, mk);
-  uint32_t fin = 0u, msk = 0u;
+  uint32_t key[C], fin = 0u;
 #pragma unroll
   for (int c = 0; c < C; ++c) {
-    fin |= (finite_f32(x[c]) ? 1u : 0u) << c;
-    msk |= (mk[c] ? 1u : 0u) << c;
+    key[c] = keys[c];
+    fin |= (key[c] <= range ? 1u : 0u) << c;
   }
-  int base[V];
-  const int m = compact_bases<NT, V>(fin, base, scan64);  // its barriers publish the bitmap clear
+  int base[V], m;
+  const uint32_t diff = compact_bits<NT, V>(key, fin, base, m, scan64);  // its barriers publish the bitmap clear
 #pragma unroll
   for (int j = 0; j < V; ++j) {
     int p = base[j];
@@ -119,8 +151,8 @@ __device__ __noinline__ void pscan_radix(const float* __restrict__ X, const uint
     for (int k = 0; k < 4; ++k) {
       const int c = 4 * j + k;
       if ((fin >> c) & 1u) {
-        k0[p] = key_f32(x[c]);
-        i0[p] = static_cast<uint16_t>((4 * (j * NT + tid) + k) | (((msk >> c) & 1u) << 15));
+        k0[p] = key[c];
+        i0[p] = static_cast<uint16_t>((4 * (j * NT + tid) + k) | (((~out_of_mask >> c) & 1u) << 15));
         ++p;
       }
     }
@@ -128,7 +160,7 @@ __device__ __noinline__ void pscan_radix(const float* __restrict__ X, const uint
   __syncthreads();
   uint32_t* ks;
   uint16_t* is;
-  block_radix_sort<NT, C, uint32_t>(k0, i0, k1, i1, m, sm + L.scratch, &ks, &is);
+  block_radix_sort_bits<NT, C, uint32_t>(k0, i0, k1, i1, m, diff, sm + L.scratch, &ks, &is);
   uint16_t* S = (is == i0) ? i1 : i0;                                // group start per sorted position
   uint32_t* O = (ks == k0) ? k1 : k0;                                // two ranks per column
   uint16_t* Cn = reinterpret_cast<uint16_t*>(ks);                    // m + 1 entries, over the sorted keys
@@ -234,7 +266,10 @@ __global__ void __launch_bounds__(NT, kSmThreads / NT) k_csr(const float* __rest
   }
   SpreadTotals T;
   if (!spread_place<NT, V>(key, L, sm, W, T)) {
-    csr_radix<NT, V>(X, mask, N, desc, out, sm);
+    uint32_t kk[C];  // (the keys stay in registers but for this call)
+#pragma unroll
+    for (int c = 0; c < C; ++c) kk[c] = key[c];
+    csr_radix<NT, V>(kk, T.range, N, out + row, sm);
     return;
   }
   spread_positions<NT, V, false>(L, sm, T.m, T.heavy, key, W);
@@ -279,7 +314,10 @@ __global__ void __launch_bounds__(NT, kSmThreads / NT) k_pscan(const float* __re
   }
   SpreadTotals T;
   if (!spread_place<NT, V>(key, L, sm, W, T)) {
-    pscan_radix<NT, V>(X, mask, N, outs, sm);
+    uint32_t kk[C];  // (the keys stay in registers but for this call)
+#pragma unroll
+    for (int c = 0; c < C; ++c) kk[c] = key[c];
+    pscan_radix<NT, V>(kk, T.range, out_of_mask, N, outs, sm);
     return;
   }
   static_assert(kSpreadMaxBucket < 512, "ties fit 9-bit fields");

@@ -273,7 +273,7 @@ FCB_DEV void scatter_cells(const uint32_t (&key)[4 * V], uint32_t range, int m, 
 // becomes the distance from the smallest valid key, above T.range for the
 // invalid cells.  On true, W[c] of a valid cell is its bucket's start | size
 // << 14 and mem its words (scatter_cells).  On false (crowded buckets) shared memory holds nothing
-// of use.  Uniform across
+// of use, and the valid cells are still those at or below T.range, in order.  Uniform across
 // the block; every thread calls; ends with a barrier.  T.m == 0 returns true
 // with nothing placed but the pad.
 template <int NT, int V>
@@ -307,6 +307,7 @@ FCB_DEV bool spread_place(uint32_t (&key)[4 * V], const SpreadLayout<NT, V>& L, 
   __syncthreads();
   const uint32_t kmin = warps_min<NW>(red), range = warps_max<NW>(red + 32) - 1u - kmin;
   if (warps_sum<NW>(red + 64) > kSpreadMaxEqualPairs) {
+    T.range = kInvalidKey32 - 1u;  // (the keys are as they were)
     __syncthreads();  // the caller reuses the shared memory
     return false;
   }
