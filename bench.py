@@ -10,6 +10,11 @@ plus the daily Spearman IC of every factor against the forward returns.
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference]
                     [--method radix|learned]
 
+--method names the entry point: fcb_dev_rank_ic_panel (radix) or
+fcb_dev_rank_ic_panel_learned with a fitted model (learned).  Without
+statistics both rank by value-spread buckets; the learned buckets run where
+statistics are asked for, in a leg of their own.
+
 Prints one JSON line (rank 0).  ``value`` is device-resident throughput
 (inputs in HBM, CUDA events on the launching stream, inputs larger than L2
 so no flush is needed); ``e2e`` is the same metric through the C ABI host
@@ -215,7 +220,7 @@ def run_b200(args, rank, world):
     dic = torch.empty((F, T), dtype=torch.float64, device=dev)
     stream = torch.cuda.current_stream(dev)
 
-    def radix_step():
+    def plain_step():
         rc = lib.fcb_dev_rank_ic_panel(dX.data_ptr(), dR.data_ptr(), dfm.data_ptr(), drm.data_ptr(), F, T, N,
                                        MIN_VALID, dranks.data_ptr(), dic.data_ptr(), 0, stream.cuda_stream)
         nat.check(rc, "fcb_dev_rank_ic_panel")
@@ -223,8 +228,8 @@ def run_b200(args, rank, world):
     learn = None
     if method == 1:
         import fcb200
-        # exact radix ranks of the earlier dates are the training labels
-        radix_step()
+        # exact ranks of the earlier dates are the training labels
+        plain_step()
         torch.cuda.synchronize(dev)
         model = fcb200.CdfModel(F, seed=20261203)
         tfit = min(T, 250)
@@ -239,7 +244,7 @@ def run_b200(args, rank, world):
 
     def step(stats=None):
         if learn is None:
-            radix_step()
+            plain_step()
             return
         rc = lib.fcb_dev_rank_ic_panel_learned(dX.data_ptr(), dR.data_ptr(), dfm.data_ptr(), drm.data_ptr(), F, T,
                                                N, MIN_VALID, dranks.data_ptr(), dic.data_ptr(),
@@ -274,18 +279,19 @@ def run_b200(args, rank, world):
     timed_ic = dic.cpu().numpy()
     learned_info = None
     if learn is not None:
-        step(learn["stats"].data_ptr())  # the learned buckets' statistics, once, outside the timed steps
+        # the learned buckets (they run where statistics are asked for), once:
+        # their ranks and IC against the timed steps', bit for bit
+        dranks.zero_()
+        dic.zero_()
+        step(learn["stats"].data_ptr())
         torch.cuda.synchronize(dev)
         st = learn["stats"].cpu().numpy()
         codes = st[..., 0]
-        # bit-exactness of the whole learned output against the radix path
-        radix_step()
-        torch.cuda.synchronize(dev)
         exact = bool(np.array_equal(timed_ranks.view(np.uint32), dranks.cpu().numpy().view(np.uint32))) and \
             ic_bitwise(timed_ic, dic.cpu().numpy())
-        # learned vs radix under the same conditions: alternating windows of
-        # max(K, 20) steps each, three rounds, medians (the headline `value`
-        # above is the contract's K-step measurement)
+        # learned buckets vs value-spread buckets under the same conditions:
+        # alternating windows of max(K, 20) steps each, three rounds, medians
+        # (the headline `value` above is the contract's K-step measurement)
         e2 = torch.cuda.Event(enable_timing=True)
         e3 = torch.cuda.Event(enable_timing=True)
         n_cmp = max(args.steps, 20)
@@ -299,23 +305,22 @@ def run_b200(args, rank, world):
             torch.cuda.synchronize(dev)
             return e2.elapsed_time(e3) / n_cmp
 
-        rounds = [(window(step), window(radix_step)) for _ in range(3)]
-        learned_ms_cmp = sorted(r[0] for r in rounds)[1]
-        radix_ms = sorted(r[1] for r in rounds)[1]
-        saved = radix_ms - learned_ms_cmp
-        learned_info = {"fit_ms": learn["fit_ms"], "train_dates": learn["train_dates"],
+        rounds = [(window(lambda: step(learn["stats"].data_ptr())), window(plain_step)) for _ in range(3)]
+        learned_ms = sorted(r[0] for r in rounds)[1]
+        plain_ms = sorted(r[1] for r in rounds)[1]
+        learned_info = {"what": "the learned buckets (fcb_dev_rank_ic_panel_learned with statistics), beside the timed "
+                                "steps' value-spread buckets",
+                        "fit_ms": learn["fit_ms"], "train_dates": learn["train_dates"],
                         "fit": "1500 Adam steps on 64 samples per (factor, date) of dates [0, 250), once, "
                                "before the timed steps (not in ms_per_step)",
-                        "break_even_steps": (learn["fit_ms"] / saved) if saved > 0 else None,
                         "learned_fraction": float((codes == 1).mean()),
                         "fallback_overflow": float((codes == 2).mean()),
                         "fallback_judge": float((codes == 3).mean()),
                         "fallback_scale": float((codes == 4).mean()),
                         "mean_max_bucket": float(st[..., 1][codes == 1].mean()) if (codes == 1).any() else None,
-                        "bit_exact_vs_radix": exact, "radix_ms_per_step": radix_ms,
-                        "learned_ms_per_step_paired": learned_ms_cmp,
-                        "comparison": f"median of 3 alternating windows of {n_cmp} steps each",
-                        "speedup_vs_radix": radix_ms / learned_ms_cmp}
+                        "bit_exact_vs_timed_steps": exact, "learned_ms_per_step": learned_ms,
+                        "plain_ms_per_step": plain_ms,
+                        "comparison": f"median of 3 alternating windows of {n_cmp} steps each"}
 
     # e2e: host entry point, pinned buffers, copies in the timed region
     e2e_s = e2e_ok = e2e_floor = None
@@ -415,7 +420,7 @@ def run_b200(args, rank, world):
 # of each kernel at T=600: dram__bytes_read.sum + dram__bytes_write.sum.
 # Traffic grows with the number of dates at fixed N and F, so the bench's step
 # is that times T.
-TRAFFIC_PER_DATE = dict.fromkeys(("learned", "radix"), (156.102144e6 + 108.951808e6 + 15.078656e6) / 600)
+TRAFFIC_PER_DATE = (156.102144e6 + 108.951808e6 + 15.078656e6) / 600
 
 
 def transfer_floor(h2d_bytes, d2h_bytes, dev, reps=3):
@@ -472,14 +477,15 @@ def finish(args, world, X, R, fm, rm, ms, e2e_s, e2e_ok, clk, dev, learned_info=
     peak, peak_kind = measured_peaks()
     bytes_launch = algorithmic_bytes(F, T, N)
     achieved = bytes_launch / (ms / 1e3) / 1e9
-    traffic = TRAFFIC_PER_DATE[args.method] * T if (N, F) == (5000, 12) else None
+    traffic = TRAFFIC_PER_DATE * T if (N, F) == (5000, 12) else None
     res = {
         "metric": METRIC, "value": job_throughput(world, cells, ms_all), "unit": "Gelem/s",
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_all,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic (seeded stand-in for the 1218x5000x12 corpus panel)",
         "config": {"workload": "cs_rank + rolling_ic(min_valid=30), F=12 factor panels vs one "
-                               "forward-return panel", "T": T, "N": N, "F": F, "method": args.method,
+                               "forward-return panel", "T": T, "N": N, "F": F, "method": "value-spread buckets",
+                   "entry": "fcb_dev_rank_ic_panel_learned" if args.method == "learned" else "fcb_dev_rank_ic_panel",
                    "parallelism": f"replicas{world}",
                    "l2": "inputs (292 MB factors) larger than the 126 MB L2; no flush"},
         "e2e": None if e2e_s is None else {"value": world * cells / e2e_all / 1e9, "unit": "Gelem/s",
@@ -593,7 +599,7 @@ def bench_c2_stages(dX, X, fm, dev, rank_ic_ms, factor_corr_ms, steps=3):
             "cs_rank_ms_all_planes": cs_ms, "parameter_scan_ms_all_planes": scan,
             "rank_ic_ms_all_planes": rank_ic_ms, "factor_corr_ms": factor_corr_ms,
             "pipeline_ms": scan + rank_ic_ms + factor_corr_ms,
-            "pipeline": "parameter_scan (4 groups) + cs_rank/rolling_ic (fused, learned) + factor_corr (f64), "
+            "pipeline": "parameter_scan (4 groups) + cs_rank/rolling_ic (fused) + factor_corr (f64), "
                         "device-resident kernels"}
 
 
@@ -631,11 +637,8 @@ def bench_batch(dev, steps=5, warmup=2, tune_cache=None, cpu_sample=True):
     """Batched uneven panels: one autotuned CUDA-graph replay of the batched
     rank+IC kernels + per-panel factor_corr, against the same work issued one
     panel at a time.  Device-resident inputs (8.8 GB of factors, far above
-    L2).  Rank + IC use learned splitters: one CdfModel for the 8 factors,
-    fitted once (timed, outside the replays) on the exact radix ranks of
-    panel 0's first 250 dates and shared by every panel (the model works on
-    per-date standardised values, so it does not depend on a panel's T or N);
-    the same batch without the model is timed as the radix replay."""
+    L2).  Ranks by value-spread buckets; the batch takes no model into
+    account."""
     import torch
     import fcb200
     from fcb200 import _native as nat
@@ -643,25 +646,6 @@ def bench_batch(dev, steps=5, warmup=2, tune_cache=None, cpu_sample=True):
     cells = sum(int(p["X"].numel()) for p in panels)
     torch.cuda.synchronize(dev)
     stream = torch.cuda.current_stream(dev)
-    # the radix batch first (its replay is the comparison), then the model
-    # fitted on panel 0's exact ranks
-    b_rx = fcb200.Batch(panels, min_valid=MIN_VALID)
-    p0 = panels[0]
-    F0, T0, N0 = (int(v) for v in p0["X"].shape)
-    nat.check(nat.lib().fcb_dev_rank_ic_panel(p0["X"].data_ptr(), p0["R"].data_ptr(), p0["fmask"].data_ptr(),
-                                              p0["rmask"].data_ptr(), F0, T0, N0, MIN_VALID,
-                                              p0["ranks"].data_ptr(), p0["ic"].data_ptr(), 0, stream.cuda_stream),
-              "fcb_dev_rank_ic_panel")
-    model = fcb200.CdfModel(F0, seed=20261205)
-    f0 = torch.cuda.Event(enable_timing=True)
-    f1 = torch.cuda.Event(enable_timing=True)
-    f0.record(stream)
-    model.fit(p0["X"], p0["ranks"], T0, N0, 0, min(T0, 250), steps=1500, lr=3e-3, stream=stream.cuda_stream)
-    f1.record(stream)
-    torch.cuda.synchronize(dev)
-    fit_ms = f0.elapsed_time(f1)
-    for p in panels:
-        p["model"] = model
     b = fcb200.Batch(panels, min_valid=MIN_VALID)
     t0 = time.perf_counter()
     # with a cache file, a second run takes the tuned configuration without
@@ -682,10 +666,6 @@ def bench_batch(dev, steps=5, warmup=2, tune_cache=None, cpu_sample=True):
         torch.cuda.synchronize(dev)
         return e0.elapsed_time(e1) / steps
 
-    b_rx.config = cfg
-    ms_graph_rx = timed(b_rx.run)
-    b_rx.status()
-    b_rx.close()
     ms_graph = timed(b.run)
     b.status()
     ic_g = [p["ic"].clone() for p in panels]
@@ -709,16 +689,14 @@ def bench_batch(dev, steps=5, warmup=2, tune_cache=None, cpu_sample=True):
                        "cs_rank + rolling_ic(30) + factor_corr per panel",
            "cells": cells, "unit": "Gelem/s",
            # kernels: per kernel variant, the returns pass and the rank pass over all its
-           # panels; for all panels together, factor_corr's column pass + merge, Gram pass +
-           # finalize and the four fallback kernels (every pool here has 4096 rows or more;
-           # they exit at once when no pair is flagged); the per-panel arm runs, for each
-           # panel, those two rank kernels and the eight factor_corr kernels
-           "method": "learned splitters, one CdfModel (F=8) fitted on panel 0 and shared by every panel",
-           "fit_ms": fit_ms,
+           # panels; for all panels together, factor_corr's column pass + merge, the two forms
+           # of its Gram pass (of each panel one returns at once) + finalize and the four
+           # fallback kernels (every pool here has 4096 rows or more; they exit at once when no
+           # pair is flagged); the per-panel arm runs, for each panel, those two rank kernels
+           # and eight factor_corr kernels (the merge is in the column pass)
+           "method": "value-spread buckets",
            "graph": {"ms": ms_graph, "value": cells / (ms_graph / 1e3) / 1e9,
-                     "kernels_per_replay": 2 * len(variants) + 8},
-           "graph_radix": {"ms": ms_graph_rx, "value": cells / (ms_graph_rx / 1e3) / 1e9},
-           "learned_speedup_vs_radix_graph": ms_graph_rx / ms_graph,
+                     "kernels_per_replay": 2 * len(variants) + 9},
            "per_panel": {"ms": ms_pp, "value": cells / (ms_pp / 1e3) / 1e9,
                          "kernels_per_step": sum((2 if p["X"].shape[0] >= 2 else 1) + 8 for p in panels)},
            "speedup_graph_vs_per_panel": ms_pp / ms_graph,
@@ -788,8 +766,8 @@ def bench_c5(dev, T=5000, N=8000, F=128, Tb=250, seed=20261206, cpu_sample=True,
     F=128: 5.12 G cells, 20.5 GB of f32 factors, device-resident in blocks of
     250 dates), two end-to-end runs timed by CUDA events around the whole
     block loop:
-      radix    every block ranked by the plain radix path;
-      learned  the first `head` blocks are ranked by radix; the training
+      plain    every block ranked by the plain path (value-spread buckets);
+      learned  the first `head` blocks are ranked by it; the training
                samples are drawn from block 0's exact ranks and the networks
                are fitted (`fit_steps` Adam steps) on a second stream while
                blocks 1 .. head-1 are ranked (overlap_fit; otherwise in line
@@ -799,7 +777,7 @@ def bench_c5(dev, T=5000, N=8000, F=128, Tb=250, seed=20261206, cpu_sample=True,
                into the idle table slot while block b + 1 is ranked; block
                b + 2 waits for it on the device and ranks with the new table.
     Every fit is inside the learned figure.  An untimed pass then compares
-    the learned output of every learned block with the radix output bit for
+    the learned output of every learned block with the plain output bit for
     bit."""
     import torch
     import fcb200
@@ -821,9 +799,9 @@ def bench_c5(dev, T=5000, N=8000, F=128, Tb=250, seed=20261206, cpu_sample=True,
     ic = torch.empty((F, Tb), dtype=torch.float64, device=dev)
     stats = torch.zeros((nb, F, Tb, 4), dtype=torch.int32, device=dev)
 
-    def radix(X, R, fm, rm, out):
+    def plain(X, R, fm, rm, out):
         nat.check(lib.fcb_dev_rank_ic_panel(X.data_ptr(), R.data_ptr(), fm.data_ptr(), rm.data_ptr(), F, Tb, N,
-                                            MIN_VALID, out.data_ptr(), ic.data_ptr(), 0, s), "radix")
+                                            MIN_VALID, out.data_ptr(), ic.data_ptr(), 0, s), "plain")
 
     def learned(model, b, X, R, fm, rm, out):
         nat.check(lib.fcb_dev_rank_ic_panel_learned(X.data_ptr(), R.data_ptr(), fm.data_ptr(), rm.data_ptr(), F,
@@ -831,19 +809,19 @@ def bench_c5(dev, T=5000, N=8000, F=128, Tb=250, seed=20261206, cpu_sample=True,
                                                     256, stats[b].data_ptr(), s), "learned")
 
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
-    # ---- radix run (per-block events for the same-blocks comparison)
+    # ---- plain run (per-block events for the same-blocks comparison)
     bev = [torch.cuda.Event(enable_timing=True) for _ in range(nb + 1)]
     bev[0].record(stream)
     for b, (X, R, fm, rm) in enumerate(blocks):
-        radix(X, R, fm, rm, ranks)
+        plain(X, R, fm, rm, ranks)
         bev[b + 1].record(stream)
     torch.cuda.synchronize(dev)
-    t_radix = bev[0].elapsed_time(bev[nb])
-    t_radix_lb = bev[head].elapsed_time(bev[nb])
+    t_plain = bev[0].elapsed_time(bev[nb])
+    t_plain_lb = bev[head].elapsed_time(bev[nb])
     # ---- learned run, every fit included
     model = fcb200.CdfModel(F, seed=seed)
     # a model allocates its sample buffer on its first sample call: make one
-    # (on the last radix block's ranks, overwritten by the timed call) before
+    # (on the last plain block's ranks, overwritten by the timed call) before
     # the timing, so that no host-side allocation sits inside it
     model.sample(blocks[-1][0], ranks, Tb, N, 0, Tb, stream=s)
     torch.cuda.synchronize(dev)
@@ -853,7 +831,7 @@ def bench_c5(dev, T=5000, N=8000, F=128, Tb=250, seed=20261206, cpu_sample=True,
     ev[0].record(stream)
     for b, (X, R, fm, rm) in enumerate(blocks):
         if b < head:
-            radix(X, R, fm, rm, ranks)
+            plain(X, R, fm, rm, ranks)
             if b == 0:
                 model.sample(X, ranks, Tb, N, 0, Tb, stream=s)
                 fit_stream = side if overlap_fit else stream
@@ -885,12 +863,12 @@ def bench_c5(dev, T=5000, N=8000, F=128, Tb=250, seed=20261206, cpu_sample=True,
     t_learn_lb = ev[1].elapsed_time(ev[2])
     t_fit0 = ev[0].elapsed_time(ev[1])
     codes = stats[head:, ..., 0].flatten().cpu().numpy()
-    # ---- untimed exactness pass: learned (final model) vs radix, every block
+    # ---- untimed exactness pass: learned (final model) vs plain, every block
     exact = True
     for b, (X, R, fm, rm) in enumerate(blocks):
         if b < head:
             continue
-        radix(X, R, fm, rm, ranks)
+        plain(X, R, fm, rm, ranks)
         ic_r = ic.clone()
         learned(model, b, X, R, fm, rm, ranks2)
         exact = exact and bool(torch.equal(ranks.view(torch.int32), ranks2.view(torch.int32))) and \
@@ -899,21 +877,21 @@ def bench_c5(dev, T=5000, N=8000, F=128, Tb=250, seed=20261206, cpu_sample=True,
     lb_cells = F * (T - head * Tb) * N
     res = {"workload": f"learned splitters, streaming: T={T}, N={N}, F={F} ({F * T * N / 1e9:.2f} G cells, "
                        f"{F * T * N * 4 / 1e9:.1f} GB f32), blocks of {Tb} dates; a {fit_steps}-step fit on "
-                       f"block 0's exact ranks " + (f"overlapped with radix blocks 1-{head - 1}" if overlap_fit
+                       f"block 0's exact ranks " + (f"overlapped with plain blocks 1-{head - 1}" if overlap_fit
                                                     else "in line") +
                        f", learned from block {head}; a 100-step refit after every {refit_every}th learned "
                        f"block, overlapped with the next block",
-           "radix_gelem_s": F * T * N / (t_radix / 1e3) / 1e9,
+           "plain_gelem_s": F * T * N / (t_plain / 1e3) / 1e9,
            "learned_incl_fit_gelem_s": F * T * N / (t_learn_all / 1e3) / 1e9,
            "learned_blocks_gelem_s": lb_cells / (t_learn_lb / 1e3) / 1e9,
-           "radix_same_blocks_gelem_s": lb_cells / (t_radix_lb / 1e3) / 1e9,
-           "speedup_vs_radix_same_blocks_incl_refits": t_radix_lb / t_learn_lb,
-           "speedup_vs_radix_whole_run_incl_all_fits": t_radix / t_learn_all,
-           "initial_fit_and_radix_blocks_ms": t_fit0, "refits_overlapped": refits, "table_swaps": swaps,
+           "plain_same_blocks_gelem_s": lb_cells / (t_plain_lb / 1e3) / 1e9,
+           "speedup_vs_plain_same_blocks_incl_refits": t_plain_lb / t_learn_lb,
+           "speedup_vs_plain_whole_run_incl_all_fits": t_plain / t_learn_all,
+           "initial_fit_and_plain_blocks_ms": t_fit0, "refits_overlapped": refits, "table_swaps": swaps,
            "learned_fraction": float((codes == 1).mean()),
            "fallback_overflow": float((codes == 2).mean()), "fallback_judge": float((codes == 3).mean()),
            "fallback_scale": float((codes == 4).mean()),
-           "bit_exact_vs_radix": exact}
+           "bit_exact_vs_plain": exact}
     if cpu_sample:
         from oracle import fc_oracle as O
         X, R, fm, rm = blocks[2]
@@ -1083,7 +1061,7 @@ def main():
     ap.add_argument("--impl", choices=["b200", "reference"], default="b200")
     ap.add_argument("--method", choices=["radix", "learned"], default="learned")
     ap.add_argument("--learn-cap", type=int, default=256,
-                    help="largest bucket the learned rank kernel ranks itself (larger ones go to radix)")
+                    help="largest bucket the learned rank kernel ranks itself (larger ones go to the plain kernel)")
     ap.add_argument("--no-stock-corr", action="store_true", help="skip the stock_corr precision-form leg")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true", help="skip the host-buffer leg (profiling runs)")
