@@ -21,7 +21,7 @@
 //
 // Measured on a B200, 6.1 M rows x 12 factors f32 with a mask and 1 % missing
 // cells: 143 us (the staged pass took 673; memory alone 46, the FP64 sums 35),
-// factor_corr 1405 -> 217 us a call with the sampled shift and the two-pass
+// factor_corr 1405 -> 219 us a call with the sampled shift and the two-pass
 // recomputation kept for sums that fall short.  What bounds it is the issue of
 // 300 instructions per 32 rows (102 FP64; the rest converts, tests and selects)
 // and the queue, at 8 warps per SM of 255 registers: the 90 sums of a thread

@@ -13,7 +13,7 @@
 // that loads the library holds it until the process exits.
 //
 // The array fixes the row partition at kColBlocks / kGramBlocks blocks, where
-// fcb_dev_factor_corr sizes it from the pool (up to 592 / 888 blocks): the
+// fcb_dev_factor_corr sizes it from the pool (up to 296 / 888 blocks): the
 // partial sums are added in a different order, so the two entry points agree
 // within 1e-12 per output rather than bit for bit (and a pair right at the
 // cancellation gate may take the two-pass fallback in one and not the other;

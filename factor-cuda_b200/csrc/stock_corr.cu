@@ -23,14 +23,14 @@
 // (src/stock_corr_impl.cuh:102-132), and the two-pass fallback of the flagged
 // pairs (two_pass_centered, src/stock_corr_impl.cuh:150-201; _two_pass_corr,
 // fc/_cpu_core.py:111-137).
-// Measured on a B200, 1218 x 2000 f32 masked (7 % missing, 6400 flagged pairs):
-// 2.71 ms -> 0.43 ms a call; k_sc_gram 229 us (from 1905; FP64 tensor pipe,
-// 150 us at its peak, and the finalize on the same pipe), k_sc_pairsum 123
-// (shared-memory bandwidth), statistics, copies and lists 43 (from 103).
+// Measured on a B200, 1218 x 2000 f32 masked (7 % missing): 2.71 ms -> 0.44 ms a
+// call; k_sc_gram 218 us (from 1905; FP64 tensor pipe, 150 us at its peak, and
+// the finalize on the same pipe), k_sc_pairsum 120 (shared-memory bandwidth),
+// k_sc_direct 10, statistics, copies and lists 38 (from 103).
 // 64 x 32 tiles, four CTAs per SM: 64 x 64 tiles take 267-294 us, their last
 // wave being nearly empty.  Against 80-bit sums the rms error of a correlation
-// is 2.6e-17 (2.8e-17 with the six products): every long sum is a sum of short
-// ones, single chains over all dates gave 1.1e-16.
+// of 0.1 is 2.4e-17 (2.7e-17 with the six products): every long sum is a sum of
+// short ones, single chains over all dates gave 1.1e-16.
 // The domain check and the full-validity flag stay on the device: the later
 // kernels return at once when the panel is out of the domain, and the host
 // reads the summary once, at the end.

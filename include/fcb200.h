@@ -151,7 +151,7 @@ int fcb_rolling_ic(const void* f, int f_dtype, const void* r, int r_dtype, const
  * mask (T,N) broadcast to every factor.  x is f32 or f64.  fallback_out
  * (NULL = off) receives F*F bytes, 1 where the pair fails the cancellation
  * gate (its value comes from centred sums or, where these fall short, from the
- * two-pass compensated recomputation).
+ * two-pass compensated recomputation), and 0 for every other pair.
  * Replaces factor_corr_gpu (src/factor_corr.cuh:46-49).
  * Returns -1 null/dim, -2 T*N > INT32_MAX, -3 F > 128. */
 int fcb_factor_corr(const void* x, int dtype, const uint8_t* mask, int T, int N, int F, double* out,
@@ -257,10 +257,11 @@ int fcb_dev_corr_domain(const void* d_x, int dtype, const uint8_t* d_mask, int T
  * CDF network per factor (1 -> 32 -> 32 -> 1, tanh, sigmoid output) trained
  * on the GPU by this library's forward/backward kernels, and its tabulated
  * monotone CDF.  The learned rank path scatters each cross-section into
- * buckets by that CDF and ranks each bucket exactly; every date is checked
- * (strictly increasing (value, column) order over the whole output) and any
- * failure, bucket above `cap` or unusable scale falls back to the plain path,
- * so ranks and IC are bit-identical to it. */
+ * buckets by that CDF and ranks each bucket exactly.  A table that is not
+ * non-decreasing (one factor: ranked keys out of order), a bucket above `cap`
+ * or an unusable scale sends the section to the plain path, so ranks and IC are
+ * bit-identical to it.  It runs where outcome statistics are asked for and in
+ * fcb_rank_ic_panel's method 1; elsewhere the plain path is faster. */
 #define FCB_CDF_PARAMS 1153
 #define FCB_CDF_KNOTS 1024
 typedef struct fcb_cdf_model fcb_cdf_model;
@@ -419,9 +420,9 @@ typedef struct fcb_panel {
 } fcb_panel;
 
 /* Scheduling knobs.  None of them changes a result.  f32 panels: a panel of
- * width N runs in the narrowest kernel variant whose range holds it: up to
- * 1024 and 2048 (N <= nt_small_max), 3072 and 5120 (N <= nt_mid_max), 8192,
- * 16384; ctas_per_sm and learn_cap are not used.
+ * width N runs in the narrowest kernel variant whose range holds it: up to 512,
+ * 768, 1024, 1536 and 2048 (N <= nt_small_max), 3072 and 5120 (N <= nt_mid_max),
+ * 8192, 16384; ctas_per_sm and learn_cap are not used.
  * f64 panels: size classes of 256 / 512 / 1024-thread persistent CTAs. */
 typedef struct fcb_batch_config {
   int nt_small_max;  /* f64: largest N ranked by 256-thread CTAs (1..4096)       */
