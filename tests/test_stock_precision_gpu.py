@@ -60,3 +60,22 @@ def test_means_far_from_zero_in_long_panels(T, miss):
     N = 32
     r, X = common(T, N, T)
     assert rms_error(X + 1.0, r.random((T, N)) >= miss) < 1.3 * ULP
+
+
+def test_more_direct_sums_than_the_list_holds():
+    """Five of six pairs lose most of a column's squares: 640000 ordered pairs, more than twice the list of those that
+    are summed apart."""
+    import torch
+
+    import fcb200
+    from conftest import corr_match
+    from oracle import fc_oracle as O
+    r = np.random.default_rng(2)
+    T, N = 60, 800
+    X = 0.02 * r.standard_normal((T, N))
+    m = np.ones((T, N), bool)
+    d = np.arange(N) % 6
+    m[:6] = np.arange(6)[:, None] == d[None, :]     # of the first six dates a column has one, with an outlier
+    X[d, np.arange(N)] = 0.2 * np.sign(r.standard_normal(N))
+    got = fcb200.stock_corr(torch.from_numpy(X).cuda(), torch.from_numpy(m).cuda()).cpu().numpy()
+    assert corr_match(got, O.stock_corr(X, m))
