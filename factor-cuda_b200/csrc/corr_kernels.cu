@@ -111,8 +111,9 @@ FCB_DEV Blk launch_blk() {
 
 // Per-block column partials over a contiguous range of the sampled rows (every
 // ms-th; R, sr and the mask index count in sampled rows): count and Kahan sum of
-// each factor and, up to kFcRegMaxF factors, the rows with some valid factor.  Rows are visited in increasing order within each thread's strided
-// slice; partials are merged in a fixed order by k_fc_colfinal.
+// each factor and, up to kFcRegMaxF factors, the rows with some valid factor.
+// Rows are visited in increasing order within each thread's strided slice;
+// partials are merged in a fixed order (fc_colfinal_body).
 template <typename TIN>
 FCB_DEV void fc_colpart_body(const TIN* __restrict__ X, const uint8_t* __restrict__ mask, long long R, int F,
                              long long sr, long long sf, long long ms, long long rows_per_block,
